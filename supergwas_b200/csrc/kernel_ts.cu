@@ -56,7 +56,6 @@ constexpr int TS_XST_MAX = 12;
 __host__ __device__ constexpr int ts_ug(int N) { return N <= 80 ? 2 : 1; }
 __host__ __device__ constexpr int ts_threads(int N) { return 32 * (8 + 4 * ts_ug(N) + 2); }
 constexpr int TS_LU = 3, TS_LY = 5;
-constexpr uint32_t TS_XBYTES = TS_TM * 128;  // one box: 128 rows x 128 bytes
 constexpr int TS_WARP_UNPACK0 = 8;  // then the unpack groups, the producer, the MMA warp
 constexpr int TS_MAXSLOT = 3;
 
@@ -68,10 +67,10 @@ __host__ __device__ constexpr int ts_nslot(int N) {
 struct TsSmem {  // offsets from the 1024-aligned base
   uint32_t x, b, bars, tmem, abort, total;
 };
-__host__ __device__ inline TsSmem ts_smem(int b_bytes, int xst) {
+__host__ __device__ inline TsSmem ts_smem(int b_bytes, int xst, int rb) {
   TsSmem L;
   L.x = 0;
-  L.b = xst * TS_XBYTES;
+  L.b = xst * TS_TM * rb;
   L.bars = L.b + ((b_bytes + 127) / 128) * 128;
   L.tmem = L.bars + 8 * (2 * TS_XST_MAX + 2 * TS_MAXSLOT + 4 + 2);
   L.abort = L.tmem + 8;
@@ -79,10 +78,10 @@ __host__ __device__ inline TsSmem ts_smem(int b_bytes, int xst) {
   return L;
 }
 
-template <int N, bool DROP0, bool GATE>
+template <int N, bool DROP0, bool GATE, bool WIDE>
 __global__ void __launch_bounds__(ts_threads(N), 1)
     ts_kernel(const __grid_constant__ CUtensorMap tmap, unsigned long long m, int nbox, int nsub, int xst,
-              const int8_t* __restrict__ Bimg, int b_bytes, const __grid_constant__ EpiParams P,
+              int row_bytes, const int8_t* __restrict__ Bimg, int b_bytes, const __grid_constant__ EpiParams P,
               const __grid_constant__ LimbMap LM, const DevOut O) {
   constexpr int UG = ts_ug(N);
   constexpr int TS_WARP_PROD = TS_WARP_UNPACK0 + 4 * UG, TS_WARP_MMA = TS_WARP_PROD + 1;
@@ -96,7 +95,12 @@ __global__ void __launch_bounds__(ts_threads(N), 1)
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* gbase = smem_raw + (base - raw);
-  const TsSmem L = ts_smem(b_bytes, xst);
+  // WIDE: boxes of 128 swizzled bytes per row; otherwise a box holds whole
+  // rows of row_bytes < 128 (a run-time width would cost the wide case 1 %)
+  const int rb = WIDE ? 128 : row_bytes;
+  constexpr uint32_t swz = WIDE ? 7u : 0u;
+  const uint32_t xbytes = TS_TM * (uint32_t)rb;  // one box: 128 rows
+  const TsSmem L = ts_smem(b_bytes, xst, rb);
   const uint32_t sx = base + L.x, sb = base + L.b;
   const uint32_t x_full = base + L.bars, x_empty = x_full + 8 * TS_XST_MAX;
   const uint32_t a_full = x_empty + 8 * TS_XST_MAX, a_empty = a_full + 8 * TS_MAXSLOT;
@@ -162,8 +166,8 @@ __global__ void __launch_bounds__(ts_threads(N), 1)
             ok = false;
             break;
           }
-          mbar_arrive_expect_tx(x_full + 8 * xr.slot, TS_XBYTES);
-          tma_load_2d(sx + xr.slot * TS_XBYTES, &tmap, bx * 128, (int)(tile * TS_TM), x_full + 8 * xr.slot);
+          mbar_arrive_expect_tx(x_full + 8 * xr.slot, xbytes);
+          tma_load_2d(sx + xr.slot * xbytes, &tmap, bx * 128, (int)(tile * TS_TM), x_full + 8 * xr.slot);
           issued[xr.slot] = true;
           last_phase[xr.slot] = xr.phase;
         }
@@ -265,7 +269,8 @@ __global__ void __launch_bounds__(ts_threads(N), 1)
             ok = false;
             break;
           }
-          const uint32_t xrow = sx + xr.slot * TS_XBYTES + r * 128;
+          const uint32_t xrow = sx + xr.slot * xbytes + r * rb;
+          const uint32_t rx = r & swz;
           const uint32_t a_t = tmem + lane_base + A0 + ar.slot * 128;
           const int c0 = kc - bx * (TS_BOX / TS_KS);
           // 16 bytes (128 samples) of row r per sub-stage; 128-byte swizzle:
@@ -281,7 +286,7 @@ __global__ void __launch_bounds__(ts_threads(N), 1)
             for (int sub = 0; sub < TS_SUPER; ++sub)
               asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
                            : "=r"(w[sub][0]), "=r"(w[sub][1]), "=r"(w[sub][2]), "=r"(w[sub][3])
-                           : "r"(xrow + (((c0 + sub) ^ (r & 7)) << 4)));
+                           : "r"(xrow + (((c0 + sub) ^ rx) << 4)));
 #pragma unroll
             for (int sub = 0; sub < TS_SUPER; ++sub) {
               uint32_t o[32];
@@ -293,7 +298,7 @@ __global__ void __launch_bounds__(ts_threads(N), 1)
               uint4 v;
               asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
                            : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                           : "r"(xrow + (((c0 + sub) ^ (r & 7)) << 4)));
+                           : "r"(xrow + (((c0 + sub) ^ rx) << 4)));
               const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
               uint32_t o[32];
               unpack_stage(w4, o);
@@ -400,22 +405,38 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   return fn;
 }
 
+// Bytes of a packed row in one TMA box: 128 (1024 samples), or the whole row
+// where it is shorter.  A short row's box is not swizzled: its rows lie
+// wpk * 8 bytes apart in shared memory, where a warp's 16-byte reads take up
+// to 4 times as long (64-byte rows), a few cycles per 128-sample stage.
+// Against the smem-A kernel, which those rows took before (one 128-thread
+// block per SM, load, unpack, MMA and epilogue one after another): 1e7 k-mers
+// at n = 700, r = 8+1 in 0.56 ms instead of 3.38 ms, 1e6 at n = 200, r = 5+1
+// in 0.10 instead of 0.25 ms (whole calls).
+static int ts_box_bytes(int wpk) { return wpk * 8 < 128 ? wpk * 8 : 128; }
+
 bool ts_supported(int N, int limbs_u, int limbs_y, int kpad, int wpk) {
   if (limbs_u != TS_LU || limbs_y != TS_LY) return false;
   if (N < 16 || N > 128 || N % 16) return false;
   if (ts_nslot(N) < 2) return false;
-  if ((size_t)kpad * N > 128 * 1024) return false;  // B stays resident in shared memory
-  if (wpk * 8 < 128) return false;                   // one TMA box row is 128 bytes
+  // the whole image stays in shared memory, beside two boxes at least: up to
+  // 195 KB, with the ring as deep as the rest allows (1e7 k-mers at n = 2000,
+  // r = 20+1, 160 KB and 4 boxes: 1.24 ms; the smem-A kernel takes 8.3 ms)
+  int dev = 0, optin = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+    return false;
+  if (ts_smem(kpad * N, 2, ts_box_bytes(wpk)).total + 1024 > (uint32_t)optin) return false;
   return encode_fn() != nullptr;
 }
 
 // Boxes of the packed-row ring that fit next to the B image (at least 2).
-static int ts_ring_depth(int b_bytes) {
+static int ts_ring_depth(int b_bytes, int rb) {
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) optin = 0;
   int x = TS_XST_MAX;
-  while (x > 2 && ts_smem(b_bytes, x).total + 1024 > (uint32_t)optin) --x;
+  while (x > 2 && ts_smem(b_bytes, x, rb).total + 1024 > (uint32_t)optin) --x;
   if (const char* v = std::getenv("KG_TS_XST")) {
     const int want = std::atoi(v);
     if (want >= 2 && want < x) x = want;
@@ -423,22 +444,31 @@ static int ts_ring_depth(int b_bytes) {
   return x;
 }
 
-template <int N, bool D0, bool GATE>
-static cudaError_t launch_ts_t(const LaunchTs& L, const CUtensorMap& tm, cudaStream_t st) {
+template <int N, bool D0, bool GATE, bool WIDE>
+static cudaError_t launch_ts_w(const LaunchTs& L, const CUtensorMap& tm, cudaStream_t st) {
   const int b_bytes = L.kpad * N;
-  const int xst = ts_ring_depth(b_bytes);
-  const size_t smem = ts_smem(b_bytes, xst).total + 1024;
+  const int rb = ts_box_bytes(L.wpk);
+  const int xst = ts_ring_depth(b_bytes, rb);
+  const size_t smem = ts_smem(b_bytes, xst, rb).total + 1024;
   cudaError_t e =
-      cudaFuncSetAttribute(ts_kernel<N, D0, GATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(ts_kernel<N, D0, GATE, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const unsigned long long tiles = (L.m + TS_TM - 1) / TS_TM;
   unsigned long long grid = (unsigned long long)L.num_sms;
   if (grid > tiles) grid = tiles;
-  const int nbox = (L.wpk * 8 + 127) / 128;
-  const int nsub = L.kpad / TS_KS;
-  ts_kernel<N, D0, GATE><<<(unsigned)grid, ts_threads(N), smem, st>>>(tm, L.m, nbox, nsub, xst, L.Bimg, b_bytes,
+  // 128-sample sub-stages: those of the image that a row reaches (kpad is
+  // rounded up further; the image is zero past the row's samples)
+  const int nsub = L.kpad / TS_KS < L.wpk / 2 ? L.kpad / TS_KS : L.wpk / 2;
+  const int nbox = (nsub * 16 + 127) / 128;
+  ts_kernel<N, D0, GATE, WIDE><<<(unsigned)grid, ts_threads(N), smem, st>>>(tm, L.m, nbox, nsub, xst, rb, L.Bimg, b_bytes,
                                                                    *L.P, *L.LM, *L.O);
   return cudaGetLastError();
+}
+
+template <int N, bool D0, bool GATE>
+static cudaError_t launch_ts_t(const LaunchTs& L, const CUtensorMap& tm, cudaStream_t st) {
+  return ts_box_bytes(L.wpk) == 128 ? launch_ts_w<N, D0, GATE, true>(L, tm, st)
+                                    : launch_ts_w<N, D0, GATE, false>(L, tm, st);
 }
 
 cudaError_t launch_ts(const LaunchTs& L, cudaStream_t st) {
@@ -448,10 +478,12 @@ cudaError_t launch_ts(const LaunchTs& L, cudaStream_t st) {
   const cuuint64_t rowbytes = (cuuint64_t)L.wpk * 8;
   cuuint64_t gdim[2] = {rowbytes, (cuuint64_t)L.m};
   cuuint64_t gstride[1] = {rowbytes};
-  cuuint32_t box[2] = {128, TS_TM};
+  const int rb = ts_box_bytes(L.wpk);
+  cuuint32_t box[2] = {(cuuint32_t)rb, TS_TM};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = enc(&tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)L.x, gdim, gstride, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   rb == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return cudaErrorInvalidValue;
   const bool d0 = L.drop0;

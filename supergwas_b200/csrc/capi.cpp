@@ -193,6 +193,7 @@ int kg_set_structure_ex(kg_ctx* ctx, const double* U, int n, int k, const double
     KG_CUDA(cudaStreamSynchronize(ctx->stream), "refinement tables");
     P.refine = 1;
     P.r2_ref = -std::expm1(-kg::REFINE_CHISQ / (double)n);
+    kg::set_refine_need(P);
     e = kg::make_limbs(p, sample_pos, n_row, ctx->opts.limbs_u, ctx->opts.limbs_y, kg::tc_kc(), ctx->limbs);
     if (!e.empty()) return ctx->fail(KG_ERR_UNSUPPORTED, e);
     if (!kg::tc_supported_n(ctx->limbs.N))
@@ -211,6 +212,7 @@ int kg_set_structure_ex(kg_ctx* ctx, const double* U, int n, int k, const double
       LM.scale[j] = ctx->limbs.scale[j];
     }
     kg::set_limb_consts(LM);
+    if (ctx->opts.limbs_u == 3 && ctx->opts.limbs_y == 5) kg::set_screen(P, LM, p.drop0 && k > 0);
     dfree(ctx->dB);
     KG_CUDA(cudaMalloc((void**)&ctx->dB, img.size()), "cudaMalloc(B)");
     KG_CUDA(cudaMemcpy(ctx->dB, img.data(), img.size(), cudaMemcpyHostToDevice), "copy B");
@@ -497,7 +499,7 @@ int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64
     const bool want_ss = force && std::string(force) == "ss";
     const bool ts_ok = kg::ts_supported(ctx->limbs.N, ctx->opts.limbs_u, ctx->opts.limbs_y, ctx->limbs.Kpad,
                                         (int)wpk) &&
-                       ((uintptr_t)dx % 16) == 0;
+                       ((uintptr_t)dx % 16) == 0 && m <= 0x7fffff00ull;  // 31-bit row coordinates
     if (force && std::string(force) == "ts" && !ts_ok)
       return ctx->fail(KG_ERR_UNSUPPORTED, "KG_KERNEL=ts: shape not supported by the TMEM-A kernel");
     if (ts_ok && !want_ss) {

@@ -28,6 +28,19 @@ __device__ __forceinline__ double magic_raw(long long v) {
 }
 __device__ __forceinline__ double i2d_exact(long long v) { return magic_raw(v) - MAGIC_BIAS; }
 
+// a * B + c, 32 x 32 -> 64 bits in one multiply-add.  B is an immediate: from
+// a register each use cost a move on the uniform datapath.
+template <int B>
+__device__ __forceinline__ long long mad_wide(uint32_t a, long long c) {
+  long long d;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "n"(B), "l"(c));
+  return d;
+}
+// The integer 65536 hi + 256 mid + lo of three int32 limb sums.
+__device__ __forceinline__ long long limb3(uint32_t hi, uint32_t mid, uint32_t lo) {
+  return mad_wide<65536>(hi, mad_wide<256>(mid, (long long)(int)lo));
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
@@ -45,6 +58,15 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// count arrivals by each lane with p set, without a branch.
+__device__ __forceinline__ void mbar_arrive_if(uint32_t bar, bool p, uint32_t count = 1) {
+  asm volatile(
+      "{\n\t.reg .pred P1;\n\t"
+      "setp.ne.u32 P1, %1, 0;\n\t"
+      "@P1 mbarrier.arrive.shared::cta.b64 _, [%0], %2;\n\t}" ::"r"(bar),
+      "r"((uint32_t)p), "r"(count)
+      : "memory");
 }
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   uint32_t ok;
@@ -235,13 +257,13 @@ __device__ __forceinline__ void unpack_stage(const uint32_t (&w)[4], uint32_t (&
 }
 
 // Bounded wait that also gives up when another role has aborted.  The first
-// test is inline (the common case: the phase is already complete); the
+// test is inline (the common case: the phase is already complete), the rest a
+// call, so that the waits of all roles do not fill the instruction cache; the
 // abort flag and the clock are read only every 16 failed tests.  limit_ns:
 // how long to wait before giving up (a launch parameter, see wait_limit).
-__device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, volatile int* abort,
-                                        unsigned long long* counters, unsigned code,
-                                        unsigned long long limit_ns = WAIT_LIMIT_NS) {
-  if (mbar_try(bar, parity)) return true;
+static __device__ __forceinline__ bool wait_more(uint32_t bar, uint32_t parity, volatile int* abort,
+                                              unsigned long long* counters, unsigned code,
+                                              unsigned long long limit_ns) {
   const unsigned long long t0 = gtimer_ns();
   for (uint32_t it = 1;; ++it) {
     if (mbar_try_sleep(bar, parity)) return true;
@@ -254,6 +276,11 @@ __device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, vol
       }
     }
   }
+}
+__device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, volatile int* abort,
+                                        unsigned long long* counters, unsigned code,
+                                        unsigned long long limit_ns = WAIT_LIMIT_NS) {
+  return mbar_try(bar, parity) || wait_more(bar, parity, abort, counters, code, limit_ns);
 }
 
 // The pipeline wait limit of a launch: the caller's value, or WAIT_LIMIT_NS
@@ -445,6 +472,21 @@ __device__ __forceinline__ void finish_kmer_fast(const EpiParams& P, const DevOu
   emit_kmer(O, local, valid, tested, hit, cand, T, p, effect, xxM, xyM, 0.0);
 }
 
+// Whether a tested k-mer of the split form goes to the FP64 refinement in a
+// launch that returns emitted rows only: r2 = q / den at least r2_ref, and not
+// so far below the emit cut that refining cannot matter.  The limbs of U are
+// rounded to 2^-23 of a column's largest value, which in the worst case (every
+// rounding of one sign) moves xxM by under 1 % of c(n - c)/n / 50 (up to 12,000
+// samples, 33 columns), so the 10 % below the cut hold where xxM is at least
+// that 50th.
+// Refining every k-mer from chi-square 12 up took 0.1 ms per 4e7 k-mers at
+// n = 1000 (5e-4 of them, 20 KB of byte tables each); from 0.9 of the cut at
+// p = 1e-6 it is 4e-6 of them.
+__device__ __forceinline__ bool may_refine(const EpiParams& P, double cd, double xxM, double q, double den) {
+  return q >= P.r2_ref * den &&
+         (q >= P.r2_need * den || !(xxM >= 0.02 * cd * ((double)P.n - cd) / (double)P.n));
+}
+
 // Fast screen of one k-mer for kernels that count tested k-mers in a
 // register (tested_local, flushed once per warp by the caller): in the common
 // case (no hit, no refinement candidate in the warp) it costs one ballot.
@@ -465,7 +507,7 @@ __device__ __forceinline__ void finish_kmer_lean(const EpiParams& P, const DevOu
   const double xyM = P.b * cd + ey;
   const double q = xyM * xyM, den = xxM * P.yyM;
   const bool ok = tested && xxM > eps && P.yyM > eps;
-  const bool cand = ok && P.refine && q >= P.r2_ref * den;
+  const bool cand = ok && P.refine && may_refine(P, cd, xxM, q, den);
   const bool maybe = ok && !cand && q >= P.r2_cand * den;
   if (__ballot_sync(0xffffffffu, cand || maybe) == 0u) return;
   double T = 0, p = 1, effect = 0;
@@ -480,6 +522,55 @@ __device__ __forceinline__ void finish_kmer_lean(const EpiParams& P, const DevOu
     hit = p <= P.p_thresh;
   }
   emit_rare(O, local, hit, cand, T, p, effect);
+}
+
+// A limb sum (int64) shifted right by s < 32 into 32 bits, as a float.
+__device__ __forceinline__ float shifted_float(long long v, int s) {
+  return (float)(int)__funnelshift_r((uint32_t)v, (uint32_t)((unsigned long long)v >> 32), s);
+}
+
+// Single-precision screen of one k-mer from its limb sums d (count, 5 y' limbs,
+// then 3 limbs per U column 1 .. ku; the intercept in double only).  Returns
+//   0  not tested;
+//   1  tested, and certainly neither a row to emit nor a refinement candidate;
+//   2  undecided: the FP64 statistic decides.
+// FP64 instructions and the MMAs share one pipe (ncu: pipe_shared), so an FP64
+// instruction waits for the MMA in the pipe, ~36 cycles beside N = 64: the
+// FP64 statistic of 16 U columns took 3100 cycles per 128-k-mer tile.  The
+// screen uses the integer, conversion and FP32 pipes only.  Errors, relative to
+// what is compared: a limb sum shifted into 32 bits is good to 2^-20 of its
+// column's largest value per 1024 samples, and columns of U (and y' over
+// ||y - mean||) hold no value above 1.  With xxM at least 0.02 c(n - c)/n the
+// r2 compared here is within 1 % of the exact one (up to 12,000 samples, 64
+// columns); the cut it is compared with is 10 % low.  The correlation is
+// within 1e-5 per 1024 samples; gate_lo and gate_hi leave 1e-4.
+// PAIRS: no correlation gate, and c = n is left to the FP64 form.
+template <int KU_MAX, int LAST, bool GATE, bool PAIRS>
+__device__ __forceinline__ int screen_kmer(const ScreenParams& S, int n, const uint32_t* d, int ku, bool valid) {
+  const int c = (-(int)d[0]) >> 7;
+  const float cf = (float)c;
+  const float xcn = (float)(c * (n - c)) * S.inv_n;
+  const long long vy = mad_wide<(1 << 24)>(d[1], limb3(d[2], d[3], d[4]));
+  const float ey = shifted_float(vy, S.shift + 8) * S.sy;
+  float ss = 0.0f, gs = 0.0f;
+#pragma unroll
+  for (int jj = 0; jj < KU_MAX; ++jj) {
+    if (jj >= KU_MAX - LAST && jj >= ku) break;
+    const int o = 6 + 3 * jj;
+    const float e = shifted_float(limb3(d[o], d[o + 1], d[o + 2]), S.shift) * S.su[jj + 1];
+    ss = fmaf(e, e, ss);
+    if (GATE) gs = fmaf(S.g[jj + 1], e, gs);
+  }
+  const bool in = valid && c > 0 && (PAIRS || c < n);
+  if (!in) return 0;
+  if (GATE) {
+    const float xyc = fmaf(S.kappa, cf, ey + gs);
+    const float q = xyc * xyc;
+    if (q < S.gate_lo * xcn) return 0;
+    if (!(q > S.gate_hi * xcn)) return 2;
+  }
+  const float xxM = xcn - ss, xyM = fmaf(S.b, cf, ey);
+  return xxM >= 0.02f * xcn && xcn > 0.0f && xyM * xyM < S.cut * xxM ? 1 : 2;
 }
 
 // Adds the per-thread tested counts of a warp to counters[0].

@@ -1,40 +1,56 @@
 // kernel_ts.cu -- split-precision association kernel with the unpacked x
 // operand held in tensor memory.
 //
-// One persistent CTA per SM, warp-specialised (576 threads; 448 for N > 80):
-//   warps 0-7   epilogue, two groups of four (one warp per TMEM lane quarter),
-//               group e owning accumulator buffer e, i.e. every other tile:
-//               tcgen05.ld of the int32 accumulators (one TMEM lane = one
-//               k-mer), exact limb recombination, FP64 statistics,
-//               warp-aggregated hit compaction;
-//   warps 8-15  unpack, two groups of four taking super-stages in turn (one
-//               group for N > 80, so that the epilogue keeps its registers): read
-//               128 samples of a packed row from the TMA-filled shared tile
-//               and write them as int8 (0 / -128, or 0 / 64 against -2x the
-//               B digits) straight into a TMEM A slot with tcgen05.st -- the
-//               unpacked operand never touches shared memory;
-//   warp 16     producer (12 for N > 80): one 2-D TMA load (128 rows x 128 bytes, 128-byte
-//               swizzle, no multicast) per 1024 samples of a 128-k-mer tile;
-//   warp 17     MMA (13 for N > 80): tcgen05.mma kind::i8, A from TMEM, B (the int8 limbs of
-//               the centred structure and phenotype columns, resident in
-//               shared memory for the whole launch) from a smem descriptor.
+// One persistent CTA per SM, warp-specialised (736 threads; 608 for N = 80,
+// 480 above):
+//   epilogue  8 warps, two groups of four (one warp per TMEM lane quarter),
+//             group e owning accumulator buffer e, i.e. every other tile:
+//             tcgen05.ld of the int32 accumulators (one TMEM lane = one
+//             k-mer), then the single-precision screen (screen_kmer), and for
+//             warps holding a k-mer that it cannot decide the exact limb
+//             recombination and FP64 statistic; warp-aggregated hits;
+//   unpack    groups of four warps, one per TMEM A slot (one group for
+//             N > 80, so that the epilogue keeps its registers), taking
+//             super-stages in turn: read 128 samples of a packed row from the
+//             TMA-filled shared tile and write them as int8 (0 / -128, or
+//             0 / 64 against -2x the B digits) straight into the slot with
+//             tcgen05.st -- the unpacked operand never touches shared memory;
+//   producer  one warp: one 2-D TMA load (128 rows x 128 bytes, 128-byte
+//             swizzle, no multicast; whole rows where they are shorter) per
+//             1024 samples of a 128-k-mer tile;
+//   MMA       two warps taking alternate tiles: tcgen05.mma kind::i8, A from
+//             TMEM, B (the int8 limbs of the centred structure and phenotype
+//             columns, resident in shared memory for the whole launch) from a
+//             smem descriptor.
 // Tile = 128 k-mers (M), N = 16..128 limb columns.
 //
-// The MMA-issuing thread is the critical path: on B200 a kind::i8 M=128
-// N=64 K=32 MMA occupies the tensor pipe 32 cycles (16384 int8 ops per SM
-// cycle), and every barrier test, commit or runtime division between MMAs
-// adds its latency on top.  So the
-// A operand moves in super-stages of 512 samples (4 sub-stages of 128
-// samples = 128 TMEM columns = 16 MMAs) with one barrier wait and one
-// commit each, and every ring index is a compile-time-bounded counter.
+// A kind::i8 M=128 N=64 K=32 MMA occupies the tensor pipe 32 cycles (16384
+// int8 ops per SM cycle), and every barrier test, commit or runtime division
+// between MMAs adds its latency on top.  So the A operand moves in
+// super-stages of 512 samples (4 sub-stages of 128 samples = 128 TMEM columns
+// = 16 MMAs) with one barrier wait and one commit each.
 // TMEM (512 columns): two accumulators of N columns, then NSLOT super-slots.
+//
+// What bounds it (n = 1000, r = 16+1, N = 64; ncu and copies with a role's work
+// left out): 11.8 SM-cycles per k-mer against 8 of MMAs; the tensor pipe is
+// 74 % active, the ALU pipe of the unpack's masks (2 cycles per warp
+// instruction) 60 %, instruction issue 67 %; 11.0 without the epilogue's
+// arithmetic, 8.3 with the unpack alone.  4e7 k-mers take 1.62 ms.  Before
+// (2.19 ms): the FP64 statistic of every k-mer in the epilogue, whose FP64
+// instructions share a pipe with the MMAs (3100 cycles per tile; with the
+// screen 2.06 ms); one MMA warp, 400 of its 1850 cycles per tile in barrier
+// tests that the pipe's queue of six MMAs does not cover (two: 1.93 ms); every
+// k-mer of chi-square 12 and up refined (1.67 ms); unpack groups that visited
+// every box and took super-stages in a 64-bit loop (1.62 ms).
 //
 // The accumulators hold -128 * sum_i x_i * digit_l(i) for every limb l; the
 // epilogue recombines the limbs exactly in int64, scales by 2^-s / 128, and
-// evaluates the reference's statistic (src/kgwas.cpp:44-56, 182-218) in FP64.
+// evaluates the reference's statistic (src/kgwas.cpp:44-56, 182-218) in FP64,
+// for the k-mers that the screen leaves.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 
@@ -51,18 +67,18 @@ constexpr int TS_BOX = 1024;       // samples per TMA box (128 bytes)
 // holds, up to TS_XST_MAX (chosen at launch).  HBM latency under this load is
 // ~2 us, so 4 boxes (64 KB per SM) cap the row stream near 4.3 TB/s.
 constexpr int TS_XST_MAX = 12;
-// Unpack groups (taking super-stages in turn): two while the epilogue fits
-// the register budget of 18 warps, one for wide N.
-__host__ __device__ constexpr int ts_ug(int N) { return N <= 80 ? 2 : 1; }
-__host__ __device__ constexpr int ts_threads(int N) { return 32 * (8 + 4 * ts_ug(N) + 2); }
-constexpr int TS_LU = 3, TS_LY = 5;
-constexpr int TS_WARP_UNPACK0 = 8;  // then the unpack groups, the producer, the MMA warp
 constexpr int TS_MAXSLOT = 3;
-
 // Super-slots of 128 TMEM columns left after the two N-column accumulators.
 __host__ __device__ constexpr int ts_nslot(int N) {
   return (512 - 2 * N) / 128 > TS_MAXSLOT ? TS_MAXSLOT : (512 - 2 * N) / 128;
 }
+// Unpack groups, taking super-stages in turn: one per slot, so that a group
+// always fills the same slot and waits for every release of it; one for wide
+// N, so that the epilogue keeps its registers.
+__host__ __device__ constexpr int ts_ug(int N) { return N <= 80 ? ts_nslot(N) : 1; }
+__host__ __device__ constexpr int ts_threads(int N) { return 32 * (8 + 4 * ts_ug(N) + 3); }
+constexpr int TS_LU = 3, TS_LY = 5;
+constexpr int TS_WARP_UNPACK0 = 8;  // then the unpack groups, the producer, two MMA warps
 
 struct TsSmem {  // offsets from the 1024-aligned base
   uint32_t x, b, bars, tmem, abort, total;
@@ -72,7 +88,7 @@ __host__ __device__ inline TsSmem ts_smem(int b_bytes, int xst, int rb) {
   L.x = 0;
   L.b = xst * TS_TM * rb;
   L.bars = L.b + ((b_bytes + 127) / 128) * 128;
-  L.tmem = L.bars + 8 * (2 * TS_XST_MAX + 2 * TS_MAXSLOT + 4 + 2);
+  L.tmem = L.bars + 8 * (2 * TS_XST_MAX + 2 * TS_MAXSLOT + 4 + 5);
   L.abort = L.tmem + 8;
   L.total = L.abort + 8;
   return L;
@@ -81,7 +97,7 @@ __host__ __device__ inline TsSmem ts_smem(int b_bytes, int xst, int rb) {
 template <int N, bool DROP0, bool GATE, bool WIDE>
 __global__ void __launch_bounds__(ts_threads(N), 1)
     ts_kernel(const __grid_constant__ CUtensorMap tmap, unsigned long long m, int nbox, int nsub, int xst,
-              int row_bytes, const int8_t* __restrict__ Bimg, int b_bytes, const __grid_constant__ EpiParams P,
+              int ug, int row_bytes, const int8_t* __restrict__ Bimg, int b_bytes, const __grid_constant__ EpiParams P,
               const __grid_constant__ LimbMap LM, const DevOut O) {
   constexpr int UG = ts_ug(N);
   constexpr int TS_WARP_PROD = TS_WARP_UNPACK0 + 4 * UG, TS_WARP_MMA = TS_WARP_PROD + 1;
@@ -105,10 +121,11 @@ __global__ void __launch_bounds__(ts_threads(N), 1)
   const uint32_t x_full = base + L.bars, x_empty = x_full + 8 * TS_XST_MAX;
   const uint32_t a_full = x_empty + 8 * TS_XST_MAX, a_empty = a_full + 8 * TS_MAXSLOT;
   const uint32_t acc_full = a_empty + 8 * TS_MAXSLOT, acc_empty = acc_full + 16, b_full = acc_empty + 16;
-  const uint32_t drain = b_full + 8;
+  const uint32_t drain = b_full + 8, turn = drain + 16;
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(gbase + L.tmem);
   volatile int* s_abort = reinterpret_cast<volatile int*>(gbase + L.abort);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // warp-uniform values as such: the roles' loops then run on the uniform datapath
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int nsp = (nsub + TS_SUPER - 1) / TS_SUPER;  // super-stages per tile
 
   if (warp == 0) {
@@ -119,7 +136,7 @@ __global__ void __launch_bounds__(ts_threads(N), 1)
   if (tid == 32) {
     for (int s = 0; s < xst; ++s) {
       mbar_init(x_full + 8 * s, 1);
-      mbar_init(x_empty + 8 * s, 4 * UG);  // every unpack warp
+      mbar_init(x_empty + 8 * s, 8);  // four warps, twice
     }
     for (int t = 0; t < NSLOT; ++t) {
       mbar_init(a_full + 8 * t, 4);   // the four warps of one unpack group
@@ -130,14 +147,17 @@ __global__ void __launch_bounds__(ts_threads(N), 1)
       mbar_init(acc_empty + 8 * b, 4);  // the four warps of epilogue group b
     }
     mbar_init(b_full, 1);
-    mbar_init(drain, 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(drain + 8 * b, 1);
+      mbar_init(turn + 8 * b, 1);
+    }
     *s_abort = 0;
     mbar_fence_init();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *s_tmem;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *s_tmem, 0);
   const unsigned long long ntiles = (m + TS_TM - 1) / TS_TM;
   const unsigned long long lim = wait_limit(O.wait_ns);
 
@@ -177,29 +197,44 @@ __global__ void __launch_bounds__(ts_threads(N), 1)
       for (int s = 0; s < xst; ++s)
         if (issued[s]) mbar_wait(x_full + 8 * s, last_phase[s], O.counters, ERR_TIMEOUT_FULL);
     }
-  } else if (warp == TS_WARP_MMA) {
+  } else if (warp >= TS_WARP_MMA) {
     // ----------------------------------------------------------------- MMA
-    // The whole warp runs the loop (warp-uniform control flow and operands);
-    // one elected lane issues the MMAs and the commits that track them.
+    // Two warps take alternate tiles, warp w accumulator w: an issuing thread
+    // spends 20-30 cycles per MMA and ~100 per barrier test, which the other
+    // warp's MMAs cover.  Each whole warp runs its loop (warp-uniform control
+    // flow and operands); one elected lane issues the MMAs and the commits
+    // that track them.  The super-stages' barriers are waited for in order
+    // across both warps (a warp passes `turn` on once it has seen its tile's
+    // last super-stage full): a parity wait is only sound for a waiter that
+    // is less than a lap of the ring ahead.
     const bool leader = elect_one();
+    const uint32_t b = (uint32_t)(warp - TS_WARP_MMA);
     bool ok = __all_sync(0xffffffffu, wait_or_abort(b_full, 0, s_abort, O.counters, ERR_TIMEOUT_FULL, lim));
     const uint64_t bdesc0 = sdesc_noswz(sb, N * 16, 128);
+    const uint32_t d_t = tmem + b * N;
     Ring<NSLOT> ar;
-    uint32_t i = 0;
-    for (unsigned long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++i) {
-      const uint32_t b = i & 1u;
-      if (i >= 2 && !__all_sync(0xffffffffu, wait_or_abort(acc_empty + 8 * b, ((i >> 1) - 1) & 1u, s_abort, O.counters,
-                                                     ERR_TIMEOUT_MMA, lim))) {
+    if (b)
+      for (int sp = 0; sp < nsp; ++sp) ar.next();  // the first tile is the other warp's
+    uint32_t i = 0;  // tiles of this warp
+    for (unsigned long long tile = blockIdx.x + (unsigned long long)b * gridDim.x; tile < ntiles && ok;
+         tile += 2ull * gridDim.x, ++i) {
+      if (i >= 1 && !__all_sync(0xffffffffu, wait_or_abort(acc_empty + 8 * b, (i - 1) & 1u, s_abort, O.counters,
+                                                           ERR_TIMEOUT_MMA, lim))) {
         ok = false;
         break;
       }
-      const uint32_t d_t = tmem + b * N;
+      if ((b || i >= 1) && !__all_sync(0xffffffffu, wait_or_abort(turn + 8 * b, b ? i & 1u : (i - 1) & 1u, s_abort,
+                                                                  O.counters, ERR_TIMEOUT_MMA, lim))) {
+        ok = false;
+        break;
+      }
       uint64_t bd = bdesc0;
       for (int sp = 0; sp < nsp; ++sp, ar.next()) {
         if (!__all_sync(0xffffffffu, wait_or_abort(a_full + 8 * ar.slot, ar.phase, s_abort, O.counters, ERR_TIMEOUT_MMA, lim))) {
           ok = false;
           break;
         }
+        mbar_arrive_if(turn + 8 * (b ^ 1u), leader && sp + 1 == nsp);
         tc_fence_after();
         const int nsub_here = nsub - sp * TS_SUPER < TS_SUPER ? nsub - sp * TS_SUPER : TS_SUPER;
         const uint32_t a_t = tmem + A0 + ar.slot * 128;
@@ -227,96 +262,114 @@ __global__ void __launch_bounds__(ts_threads(N), 1)
       if (!ok) break;
       if (leader) tc_commit(acc_full + 8 * b);
       __syncwarp();
+      for (int sp = 0; sp < nsp; ++sp) ar.next();  // the other warp's tile
     }
     // drain: wait (bounded) until every issued MMA has completed
     if (leader) {
-      tc_commit(drain);
-      mbar_wait(drain, 0, O.counters, ERR_TIMEOUT_MMA);
+      tc_commit(drain + 8 * b);
+      mbar_wait(drain + 8 * b, 0, O.counters, ERR_TIMEOUT_MMA);
     }
     __syncwarp();
   } else if (warp >= TS_WARP_UNPACK0) {
     // -------------------------------------------------------------- unpack
-    const int grp = (warp - TS_WARP_UNPACK0) >> 2;  // takes every other super-stage
-    const int q = warp & 3;                         // TMEM lane quarter
-    const int r = q * 32 + lane;                    // row of the tile = TMEM lane
+    // Group grp fills super-stages grp, grp + ug, ... of the CTA's stream of
+    // tiles (ug: ts_groups).  A box holds two super-stages (the last of a tile
+    // may hold one).
+    const int grp = (warp - TS_WARP_UNPACK0) >> 2;
+    const int q = warp & 3;      // TMEM lane quarter
+    const int r = q * 32 + lane;  // row of the tile = TMEM lane
+    const uint32_t rx = r & swz;
+    const uint32_t row0 = sx + r * rb;
     const uint32_t lane_base = (uint32_t)(q * 32) << 16;
-    RingN xr(xst);
+    const uint32_t xst_u = (uint32_t)xst;
+    uint32_t xslot = 0, xphase = 0;  // the box of this group's super-stage
     Ring<NSLOT> ar;
-    uint32_t turn = 0;  // super-stage counter modulo UG
-    bool ok = true;
-    for (unsigned long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-      int kc = 0;  // sub-stage of the tile
-      for (int bx = 0; bx < nbox && ok; ++bx, xr.next()) {
-        // every unpack warp waits for every box, also one holding none of its
-        // super-stages, so that its release below belongs to this fill
-        if (!__all_sync(0xffffffffu, wait_or_abort(x_full + 8 * xr.slot, xr.phase, s_abort, O.counters,
-                                            ERR_TIMEOUT_FULL, lim))) {
-          ok = false;
-          break;
-        }
-        const int kc1 = (bx + 1) * (TS_BOX / TS_KS) < nsub ? (bx + 1) * (TS_BOX / TS_KS) : nsub;
-        // super-stages never straddle a box: a box holds two of them
-        while (kc < kc1) {
-          const int ke = kc + TS_SUPER < kc1 ? kc + TS_SUPER : kc1;
-          if (UG > 1 && turn != (uint32_t)grp) {  // another group's super-stage
-            kc = ke;
-            ar.next();
-            turn = turn + 1 == (uint32_t)UG ? 0u : turn + 1;
-            continue;
-          }
-          if (ar.used && !__all_sync(0xffffffffu, wait_or_abort(a_empty + 8 * ar.slot, ar.phase ^ 1u, s_abort,
-                                                          O.counters, ERR_TIMEOUT_MMA, lim))) {
+    for (int g = 0; g < grp; ++g) ar.next();
+    uint32_t off[TS_SUPER];  // 16-byte chunks 0-3 of the row, swizzled
+#pragma unroll
+    for (int c = 0; c < TS_SUPER; ++c) off[c] = (c ^ rx) << 4;
+    const uint32_t nt32 = (uint32_t)ntiles;  // row indices fit 31 bits (TMA coordinates)
+    uint32_t tile = blockIdx.x;
+    int sp = 0;  // super-stage of the tile
+    for (int step = grp; grp < ug; step = ug) {
+      // on to this group's next super-stage, `step` further
+      int nb = -(sp >> 1);  // boxes passed over
+      for (sp += step; sp >= nsp; sp -= nsp) {
+        tile += gridDim.x;
+        nb += nbox;
+      }
+      if (tile >= nt32) break;
+      xslot += (uint32_t)(nb + (sp >> 1));
+      if (xslot >= xst_u) {
+        xslot -= xst_u;
+        xphase ^= 1u;
+      }
+      if (!__all_sync(0xffffffffu, wait_or_abort(x_full + 8 * xslot, xphase, s_abort, O.counters, ERR_TIMEOUT_FULL,
+                                                 lim)))
+        break;
+      const uint32_t xrow = row0 + xslot * xbytes;
+      const uint32_t a_t = tmem + lane_base + A0 + ar.slot * 128;
+      const uint32_t half = (uint32_t)(sp & 1) << 6;  // chunks 4-7 of the box: chunk ^ 4
+      // 16 bytes (128 samples) of row r per sub-stage; 128-byte swizzle:
+      // chunk c of row r sits at c ^ (r % 8).  Column 8qq+jj of a stage =
+      // word qq shifted left by 2*(jj/2), masked to bit 7 (jj even: byte t
+      // holds sample 8t+7-jj as 0 / -128) or bit 6 (jj odd: 0 / 64; the B
+      // image holds -2 V there), so one shift serves two columns.  The
+      // shift is a multiply so that it issues on the FMA pipe and the
+      // masks on the ALU pipe.
+      // The slot is waited for once the first sub-stage is unpacked.
+      auto slot_free = [&] {
+        return !ar.used || __all_sync(0xffffffffu, wait_or_abort(a_empty + 8 * ar.slot, ar.phase ^ 1u, s_abort,
+                                                                 O.counters, ERR_TIMEOUT_MMA, lim));
+      };
+      const int nsub_here = nsub - sp * TS_SUPER;
+      bool ok = true;
+      if (nsub_here >= TS_SUPER) {
+        uint32_t w[TS_SUPER][4];
+#pragma unroll
+        for (int sub = 0; sub < TS_SUPER; ++sub)
+          asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                       : "=r"(w[sub][0]), "=r"(w[sub][1]), "=r"(w[sub][2]), "=r"(w[sub][3])
+                       : "r"(xrow + (WIDE ? off[sub] ^ half : off[sub] + half)));
+#pragma unroll
+        for (int sub = 0; sub < TS_SUPER; ++sub) {
+          uint32_t o[32];
+          unpack_stage(w[sub], o);
+          if (sub == 0 && !slot_free()) {
             ok = false;
             break;
           }
-          const uint32_t xrow = sx + xr.slot * xbytes + r * rb;
-          const uint32_t rx = r & swz;
-          const uint32_t a_t = tmem + lane_base + A0 + ar.slot * 128;
-          const int c0 = kc - bx * (TS_BOX / TS_KS);
-          // 16 bytes (128 samples) of row r per sub-stage; 128-byte swizzle:
-          // chunk c of row r sits at c ^ (r % 8).  Column 8qq+jj of a stage =
-          // word qq shifted left by 2*(jj/2), masked to bit 7 (jj even: byte t
-          // holds sample 8t+7-jj as 0 / -128) or bit 6 (jj odd: 0 / 64; the B
-          // image holds -2 V there), so one shift serves two columns.  The
-          // shift is a multiply so that it issues on the FMA pipe and the
-          // masks on the ALU pipe.
-          if (ke - kc == TS_SUPER) {
-            uint32_t w[TS_SUPER][4];
-#pragma unroll
-            for (int sub = 0; sub < TS_SUPER; ++sub)
-              asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                           : "=r"(w[sub][0]), "=r"(w[sub][1]), "=r"(w[sub][2]), "=r"(w[sub][3])
-                           : "r"(xrow + (((c0 + sub) ^ rx) << 4)));
-#pragma unroll
-            for (int sub = 0; sub < TS_SUPER; ++sub) {
-              uint32_t o[32];
-              unpack_stage(w[sub], o);
-              tc_st32(a_t + sub * 32, o);
-            }
-          } else {
-            for (int sub = 0; sub < ke - kc; ++sub) {
-              uint4 v;
-              asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                           : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                           : "r"(xrow + (((c0 + sub) ^ rx) << 4)));
-              const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
-              uint32_t o[32];
-              unpack_stage(w4, o);
-              tc_st32(a_t + sub * 32, o);
-            }
-          }
-          kc = ke;
-          tc_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(a_full + 8 * ar.slot);
-          ar.next();
-          if (UG > 1) turn = turn + 1 == (uint32_t)UG ? 0u : turn + 1;
+          tc_st32(a_t + sub * 32, o);
         }
-        if (!ok) break;
-        // every unpack warp releases every box, whether or not it read from it
-        __syncwarp();
-        if (lane == 0) mbar_arrive(x_empty + 8 * xr.slot);
+      } else {
+        for (int sub = 0; sub < nsub_here; ++sub) {
+          uint4 v;
+          asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                       : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                       : "r"(xrow + ((uint32_t)(sub ^ rx) << 4 ^ half)));
+          const uint32_t w4[4] = {v.x, v.y, v.z, v.w};
+          uint32_t o[32];
+          unpack_stage(w4, o);
+          if (sub == 0 && !slot_free()) {
+            ok = false;
+            break;
+          }
+          tc_st32(a_t + sub * 32, o);
+        }
+      }
+      if (!ok) break;
+      tc_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      mbar_arrive_if(a_full + 8 * ar.slot, lane == 0);
+      // each warp arrives twice per box: once per super-stage, or twice for
+      // a single one
+      mbar_arrive_if(x_empty + 8 * xslot, lane == 0, (sp & 1) == 0 && sp + 1 == nsp ? 2u : 1u);
+      if (ug == NSLOT) {  // the same slot again, a lap later
+        ar.phase ^= 1u;
+        ar.used = 1;
+      } else {
+        ar.next();
       }
     }
   } else {
@@ -325,6 +378,7 @@ __global__ void __launch_bounds__(ts_threads(N), 1)
     const int q = warp & 3;
     const int r = q * 32 + lane;
     const uint32_t lane_base = (uint32_t)(q * 32) << 16;
+    const int ku = P.k - (DROP0 ? 1 : 0);  // U columns with limbs
     uint32_t jt = 0;            // tiles taken by this group
     uint32_t tested_local = 0;  // k-mers this thread tested (lean path)
     for (unsigned long long tile = blockIdx.x + (unsigned long long)e * gridDim.x; tile < ntiles;
@@ -340,9 +394,16 @@ __global__ void __launch_bounds__(ts_threads(N), 1)
       for (int c16 = 0; c16 < N / 16; ++c16) reg_fence16(d + c16 * 16);
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(acc_empty + 8 * e);
+      mbar_arrive_if(acc_empty + 8 * e, lane == 0);
       const unsigned long long local = tile * TS_TM + r;
       const bool valid = local < m;
+      if (DROP0 && P.S.on && !O.tested) {
+        const int v = screen_kmer<KU_MAX, 5, GATE, false>(P.S, P.n, d, ku, valid);
+        if (!__any_sync(0xffffffffu, v == 2)) {
+          if (v) tested_local += O.weight ? O.weight[O.kmer_offset + local] : 1u;
+          continue;
+        }
+      }
       // accumulators hold -128 * (integer limb sums).  The limbs are
       // recombined exactly in int64 and turned into doubles with the
       // bias trick (integer add + one FMA, no conversion instructions):
@@ -364,18 +425,15 @@ __global__ void __launch_bounds__(ts_threads(N), 1)
         const double s0 = P.a[0] * cd;
         ss = s0 * s0;
       }
-      // straight-line over every column slot that fits in N: slots past the
-      // phenotype's k columns have zero limbs and a = g = 0, so they add
-      // exact zeros
+      // the ku column slots in use: at least KU_MAX - 5, as N is the limb
+      // columns rounded up to 16.  e_j = V * esc exactly; every operation has
+      // one constant operand, which it reads from the parameter bank.
 #pragma unroll
       for (int jj = 0; jj < KU_MAX; ++jj) {
+        if (jj >= KU_MAX - 5 && jj >= ku) break;
         const int j = jj + (DROP0 ? 1 : 0);
         const int o = 1 + TS_LY + TS_LU * jj;
-        // biased: 1.5 * 2^52 + V as a bit pattern, V = sum_l 256^(L-1-l) d_l
-        long long Vb = (long long)(int)d[o + TS_LU - 1] + (long long)0x4338000000000000LL;
-#pragma unroll
-        for (int l = 1; l < TS_LU; ++l) Vb += (long long)(int)d[o + TS_LU - 1 - l] * (1ll << (8 * l));
-        const double e = fma(__longlong_as_double(Vb), LM.esc[j], LM.eoff[j]);
+        const double e = i2d_exact(limb3(d[o], d[o + 1], d[o + 2])) * LM.esc[j];
         const double sj = fma(P.a[j], cd, e);
         ss = fma(sj, sj, ss);
         if (GATE) gs = fma(P.g[j], e, gs);  // only the Pearson gate reads gs
@@ -444,23 +502,41 @@ static int ts_ring_depth(int b_bytes, int rb) {
   return x;
 }
 
+// Unpack groups that take part.  A parity wait is only sound for a waiter less
+// than a lap of its ring ahead.  A group that waits for the box of super-stage
+// s has filled s - ug, so the MMAs of s - 2 ug have completed, and those were
+// issued after every earlier super-stage was full: all boxes up to that one's
+// have landed.  With ug groups the ring must therefore hold at least the boxes
+// from s - 2 ug to s; where it does not (an image that leaves two or three
+// boxes), one group takes every super-stage and visits every box.
+static int ts_groups(int ug, int nsub, int xst) {
+  const int nsp = (nsub + TS_SUPER - 1) / TS_SUPER, nbox = (nsp + 1) / 2;
+  int need = 0;
+  for (int s = 0; s < nsp; ++s) {
+    const int e = s + 2 * ug;
+    need = std::max(need, e / nsp * nbox + (e % nsp) / 2 - s / 2);
+  }
+  return xst >= need ? ug : 1;
+}
+
 template <int N, bool D0, bool GATE, bool WIDE>
 static cudaError_t launch_ts_w(const LaunchTs& L, const CUtensorMap& tm, cudaStream_t st) {
   const int b_bytes = L.kpad * N;
+  // 128-sample sub-stages: those of the image that a row reaches (kpad is
+  // rounded up further; the image is zero past the row's samples)
+  const int nsub = L.kpad / TS_KS < L.wpk / 2 ? L.kpad / TS_KS : L.wpk / 2;
   const int rb = ts_box_bytes(L.wpk);
   const int xst = ts_ring_depth(b_bytes, rb);
   const size_t smem = ts_smem(b_bytes, xst, rb).total + 1024;
+  const int ug = ts_groups(ts_ug(N), nsub, xst);
   cudaError_t e =
       cudaFuncSetAttribute(ts_kernel<N, D0, GATE, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const unsigned long long tiles = (L.m + TS_TM - 1) / TS_TM;
   unsigned long long grid = (unsigned long long)L.num_sms;
   if (grid > tiles) grid = tiles;
-  // 128-sample sub-stages: those of the image that a row reaches (kpad is
-  // rounded up further; the image is zero past the row's samples)
-  const int nsub = L.kpad / TS_KS < L.wpk / 2 ? L.kpad / TS_KS : L.wpk / 2;
   const int nbox = (nsub * 16 + 127) / 128;
-  ts_kernel<N, D0, GATE, WIDE><<<(unsigned)grid, ts_threads(N), smem, st>>>(tm, L.m, nbox, nsub, xst, rb, L.Bimg, b_bytes,
+  ts_kernel<N, D0, GATE, WIDE><<<(unsigned)grid, ts_threads(N), smem, st>>>(tm, L.m, nbox, nsub, xst, ug, rb, L.Bimg, b_bytes,
                                                                    *L.P, *L.LM, *L.O);
   return cudaGetLastError();
 }

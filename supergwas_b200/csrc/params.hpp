@@ -7,6 +7,22 @@
 
 namespace kg {
 
+// Single-precision screen of one k-mer (screen_kmer in device.cuh): decides
+// from the limb sums, with room for its own rounding, that a k-mer is not
+// tested, or is tested and cannot reach the emit or the refinement cut.
+// Everything about y is relative to ||y - mean(y)||.
+struct ScreenParams {
+  int on;            // 0: every k-mer takes the FP64 statistic
+  int shift;         // limb sums are shifted right by this into 32 bits
+  float inv_n;       // 1 / n
+  float b, kappa;    // b / ynorm, kappa / ynorm
+  float cut;         // 0.9 x the lowest r2 that matters x yyM / ynorm^2
+  float gate_lo, gate_hi;  // (corr_thr -+ margin)^2
+  float sy;          // y' limb sums -> e_y / ynorm
+  float su[KMAX];    // U limb sums -> e_j
+  float g[KMAX];     // g_j / ynorm
+};
+
 // Per-phenotype constants of the epilogue (prep.hpp notation).
 struct EpiParams {
   int n, k;
@@ -14,9 +30,11 @@ struct EpiParams {
   double r2_cand;   // r2 below this cannot give p <= p_thresh (log/erfc skipped)
   int refine;       // 1: k-mers with r2 >= r2_ref go to the FP64 refinement list
   double r2_ref;
+  double r2_need;   // refinement may skip k-mers with r2 in [r2_ref, r2_need), see may_refine
   double thr2_ynorm2;  // corr_thr^2 * ynorm^2 (division-free Pearson gate)
   double a[KMAX];
   double g[KMAX];
+  ScreenParams S;
 };
 
 // Column map of the int8 limb contraction (prep.hpp LimbCols).
@@ -37,6 +55,41 @@ inline void set_limb_consts(LimbMap& L) {
   for (int j = 0; j <= KMAX; ++j) {
     L.esc[j] = -L.scale[j] / 128.0;
     L.eoff[j] = 6755399441055744.0 * L.scale[j] / 128.0;
+  }
+}
+
+// The part of the refinement range that a launch without per-k-mer outputs
+// leaves out: a k-mer whose r2 in the split form is below 0.9 of the emit cut
+// is not emitted whatever the refinement gives, as long as the split form's
+// xxM is good to a few percent (may_refine).
+inline void set_refine_need(EpiParams& P) { P.r2_need = 0.9 * P.r2_cand; }
+
+// Screen constants of a phenotype whose intercept carries no limbs (drop0)
+// and whose limb columns are those of L (3 per U column, 5 for y').  See
+// screen_kmer for the error bounds behind the margins.
+inline void set_screen(EpiParams& P, const LimbMap& L, bool drop0) {
+  ScreenParams& S = P.S;
+  S = ScreenParams();
+  double cut = P.r2_cand;
+  if (P.refine && P.r2_ref < cut) cut = P.r2_ref > P.r2_need ? P.r2_ref : P.r2_need;
+  const double yv = P.yyM / (P.ynorm * P.ynorm);
+  if (!drop0 || !(P.ynorm >= 1e-12) || !(P.ynorm < 1e150) || !(cut > 0) || !(yv > 1e-6) || P.n >= 65536) return;
+  S.on = 1;
+  while ((4 << S.shift) < P.n) ++S.shift;
+  S.inv_n = (float)(1.0 / P.n);
+  S.b = (float)(P.b / P.ynorm);
+  S.kappa = (float)(P.kappa / P.ynorm);
+  S.cut = (float)(0.9 * cut * yv);
+  const double eps = 1e-4 * (P.n > 1024 ? P.n / 1024.0 : 1.0);
+  const double lo = P.corr_thr > eps ? P.corr_thr - eps : 0.0, hi = P.corr_thr + eps;
+  S.gate_lo = (float)(lo * lo);
+  S.gate_hi = (float)(hi * hi);
+  // accumulators hold -128 x the digit sums; y' drops its lowest limb
+  const double unit = -(double)(1 << S.shift) / 128.0;
+  S.sy = (float)(unit * 65536.0 * L.scale[P.k] / P.ynorm);
+  for (int j = 1; j < P.k; ++j) {
+    S.su[j] = (float)(unit * L.scale[j]);
+    S.g[j] = (float)(P.g[j] / P.ynorm);
   }
 }
 

@@ -416,13 +416,13 @@ static cudaError_t launch_mp_t(const LaunchMp& L, const CUtensorMap& tm, cudaStr
   return cudaGetLastError();
 }
 
-bool mp_tmap(const uint64_t* x, unsigned long long m, int wpk, CUtensorMap* tm) {
+bool mp_tmap(const uint64_t* x, unsigned long long m, int wpk, CUtensorMap* tm, int rows) {
   auto enc = mp_encode_fn();
   if (!enc) return false;
   const cuuint64_t rowbytes = (cuuint64_t)wpk * 8;
   cuuint64_t gdim[2] = {rowbytes, (cuuint64_t)m};
   cuuint64_t gstride[1] = {rowbytes};
-  cuuint32_t box[2] = {128, MP_TM};
+  cuuint32_t box[2] = {128, (cuuint32_t)rows};
   cuuint32_t estr[2] = {1, 1};
   return enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)x, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,

@@ -6,15 +6,22 @@
 // xyM = x12.y - (U^T x12).(U^T y), compute_hit.  That is exactly the
 // contraction kernel_ts.cu runs, with A = the AND of two packed rows.  A tile
 // here is 128 pairs (i, j) sharing i, j in one 128-row j-block:
-//   producer  TMA-loads the j-block's packed rows once per unit (a unit is up
-//             to `ic` consecutive i of one j-block), no multicast;
+//   producer  TMA-loads the j-block's packed rows and the unit's rows i once
+//             per unit (a unit is up to `ic` consecutive i of one j-block), no
+//             multicast;
 //   unpack    ANDs each 128-sample chunk of the resident j rows with the same
-//             chunk of row i (a warp-uniform global load) and writes the int8
-//             A operand into TMEM (unpack_stage);
-//   MMA       tcgen05.mma kind::i8 against the resident limb image;
-//   epilogue  limb recombination and the FP64 statistic; pairs that may pass
-//             the cut (chi-square >= 12) go to the FP64 refinement list,
-//             which pr_refine_kernel recomputes from byte tables.
+//             chunk of row i (one address for the warp) and writes the int8 A
+//             operand into TMEM (unpack_stage); a group per slot;
+//   MMA       tcgen05.mma kind::i8 against the resident limb image, two warps
+//             on alternate tiles;
+//   epilogue  the single-precision screen; for warps with a pair near a cut
+//             the limb recombination and FP64 statistic; pairs that may pass
+//             the emit cut go to the FP64 refinement list, which
+//             pr_refine_kernel recomputes from byte tables.
+// Roles and bounds are those of kernel_ts.cu.  2e8 pairs at n = 1000, r = 16+1
+// (whole call, rows from host memory, 47,000 pairs returned): 12.2 ms, before
+// 17.1 ms (FP64 statistic per pair, one MMA warp, rows i by global loads whose
+// first touch waited for L2 in every tile).
 // Every wait is bounded (KG_ERR_TIMEOUT), as in kernel_ts.cu.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -29,27 +36,32 @@ constexpr int PR_KS = 128;
 constexpr int PR_SUPER = 4;
 constexpr int PR_BOX = 1024;
 constexpr uint32_t PR_XBYTES = PR_TM * 128;
+// Rows i of a unit beside its j-block: one box of 32 rows per 1024 samples, in
+// the same slot of the ring.
+constexpr int PR_IC = 32;
+constexpr uint32_t PR_IBYTES = PR_IC * 128;
 constexpr int PR_LU = 3, PR_LY = 5;
 constexpr int PR_MAXSLOT = 3;
 constexpr int PR_XST_MAX = 12;
 constexpr int PR_NBOX_MAX = 8;  // rows of up to 1 KB: 8192 samples
 constexpr int PR_WARP_UNPACK0 = 8;
 
-__host__ __device__ constexpr int pr_ug(int N) { return N <= 80 ? 2 : 1; }
-__host__ __device__ constexpr int pr_threads(int N) { return 32 * (8 + 4 * pr_ug(N) + 2); }
 __host__ __device__ constexpr int pr_nslot(int N) {
   return (512 - 2 * N) / 128 > PR_MAXSLOT ? PR_MAXSLOT : (512 - 2 * N) / 128;
 }
+// Unpack groups: one per slot, as in kernel_ts.cu.
+__host__ __device__ constexpr int pr_ug(int N) { return N <= 80 ? pr_nslot(N) : 1; }
+__host__ __device__ constexpr int pr_threads(int N) { return 32 * (8 + 4 * pr_ug(N) + 3); }
 
 struct PrSmem {
   uint32_t x, b, bars, tmem, abort, total;
 };
-__host__ __device__ inline PrSmem pr_smem(int b_bytes, int xst) {
+__host__ __device__ inline PrSmem pr_smem(int b_bytes, int xst, bool ibox) {
   PrSmem L;
   L.x = 0;
-  L.b = xst * PR_XBYTES;
+  L.b = xst * (PR_XBYTES + (ibox ? PR_IBYTES : 0));
   L.bars = L.b + ((b_bytes + 127) / 128) * 128;
-  L.tmem = L.bars + 8 * (2 * PR_XST_MAX + 2 * PR_MAXSLOT + 4 + 2);
+  L.tmem = L.bars + 8 * (2 * PR_XST_MAX + 2 * PR_MAXSLOT + 4 + 5);
   L.abort = L.tmem + 8;
   L.total = L.abort + 8;
   return L;
@@ -116,7 +128,8 @@ __device__ __forceinline__ void pr_emit(const DevOutPairs& O, unsigned long long
 
 template <int N, bool DROP0>
 __global__ void __launch_bounds__(pr_threads(N), 1)
-    pairs_kernel(const __grid_constant__ CUtensorMap tmap, const uint64_t* __restrict__ x, int wpk, int nbox,
+    pairs_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap itmap, bool ibox,
+                 const uint64_t* __restrict__ x, int wpk, int nbox,
                  int nsub, int xst, const __grid_constant__ PairSched S, const int8_t* __restrict__ Bimg,
                  int b_bytes, const __grid_constant__ EpiParams P, const __grid_constant__ LimbMap LM,
                  const DevOutPairs O) {
@@ -132,15 +145,16 @@ __global__ void __launch_bounds__(pr_threads(N), 1)
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* gbase = smem_raw + (base - raw);
-  const PrSmem L = pr_smem(b_bytes, xst);
+  const PrSmem L = pr_smem(b_bytes, xst, ibox);
+  const uint32_t xslot = PR_XBYTES + (ibox ? PR_IBYTES : 0u);
   const uint32_t sx = base + L.x, sb = base + L.b;
   const uint32_t x_full = base + L.bars, x_empty = x_full + 8 * PR_XST_MAX;
   const uint32_t a_full = x_empty + 8 * PR_XST_MAX, a_empty = a_full + 8 * PR_MAXSLOT;
   const uint32_t acc_full = a_empty + 8 * PR_MAXSLOT, acc_empty = acc_full + 16, b_full = acc_empty + 16;
-  const uint32_t drain = b_full + 8;
+  const uint32_t drain = b_full + 8, turn = drain + 16;
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(gbase + L.tmem);
   volatile int* s_abort = reinterpret_cast<volatile int*>(gbase + L.abort);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int nsp = (nsub + PR_SUPER - 1) / PR_SUPER;
 
   if (warp == 0) {
@@ -162,14 +176,17 @@ __global__ void __launch_bounds__(pr_threads(N), 1)
       mbar_init(acc_empty + 8 * b, 4);
     }
     mbar_init(b_full, 1);
-    mbar_init(drain, 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(drain + 8 * b, 1);
+      mbar_init(turn + 8 * b, 1);
+    }
     *s_abort = 0;
     mbar_fence_init();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *s_tmem;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *s_tmem, 0);
   const unsigned long long lim = wait_limit(O.wait_ns);
 
   if (warp == WPROD) {
@@ -193,8 +210,10 @@ __global__ void __launch_bounds__(pr_threads(N), 1)
             ok = false;
             break;
           }
-          mbar_arrive_expect_tx(x_full + 8 * xr.slot, PR_XBYTES);
-          tma_load_2d(sx + xr.slot * PR_XBYTES, &tmap, bx * 128, (int)(U.jb * PR_TM), x_full + 8 * xr.slot);
+          mbar_arrive_expect_tx(x_full + 8 * xr.slot, xslot);
+          tma_load_2d(sx + xr.slot * xslot, &tmap, bx * 128, (int)(U.jb * PR_TM), x_full + 8 * xr.slot);
+          if (ibox)
+            tma_load_2d(sx + xr.slot * xslot + PR_XBYTES, &itmap, bx * 128, (int)U.i0, x_full + 8 * xr.slot);
           issued[xr.slot] = true;
           last_phase[xr.slot] = xr.phase;
         }
@@ -203,23 +222,34 @@ __global__ void __launch_bounds__(pr_threads(N), 1)
       for (int s = 0; s < xst; ++s)
         if (issued[s]) mbar_wait(x_full + 8 * s, last_phase[s], O.counters, ERR_TIMEOUT_FULL);
     }
-  } else if (warp == WMMA) {
+  } else if (warp >= WMMA) {
     // ----------------------------------------------------------------- MMA
+    // two warps taking alternate tiles, in the order of kernel_ts.cu
     const bool leader = elect_one();
+    const uint32_t b = (uint32_t)(warp - WMMA);
     bool ok = __all_sync(0xffffffffu, wait_or_abort(b_full, 0, s_abort, O.counters, ERR_TIMEOUT_FULL, lim));
     const uint64_t bdesc0 = sdesc_noswz(sb, N * 16, 128);
+    const uint32_t d_t = tmem + b * N;
     Ring<NSLOT> ar;
-    uint32_t v = 0;  // tiles
+    uint32_t v = 0, t = 0;  // tiles of the CTA, of this warp
     for (unsigned long long u = blockIdx.x; u < S.n_units && ok; u += gridDim.x) {
       const PairUnit U = pr_unit(S, u);
-      for (unsigned long long i = U.i0; i < U.i1 && ok; ++i, ++v) {
-        const uint32_t b = v & 1u;
-        if (v >= 2 && !__all_sync(0xffffffffu, wait_or_abort(acc_empty + 8 * b, ((v >> 1) - 1) & 1u, s_abort,
-                                                             O.counters, ERR_TIMEOUT_MMA, lim))) {
+      for (unsigned long long i = U.i0; i < U.i1; ++i, ++v) {
+        if ((v & 1u) != b) {  // the other warp's tile
+          for (int sp = 0; sp < nsp; ++sp) ar.next();
+          continue;
+        }
+        if (t >= 1 && !__all_sync(0xffffffffu, wait_or_abort(acc_empty + 8 * b, (t - 1) & 1u, s_abort, O.counters,
+                                                             ERR_TIMEOUT_MMA, lim))) {
           ok = false;
           break;
         }
-        const uint32_t d_t = tmem + b * N;
+        if ((b || t >= 1) && !__all_sync(0xffffffffu, wait_or_abort(turn + 8 * b, b ? t & 1u : (t - 1) & 1u, s_abort,
+                                                                    O.counters, ERR_TIMEOUT_MMA, lim))) {
+          ok = false;
+          break;
+        }
+        ++t;
         uint64_t bd = bdesc0;
         for (int sp = 0; sp < nsp; ++sp, ar.next()) {
           if (!__all_sync(0xffffffffu,
@@ -227,16 +257,23 @@ __global__ void __launch_bounds__(pr_threads(N), 1)
             ok = false;
             break;
           }
+          mbar_arrive_if(turn + 8 * (b ^ 1u), leader && sp + 1 == nsp);
           tc_fence_after();
           const int nsub_here = nsub - sp * PR_SUPER < PR_SUPER ? nsub - sp * PR_SUPER : PR_SUPER;
           const uint32_t a_t = tmem + A0 + ar.slot * 128;
           if (leader) {
-            uint64_t bk = bd;
-            for (int sub = 0; sub < nsub_here; ++sub) {
+            if (nsub_here == PR_SUPER) {
 #pragma unroll
-              for (int ks = 0; ks < PR_KS / 32; ++ks) {
-                tc_mma_i8_ts(d_t, a_t + sub * 32 + ks * 8, bk, IDESC, (sp | sub | ks) ? 1u : 0u);
-                bk += BSTEP;
+              for (int k = 0; k < PR_SUPER * (PR_KS / 32); ++k)
+                tc_mma_i8_ts(d_t, a_t + k * 8, bd + (uint64_t)(k * BSTEP), IDESC, (sp | k) ? 1u : 0u);
+            } else {
+              uint64_t bk = bd;
+              for (int sub = 0; sub < nsub_here; ++sub) {
+#pragma unroll
+                for (int ks = 0; ks < PR_KS / 32; ++ks) {
+                  tc_mma_i8_ts(d_t, a_t + sub * 32 + ks * 8, bk, IDESC, (sp | sub | ks) ? 1u : 0u);
+                  bk += BSTEP;
+                }
               }
             }
             tc_commit(a_empty + 8 * ar.slot);
@@ -250,12 +287,13 @@ __global__ void __launch_bounds__(pr_threads(N), 1)
       }
     }
     if (leader) {
-      tc_commit(drain);
-      mbar_wait(drain, 0, O.counters, ERR_TIMEOUT_MMA);
+      tc_commit(drain + 8 * b);
+      mbar_wait(drain + 8 * b, 0, O.counters, ERR_TIMEOUT_MMA);
     }
     __syncwarp();
   } else if (warp >= PR_WARP_UNPACK0) {
     // -------------------------------------------------------------- unpack
+    // group grp fills super-stages grp, grp + UG, ... of the CTA's tiles
     const int grp = (warp - PR_WARP_UNPACK0) >> 2;
     const int q = warp & 3;
     const int r = q * 32 + lane;
@@ -263,78 +301,85 @@ __global__ void __launch_bounds__(pr_threads(N), 1)
     const int half_row = wpk / 2;  // 16-byte chunks in a packed row
     RingN xr(xst);
     Ring<NSLOT> ar;
-    uint32_t turn = 0;
+    for (int g = 0; g < grp; ++g) ar.next();
+    int skip = grp;  // super-stages from here to this group's next one
     bool ok = true;
     for (unsigned long long u = blockIdx.x; u < S.n_units && ok; u += gridDim.x) {
       const PairUnit U = pr_unit(S, u);
-      // the unit's boxes stay resident for all its tiles
-      uint32_t bslot[PR_NBOX_MAX], bphase[PR_NBOX_MAX];
-      for (int bx = 0; bx < nbox; ++bx, xr.next()) {
-        bslot[bx] = xr.slot;
-        bphase[bx] = xr.phase;
-      }
-      for (unsigned long long i = U.i0; i < U.i1 && ok; ++i) {
-        const uint4* xi = reinterpret_cast<const uint4*>(x + i * (unsigned long long)wpk);
-        int kc = 0;
-        for (int bx = 0; bx < nbox && ok; ++bx) {
-          if (i == U.i0 && !__all_sync(0xffffffffu, wait_or_abort(x_full + 8 * bslot[bx], bphase[bx], s_abort,
-                                                                  O.counters, ERR_TIMEOUT_FULL, lim))) {
-            ok = false;
-            break;
-          }
-          const int kc1 = (bx + 1) * (PR_BOX / PR_KS) < nsub ? (bx + 1) * (PR_BOX / PR_KS) : nsub;
-          while (kc < kc1) {
-            const int ke = kc + PR_SUPER < kc1 ? kc + PR_SUPER : kc1;
-            if (UG == 2 && turn != (uint32_t)grp) {
-              kc = ke;
-              ar.next();
-              turn ^= 1u;
-              continue;
+      const int cnt = (int)(U.i1 - U.i0);
+      // the unit's boxes stay resident for all its tiles; box bx of the unit
+      // is slot slot0 + bx of the ring
+      const uint32_t slot0 = xr.slot;
+      for (int bx = 0; bx < nbox; ++bx, xr.next())
+        if (ok && !__all_sync(0xffffffffu, wait_or_abort(x_full + 8 * xr.slot, xr.phase, s_abort, O.counters,
+                                                         ERR_TIMEOUT_FULL, lim)))
+          ok = false;
+      int ii = 0, sp = skip;  // tile of the unit, super-stage of the tile
+      for (; sp >= nsp; sp -= nsp) ++ii;
+      while (ok && ii < cnt) {
+        uint32_t slot = slot0 + (uint32_t)(sp >> 1);
+        if (slot >= (uint32_t)xst) slot -= (uint32_t)xst;
+        const uint32_t box = sx + slot * xslot;
+        const uint32_t half = (uint32_t)(sp & 1) * PR_SUPER;  // first 16-byte chunk of the box
+        const int here = nsub - sp * PR_SUPER < PR_SUPER ? nsub - sp * PR_SUPER : PR_SUPER;
+        const uint32_t a_t = tmem + lane_base + A0 + ar.slot * 128;
+        // the super-stage's chunks of row i (uniform across the warp) and of
+        // the j rows, all loads in flight before the first use
+        uint4 wi[PR_SUPER], wj[PR_SUPER];
+#pragma unroll
+        for (int s4 = 0; s4 < PR_SUPER; ++s4) {
+          if (s4 < here) {
+            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                         : "=r"(wj[s4].x), "=r"(wj[s4].y), "=r"(wj[s4].z), "=r"(wj[s4].w)
+                         : "r"(box + r * 128 + (((half + s4) ^ (r & 7)) << 4)));
+            if (ibox)
+              asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                           : "=r"(wi[s4].x), "=r"(wi[s4].y), "=r"(wi[s4].z), "=r"(wi[s4].w)
+                           : "r"(box + PR_XBYTES + ii * 128 + (((half + s4) ^ (ii & 7)) << 4)));
+            else {
+              const int sub = sp * PR_SUPER + s4;
+              const uint4* xi = reinterpret_cast<const uint4*>(x + (U.i0 + ii) * (unsigned long long)wpk);
+              wi[s4] = sub < half_row ? __ldg(xi + sub) : make_uint4(0u, 0u, 0u, 0u);
             }
-            if (ar.used && !__all_sync(0xffffffffu, wait_or_abort(a_empty + 8 * ar.slot, ar.phase ^ 1u, s_abort,
-                                                                  O.counters, ERR_TIMEOUT_MMA, lim))) {
+          }
+        }
+#pragma unroll
+        for (int s4 = 0; s4 < PR_SUPER; ++s4) {
+          if (s4 < here) {
+            const uint32_t w4[4] = {wj[s4].x & wi[s4].x, wj[s4].y & wi[s4].y, wj[s4].z & wi[s4].z,
+                                    wj[s4].w & wi[s4].w};
+            uint32_t o[32];
+            unpack_stage(w4, o);
+            if (s4 == 0 && ar.used &&
+                !__all_sync(0xffffffffu, wait_or_abort(a_empty + 8 * ar.slot, ar.phase ^ 1u, s_abort, O.counters,
+                                                       ERR_TIMEOUT_MMA, lim))) {
               ok = false;
               break;
             }
-            const uint32_t xrow = sx + bslot[bx] * PR_XBYTES + r * 128;
-            const uint32_t a_t = tmem + lane_base + A0 + ar.slot * 128;
-            // the super-stage's chunks of row i (uniform across the warp) and
-            // of the j rows, all loads in flight before the first use
-            uint4 wi[PR_SUPER], wj[PR_SUPER];
-#pragma unroll
-            for (int s4 = 0; s4 < PR_SUPER; ++s4) {
-              const int sub = kc + s4;
-              wi[s4] = (sub < ke && sub < half_row) ? __ldg(xi + sub) : make_uint4(0u, 0u, 0u, 0u);
-              const int c = sub - bx * (PR_BOX / PR_KS);
-              if (sub < ke)
-                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                             : "=r"(wj[s4].x), "=r"(wj[s4].y), "=r"(wj[s4].z), "=r"(wj[s4].w)
-                             : "r"(xrow + ((c ^ (r & 7)) << 4)));
-            }
-#pragma unroll
-            for (int s4 = 0; s4 < PR_SUPER; ++s4) {
-              if (kc + s4 < ke) {
-                const uint32_t w4[4] = {wj[s4].x & wi[s4].x, wj[s4].y & wi[s4].y, wj[s4].z & wi[s4].z,
-                                        wj[s4].w & wi[s4].w};
-                uint32_t o[32];
-                unpack_stage(w4, o);
-                tc_st32(a_t + s4 * 32, o);
-              }
-            }
-            kc = ke;
-            tc_wait_st();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(a_full + 8 * ar.slot);
-            ar.next();
-            if (UG == 2) turn ^= 1u;
+            tc_st32(a_t + s4 * 32, o);
           }
         }
+        if (!ok) break;
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        mbar_arrive_if(a_full + 8 * ar.slot, lane == 0);
+        if (UG == NSLOT) {  // the same slot again, a lap later
+          ar.phase ^= 1u;
+          ar.used = 1;
+        } else {
+          ar.next();
+        }
+        for (sp += UG; sp >= nsp; sp -= nsp) ++ii;
       }
       if (!ok) break;
+      skip = (ii - cnt) * nsp + sp;
       __syncwarp();
       if (lane == 0)
-        for (int bx = 0; bx < nbox; ++bx) mbar_arrive(x_empty + 8 * bslot[bx]);
+        for (int bx = 0; bx < nbox; ++bx) {
+          const uint32_t slot = slot0 + bx < (uint32_t)xst ? slot0 + bx : slot0 + bx - (uint32_t)xst;
+          mbar_arrive(x_empty + 8 * slot);
+        }
     }
   } else {
     // ------------------------------------------------------------ epilogue
@@ -342,6 +387,7 @@ __global__ void __launch_bounds__(pr_threads(N), 1)
     const int q = warp & 3;
     const int r = q * 32 + lane;
     const uint32_t lane_base = (uint32_t)(q * 32) << 16;
+    const int ku = P.k - (DROP0 ? 1 : 0);
     uint32_t v = 0, jt = 0, evaluated = 0;
     bool ok = true;
     for (unsigned long long u = blockIdx.x; u < S.n_units && ok; u += gridDim.x) {
@@ -368,6 +414,13 @@ __global__ void __launch_bounds__(pr_threads(N), 1)
         if (lane == 0) mbar_arrive(acc_empty + 8 * e);
         const unsigned long long j = U.jb * PR_TM + r;
         const bool valid = j < S.n_kmers && j > i;
+        if (DROP0 && P.S.on) {
+          const int v2 = screen_kmer<KU_MAX, 5, false, true>(P.S, P.n, d, ku, valid);
+          if (!__any_sync(0xffffffffu, v2 == 2)) {
+            evaluated += v2 ? 1u : 0u;
+            continue;
+          }
+        }
         // limb sums hold -128 * integer sums (see kernel_ts.cu)
         const int c = (-(int)d[0]) >> 7;
         const double cd = i2d_exact(c);
@@ -385,10 +438,7 @@ __global__ void __launch_bounds__(pr_threads(N), 1)
         for (int jj = 0; jj < KU_MAX; ++jj) {
           const int col = jj + (DROP0 ? 1 : 0);
           const int o = 1 + PR_LY + PR_LU * jj;
-          long long Vb = (long long)(int)d[o + PR_LU - 1] + (long long)0x4338000000000000LL;
-#pragma unroll
-          for (int l = 1; l < PR_LU; ++l) Vb += (long long)(int)d[o + PR_LU - 1 - l] * (1ll << (8 * l));
-          const double ej = fma(__longlong_as_double(Vb), LM.esc[col], LM.eoff[col]);
+          const double ej = i2d_exact(limb3(d[o], d[o + 1], d[o + 2])) * LM.esc[col];
           const double sj = fma(P.a[col], cd, ej);
           ss = fma(sj, sj, ss);
         }
@@ -398,7 +448,7 @@ __global__ void __launch_bounds__(pr_threads(N), 1)
         const double qv = xyM * xyM, den = xxM * P.yyM;
         const bool okp = valid && c > 0 && xxM > eps && P.yyM > eps;
         evaluated += okp ? 1u : 0u;
-        const bool cand = okp && P.refine && qv >= P.r2_ref * den;
+        const bool cand = okp && P.refine && may_refine(P, cd, xxM, qv, den);
         const bool maybe = okp && !cand && qv >= P.r2_cand * den;
         if (__ballot_sync(0xffffffffu, cand || maybe) == 0u) continue;
         double T = 0, p = 1, effect = 0;
@@ -474,13 +524,20 @@ __global__ void __launch_bounds__(256) pr_refine_kernel(const uint64_t* __restri
 
 // ------------------------------------------------------------------- host
 
-static int pr_ring_depth(int b_bytes, int nbox) {
+static int pr_ring_depth(int b_bytes, int nbox, bool ibox) {
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) optin = 0;
   int x = PR_XST_MAX;
-  while (x > nbox && pr_smem(b_bytes, x).total + 1024 > (uint32_t)optin) --x;
+  while (x > nbox && pr_smem(b_bytes, x, ibox).total + 1024 > (uint32_t)optin) --x;
   return x;
+}
+
+static bool pr_fits(int b_bytes, int xst, bool ibox) {
+  int dev = 0, optin = 0;
+  cudaGetDevice(&dev);
+  return cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
+         pr_smem(b_bytes, xst, ibox).total + 1024 <= (uint32_t)optin;
 }
 
 bool pairs_supported(int N, int limbs_u, int limbs_y, int kpad, int wpk) {
@@ -493,23 +550,30 @@ bool pairs_supported(int N, int limbs_u, int limbs_y, int kpad, int wpk) {
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return false;
   // the unit's boxes plus a second unit's, so that loads overlap
-  return pr_smem(kpad * N, 2 * nbox).total + 1024 <= (uint32_t)optin;
+  return pr_smem(kpad * N, 2 * nbox, false).total + 1024 <= (uint32_t)optin;
 }
 
 template <int N, bool D0>
-static cudaError_t launch_pairs_t(const LaunchPairs& L, const CUtensorMap& tm, cudaStream_t st) {
+static cudaError_t launch_pairs_t(const LaunchPairs& L, const CUtensorMap& tm, const CUtensorMap& itm, cudaStream_t st) {
   const int b_bytes = L.kpad * N;
   const int nbox = (L.wpk * 8 + 127) / 128;
-  const int xst = pr_ring_depth(b_bytes, nbox);
+  // rows i come with the unit's boxes while two units' fit that way, else by
+  // global loads (an image of 160 KB, n = 2000 at r = 20+1)
+  bool ibox = L.S.ic <= PR_IC;
+  int xst = pr_ring_depth(b_bytes, nbox, ibox);
+  if (ibox && (xst < 2 * nbox || !pr_fits(b_bytes, xst, ibox))) {
+    ibox = false;
+    xst = pr_ring_depth(b_bytes, nbox, ibox);
+  }
   if (xst < 2 * nbox) return cudaErrorInvalidValue;
-  const size_t smem = pr_smem(b_bytes, xst).total + 1024;
+  const size_t smem = pr_smem(b_bytes, xst, ibox).total + 1024;
   cudaError_t e =
       cudaFuncSetAttribute(pairs_kernel<N, D0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   unsigned long long grid = (unsigned long long)L.num_sms;
   if (grid > L.S.n_units) grid = L.S.n_units;
   if (grid == 0) return cudaSuccess;
-  pairs_kernel<N, D0><<<(unsigned)grid, pr_threads(N), smem, st>>>(tm, L.x, L.wpk, nbox, L.kpad / PR_KS, xst, L.S,
+  pairs_kernel<N, D0><<<(unsigned)grid, pr_threads(N), smem, st>>>(tm, itm, ibox, L.x, L.wpk, nbox, L.kpad / PR_KS, xst, L.S,
                                                                    L.Bimg, b_bytes, *L.P, *L.LM, *L.O);
   return cudaGetLastError();
 }
@@ -517,11 +581,13 @@ static cudaError_t launch_pairs_t(const LaunchPairs& L, const CUtensorMap& tm, c
 cudaError_t launch_pairs(const LaunchPairs& L, cudaStream_t st) {
   if (L.S.n_units == 0) return cudaSuccess;
   CUtensorMap tm;
-  if (!mp_tmap(L.x, L.S.n_kmers, L.wpk, &tm)) return cudaErrorInvalidValue;
+  CUtensorMap itm;
+  if (!mp_tmap(L.x, L.S.n_kmers, L.wpk, &tm) || !mp_tmap(L.x, L.S.n_kmers, L.wpk, &itm, PR_IC))
+    return cudaErrorInvalidValue;
   const bool d0 = L.drop0;
   switch (L.LM->N) {
 #define KG_PR_CASE(NN) \
-  case NN: return d0 ? launch_pairs_t<NN, true>(L, tm, st) : launch_pairs_t<NN, false>(L, tm, st);
+  case NN: return d0 ? launch_pairs_t<NN, true>(L, tm, itm, st) : launch_pairs_t<NN, false>(L, tm, itm, st);
     KG_PR_CASE(16)
     KG_PR_CASE(32)
     KG_PR_CASE(48)

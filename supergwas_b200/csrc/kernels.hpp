@@ -104,8 +104,8 @@ struct LaunchMpRefine {
 bool mp_supported(int NP, int PPG, int wpk);
 size_t mp_smem_bytes(int nbox, int xs, int nb, int N);
 cudaError_t launch_mp(const LaunchMp& L, cudaStream_t st);
-// 2-D TMA map of packed rows: 128-byte x 128-row boxes, 128-byte swizzle.
-bool mp_tmap(const uint64_t* x, unsigned long long m, int wpk, CUtensorMap_st* tm);
+// 2-D TMA map of packed rows: boxes of 128 bytes x `rows` rows, 128-byte swizzle.
+bool mp_tmap(const uint64_t* x, unsigned long long m, int wpk, CUtensorMap_st* tm, int rows = 128);
 
 // B-stationary many-phenotype kernel (kernel_mpb.cu): each group's image
 // (make_b_image_ts layout, kpad x NP*PPG bytes) resident in shared memory for

@@ -545,24 +545,12 @@ __device__ __forceinline__ float shifted_float(long long v, int s) {
 // columns); the cut it is compared with is 10 % low.  The correlation is
 // within 1e-5 per 1024 samples; gate_lo and gate_hi leave 1e-4.
 // PAIRS: no correlation gate, and c = n is left to the FP64 form.
-template <int KU_MAX, int LAST, bool GATE, bool PAIRS>
-__device__ __forceinline__ int screen_kmer(const ScreenParams& S, int n, const uint32_t* d, int ku, bool valid) {
-  const int c = (-(int)d[0]) >> 7;
+template <bool GATE, bool PAIRS>
+__device__ __forceinline__ int screen_verdict(const ScreenParams& S, int n, int c, float ey, float ss, float gs,
+                                              bool valid) {
   const float cf = (float)c;
   const float xcn = (float)(c * (n - c)) * S.inv_n;
-  const long long vy = mad_wide<(1 << 24)>(d[1], limb3(d[2], d[3], d[4]));
-  const float ey = shifted_float(vy, S.shift + 8) * S.sy;
-  float ss = 0.0f, gs = 0.0f;
-#pragma unroll
-  for (int jj = 0; jj < KU_MAX; ++jj) {
-    if (jj >= KU_MAX - LAST && jj >= ku) break;
-    const int o = 6 + 3 * jj;
-    const float e = shifted_float(limb3(d[o], d[o + 1], d[o + 2]), S.shift) * S.su[jj + 1];
-    ss = fmaf(e, e, ss);
-    if (GATE) gs = fmaf(S.g[jj + 1], e, gs);
-  }
-  const bool in = valid && c > 0 && (PAIRS || c < n);
-  if (!in) return 0;
+  if (!(valid && c > 0 && (PAIRS || c < n))) return 0;
   if (GATE) {
     const float xyc = fmaf(S.kappa, cf, ey + gs);
     const float q = xyc * xyc;
@@ -571,6 +559,25 @@ __device__ __forceinline__ int screen_kmer(const ScreenParams& S, int n, const u
   }
   const float xxM = xcn - ss, xyM = fmaf(S.b, cf, ey);
   return xxM >= 0.02f * xcn && xcn > 0.0f && xyM * xyM < S.cut * xxM ? 1 : 2;
+}
+// e_y / ynorm from the y' limb sums d[1..5], without the lowest limb.
+__device__ __forceinline__ float screen_ey(const ScreenParams& S, const uint32_t* d) {
+  return shifted_float(mad_wide<(1 << 24)>(d[1], limb3(d[2], d[3], d[4])), S.shift + 8) * S.sy;
+}
+template <int KU_MAX, int LAST, bool GATE, bool PAIRS>
+__device__ __forceinline__ int screen_kmer(const ScreenParams& S, int n, const uint32_t* d, int ku, bool valid) {
+  const int c = (-(int)d[0]) >> 7;
+  const float ey = screen_ey(S, d);
+  float ss = 0.0f, gs = 0.0f;
+#pragma unroll
+  for (int jj = 0; jj < KU_MAX; ++jj) {
+    if (jj >= KU_MAX - LAST && jj >= ku) break;
+    const int o = 6 + 3 * jj;
+    const float e = shifted_float(limb3(d[o], d[o + 1], d[o + 2]), S.shift) * S.su[jj];
+    ss = fmaf(e, e, ss);
+    if (GATE) gs = fmaf(S.g[jj], e, gs);
+  }
+  return screen_verdict<GATE, PAIRS>(S, n, c, ey, ss, gs, valid);
 }
 
 // Adds the per-thread tested counts of a warp to counters[0].
@@ -680,7 +687,7 @@ __device__ __forceinline__ void mp_eval(const EpiParams& P, bool valid, int c, d
     return;
   }
   const double q = xyM * xyM, den = xxM * P.yyM;
-  if (P.refine && q >= P.r2_ref * den) {
+  if (P.refine && may_refine(P, (double)c, xxM, q, den)) {
     cand = true;
   } else if (q >= P.r2_cand * den) {
     double r2 = q / den;
@@ -691,6 +698,119 @@ __device__ __forceinline__ void mp_eval(const EpiParams& P, bool valid, int c, d
     effect = xyM / den;
     hit = p <= P.p_thresh;
   }
+}
+
+__device__ __forceinline__ void mp_emit_rare(const DevOutMP& O, int p, unsigned long long gk, int shard, bool hit,
+                                             bool cand, double T, double pv, double effect);
+
+// Accumulator columns of one phenotype slot, 48 at a time: column 0 is the
+// count, 1-5 the y' limbs, then 3 limbs per U column, so that a chunk never
+// splits a limb group.
+constexpr int MP_CH = 48;
+template <int NP, int CHUNK>
+__device__ __forceinline__ void mp_load_chunk(uint32_t taddr, uint32_t (&d)[MP_CH]) {
+#pragma unroll
+  for (int c16 = 0; c16 < MP_CH / 16; ++c16)
+    if (CHUNK * MP_CH + c16 * 16 < NP) tc_ld16p(taddr + CHUNK * MP_CH + c16 * 16, d + c16 * 16);
+  tc_wait_ld();
+#pragma unroll
+  for (int c16 = 0; c16 < MP_CH / 16; ++c16)
+    if (CHUNK * MP_CH + c16 * 16 < NP) reg_fence16(d + c16 * 16);
+}
+
+// screen_kmer for one phenotype slot of NP accumulator columns at tensor-memory
+// address taddr; the phenotype's constants come from global memory.  Slots
+// past its U columns hold zero limbs.
+template <int NP, int CHUNK, bool GATE>
+__device__ __forceinline__ void mp_screen_chunk(const ScreenParams& S, uint32_t taddr, int& c, float& ey, float& ss,
+                                                float& gs) {
+  uint32_t d[MP_CH];
+  mp_load_chunk<NP, CHUNK>(taddr, d);
+  if (CHUNK == 0) {
+    c = (-(int)d[0]) >> 7;
+    ey = screen_ey(S, d);
+  }
+  constexpr int J0 = CHUNK == 0 ? 0 : (CHUNK * MP_CH - 6) / 3;
+  constexpr int JN = (NP - 6) / 3, JE = (CHUNK * MP_CH + MP_CH - 6) / 3 < JN ? (CHUNK * MP_CH + MP_CH - 6) / 3 : JN;
+#pragma unroll
+  for (int j = J0; j < JE; ++j) {
+    const int o = 6 + 3 * j - CHUNK * MP_CH;
+    const float e = shifted_float(limb3(d[o], d[o + 1], d[o + 2]), S.shift) * __ldg(S.su + j);
+    ss = fmaf(e, e, ss);
+    if (GATE) gs = fmaf(__ldg(S.g + j), e, gs);
+  }
+}
+template <int NP, bool GATE>
+__device__ __forceinline__ int mp_screen_t(const ScreenParams& S, int n, uint32_t taddr, bool valid) {
+  int c = 0;
+  float ey = 0.0f, ss = 0.0f, gs = 0.0f;
+  mp_screen_chunk<NP, 0, GATE>(S, taddr, c, ey, ss, gs);
+  if (NP > MP_CH) mp_screen_chunk<NP, 1, GATE>(S, taddr, c, ey, ss, gs);
+  if (NP > 2 * MP_CH) mp_screen_chunk<NP, 2, GATE>(S, taddr, c, ey, ss, gs);
+  return screen_verdict<GATE, false>(S, n, c, ey, ss, gs, valid);
+}
+// Returns 2 where the phenotype has no screen.
+template <int NP>
+__device__ __forceinline__ int mp_screen(const EpiParams& P, uint32_t taddr, bool valid) {
+  if (!P.S.on) return 2;
+  return P.S.gate ? mp_screen_t<NP, true>(P.S, P.n, taddr, valid) : mp_screen_t<NP, false>(P.S, P.n, taddr, valid);
+}
+
+// The exact limb recombination and FP64 sums of one phenotype slot.
+template <int NP, int CHUNK>
+__device__ __forceinline__ void mp_exact_chunk(const MPheno* ME, uint32_t taddr, int& c, double& cd, double& ey,
+                                               double& ss, double& gs) {
+  const EpiParams& P = ME->P;
+  const int drop0 = ME->drop0;
+  uint32_t d[MP_CH];
+  mp_load_chunk<NP, CHUNK>(taddr, d);
+  if (CHUNK == 0) {
+    // limb sums hold -128 * integer sums (see kernel_ts.cu)
+    c = (-(int)d[0]) >> 7;
+    cd = i2d_exact(c);
+    long long Vy = (long long)(int)d[5];
+#pragma unroll
+    for (int l = 1; l < 5; ++l) Vy += (long long)(int)d[5 - l] * (1ll << (8 * l));
+    const double sy = ME->LM.scale[P.k];
+    ey = fma(magic_raw((-Vy) >> 7), sy, -MAGIC_BIAS * sy);
+    if (drop0) {
+      const double s0 = P.a[0] * cd;
+      ss = s0 * s0;
+    }
+  }
+  constexpr int J0 = CHUNK == 0 ? 0 : (CHUNK * MP_CH - 6) / 3;
+  constexpr int JN = (NP - 6) / 3, JE = (CHUNK * MP_CH + MP_CH - 6) / 3 < JN ? (CHUNK * MP_CH + MP_CH - 6) / 3 : JN;
+  // slots past the phenotype's k columns have zero limbs and zero constants:
+  // they add exact zeros
+#pragma unroll
+  for (int jj = J0; jj < JE; ++jj) {
+    const int o = 6 + 3 * jj - CHUNK * MP_CH;
+    const int j = jj + drop0;
+    const double ej = i2d_exact(limb3(d[o], d[o + 1], d[o + 2])) * ME->LM.esc[j];
+    const double sj = fma(P.a[j], cd, ej);
+    ss = fma(sj, sj, ss);
+    gs = fma(P.g[j], ej, gs);
+  }
+}
+// Statistic of one (k-mer, phenotype) of a resident-image kernel: the screen,
+// and the FP64 statistic for warps with a k-mer that it leaves.  Returns
+// whether the k-mer counts as tested; emits rows and candidates.  Called by
+// all 32 lanes.
+template <int NP>
+__device__ __forceinline__ bool mp_test(const DevOutMP& O, const MPheno* ME, uint32_t taddr, int p,
+                                        unsigned long long gk, int shard, bool valid) {
+  const int v = mp_screen<NP>(ME->P, taddr, valid);
+  if (!__any_sync(0xffffffffu, v == 2)) return v != 0;
+  int c = 0;
+  double cd = 0, ey = 0, ss = 0, gs = 0;
+  mp_exact_chunk<NP, 0>(ME, taddr, c, cd, ey, ss, gs);
+  if (NP > MP_CH) mp_exact_chunk<NP, 1>(ME, taddr, c, cd, ey, ss, gs);
+  if (NP > 2 * MP_CH) mp_exact_chunk<NP, 2>(ME, taddr, c, cd, ey, ss, gs);
+  bool tested, hit, cand;
+  double T, pv, effect;
+  mp_eval(ME->P, valid, c, ss, gs, ey, tested, hit, cand, T, pv, effect);
+  if (__any_sync(0xffffffffu, hit || cand)) mp_emit_rare(O, p, gk, shard, hit, cand, T, pv, effect);
+  return tested;
 }
 
 // Warp-aggregated hit records and FP64 refinement candidates (k-mer |

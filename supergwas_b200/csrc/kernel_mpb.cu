@@ -16,7 +16,10 @@
 // that image traffic.
 //
 // Warps (15):
-//   0-7     epilogue, two groups of four taking tile-visits in turn;
+//   0-7     epilogue, two groups of four taking tile-visits in turn (mp_test:
+//           the single-precision screen, FP64 near a cut; 4e6 k-mers x 16
+//           phenotypes at n = 1000, r = 16+1: 2.61 ms, 4.37 ms with the FP64
+//           statistic of every test);
 //   8-11    unpack: packed rows -> int8 A operand in TMEM, 512-sample
 //           super-stages;
 //   XP      x producer: 2-D TMA loads of the packed rows (no multicast);
@@ -38,7 +41,6 @@ constexpr int MB_SUPER = 4;
 constexpr int MB_BOX = 1024;
 constexpr int MB_XST = 4;
 constexpr uint32_t MB_XBYTES = MB_TM * 128;
-constexpr int MB_LU = 3, MB_LY = 5;
 constexpr int MB_MAXSLOT = 3;
 constexpr int MB_WARP_UNPACK0 = 8;
 
@@ -46,10 +48,6 @@ constexpr int MB_WARP_UNPACK0 = 8;
 // (2560 at n = 2000, N = 80), which one group's unpack of the tile keeps up
 // with, and 15 warps leave 128 registers a thread for the epilogue.
 __host__ __device__ constexpr int mb_ug(int) { return 1; }
-// Epilogue chunks of accumulator columns: 48 = the count, 5 y' limbs and 14
-// U columns of 3 limbs, so a chunk never splits a limb group.
-constexpr int MB_CH = 48;
-#define MB_NCH(NP_) (((NP_) + MB_CH - 1) / MB_CH)
 __host__ __device__ constexpr int mb_threads(int N) { return 32 * (8 + 4 * mb_ug(N) + 3); }
 __host__ __device__ constexpr int mb_nslot(int N) {
   return (512 - 2 * N) / 128 > MB_MAXSLOT ? MB_MAXSLOT : (512 - 2 * N) / 128;
@@ -104,7 +102,6 @@ __global__ void __launch_bounds__(mb_threads(NP * PPG), 1)
   constexpr int A0 = 512 - NSLOT * 128;
   static_assert(NSLOT >= 2 && A0 >= 2 * N, "TMEM budget");
   constexpr uint32_t IDESC = idesc_i8(MB_TM, N);
-  constexpr int KU_MAX = (NP - 1 - MB_LY) / MB_LU;
   constexpr uint32_t BSTEP = (2 * N * 16) >> 4;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -118,7 +115,7 @@ __global__ void __launch_bounds__(mb_threads(NP * PPG), 1)
   const uint32_t b_full = acc_empty + 16, b_free = b_full + 8, drain = b_free + 8;
   uint32_t* s_tmem = reinterpret_cast<uint32_t*>(gbase + L.tmem);
   volatile int* s_abort = reinterpret_cast<volatile int*>(gbase + L.abort);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int nsp = (nsub + MB_SUPER - 1) / MB_SUPER;
   const unsigned long long ntiles = (m + MB_TM - 1) / MB_TM;
   // tile-iterations of this CTA: tiles blockIdx.x + i * gridDim.x
@@ -152,7 +149,7 @@ __global__ void __launch_bounds__(mb_threads(NP * PPG), 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *s_tmem;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *s_tmem, 0);
   const unsigned long long lim = wait_limit(O.wait_ns);
 
   if (warp == WXP) {
@@ -372,78 +369,14 @@ __global__ void __launch_bounds__(mb_threads(NP * PPG), 1)
 #pragma unroll
           for (int pp = 0; pp < PPG; ++pp) {
             const int p = g * PPG + pp;
-            const bool live = p < O.n_pheno;  // warp-uniform
-            const MPheno* ME = ph + (live ? p : 0);
-            const EpiParams& P = ME->P;
-            int c = 0;
-            double cd = 0, ey = 0, ss = 0, gs = 0;
-            int drop0 = 0;
-            // The phenotype's NP accumulator columns, 48 at a time: column 0
-            // is the count, 1-5 the y' limbs, then 3 limbs per U column, so
-            // every 48-column chunk holds whole limb groups.  The buffer is
-            // released after the group's last load.
-#pragma unroll
-            for (int ch = 0; ch < MB_NCH(NP); ++ch) {
-              constexpr int CH = MB_CH;
-              const int width = NP - ch * CH < CH ? NP - ch * CH : CH;
-              uint32_t d[CH];
-              if (live) {
-#pragma unroll
-                for (int c16 = 0; c16 < CH / 16; ++c16) {
-                  if (c16 * 16 < width) {
-                    uint32_t rr[16];
-                    tc_ld16(tmem + lane_base + e * N + pp * NP + ch * CH + c16 * 16, rr);
-                    tc_wait_ld();
-#pragma unroll
-                    for (int k = 0; k < 16; ++k) d[c16 * 16 + k] = rr[k];
-                  }
-                }
-              }
-              if (pp == PPG - 1 && ch == MB_NCH(NP) - 1) {
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(acc_empty + 8 * e);
-              }
-              if (!live) continue;
-              if (ch == 0) {
-                // limb sums hold -128 * integer sums (see kernel_ts.cu)
-                c = (-(int)d[0]) >> 7;
-                cd = i2d_exact(c);
-                long long Vy = (long long)(int)d[MB_LY];
-#pragma unroll
-                for (int l = 1; l < MB_LY; ++l) Vy += (long long)(int)d[MB_LY - l] * (1ll << (8 * l));
-                const double sy = ME->LM.scale[P.k];
-                ey = fma(magic_raw((-Vy) >> 7), sy, -MAGIC_BIAS * sy);
-                drop0 = ME->drop0;
-                if (drop0) {
-                  const double s0 = P.a[0] * cd;
-                  ss = s0 * s0;
-                }
-              }
-              // slots past the phenotype's k columns have zero limbs and zero
-              // constants: they add exact zeros
-#pragma unroll
-              for (int jj = 0; jj < KU_MAX; ++jj) {
-                const int o = 1 + MB_LY + MB_LU * jj;  // first limb column of slot jj
-                if (o / CH != ch) continue;
-                const int od = o - ch * CH;
-                const int j = jj + drop0;
-                long long Vb = (long long)(int)d[od + MB_LU - 1] + (long long)0x4338000000000000LL;
-#pragma unroll
-                for (int l = 1; l < MB_LU; ++l) Vb += (long long)(int)d[od + MB_LU - 1 - l] * (1ll << (8 * l));
-                const double ej = fma(__longlong_as_double(Vb), ME->LM.esc[j], ME->LM.eoff[j]);
-                const double sj = fma(P.a[j], cd, ej);
-                ss = fma(sj, sj, ss);
-                gs = fma(P.g[j], ej, gs);
-              }
-            }
-            if (!live) continue;
-            bool tested, hit, cand;
-            double T, pv, effect;
-            mp_eval(P, valid, c, ss, gs, ey, tested, hit, cand, T, pv, effect);
-            cnt[pp] += tested ? wt : 0u;
-            if (__any_sync(0xffffffffu, hit || cand)) mp_emit_rare(O, p, gk, shard, hit, cand, T, pv, effect);
+            if (p < O.n_pheno &&  // warp-uniform
+                mp_test<NP>(O, ph + p, tmem + lane_base + e * N + pp * NP, p, gk, shard, valid))
+              cnt[pp] += wt;
           }
+          // the accumulator is released after its last load
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acc_empty + 8 * e);
         }
         mb_flush<PPG>(O, g, cur, cnt);
       }

@@ -21,7 +21,11 @@
 //
 // Roles (15 warps per CTA, both CTAs):
 //   0-7   epilogue, two groups of four taking pair-tile visits in turn: the
-//         accumulators of both phenotypes for this CTA's 128 k-mers;
+//         accumulators of both phenotypes for this CTA's 128 k-mers (mp_test:
+//         the single-precision screen, FP64 for warps with a k-mer near a
+//         cut).  2e6 k-mers x 16 phenotypes at n = 2000, r = 20+1: 2.61 ms,
+//         89 % of the nominal int8 rate; 3.74 ms with the FP64 statistic of
+//         every test, whose instructions wait for the MMAs' pipe;
 //   8-11  unpack: packed rows -> int8 A operand in this CTA's tensor memory,
 //         256-sample stages (64 columns);
 //   XP    row producer: 2-D TMA loads of this CTA's 128 rows (no multicast);
@@ -49,10 +53,7 @@ constexpr int M2_SUPER = 2;                   // sub-stages per stage (64 column
 constexpr int M2_BOX = 1024;                  // samples per TMA box (128 bytes)
 constexpr int M2_XST = 4;                     // row boxes in flight per CTA
 constexpr uint32_t M2_XBYTES = M2_TM * 128;
-constexpr int M2_LU = 3, M2_LY = 5;
 constexpr int M2_MAXSLOT = 4;
-constexpr int M2_CH = 48;                     // epilogue chunk (whole limb groups)
-#define M2_NCH(NP_) (((NP_) + M2_CH - 1) / M2_CH)
 constexpr int M2_THREADS = 32 * (8 + 4 + 3);
 constexpr int M2_WXP = 12, M2_WBP = 13, M2_WMMA = 14;
 
@@ -168,7 +169,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(M2_THREADS, 1)
   constexpr int A0 = 512 - NSLOT * 64;
   static_assert(NSLOT >= 2 && A0 >= 2 * N, "TMEM budget");
   constexpr uint32_t IDESC = idesc_i8(2 * M2_TM, N);
-  constexpr int KU_MAX = (NP - 1 - M2_LY) / M2_LU;
   constexpr uint32_t BSTEP = (2 * NP * 16) >> 4;  // one K = 32 step of this CTA's NP-column half
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -185,7 +185,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(M2_THREADS, 1)
   const uint32_t rank = cta_rank_in_cluster();
   const bool lead = rank == 0;
   const uint32_t peer_abort = peer_addr(base + L.abort, rank ^ 1u);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int nsp = (nsub + M2_SUPER - 1) / M2_SUPER;
   const unsigned long long lim = wait_limit(O.wait_ns);
   // pair-tiles of 256 k-mers; this pair visits pt = pair, pair + npairs, ...
@@ -222,7 +222,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(M2_THREADS, 1)
   __syncthreads();
   cluster_sync_all();  // barriers, flags and tensor memory of both CTAs are in place
   tc_fence_after();
-  const uint32_t tmem = *s_tmem;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *s_tmem, 0);
 
   if (warp == M2_WXP) {
     // ------------------------------------------------------- row producer
@@ -444,74 +444,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(M2_THREADS, 1)
 #pragma unroll
           for (int pp = 0; pp < 2; ++pp) {
             const int p = 2 * g + pp;
-            const bool live = p < O.n_pheno;  // warp-uniform
-            const MPheno* ME = ph + (live ? p : 0);
-            const EpiParams& P = ME->P;
-            int c = 0;
-            double cd = 0, ey = 0, ss = 0, gs = 0;
-            int drop0 = 0;
-            // the phenotype's NP accumulator columns, 48 at a time (column 0
-            // the count, 1-5 the y' limbs, then 3 limbs per U column: every
-            // chunk holds whole limb groups); the accumulator is released
-            // after the last load
-#pragma unroll
-            for (int ch = 0; ch < M2_NCH(NP); ++ch) {
-              constexpr int CH = M2_CH;
-              const int width = NP - ch * CH < CH ? NP - ch * CH : CH;
-              uint32_t d[CH];
-#pragma unroll
-              for (int c16 = 0; c16 < CH / 16; ++c16) {
-                if (c16 * 16 < width) {
-                  uint32_t rr[16];
-                  tc_ld16(tmem + lane_base + e * N + pp * NP + ch * CH + c16 * 16, rr);
-                  tc_wait_ld();
-#pragma unroll
-                  for (int k = 0; k < 16; ++k) d[c16 * 16 + k] = rr[k];
-                }
-              }
-              if (pp == 1 && ch == M2_NCH(NP) - 1) {
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(lead_acc_empty + 8 * e);
-              }
-              if (!live) continue;
-              if (ch == 0) {
-                // limb sums hold -128 * integer sums (see kernel_ts.cu)
-                c = (-(int)d[0]) >> 7;
-                cd = i2d_exact(c);
-                long long Vy = (long long)(int)d[M2_LY];
-#pragma unroll
-                for (int l = 1; l < M2_LY; ++l) Vy += (long long)(int)d[M2_LY - l] * (1ll << (8 * l));
-                const double sy = ME->LM.scale[P.k];
-                ey = fma(magic_raw((-Vy) >> 7), sy, -MAGIC_BIAS * sy);
-                drop0 = ME->drop0;
-                if (drop0) {
-                  const double s0 = P.a[0] * cd;
-                  ss = s0 * s0;
-                }
-              }
-#pragma unroll
-              for (int jj = 0; jj < KU_MAX; ++jj) {
-                const int o = 1 + M2_LY + M2_LU * jj;  // first limb column of slot jj
-                if (o / CH != ch) continue;
-                const int od = o - ch * CH;
-                const int j = jj + drop0;
-                long long Vb = (long long)(int)d[od + M2_LU - 1] + (long long)0x4338000000000000LL;
-#pragma unroll
-                for (int l = 1; l < M2_LU; ++l) Vb += (long long)(int)d[od + M2_LU - 1 - l] * (1ll << (8 * l));
-                const double ej = fma(__longlong_as_double(Vb), ME->LM.esc[j], ME->LM.eoff[j]);
-                const double sj = fma(P.a[j], cd, ej);
-                ss = fma(sj, sj, ss);
-                gs = fma(P.g[j], ej, gs);
-              }
-            }
-            if (!live) continue;
-            bool tested, hit, cand;
-            double T, pv, effect;
-            mp_eval(P, valid, c, ss, gs, ey, tested, hit, cand, T, pv, effect);
-            cnt[pp] += tested ? wt : 0u;
-            if (__any_sync(0xffffffffu, hit || cand)) mp_emit_rare(O, p, gk, shard, hit, cand, T, pv, effect);
+            if (p < O.n_pheno &&  // warp-uniform
+                mp_test<NP>(O, ph + p, tmem + lane_base + e * N + pp * NP, p, gk, shard, valid))
+              cnt[pp] += wt;
           }
+          // the accumulator is released after its last load
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(lead_acc_empty + 8 * e);
         }
         m2_flush(O, g, cur, cnt);
       }

@@ -11,7 +11,7 @@ namespace kg {
 // from the limb sums, with room for its own rounding, that a k-mer is not
 // tested, or is tested and cannot reach the emit or the refinement cut.
 // Everything about y is relative to ||y - mean(y)||.
-struct ScreenParams {
+struct alignas(16) ScreenParams {
   int on;            // 0: every k-mer takes the FP64 statistic
   int shift;         // limb sums are shifted right by this into 32 bits
   float inv_n;       // 1 / n
@@ -19,8 +19,10 @@ struct ScreenParams {
   float cut;         // 0.9 x the lowest r2 that matters x yyM / ynorm^2
   float gate_lo, gate_hi;  // (corr_thr -+ margin)^2
   float sy;          // y' limb sums -> e_y / ynorm
-  float su[KMAX];    // U limb sums -> e_j
-  float g[KMAX];     // g_j / ynorm
+  int gate;          // corr_thr > 0
+  int pad[2];
+  float su[KMAX];    // limb sums of U column j + 1 -> e_(j+1) (column 0: the intercept)
+  float g[KMAX];     // g_(j+1) / ynorm
 };
 
 // Per-phenotype constants of the epilogue (prep.hpp notation).
@@ -84,12 +86,13 @@ inline void set_screen(EpiParams& P, const LimbMap& L, bool drop0) {
   const double lo = P.corr_thr > eps ? P.corr_thr - eps : 0.0, hi = P.corr_thr + eps;
   S.gate_lo = (float)(lo * lo);
   S.gate_hi = (float)(hi * hi);
+  S.gate = P.corr_thr > 0.0;
   // accumulators hold -128 x the digit sums; y' drops its lowest limb
   const double unit = -(double)(1 << S.shift) / 128.0;
   S.sy = (float)(unit * 65536.0 * L.scale[P.k] / P.ynorm);
   for (int j = 1; j < P.k; ++j) {
-    S.su[j] = (float)(unit * L.scale[j]);
-    S.g[j] = (float)(P.g[j] / P.ynorm);
+    S.su[j - 1] = (float)(unit * L.scale[j]);
+    S.g[j - 1] = (float)(P.g[j] / P.ynorm);
   }
 }
 

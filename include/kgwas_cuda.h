@@ -211,7 +211,7 @@ typedef struct kg_tile_shape {
     int groups;   /* MMA groups                                              */
     int kpad;     /* samples per image (padded)                              */
     int bt;       /* kernel 1: tile-iterations per L2 block of the last launch */
-    int xs, nb;   /* kernel 2: resident row tiles, image ring stages         */
+    int xs, nb;   /* kernel 2: row tiles at a time, image ring stages        */
 } kg_tile_shape;
 int kg_multi_shape(const kg_ctx* ctx, kg_tile_shape* out);
 
@@ -255,8 +255,9 @@ int kg_pairs_run_host(kg_ctx* ctx, const uint64_t* xbits, uint64_t n_kmers, uint
 int kg_last_launch_count(const kg_ctx* ctx);
 
 /* Which association kernel the last launch used: "ts" (tensor cores, x
- * unpacked into tensor memory), "ss" (tensor cores, x unpacked into shared
- * memory; shapes the first does not cover) or "fp64" (CUDA cores). */
+ * unpacked into tensor memory), "tb" (the same with the limb image streamed,
+ * where it does not fit shared memory), "ss" (tensor cores, x unpacked into
+ * shared memory; other limb counts, unaligned rows) or "fp64". */
 const char* kg_last_kernel(const kg_ctx* ctx);
 
 /* Rows the last kg_run_host tested on the device when it used runs of equal

@@ -89,6 +89,7 @@ void kg_destroy(kg_ctx* ctx) {
   dfree(ctx->dT);
   dfree(ctx->dB);
   dfree(ctx->dBts);
+  dfree(ctx->dPh1);
   dfree(ctx->dCounters);
   dfree(ctx->dHits);
   dfree(ctx->dCand);
@@ -220,6 +221,16 @@ int kg_set_structure_ex(kg_ctx* ctx, const double* U, int n, int k, const double
     dfree(ctx->dBts);
     KG_CUDA(cudaMalloc((void**)&ctx->dBts, img.size()), "cudaMalloc(B)");
     KG_CUDA(cudaMemcpy(ctx->dBts, img.data(), img.size(), cudaMemcpyHostToDevice), "copy B");
+    dfree(ctx->dPh1);
+    if (ctx->opts.limbs_u == 3 && ctx->opts.limbs_y == 5 &&
+        !kg::ts_supported(ctx->limbs.N, 3, 5, ctx->limbs.Kpad, std::max(16, (n_row + 63) / 64))) {
+      kg::MPheno ph{};
+      ph.P = P;
+      ph.LM = LM;
+      ph.drop0 = p.drop0 && k > 0;
+      KG_CUDA(cudaMalloc((void**)&ctx->dPh1, sizeof(ph)), "cudaMalloc(phenotype)");
+      KG_CUDA(cudaMemcpy(ctx->dPh1, &ph, sizeof(ph), cudaMemcpyHostToDevice), "copy");
+    }
   }
   ctx->have_structure = true;
   return KG_OK;
@@ -497,9 +508,12 @@ int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64
     KG_CUDA(cudaMemsetAsync(ctx->dCounters + 3, 0, sizeof(unsigned long long), st), "memset");
     const char* force = std::getenv("KG_KERNEL");
     const bool want_ss = force && std::string(force) == "ss";
-    const bool ts_ok = kg::ts_supported(ctx->limbs.N, ctx->opts.limbs_u, ctx->opts.limbs_y, ctx->limbs.Kpad,
-                                        (int)wpk) &&
-                       ((uintptr_t)dx % 16) == 0 && m <= 0x7fffff00ull;  // 31-bit row coordinates
+    // 16-byte aligned rows with 31-bit row coordinates: the TMA kernels
+    const bool tma_ok = ((uintptr_t)dx % 16) == 0 && m <= 0x7fffff00ull;
+    const bool ts_ok = tma_ok && kg::ts_supported(ctx->limbs.N, ctx->opts.limbs_u, ctx->opts.limbs_y, ctx->limbs.Kpad,
+                                                  (int)wpk);
+    // an image that leaves shared memory no room for rows is streamed
+    const bool tb_ok = tma_ok && !ts_ok && ctx->dPh1 && kg::tb_supported(ctx->limbs.N, (int)wpk);
     if (force && std::string(force) == "ts" && !ts_ok)
       return ctx->fail(KG_ERR_UNSUPPORTED, "KG_KERNEL=ts: shape not supported by the TMEM-A kernel");
     if (ts_ok && !want_ss) {
@@ -507,6 +521,11 @@ int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64
                      &ctx->LM, &O, ctx->num_sms};
       e = kg::launch_ts(L, st);
       ctx->last_kernel = "ts";
+    } else if (tb_ok && !want_ss) {
+      kg::LaunchTb L{dx, m, (int)wpk, ctx->limbs.Kpad, ctx->limbs.N, 1, 1, ctx->dBts, ctx->dPh1, nullptr, &O,
+                     ctx->num_sms};
+      e = kg::launch_tb(L, st);
+      ctx->last_kernel = "tb";
     } else {
       kg::LaunchTc L{dx, m, (int)wpk, ctx->nchunk, ctx->dB, &ctx->P, &ctx->LM, &O, ctx->num_sms};
       e = kg::launch_tc(L, st);

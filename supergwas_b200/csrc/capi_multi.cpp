@@ -40,17 +40,6 @@ void drop_graph(Multi& M) {
   M.g_seen = 0;
 }
 
-// Resident x tiles and B ring stages that fit the shared memory.
-void pick_shape(Multi& M, int nbox, int xs_pref, int nb_pref) {
-  const size_t budget = 220 * 1024;
-  const int N = M.PPG * M.NP;
-  int xs = xs_pref, nb = nb_pref;
-  while (xs > 1 && kg::mp_smem_bytes(nbox, xs, 2, N) > budget) --xs;
-  while (nb > 2 && kg::mp_smem_bytes(nbox, xs, nb, N) > budget) --nb;
-  M.xs = xs;
-  M.nb = nb;
-}
-
 int ensure_multi_out(kg_ctx* ctx, int n_shards, unsigned long long hit_cap) {
   Multi& M = ctx->mp;
   const size_t need = (size_t)n_shards * M.np;
@@ -140,8 +129,10 @@ int enqueue_multi(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uns
     kg::LaunchMpb L{dx, m, (int)wpk, M.kpad, M.NP, M.PPG, M.G, (int)bt, M.dB, M.dPh, &O, ctx->num_sms};
     e = M.kern == 2 ? kg::launch_mpb2(L, st) : kg::launch_mpb(L, st);
   } else {
-    kg::LaunchMp L{dx, m, (int)wpk, M.kpad, M.NP, M.PPG, M.G, M.xs, M.nb, 0, 0, M.dB, M.dPh, &O, ctx->num_sms};
-    e = kg::launch_mp(L, st);
+    M.xs = kg::tb_tiles(m, ctx->num_sms);
+    M.nb = kg::tb_ring(M.NP * M.PPG);
+    kg::LaunchTb L{dx, m, (int)wpk, M.kpad, M.NP, M.PPG, M.G, M.dB, M.dPh, &O, nullptr, ctx->num_sms};
+    e = kg::launch_tb(L, st);
   }
   if (e != cudaSuccess) return ctx->cuda_fail(e, "multi-phenotype kernel launch");
   kg::LaunchMpRefine R{dx, (int)wpk, M.dV, M.nsteps * 128, M.cm, M.vstride, M.dPh, &O, ctx->num_sms, M.dT};
@@ -165,37 +156,29 @@ int reset_outputs(kg_ctx* ctx, cudaStream_t st) {
 //   per MMA) and, where one phenotype fills an MMA group, the SM-pair kernel
 //   (mpb2, two phenotypes per M = 256 MMA), each with L2 blocks of 0.5x, 1x
 //   and 2x the 48 MB rule;
-//   image streamed from L2 (mp): resident x tiles x B ring stages.
+//   an image that does not fit is streamed (kernel_tb.cu): nothing to choose.
 // KG_MP_KERNEL=mp|mpb|mpb2 restricts the search to one kernel.
 int autotune(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, cudaStream_t st) {
   Multi& M = ctx->mp;
   const int nbox = ((int)wpk * 8 + 127) / 128;
   if (M.tuned && M.tuned_nbox == nbox) return KG_OK;
   struct Cand {
-    int kern, xs, nb, bt_scale;
+    int kern, bt_scale;
   };
   std::vector<Cand> cands;
   const char* only = std::getenv("KG_MP_KERNEL");
   auto allowed = [&](const char* k) { return !only || std::string(only) == k; };
   if (M.stationary && !(only && std::string(only) == "mp")) {
     for (int s : {2, 1, 4}) {
-      if (allowed("mpb")) cands.push_back({1, 1, 4, s});
-      if (M.pair_ok && allowed("mpb2")) cands.push_back({2, 1, 4, s});
+      if (allowed("mpb")) cands.push_back({1, s});
+      if (M.pair_ok && allowed("mpb2")) cands.push_back({2, s});
     }
-    if (cands.empty()) cands.push_back({1, 1, 4, 2});  // the requested kernel does not fit these phenotypes
+    if (cands.empty()) cands.push_back({1, 2});  // the requested kernel does not fit these phenotypes
   }
-  if (cands.empty()) {
-    if (const char* v = std::getenv("KG_MP_SHAPE")) {  // "xs,nb": fixed shape, no tuning
-      int xs = 1, nb = 4;
-      if (std::sscanf(v, "%d,%d", &xs, &nb) == 2) cands.push_back({0, std::max(1, std::min(2, xs)), std::max(2, std::min(8, nb)), 2});
-    }
-    if (cands.empty())
-      for (const Cand& c : {Cand{0, 1, 4, 2}, Cand{0, 1, 8, 2}, Cand{0, 2, 4, 2}, Cand{0, 2, 8, 2}}) cands.push_back(c);
-  }
+  if (cands.empty()) cands.push_back({0, 2});
   if (cands.size() == 1) {
     M.kern = cands[0].kern;
     M.bt_scale = cands[0].bt_scale;
-    pick_shape(M, nbox, cands[0].xs, cands[0].nb);
     M.tuned = true;
     M.tuned_nbox = nbox;
     return KG_OK;
@@ -209,8 +192,6 @@ int autotune(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, cudaStre
   for (const Cand& c : cands) {
     M.kern = c.kern;
     M.bt_scale = c.bt_scale;
-    pick_shape(M, nbox, c.xs, c.nb);
-    if (c.kern == 0 && (M.xs != c.xs || M.nb != c.nb)) continue;  // does not fit
     int rc = reset_outputs(ctx, st);
     if (rc) return rc;
     if ((rc = enqueue_multi(ctx, dx, sample, wpk, 0, st))) return rc;  // warm
@@ -229,7 +210,6 @@ int autotune(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, cudaStre
   cudaEventDestroy(b);
   M.kern = win.kern;
   M.bt_scale = win.bt_scale;
-  pick_shape(M, nbox, win.xs, win.nb);
   M.tuned = true;
   M.tuned_nbox = nbox;
   return KG_OK;

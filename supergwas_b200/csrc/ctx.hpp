@@ -68,7 +68,7 @@ struct Multi {
   int PPG = 1;          // phenotypes per group (one MMA of NP * PPG columns)
   bool stationary = false;  // the group image fits in shared memory: kernel_mpb.cu
   bool pair_ok = false;     // kernel_mpb2.cu can run these phenotypes (PPG = 1 images)
-  int kern = 0;             // chosen kernel: 0 image streamed (mp), 1 image resident (mpb), 2 SM pair (mpb2)
+  int kern = 0;             // chosen kernel: 0 image streamed (tb), 1 image resident (mpb), 2 SM pair (mpb2)
   int bt_scale = 2;         // tile-iterations per L2 block: the 48 MB rule times bt_scale / 2
   int8_t* dB = nullptr;
   kg::MPheno* dPh = nullptr;
@@ -87,7 +87,7 @@ struct Multi {
   std::vector<kg_phit> hits;
   std::vector<uint64_t> tested;
   unsigned long long counters[4] = {0, 0, 0, 0};
-  // launch shape chosen by the autotuner: x tiles resident, B ring stages
+  // shape of the last streamed-image launch: tiles per item, image chunks in the ring
   int xs = 1, nb = 4;
   int bt = 0;  // B-stationary kernel: tile-iterations per L2 block of the last launch
   bool tuned = false;
@@ -124,7 +124,8 @@ struct kg_ctx {
   double* dT = nullptr;      // byte tables of V for the split form's FP64 refinement
   int cm = 0, nsteps = 0;
   int8_t* dB = nullptr;      // B image of the smem-A kernel
-  int8_t* dBts = nullptr;    // B image of the TMEM-A kernel
+  int8_t* dBts = nullptr;    // B image of the TMEM-A kernels
+  kg::MPheno* dPh1 = nullptr;  // the phenotype's constants for the streamed-image kernel
   int nchunk = 0;
   // outputs on the device
   unsigned long long* dCounters = nullptr;

@@ -75,21 +75,25 @@ cudaError_t launch_ts(const LaunchTs& L, cudaStream_t st);
   X(16, 1) X(16, 2) X(16, 4) X(16, 8) X(32, 1) X(32, 2) X(32, 4) X(48, 1) X(48, 2) X(64, 1) \
   X(64, 2) X(80, 1) X(96, 1) X(112, 1) X(128, 1)
 
-struct LaunchMp {
+// Streamed image (kernel_tb.cu): tiles in pairs against a limb image that does
+// not fit shared memory, one phenotype (O1) or many (O).
+struct LaunchTb {
   const uint64_t* x;          // packed rows (device), 16-byte aligned
   unsigned long long m;
   int wpk;
-  int kpad;                   // samples per phenotype group image (multiple of 128)
-  int NP;                     // columns per phenotype slot (multiple of 16, <= 128)
-  int PPG;                    // phenotypes per group (KG_MP_GROUPS)
-  int G;                      // phenotype groups
-  int xs, nb;                 // resident x tiles (1-2), B ring stages (2-8)
-  int splits, nacc;           // split-K accumulators, accumulator buffers (0: default)
-  const int8_t* Bimg;         // G x (kpad/128) chunks of 128 x N bytes (device)
+  int kpad;                   // samples per group image (multiple of 128)
+  int NP, PPG, G;             // columns per phenotype slot, phenotypes per group (KG_MP_GROUPS), groups
+  const int8_t* Bimg;         // G images of kpad x NP*PPG bytes in the make_b_image_ts layout (device)
   const MPheno* ph;           // per-phenotype constants (device)
   const DevOutMP* O;
+  const DevOut* O1;           // one phenotype: its outputs (O unused)
   int num_sms;
 };
+bool tb_supported(int N, int wpk);
+int tb_tiles(unsigned long long m, int num_sms);  // tiles per item of a launch
+int tb_ring(int N);                               // image chunks in the ring
+cudaError_t launch_tb(const LaunchTb& L, cudaStream_t st);
+
 struct LaunchMpRefine {
   const uint64_t* x;
   int wpk;
@@ -101,9 +105,7 @@ struct LaunchMpRefine {
   int num_sms;
   const double* T = nullptr;  // byte tables of V, refine_table_len(vrows, cm) doubles per phenotype
 };
-bool mp_supported(int NP, int PPG, int wpk);
-size_t mp_smem_bytes(int nbox, int xs, int nb, int N);
-cudaError_t launch_mp(const LaunchMp& L, cudaStream_t st);
+bool mp_supported(int NP, int PPG, int wpk);  // shapes of the many-phenotype kernels
 // 2-D TMA map of packed rows: boxes of 128 bytes x `rows` rows, 128-byte swizzle.
 bool mp_tmap(const uint64_t* x, unsigned long long m, int wpk, CUtensorMap_st* tm, int rows = 128);
 

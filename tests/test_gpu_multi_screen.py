@@ -1,6 +1,6 @@
-"""The many-phenotype kernels with a resident image decide most (k-mer,
-phenotype) tests in single precision; counts and rows must equal the streamed
-kernel's, which evaluates the FP64 statistic for every one."""
+"""The many-phenotype kernels decide most (k-mer, phenotype) tests in single
+precision; counts and rows must equal those of the single-phenotype smem-A
+kernel, which evaluates the FP64 statistic for every k-mer."""
 import numpy as np
 import pytest
 
@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("thr,lt", [(0.0, 6.0), (0.2, 1.0), (0.2, 6.0), (0.0, 3.0)])
 @pytest.mark.parametrize("n,ks", [(300, (1, 3)), (300, (7, 2)), (900, (12, 15)), (1500, (22, 3)), (1200, (33, 41)),
                                   (700, (28, 30))], ids=lambda v: str(v))
-def test_screened_tests_equal_streamed_kernel(built, n, ks, thr, lt, monkeypatch):
+def test_screened_tests_equal_smem_kernel(built, n, ks, thr, lt, monkeypatch):
     rng = np.random.default_rng(n + ks[0])
     pop = np.arange(n) * 4 // n
     y0 = rng.standard_normal(n) + 0.5 * pop
@@ -34,7 +34,20 @@ def test_screened_tests_equal_streamed_kernel(built, n, ks, thr, lt, monkeypatch
         with api.Kgwas(corr_threshold=thr, log10_thresh=lt) as g:
             g.set_phenotypes(phenos, n)
             out[kern] = g.run_multi_host(X, shards)
-    assert out["mp"][1].shape[0] > 0
-    for kern in ("mpb", "mpb2"):
-        assert np.array_equal(out[kern][0], out["mp"][0]), kern
-        assert np.array_equal(out[kern][1], out["mp"][1]), kern
+    monkeypatch.setenv("KG_KERNEL", "ss")
+    bounds = list(shards.astype(int)) + [X.shape[0]]
+    total = 0
+    for p, (U, y, keep) in enumerate(phenos):
+        with api.Kgwas(corr_threshold=thr, log10_thresh=lt) as g:
+            g.set_structure(U, y, keep, n)
+            for s in range(3):
+                ref = g.run_host(X[bounds[s]:bounds[s + 1]])
+                total += ref.hits.shape[0]
+                for kern, (tested, hits) in out.items():
+                    assert tested[s, p] == ref.n_tested, (kern, p, s)
+                    h = hits[(hits["pheno"] == p) & (hits["shard"] == s)]
+                    assert np.array_equal(h["kmer"], ref.hits["kmer"] + np.uint64(bounds[s])), (kern, p, s)
+                    for f in ("effect", "pval", "chisq"):
+                        assert np.array_equal(h[f], ref.hits[f]), (kern, p, s, f)
+            assert g.last_kernel() == "ss"
+    assert total > 0

@@ -10,7 +10,7 @@ A step = one pass of the association test over the whole batch: pre-filter,
 U^T x and x.y' contraction, chi-square and p, hit compaction, count.
 ``value`` times the split-precision tensor-core kernel with the batch resident
 in HBM; ``e2e`` times kg_run_host from pinned host memory (host-to-device
-copies inside the timed region); ``fp64_form`` is the plain FP64 CUDA-core
+copies inside the timed region); ``fp64_form`` is the FP64
 kernel on the same batch.  The batch (25.6 GB) is far larger than L2 (126 MB),
 so no L2 flush is needed between steps.
 
@@ -293,7 +293,7 @@ def run_ours(args):
     clocks = ck.summary()
     t_split = sum(per) / 1e3
 
-    # plain FP64 form on the same batch
+    # FP64 form on the same batch
     f = api.Kgwas(device=local, precision="fp64", corr_threshold=0.0, log10_thresh=6.0)
     f.set_structure(U, y, keep, n)
     fsteps = max(1, min(args.steps, 3))
@@ -329,7 +329,7 @@ def run_ours(args):
     # measured peaks of the FP64 form and of the host link
     fp64_peak = api.probe_fp64_tflops(local)
     h2d_peak = api.probe_h2d_gbs(local, 1 << 30, 8)
-    # plain FP64 form at n=1000, m=5e7, r=10+1
+    # FP64 form at n=1000, m=5e7, r=10+1
     leg_fp64 = None if args.no_legs else fp64_config2_leg(X, local, rank, 3, 3, fp64_peak)
     acc = accuracy_report(X, min(m, args.acc_kmers), wpk, U, y, keep, n) if rank == 0 else None
     # batched 64 phenotypes (n=2000, m=1e8, r=20+1) on a batch of its own
@@ -386,8 +386,9 @@ def run_ours(args):
                                     "useful_columns": "54 of N=64 (count, 5 y' limbs, 16 x 3 U limbs)"}},
             "fp64_form": {"value": ftested / t_fp64, "unit": "k-mer tests/s", "ms_per_step": 1e3 * t_fp64,
                           "split_speedup": value / world / (ftested / t_fp64),
-                          "fp64_tflops": 2.0 * m * (((n + 127) // 128) * 128) * 20 / t_fp64 / 1e12,
-                          "fp64_frac": 2.0 * m * (((n + 127) // 128) * 128) * 20 / t_fp64 / 1e12 / fp64_peak},
+                          # the multiply-adds of a plain FP64 evaluation; the form runs in exact
+                          # int8 limbs on the tensor cores
+                          "equivalent_fp64_tflops": 2.0 * m * n * (r + 2) / t_fp64 / 1e12},
             "fp64_config2": leg_fp64,
             "files_cols": leg_files,
             "batched": leg_batched,
@@ -515,10 +516,11 @@ FP64_CFG2 = dict(n=1000, m=50_000_000, r=10, n_causal=50, missing=0.05, seed=45)
 
 
 def fp64_config2_leg(X, local, rank, steps, warmup, fp64_peak):
-    """Plain FP64 form at n=1000, m=5e7, r=10+1 (50 causal k-mers): the first
+    """FP64 form at n=1000, m=5e7, r=10+1 (50 causal k-mers): the first
     5e7 rows of the device batch (same generator, 8 subpopulations) with a
-    structure of 10 PCs and its own phenotype.  HBM GB/s of the packed rows
-    and FP64 TFLOP/s against the measured DFMA peak."""
+    structure of 10 PCs and its own phenotype.  HBM GB/s of the packed rows,
+    and the rate of a plain FP64 evaluation's multiply-adds beside the measured
+    DFMA peak (the form runs in exact int8 limbs on the tensor cores)."""
     import torch
     from supergwas_b200 import api, synth_gpu
     C = FP64_CFG2
@@ -531,17 +533,14 @@ def fp64_config2_leg(X, local, rank, steps, warmup, fp64_peak):
         f.set_structure(U, y, keep, n)
         tested, per, launches = time_device(f, Xc, m, wpk, steps, warmup, st)
     t = sum(per) / steps / 1e3
-    cm = 16                       # FP64 columns [count, d_0..d_10, d_y] padded to the kernel's 16
-    kpad = ((n + 127) // 128) * 128
-    flops = 2.0 * m * kpad * cm   # one FMA per (sample, column) per k-mer, padding included
+    flops = 2.0 * m * n * (r + 2)  # one FMA per (sample, column) per k-mer
     alg_bytes = m * ((n + 7) // 8)
     return {"value": tested / t, "unit": "k-mer tests/s", "ms_per_step": 1e3 * t, "steps": steps,
             "warmup": warmup, "gpu_launches": launches,
             "config": {"workload": f"fp64 form: n={n} (5% unphenotyped), m={m}, r={r}+1, 1 phenotype "
                                    f"({C['n_causal']} causal), CORR_THRESHOLD=0"},
             "hbm_gbs": alg_bytes / t / 1e9,
-            "fp64": {"achieved_tflops": flops / t / 1e12, "peak_tflops": fp64_peak,
-                     "frac": (flops / t / 1e12 / fp64_peak) if fp64_peak else None,
+            "fp64": {"equivalent_tflops": flops / t / 1e12, "dfma_peak_tflops": fp64_peak,
                      "peak_source": "measured (kg_probe_fp64_tflops: DFMA chains on every SM)"}}
 
 
@@ -559,7 +558,7 @@ def run_streaming(args):
     device generator writes chunk c+1 and copies it into the other pinned
     buffer (device-to-host, the other direction of the link) while chunk c
     streams in.  --steps chunks are timed (the per-chunk rate is steady; the
-    line extrapolates the whole 1e9).  Also: the plain FP64 form on a
+    line extrapolates the whole 1e9).  Also: the FP64 form on a
     device-resident sample of every phenotype, the split form's accuracy
     against the FP64 oracle, and the reference kgwas on a slice."""
     import threading
@@ -639,7 +638,7 @@ def run_streaming(args):
         rel = np.abs(T1 - T0) / np.maximum(T0, 1e-300)
         acc.append({"pheno": p, "n": int(keep.size), "tested_identical": bool(same),
                     "mlog10p_abs_max": float(ml.max()), "chisq_rel_p99": float(np.percentile(rel, 99))})
-    # plain FP64 form, every phenotype, on a device-resident sample (the last chunk's rows)
+    # FP64 form, every phenotype, on a device-resident sample (the last chunk's rows)
     m64 = min(per, W["fp64_kmers"])
     dgen[:m64].copy_(hbuf[(nchunks - 1) % 2][:m64])
     st = torch.cuda.Stream()

@@ -45,7 +45,10 @@ extern "C" {
 #define KG_PREC_SPLIT_I8 0  /* tcgen05 kind::i8: x exact in int8, U/y' split
                                into signed int8 limbs, exact int32 TMEM
                                accumulation, FP64 epilogue (default)        */
-#define KG_PREC_FP64     1  /* plain FP64 on CUDA cores                      */
+#define KG_PREC_FP64     1  /* FP64: U to 54 and y' to 62 bits of each column's
+                               largest value in int8 limbs, exact sums rounded
+                               once, FP64 statistic; FP64 on CUDA cores for
+                               structures wider than 256 limb columns        */
 
 typedef struct kg_ctx kg_ctx;
 

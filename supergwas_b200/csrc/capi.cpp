@@ -19,6 +19,59 @@
 
 using namespace kgctx;
 
+namespace {
+
+// The FP64 form's operand for the tensor cores (ctx->dV holds the columns): the
+// limb image and the phenotype's constants.  Leaves f64_N at 0 where the
+// structure is too wide or the device lacks the kernels: the CUDA-core kernel
+// runs then.
+int set_f64_limbs(kg_ctx* ctx, int n_row) {
+  const kg::Prepared& p = ctx->prep;
+  const int n = p.n, k = p.k;
+  int major = 0, minor = 0;
+  cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, ctx->opts.device);
+  cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, ctx->opts.device);
+  std::vector<double> mx((size_t)k + 1, 0.0);
+  for (int j = 0; j <= k; ++j)
+    for (int i = 0; i < n; ++i) mx[j] = std::max(mx[j], std::fabs(p.d[(size_t)j * n + i]));
+  // the intercept's centred part is left out only where it is rounding noise of
+  // U itself: below 1e-14 it moves xxM by less than a rounding of the count
+  const bool drop0 = k > 0 && mx[0] <= 1e-14 * std::fabs(p.a[0]);
+  const int N = kg::f64_limb_cols(k, drop0);
+  const int wpk = ((n_row + 63) / 64 + 1) / 2 * 2;
+  if (major != 10 || minor != 0 || !kg::f64_limbs_supported(N, n_row, wpk)) return KG_OK;
+  kg::MPheno ph{};
+  ph.P = ctx->P;
+  ph.drop0 = drop0;
+  double up[kg::KMAX + 1] = {};
+  for (int j = drop0; j <= k; ++j) {
+    // half the largest magnitude of the limbs, as in make_limbs
+    const double lim = 127.0 * std::ldexp(1.0, 8 * (j == k ? 7 : 6) - 1);
+    int s = 0;
+    if (mx[j] > 0) {
+      std::frexp(lim / mx[j], &s);
+      --s;
+    }
+    if (s > 1000 || s < -1000) return KG_OK;
+    up[j] = std::ldexp(1.0, s);
+    ph.LM.scale[j] = std::ldexp(1.0, -s);
+  }
+  kg::set_limb_consts(ph.LM);
+  kg::set_screen64(ph.P, ph.LM, drop0);
+  const int kpad = ctx->nsteps * 128;
+  const size_t img = (size_t)kpad * N;
+  dfree(ctx->dBts);
+  KG_CUDA(cudaMalloc((void**)&ctx->dBts, img + sizeof(ph)), "cudaMalloc(B)");  // kpad * N: a multiple of 2048
+  kg::LaunchF64Image L{ctx->dV, kpad, ctx->cm, k, drop0, kpad, N, up, ctx->dBts};
+  KG_CUDA(kg::launch_f64_image(L, ctx->stream), "limb image");
+  KG_CUDA(cudaMemcpyAsync(ctx->dBts + img, &ph, sizeof(ph), cudaMemcpyHostToDevice, ctx->stream), "copy");
+  KG_CUDA(cudaStreamSynchronize(ctx->stream), "limb image");
+  ctx->f64_N = N;
+  return KG_OK;
+}
+
+}  // namespace
+
 extern "C" {
 
 const char* kg_version(void) { return KG_VERSION; }
@@ -182,6 +235,10 @@ int kg_set_structure_ex(kg_ctx* ctx, const double* U, int n, int k, const double
     dfree(ctx->dV);
     KG_CUDA(cudaMalloc((void**)&ctx->dV, V.size() * sizeof(double)), "cudaMalloc(V)");
     KG_CUDA(cudaMemcpy(ctx->dV, V.data(), V.size() * sizeof(double), cudaMemcpyHostToDevice), "copy V");
+  }
+  ctx->f64_N = 0;
+  if (ctx->opts.precision == KG_PREC_FP64) {
+    if (int rc = set_f64_limbs(ctx, n_row)) return rc;
   }
   if (ctx->opts.precision == KG_PREC_SPLIT_I8) {
     // byte tables of V for the FP64 refinement of high-chi-square k-mers
@@ -500,8 +557,18 @@ int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64
   }
   cudaError_t e;
   if (ctx->opts.precision == KG_PREC_FP64) {
-    kg::LaunchFp64 L{dx, m, (int)wpk, ctx->dV, ctx->nsteps, ctx->cm, &ctx->P, &O, ctx->num_sms};
-    e = kg::launch_fp64(L, st);
+    const char* force = std::getenv("KG_KERNEL");
+    if (ctx->f64_N && ((uintptr_t)dx % 16) == 0 && m <= 0x7fffff00ull &&
+        kg::f64_limbs_supported(ctx->f64_N, ctx->n_row, (int)wpk) && !(force && std::string(force) == "fp64cores")) {
+      const int kpad = ctx->nsteps * 128;
+      kg::LaunchTb L{dx, m, (int)wpk, kpad, ctx->f64_N, 1, 1, ctx->dBts,
+                     reinterpret_cast<const kg::MPheno*>(ctx->dBts + (size_t)kpad * ctx->f64_N), nullptr, &O,
+                     ctx->num_sms, true};
+      e = kg::launch_tb(L, st);
+    } else {
+      kg::LaunchFp64 L{dx, m, (int)wpk, ctx->dV, ctx->nsteps, ctx->cm, &ctx->P, &O, ctx->num_sms};
+      e = kg::launch_fp64(L, st);
+    }
     ctx->last_kernel = "fp64";
   } else {
     // refinement candidates of this launch start from zero

@@ -127,6 +127,7 @@ struct kg_ctx {
   int8_t* dBts = nullptr;    // B image of the TMEM-A kernels
   kg::MPheno* dPh1 = nullptr;  // the phenotype's constants for the streamed-image kernel
   int nchunk = 0;
+  int f64_N = 0;             // limb columns of the FP64 form (dBts holds image and constants); 0: CUDA cores
   // outputs on the device
   unsigned long long* dCounters = nullptr;
   kg_hit* dHits = nullptr;

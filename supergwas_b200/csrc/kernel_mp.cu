@@ -90,10 +90,12 @@ bool mp_tmap(const uint64_t* x, unsigned long long m, int wpk, CUtensorMap* tm, 
   const cuuint64_t rowbytes = (cuuint64_t)wpk * 8;
   cuuint64_t gdim[2] = {rowbytes, (cuuint64_t)m};
   cuuint64_t gstride[1] = {rowbytes};
-  cuuint32_t box[2] = {128, (cuuint32_t)rows};
+  // rows shorter than a 128-byte box: whole rows, not swizzled
+  const bool wide = rowbytes >= 128;
+  cuuint32_t box[2] = {wide ? 128u : (cuuint32_t)rowbytes, (cuuint32_t)rows};
   cuuint32_t estr[2] = {1, 1};
   return enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, (void*)x, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             wide ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 

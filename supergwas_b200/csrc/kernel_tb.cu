@@ -40,9 +40,10 @@ namespace kg {
 constexpr int TB_TM = 128;
 constexpr int TB_KS = 128;     // samples per sub-stage (4 MMAs)
 constexpr int TB_SUPER = 4;    // sub-stages per super-stage
-constexpr int TB_CHUNK = 2;    // sub-stages per image chunk
+// Sub-stages per image chunk: one for the widest images of the FP64 form, whose
+// ring of three chunks of two would not fit.
+__host__ __device__ constexpr int tb_chunk(int N) { return N > 192 ? 1 : 2; }
 constexpr int TB_UG = 2;       // unpack groups = A slots of 128 TMEM columns
-constexpr uint32_t TB_XBYTES = TB_TM * 128;
 constexpr int TB_XST_MAX = 6, TB_XST_MIN = 4, TB_NB_MAX = 8, TB_NB_MIN = 3;
 constexpr int TB_WUNP = 4, TB_WXP = TB_WUNP + 4 * TB_UG, TB_WBP = TB_WXP + 1, TB_WMMA = TB_WBP + 1;
 constexpr int TB_THREADS = 32 * (TB_WMMA + 2);
@@ -51,11 +52,11 @@ constexpr int TB_A0 = 512 - TB_UG * 128;
 struct TbSmem {
   uint32_t x, b, bars, tmem, abort, total;
 };
-__host__ __device__ inline TbSmem tb_smem(int N, int xst, int nb) {
+__host__ __device__ inline TbSmem tb_smem(int N, int xst, int nb, int rb) {
   TbSmem L;
   L.x = 0;
-  L.b = (uint32_t)xst * TB_XBYTES;
-  L.bars = L.b + (uint32_t)nb * TB_CHUNK * TB_KS * N;
+  L.b = (uint32_t)xst * TB_TM * rb;
+  L.bars = L.b + (uint32_t)nb * tb_chunk(N) * TB_KS * N;
   L.tmem = L.bars + 8 * (2 * TB_XST_MAX + 2 * TB_NB_MAX + 2 * TB_UG + 4 + 2);
   L.abort = L.tmem + 8;
   L.total = L.abort + 8;
@@ -92,23 +93,158 @@ __device__ __forceinline__ void tb_single(const DevOut& O, const MPheno* ME, uin
   else finish_kmer_lean(P, O, local, valid, c, cd, ss, gs, ey, tested_local);
 }
 
-// SINGLE: one phenotype (G = 1), results to O1; otherwise to O.
-template <int NP, int PPG, bool SINGLE>
+// ---------------------------------------------------- FP64 form in limbs
+// Columns: the count, 8 limbs of y', 7 of every U column with limbs (62 and 54
+// bits below the column's largest value, so at least what a double holds of
+// it).  The sums are exact and rounded once, where fp64_kernel rounds after
+// every sample: the error against 64 bits is that of fp64_kernel or below it
+// (8.2e-14 and 3.1e-13 in p-values at n = 1000 were the same on both).
+// fp64_kernel does n (k + 2) FP64 multiply-adds per k-mer, half of whose time
+// goes to broadcasting the columns from shared memory; here they are int8 MMAs
+// of 8 + 7 k columns.  5e6 k-mers, r = 10+1, n = 1000: 9.70 -> 0.37 ms; 3e5 at
+// n = 5000, r = 32+1: 6.79 -> 0.22 ms; 5e6 at n = 200, r = 5+1: 1.25 -> 0.16 ms.
+constexpr int F64_LY = 8, F64_LU = 7;
+
+__device__ __forceinline__ long long limb4(const uint32_t* d) {
+  return mad_wide<(1 << 24)>(d[0], limb3(d[1], d[2], d[3]));
+}
+
+// Reads the N accumulator columns at taddr, 32 at a time, and hands over the
+// count and y' (first(d)) and then the 7 limbs of each of the ku U columns
+// (column(j, d)) as they arrive.
+template <int N, class F, class G>
+__device__ __forceinline__ void f64_columns(uint32_t taddr, int ku, F first, G column) {
+  constexpr int KU = (N - 1 - F64_LY) / F64_LU;
+  uint32_t d[N];
+#pragma unroll
+  for (int q = 0; q < N; q += 32) {
+#pragma unroll
+    for (int c16 = q; c16 < q + 32 && c16 < N; c16 += 16) tc_ld16p(taddr + c16, d + c16);
+    tc_wait_ld();
+#pragma unroll
+    for (int c16 = q; c16 < q + 32 && c16 < N; c16 += 16) reg_fence16(d + c16);
+    if (q == 0) first(d);
+#pragma unroll
+    for (int j = 0; j < KU; ++j) {
+      const int o = 1 + F64_LY + F64_LU * j;
+      // N is rounded up to 16: at most two groups past the last column
+      if (o + F64_LU - 1 >= q && o + F64_LU - 1 < q + 32 && (j < KU - 2 || j < ku)) column(j, d + o);
+    }
+  }
+}
+
+template <int N, bool GATE>
+__device__ __forceinline__ int f64_screen(const EpiParams& P, uint32_t taddr, int ku, bool valid) {
+  const ScreenParams& S = P.S;
+  int c = 0;
+  float ey = 0.0f, ss = 0.0f, gs = 0.0f;
+  f64_columns<N>(
+      taddr, ku,
+      [&](const uint32_t* d) {
+        c = (-(int)d[0]) >> 7;
+        ey = shifted_float(limb4(d + 1), S.shift + 8) * S.sy;
+      },
+      [&](int j, const uint32_t* d) {
+        const float e = shifted_float(limb4(d), S.shift + 8) * __ldg(S.su + j);
+        ss = fmaf(e, e, ss);
+        if (GATE) gs = fmaf(__ldg(S.g + j), e, gs);
+      });
+  return screen_verdict<GATE, false>(S, P.n, c, ey, ss, gs, valid);
+}
+
+// One phenotype in the FP64 form: the sums of fp64_kernel (kernels.cu), each
+// rounded once, then its statistic.  Without per-k-mer outputs the screen
+// decides most k-mers first.
+template <int N>
+__device__ __forceinline__ void tb_single64(const DevOut& O, const MPheno* ME, uint32_t taddr,
+                                            unsigned long long local, bool valid, uint32_t& tested_local) {
+  const EpiParams& P = ME->P;
+  const int drop0 = ME->drop0, ku = P.k - drop0;
+  if (!O.tested && P.S.on) {
+    const int v = P.S.gate ? f64_screen<N, true>(P, taddr, ku, valid) : f64_screen<N, false>(P, taddr, ku, valid);
+    if (!__any_sync(0xffffffffu, v == 2)) {
+      if (v) tested_local += O.weight ? O.weight[O.kmer_offset + local] : 1u;
+      return;
+    }
+  }
+  int c = 0;
+  double cd = 0, ey = 0, ss = 0, gs = 0;
+  f64_columns<N>(
+      taddr, ku,
+      [&](const uint32_t* d) {
+        c = (-(int)d[0]) >> 7;
+        cd = i2d_exact(c);
+        const double sy = ME->LM.esc[P.k];
+        ey = fma(i2d_exact(limb4(d + 1)), sy * 4294967296.0, i2d_exact(limb4(d + 5)) * sy);
+        if (drop0) {
+          const double s0 = P.a[0] * cd;
+          ss = s0 * s0;
+        }
+      },
+      [&](int jj, const uint32_t* d) {
+        const int j = jj + drop0;
+        const double su = ME->LM.esc[j];
+        const double e = fma(i2d_exact(limb4(d)), su * 16777216.0, i2d_exact(limb3(d[4], d[5], d[6])) * su);
+        const double sj = fma(P.a[j], cd, e);
+        ss = fma(sj, sj, ss);
+        gs = fma(P.g[j], e, gs);
+      });
+  finish_kmer(P, O, local, valid, c, ss, gs, ey);
+}
+
+// The image of the FP64 form from the FP64 columns V (row = sample position:
+// count, d_0 .. d_{k-1}, d_y, cm apart), in the layout and with the digits
+// (of v, or of -2 v where a sample enters as 64 x) of put_b_image_ts.  One
+// thread per sample position and logical column (0: count, 1: y', 2 + j: U
+// column j + drop0).
+struct F64Scales {
+  double up[KMAX + 1];  // 2^s of U column j; [k]: y'
+};
+__global__ void __launch_bounds__(128) f64_image_kernel(const double* __restrict__ V, int vrows, int cm, int k,
+                                                        int drop0, int kpad, int N,
+                                                        const __grid_constant__ F64Scales S,
+                                                        int8_t* __restrict__ img) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, col = blockIdx.y;
+  if (i >= kpad) return;
+  const int a = i >> 7, q = (i >> 5) & 3, t = (i >> 3) & 3, jj = 7 - (i & 7);
+  const int kap = 128 * a + 4 * (8 * q + jj) + t;
+  const int j = col < 2 ? k : col - 2 + drop0;  // U column (k: y')
+  const int vc = col == 0 ? 0 : 1 + j;
+  const int L = col == 0 ? 1 : col == 1 ? F64_LY : F64_LU;
+  const int first = col == 0 ? 0 : col == 1 ? 1 : 1 + F64_LY + F64_LU * (col - 2);
+  long long v = 0;
+  if (i < vrows) v = __double2ll_rn(V[(size_t)i * cm + vc] * (col == 0 ? 1.0 : S.up[j]));
+  if (jj & 1) v *= -2;
+  for (int l = L - 1; l >= 0; --l) {
+    const int8_t digit = (int8_t)(v & 255);  // balanced: [-128, 127]
+    v = (v - digit) >> 8;
+    const int cc = first + l;
+    img[(size_t)(kap >> 4) * (N * 16) + (size_t)(cc >> 3) * 128 + (size_t)(cc & 7) * 16 + (kap & 15)] = digit;
+  }
+}
+
+// FORM: TB_MANY phenotypes to O; TB_ONE phenotype (G = 1) to O1; TB_ONE64 the
+// same in the FP64 form.
+enum { TB_MANY, TB_ONE, TB_ONE64 };
+template <int NP, int PPG, int FORM>
 __global__ void __launch_bounds__(TB_THREADS, 1)
     tb_kernel(const __grid_constant__ CUtensorMap tmap, unsigned long long m, int nbox, int nsub, int G, int T,
-              int xst, int nb, const int8_t* __restrict__ Bimg, unsigned long long img_bytes,
+              int xst, int nb, int rb, const int8_t* __restrict__ Bimg, unsigned long long img_bytes,
               const MPheno* __restrict__ ph, const DevOutMP O, const DevOut O1) {
   constexpr int N = NP * PPG;
-  static_assert(N <= 128 && N % 16 == 0, "group width");
+  static_assert(N <= (FORM == TB_ONE64 ? 256 : 128) && N % 16 == 0, "group width");  // T * N <= 256
+  constexpr bool SINGLE = FORM != TB_MANY;
   constexpr uint32_t IDESC = idesc_i8(TB_TM, N);
   constexpr uint32_t BSTEP = (2 * N * 16) >> 4;             // descriptor step of one K = 32 MMA
+  constexpr int TB_CHUNK = tb_chunk(N);
   constexpr uint32_t BCH = (uint32_t)TB_CHUNK * TB_KS * N;  // bytes of one image chunk
   constexpr int NK = TB_CHUNK * (TB_KS / 32);               // MMAs per chunk
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* gbase = smem_raw + (base - raw);
-  const TbSmem L = tb_smem(N, xst, nb);
+  const uint32_t xbytes = TB_TM * (uint32_t)rb, swz = rb == 128 ? 7u : 0u;  // boxes as in kernel_ts.cu
+  const TbSmem L = tb_smem(N, xst, nb, rb);
   const uint32_t sx = base + L.x, sb = base + L.b;
   const uint32_t x_full = base + L.bars, x_empty = x_full + 8 * TB_XST_MAX;
   const uint32_t b_full = x_empty + 8 * TB_XST_MAX, b_empty = b_full + 8 * TB_NB_MAX;
@@ -177,9 +313,9 @@ __global__ void __launch_bounds__(TB_THREADS, 1)
                 ok = false;
                 break;
               }
-              mbar_arrive_expect_tx(x_full + 8 * xr.slot, TB_XBYTES);
+              mbar_arrive_expect_tx(x_full + 8 * xr.slot, xbytes);
               // rows past the last k-mer (an odd tile's partner) read as zero
-              tma_load_2d(sx + xr.slot * TB_XBYTES, &tmap, bx * 128, (int)((tg * (uint32_t)T + t) * TB_TM),
+              tma_load_2d(sx + xr.slot * xbytes, &tmap, bx * 128, (int)((tg * (uint32_t)T + t) * TB_TM),
                           x_full + 8 * xr.slot);
               issued[xr.slot] = true;
               last_phase[xr.slot] = xr.phase;
@@ -302,8 +438,8 @@ __global__ void __launch_bounds__(TB_THREADS, 1)
     const int grp = (warp - TB_WUNP) >> 2;
     const int q = warp & 3;
     const int r = q * 32 + lane;
-    const uint32_t rx = r & 7;
-    const uint32_t row0 = sx + r * 128;
+    const uint32_t rx = r & swz;
+    const uint32_t row0 = sx + r * rb;
     const uint32_t a_t = tmem + ((uint32_t)(q * 32) << 16) + TB_A0 + grp * 128;
     uint32_t off[TB_SUPER];
 #pragma unroll
@@ -331,7 +467,7 @@ __global__ void __launch_bounds__(TB_THREADS, 1)
       }
       if (!__all_sync(0xffffffffu, wait_or_abort(x_full + 8 * xslot, xphase, s_abort, counters, ERR_TIMEOUT_FULL, lim)))
         break;
-      const uint32_t xrow = row0 + xslot * TB_XBYTES;
+      const uint32_t xrow = row0 + xslot * xbytes;
       const uint32_t half = (uint32_t)(sp & 1) << 6;
       auto slot_free = [&] {
         return !used || __all_sync(0xffffffffu, wait_or_abort(a_empty + 8 * grp, aphase ^ 1u, s_abort, counters,
@@ -402,7 +538,9 @@ __global__ void __launch_bounds__(TB_THREADS, 1)
           const unsigned long long local = (unsigned long long)(tg * (uint32_t)T + t) * TB_TM + r;
           const bool valid = local < m;
           const uint32_t acc = tmem + lane_base + t * N;
-          if (SINGLE) {
+          if constexpr (FORM == TB_ONE64) {
+            tb_single64<N>(O1, ph, acc, local, valid, tested_local);
+          } else if constexpr (FORM == TB_ONE) {
             tb_single<N>(O1, ph, acc, local, valid, tested_local);
           } else {
             const unsigned long long gk = O.kmer_offset + local;
@@ -431,12 +569,12 @@ __global__ void __launch_bounds__(TB_THREADS, 1)
 
 // Ring sizes: as many image chunks as fit beside TB_XST_MIN row boxes, then two
 // more boxes where they still fit.  False where even the smallest rings do not fit.
-static bool tb_rings(int N, int& xst, int& nb) {
+static bool tb_rings(int N, int rb, int& xst, int& nb) {
   int dev = 0, optin = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
     return false;
-  auto fits = [&](int x, int n) { return tb_smem(N, x, n).total + 1024 <= (uint32_t)optin; };
+  auto fits = [&](int x, int n) { return tb_smem(N, x, n, rb).total + 1024 <= (uint32_t)optin; };
   xst = TB_XST_MIN;
   nb = TB_NB_MAX;
   while (nb >= TB_NB_MIN && !fits(xst, nb)) --nb;
@@ -445,38 +583,61 @@ static bool tb_rings(int N, int& xst, int& nb) {
   return true;
 }
 
+static int tb_box_bytes(int wpk) { return wpk * 8 < 128 ? wpk * 8 : 128; }
+
 bool tb_supported(int N, int wpk) {
   int xst, nb;
-  return N >= 16 && N <= 128 && N % 16 == 0 && wpk * 8 >= 128 && tb_rings(N, xst, nb);
+  return N >= 16 && N <= 128 && N % 16 == 0 && wpk * 8 >= 128 && tb_rings(N, 128, xst, nb);
 }
 
 int tb_tiles(unsigned long long m, int num_sms) { return (m + TB_TM - 1) / TB_TM > (unsigned)num_sms ? 2 : 1; }
 
 int tb_ring(int N) {
   int xst, nb;
-  return tb_rings(N, xst, nb) ? nb : 0;
+  return tb_rings(N, 128, xst, nb) ? nb : 0;
 }
 
-template <int NP, int PPG, bool SINGLE>
+int f64_limb_cols(int k, bool drop0) {
+  const int used = 1 + F64_LY + F64_LU * (k - (drop0 ? 1 : 0));
+  return (used + 15) / 16 * 16;
+}
+
+bool f64_limbs_supported(int N, int n_row, int wpk) {
+  int xst, nb;
+  return N <= 256 && n_row <= 12288 && tb_rings(N, tb_box_bytes(wpk), xst, nb);
+}
+
+cudaError_t launch_f64_image(const LaunchF64Image& L, cudaStream_t st) {
+  F64Scales S{};
+  for (int j = 0; j <= L.k; ++j) S.up[j] = L.up[j];
+  cudaError_t e = cudaMemsetAsync(L.img, 0, (size_t)L.kpad * L.N, st);
+  if (e != cudaSuccess) return e;
+  const dim3 grid((unsigned)((L.kpad + 127) / 128), (unsigned)(2 + L.k - (L.drop0 ? 1 : 0)));
+  f64_image_kernel<<<grid, 128, 0, st>>>(L.V, L.vrows, L.cm, L.k, L.drop0 ? 1 : 0, L.kpad, L.N, S, L.img);
+  return cudaGetLastError();
+}
+
+template <int NP, int PPG, int FORM>
 static cudaError_t launch_tb_t(const LaunchTb& L, const CUtensorMap& tm, cudaStream_t st) {
   constexpr int N = NP * PPG;
+  const int rb = tb_box_bytes(L.wpk);
   int xst, nb;
-  if (!tb_rings(N, xst, nb)) return cudaErrorInvalidValue;
-  const size_t smem = tb_smem(N, xst, nb).total + 1024;
+  if (!tb_rings(N, rb, xst, nb)) return cudaErrorInvalidValue;
+  const size_t smem = tb_smem(N, xst, nb, rb).total + 1024;
   cudaError_t e =
-      cudaFuncSetAttribute(tb_kernel<NP, PPG, SINGLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(tb_kernel<NP, PPG, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  const int T = tb_tiles(L.m, L.num_sms);
+  const int T = N <= 128 ? tb_tiles(L.m, L.num_sms) : 1;
   const unsigned long long groups = (L.m + (unsigned long long)TB_TM * T - 1) / ((unsigned long long)TB_TM * T);
   const unsigned grid = (unsigned)std::min<unsigned long long>(groups, (unsigned long long)L.num_sms);
   // the 128-sample sub-stages of the image that a row reaches
   const int nsub = std::min(L.kpad / TB_KS, L.wpk / 2), nbox = (nsub * 16 + 127) / 128;
   DevOutMP O{};
   DevOut O1{};
-  if (SINGLE) O1 = *L.O1;
-  else O = *L.O;
-  tb_kernel<NP, PPG, SINGLE><<<grid, TB_THREADS, smem, st>>>(tm, L.m, nbox, nsub, L.G, T, xst, nb, L.Bimg,
-                                                             (unsigned long long)L.kpad * N, L.ph, O, O1);
+  if (FORM == TB_MANY) O = *L.O;
+  else O1 = *L.O1;
+  tb_kernel<NP, PPG, FORM><<<grid, TB_THREADS, smem, st>>>(tm, L.m, nbox, nsub, L.G, T, xst, nb, rb, L.Bimg,
+                                                           (unsigned long long)L.kpad * N, L.ph, O, O1);
   return cudaGetLastError();
 }
 
@@ -484,9 +645,31 @@ cudaError_t launch_tb(const LaunchTb& L, cudaStream_t st) {
   if (L.m == 0) return cudaSuccess;
   CUtensorMap tm;
   if (!mp_tmap(L.x, L.m, L.wpk, &tm)) return cudaErrorInvalidValue;
+  if (L.fp64) {
+#define KG_TB_CASE(NN) \
+  if (L.NP == NN) return launch_tb_t<NN, 1, TB_ONE64>(L, tm, st);
+    KG_TB_CASE(16)
+    KG_TB_CASE(32)
+    KG_TB_CASE(48)
+    KG_TB_CASE(64)
+    KG_TB_CASE(80)
+    KG_TB_CASE(96)
+    KG_TB_CASE(112)
+    KG_TB_CASE(128)
+    KG_TB_CASE(144)
+    KG_TB_CASE(160)
+    KG_TB_CASE(176)
+    KG_TB_CASE(192)
+    KG_TB_CASE(208)
+    KG_TB_CASE(224)
+    KG_TB_CASE(240)
+    KG_TB_CASE(256)
+#undef KG_TB_CASE
+    return cudaErrorInvalidValue;
+  }
   if (L.O1) {
 #define KG_TB_CASE(NN) \
-  if (L.NP == NN) return launch_tb_t<NN, 1, true>(L, tm, st);
+  if (L.NP == NN) return launch_tb_t<NN, 1, TB_ONE>(L, tm, st);
     KG_TB_CASE(16)
     KG_TB_CASE(32)
     KG_TB_CASE(48)
@@ -499,7 +682,7 @@ cudaError_t launch_tb(const LaunchTb& L, cudaStream_t st) {
     return cudaErrorInvalidValue;
   }
 #define KG_TB_CASE(NP_, PPG_) \
-  if (L.NP == NP_ && L.PPG == PPG_) return launch_tb_t<NP_, PPG_, false>(L, tm, st);
+  if (L.NP == NP_ && L.PPG == PPG_) return launch_tb_t<NP_, PPG_, TB_MANY>(L, tm, st);
   KG_MP_GROUPS(KG_TB_CASE)
 #undef KG_TB_CASE
   return cudaErrorInvalidValue;

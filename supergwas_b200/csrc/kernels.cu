@@ -1,6 +1,8 @@
 // kernels.cu -- the association kernels.
 //
-//   fp64_kernel  : plain FP64 form on CUDA cores.  One thread per k-mer;
+//   fp64_kernel  : FP64 form on CUDA cores, for what the limb form of
+//                  kernel_tb.cu does not take (more than 256 limb columns,
+//                  unaligned rows).  One thread per k-mer;
 //                  the contraction columns (phenotyped-sample indicator, then
 //                  the centred structure and phenotype columns) are staged
 //                  through shared memory 128 samples at a time and every lane

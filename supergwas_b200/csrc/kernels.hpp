@@ -88,7 +88,20 @@ struct LaunchTb {
   const DevOutMP* O;
   const DevOut* O1;           // one phenotype: its outputs (O unused)
   int num_sms;
+  bool fp64 = false;          // one phenotype in the FP64 form (image of launch_f64_image)
 };
+// The FP64 form on the tensor cores: U columns in 7 limbs, y' in 8.
+struct LaunchF64Image {
+  const double* V;            // FP64 columns (LaunchFp64::V), vrows x cm
+  int vrows, cm, k;
+  bool drop0;                 // U column 0 has no limbs
+  int kpad, N;                // f64_limb_cols columns
+  const double* up;           // k + 1 scales 2^s (powers of two) of the columns, y' last
+  int8_t* img;                // kpad x N bytes (device)
+};
+int f64_limb_cols(int k, bool drop0);
+bool f64_limbs_supported(int N, int n_row, int wpk);
+cudaError_t launch_f64_image(const LaunchF64Image& L, cudaStream_t st);
 bool tb_supported(int N, int wpk);
 int tb_tiles(unsigned long long m, int num_sms);  // tiles per item of a launch
 int tb_ring(int N);                               // image chunks in the ring

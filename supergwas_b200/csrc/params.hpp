@@ -96,6 +96,15 @@ inline void set_screen(EpiParams& P, const LimbMap& L, bool drop0) {
   }
 }
 
+// The same for limb columns of the FP64 form (7 limbs per U column, 8 for y'),
+// of which the screen reads the four highest.
+inline void set_screen64(EpiParams& P, const LimbMap& L, bool drop0) {
+  set_screen(P, L, drop0);
+  const double f = 65536.0 * 65536.0;  // 2^8 of the shift, 256^3 of the lower limbs
+  for (int j = 0; j < KMAX; ++j) P.S.su[j] = (float)(P.S.su[j] * f);
+  P.S.sy = (float)(P.S.sy * (f * 256.0 / 65536.0));
+}
+
 // Device outputs of one launch.
 struct DevOut {
   unsigned long long* counters;  // [0] tested, [1] hits, [2] error bits, [3] refinement candidates

@@ -208,12 +208,14 @@ typedef struct kg_tile_shape {
     int kernel;   /* 1: each group's limb image resident in shared memory;
                      2: images streamed from L2;
                      3: pairs of SMs (cta_group::2), two phenotypes per M = 256
-                        MMA, one phenotype's image resident in each SM       */
+                        MMA, one phenotype's image resident in each SM;
+                     4: 4-bit screen, each group's image resident; undecided
+                        tests go to the FP64 refinement                      */
     int np;       /* limb columns per phenotype slot                         */
     int ppg;      /* phenotypes per MMA group (MMA N = np * ppg)             */
     int groups;   /* MMA groups                                              */
     int kpad;     /* samples per image (padded)                              */
-    int bt;       /* kernel 1: tile-iterations per L2 block of the last launch */
+    int bt;       /* kernels 1, 4: tile-iterations per L2 block of the last launch */
     int xs, nb;   /* kernel 2: row tiles at a time, image ring stages        */
 } kg_tile_shape;
 int kg_multi_shape(const kg_ctx* ctx, kg_tile_shape* out);

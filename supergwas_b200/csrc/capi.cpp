@@ -70,6 +70,35 @@ int set_f64_limbs(kg_ctx* ctx, int n_row) {
   return KG_OK;
 }
 
+// Image and constants of the 4-bit screen, where it applies: one limb per U
+// column, or two where one leaves too much (columns with outliers).
+int set_screen4(kg_ctx* ctx, const int32_t* sample_pos, int n_row) {
+  const kg::Prepared& p = ctx->prep;
+  if (!p.drop0 || p.k < 1) return KG_OK;
+  const bool gate = ctx->P.corr_thr > 0.0;
+  const int kpad = (n_row + 255) / 256 * 256, wpk = (n_row + 63) / 64;
+  for (int lu = 1; lu <= 2; ++lu) {
+    const int N = kg::fs_width(gate, lu, p.k - 1);
+    if (!kg::fs_supported(N, kpad, wpk + (wpk & 1))) continue;
+    kg::FsCols C;
+    kg::make_fs_cols(p, sample_pos, n_row, lu, gate, C);
+    kg::FsPheno F;
+    if (!kgctx::fill_fs(F, ctx->P, p, C, lu, gate)) continue;
+    const size_t bytes = (size_t)kpad * N / 2;
+    std::vector<uint8_t> img(bytes + sizeof(F), 0);
+    kg::put_fs_image(C, 0, N, img.data());
+    std::memcpy(img.data() + bytes, &F, sizeof(F));
+    dfree(ctx->dFs);
+    KG_CUDA(cudaMalloc((void**)&ctx->dFs, img.size()), "cudaMalloc(screen)");
+    KG_CUDA(cudaMemcpy(ctx->dFs, img.data(), img.size(), cudaMemcpyHostToDevice), "copy screen");
+    ctx->fs_N = N;
+    ctx->fs_lu = lu;
+    ctx->fs_kpad = kpad;
+    return KG_OK;
+  }
+  return KG_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -143,6 +172,7 @@ void kg_destroy(kg_ctx* ctx) {
   dfree(ctx->dB);
   dfree(ctx->dBts);
   dfree(ctx->dPh1);
+  dfree(ctx->dFs);
   dfree(ctx->dCounters);
   dfree(ctx->dHits);
   dfree(ctx->dCand);
@@ -237,6 +267,7 @@ int kg_set_structure_ex(kg_ctx* ctx, const double* U, int n, int k, const double
     KG_CUDA(cudaMemcpy(ctx->dV, V.data(), V.size() * sizeof(double), cudaMemcpyHostToDevice), "copy V");
   }
   ctx->f64_N = 0;
+  ctx->fs_N = 0;
   if (ctx->opts.precision == KG_PREC_FP64) {
     if (int rc = set_f64_limbs(ctx, n_row)) return rc;
   }
@@ -288,6 +319,7 @@ int kg_set_structure_ex(kg_ctx* ctx, const double* U, int n, int k, const double
       KG_CUDA(cudaMalloc((void**)&ctx->dPh1, sizeof(ph)), "cudaMalloc(phenotype)");
       KG_CUDA(cudaMemcpy(ctx->dPh1, &ph, sizeof(ph), cudaMemcpyHostToDevice), "copy");
     }
+    if (int rc = set_screen4(ctx, sample_pos, n_row)) return rc;
   }
   ctx->have_structure = true;
   return KG_OK;
@@ -583,7 +615,23 @@ int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64
     const bool tb_ok = tma_ok && !ts_ok && ctx->dPh1 && kg::tb_supported(ctx->limbs.N, (int)wpk);
     if (force && std::string(force) == "ts" && !ts_ok)
       return ctx->fail(KG_ERR_UNSUPPORTED, "KG_KERNEL=ts: shape not supported by the TMEM-A kernel");
-    if (ts_ok && !want_ss) {
+    if (ctx->fs_N && tma_ok && !stats && !force && kg::fs_supported(ctx->fs_N, ctx->fs_kpad, (int)wpk)) {
+      kg::LaunchFs L{};
+      L.x = dx;
+      L.m = m;
+      L.wpk = (int)wpk;
+      L.kpad = ctx->fs_kpad;
+      L.NP = ctx->fs_N;
+      L.PPG = L.G = 1;
+      L.lu = ctx->fs_lu;
+      L.gate = ctx->P.corr_thr > 0.0;
+      L.Bimg = ctx->dFs;
+      L.ph = reinterpret_cast<const kg::FsPheno*>(ctx->dFs + (size_t)ctx->fs_kpad * ctx->fs_N / 2);
+      L.O1 = &O;
+      L.num_sms = ctx->num_sms;
+      e = kg::launch_fs(L, st);
+      ctx->last_kernel = "ts";
+    } else if (ts_ok && !want_ss) {
       kg::LaunchTs L{dx, m, (int)wpk, ctx->limbs.Kpad, ctx->prep.drop0 && ctx->P.k > 0, ctx->dBts, &ctx->P,
                      &ctx->LM, &O, ctx->num_sms};
       e = kg::launch_ts(L, st);

@@ -1,9 +1,11 @@
 // capi_multi.cpp -- the many-phenotype entry points of include/kgwas_cuda.h.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "ctx.hpp"
@@ -17,6 +19,8 @@ void free_multi(kg_ctx* ctx) {
   if (M.graph) cudaGraphExecDestroy(M.graph);
   M.graph = nullptr;
   dfree(M.dB);
+  dfree(M.dFs);
+  M.fs_NP = 0;
   dfree(M.dPh);
   dfree(M.dV);
   dfree(M.dT);
@@ -115,7 +119,29 @@ int enqueue_multi(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uns
   kg::DevOutMP O = dev_out(ctx, offset);
   KG_CUDA(cudaMemsetAsync(M.dCounters + 3, 0, sizeof(unsigned long long), st), "memset");
   cudaError_t e;
-  if (M.kern >= 1) {
+  if (M.kern == 3) {
+    // a block's packed rows (every CTA's) stay in L2 across the passes
+    const unsigned long long grid = std::min<unsigned long long>((m + 127) / 128, (unsigned long long)ctx->num_sms);
+    unsigned long long bt = (64ull << 20) / std::max<unsigned long long>(1, grid * 128ull * wpk * 8);
+    if (const char* v = std::getenv("KG_MP_BT")) bt = (unsigned long long)std::max(1, std::atoi(v));
+    M.bt = (int)std::max<unsigned long long>(1, std::min<unsigned long long>(bt, 1024));
+    kg::LaunchFs L{};
+    L.x = dx;
+    L.m = m;
+    L.wpk = (int)wpk;
+    L.kpad = M.fs_kpad;
+    L.NP = M.fs_NP;
+    L.PPG = M.fs_PPG;
+    L.G = M.fs_G;
+    L.lu = 1;
+    L.gate = ctx->opts.corr_threshold > 0.0;
+    L.bt = M.bt;
+    L.Bimg = M.dFs;
+    L.ph = reinterpret_cast<const kg::FsPheno*>(M.dFs + (size_t)M.fs_G * M.fs_kpad * M.fs_NP * M.fs_PPG / 2);
+    L.O = &O;
+    L.num_sms = ctx->num_sms;
+    e = kg::launch_fs(L, st);
+  } else if (M.kern >= 1) {
     // tile-iterations per block: the block's packed rows (every CTA's) stay in L2
     // across the G passes; the autotuner scales the 48 MB rule by bt_scale / 2
     const unsigned long long tiles = (m + 127) / 128;
@@ -161,12 +187,17 @@ int reset_outputs(kg_ctx* ctx, cudaStream_t st) {
 int autotune(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, cudaStream_t st) {
   Multi& M = ctx->mp;
   const int nbox = ((int)wpk * 8 + 127) / 128;
-  if (M.tuned && M.tuned_nbox == nbox) return KG_OK;
+  const char* only = std::getenv("KG_MP_KERNEL");
+  // the 4-bit screen has one launch shape (rows of 31-bit index, as its TMA loads take)
+  if (!only && M.fs_NP && m <= 0x7fffff00ull && kg::fs_supported(M.fs_NP * M.fs_PPG, M.fs_kpad, (int)wpk)) {
+    M.kern = 3;
+    return KG_OK;
+  }
+  if (M.kern != 3 && M.tuned && M.tuned_nbox == nbox) return KG_OK;
   struct Cand {
     int kern, bt_scale;
   };
   std::vector<Cand> cands;
-  const char* only = std::getenv("KG_MP_KERNEL");
   auto allowed = [&](const char* k) { return !only || std::string(only) == k; };
   if (M.stationary && !(only && std::string(only) == "mp")) {
     for (int s : {2, 1, 4}) {
@@ -236,6 +267,60 @@ int collect_multi(kg_ctx* ctx, uint64_t m, kg_multi_result* res) {
     res->n_hits = nh;
     res->hits = M.hits.data();
   }
+  return KG_OK;
+}
+
+// Group images and constants of the 4-bit screen (one limb per U column), where
+// every phenotype has them; the slots are as wide as the widest phenotype
+// needs, and as many phenotypes share a group as fit.
+int set_screen4_multi(kg_ctx* ctx, const kg_pheno* ph, const std::vector<kg::Prepared>& prep,
+                      const std::vector<kg::MPheno>& mph, int n_row) {
+  Multi& M = ctx->mp;
+  const int np = (int)prep.size(), kpad = (n_row + 255) / 256 * 256;
+  const bool gate = ctx->opts.corr_threshold > 0.0;
+  M.fs_NP = 0;
+  int ku = 0;
+  for (const kg::Prepared& p : prep) {
+    if (!p.drop0 || p.k < 1) return KG_OK;
+    ku = std::max(ku, p.k - 1);
+  }
+  const int NP = kg::fs_width(gate, 1, ku);
+  int PPG = 0;
+#define KG_FS_CASE(NP_, PPG_) \
+  if (NP == NP_ && (PPG == 0 || PPG < np) && kg::fs_supported(NP_ * PPG_, kpad, 16)) PPG = PPG_;
+  KG_FS_GROUPS(KG_FS_CASE)
+#undef KG_FS_CASE
+  if (!PPG) return KG_OK;
+  const int N = NP * PPG, G = (np + PPG - 1) / PPG;
+  const size_t img_bytes = (size_t)kpad * N / 2;
+  std::vector<uint8_t> img((size_t)G * img_bytes + (size_t)np * sizeof(kg::FsPheno), 0);
+  std::atomic<int> next{0}, bad{0};
+  auto work = [&] {
+    for (int p; (p = next.fetch_add(1)) < np && !bad.load();) {
+      kg::FsCols C;
+      kg::make_fs_cols(prep[p], ph[p].sample_pos, n_row, 1, gate, C);
+      kg::FsPheno F;
+      if (!fill_fs(F, mph[p].P, prep[p], C, 1, gate)) {
+        bad.store(1);
+        return;
+      }
+      // two columns share no byte: a byte holds two samples of one column
+      kg::put_fs_image(C, (p % PPG) * NP, N, img.data() + (size_t)(p / PPG) * img_bytes);
+      std::memcpy(img.data() + (size_t)G * img_bytes + (size_t)p * sizeof(F), &F, sizeof(F));
+    }
+  };
+  const int nt = std::max(1, std::min<int>({8, (int)std::thread::hardware_concurrency(), np}));
+  std::vector<std::thread> th;
+  for (int t = 1; t < nt; ++t) th.emplace_back(work);
+  work();
+  for (auto& t : th) t.join();
+  if (bad.load()) return KG_OK;
+  KG_CUDA(cudaMalloc((void**)&M.dFs, img.size()), "cudaMalloc(screen)");
+  KG_CUDA(cudaMemcpy(M.dFs, img.data(), img.size(), cudaMemcpyHostToDevice), "copy screen");
+  M.fs_NP = NP;
+  M.fs_PPG = PPG;
+  M.fs_G = G;
+  M.fs_kpad = kpad;
   return KG_OK;
 }
 
@@ -369,13 +454,17 @@ int kg_set_phenotypes(kg_ctx* ctx, const kg_pheno* ph, int np, int n_row) {
   kg::LaunchTable LT{M.dV, vrows, cm, (unsigned long long)M.vstride, np, M.dT};
   KG_CUDA(kg::launch_refine_table(LT, ctx->stream), "refinement tables");
   KG_CUDA(cudaStreamSynchronize(ctx->stream), "refinement tables");
-  return KG_OK;
+  return set_screen4_multi(ctx, ph, prep, mph, n_row);
 }
 
 int kg_multi_shape(const kg_ctx* ctx, kg_tile_shape* out) {
   if (!ctx || !out) return KG_ERR_INVALID;
   const Multi& M = ctx->mp;
   if (M.np <= 0) return KG_ERR_STATE;
+  if (M.kern == 3) {
+    *out = kg_tile_shape{4, M.fs_NP, M.fs_PPG, M.fs_G, M.fs_kpad, M.bt, 1, 0};
+    return KG_OK;
+  }
   out->kernel = M.kern == 2 ? 3 : M.kern == 1 ? 1 : 2;
   out->np = M.NP;
   out->ppg = M.kern == 2 ? 2 : M.PPG;

@@ -62,14 +62,66 @@ inline void fill_epi(kg::EpiParams& P, const kg::Prepared& p, const kg_opts& o, 
   }
 }
 
+// Constants of the 4-bit screen for one phenotype (fs_verdict).  False where
+// the screen does not apply: the intercept has limbs, the structure or the
+// phenotype is degenerate, or so much may pass (thresholds at which rows of
+// chi-square below REFINE_CHISQ are emitted, residuals that leave the cut or the
+// gate vague) that refining it would cost more than the screen saves: a
+// refinement reads n / 8 table rows, 20 KB at n = 1000, r = 16+1, so 1e-3 of the
+// k-mers cost as much as the screen of all of them (1e8: 1e5 and 2.2 ms).
+inline bool fill_fs(kg::FsPheno& F, const kg::EpiParams& P, const kg::Prepared& p, const kg::FsCols& C, int lu,
+                    bool gate) {
+  F = kg::FsPheno();
+  const double r2_ref = -std::expm1(-kg::REFINE_CHISQ / (double)p.n);
+  const double yv = P.yyM / (P.ynorm * P.ynorm);
+  if (!p.drop0 || p.k < 1 || !(std::fabs(P.a[0] * P.a[0] * p.n - 1.0) <= 1e-6) || p.n >= 65536 || !(P.ynorm >= 1e-12) || !(P.ynorm < 1e150) || !(yv > 1e-6) ||
+      !(P.r2_cand >= r2_ref) || !(P.r2_cand < 1.0) || P.refine == 0)
+    return false;
+  F.n = p.n;
+  F.ku = p.k - 1;
+  F.inv_n = (float)(1.0 / p.n);
+  const double cut = P.r2_cand * yv;
+  F.cut = (float)(cut * (1.0 - 1e-4));
+  F.b = (float)(P.b / P.ynorm);
+  F.kappa = (float)(P.kappa / P.ynorm);
+  F.thr = (float)P.corr_thr;
+  // the columns' norms, for the rounding of single-precision sums and scales
+  // (a few 2^-24 of each term): 1e-5 of them
+  double fu = 0, fy = 0, fg = P.ynorm;
+  for (int j = 1; j < p.k; ++j)
+    for (int i = 0; i < p.n; ++i) fu += p.d[(size_t)j * p.n + i] * p.d[(size_t)j * p.n + i];
+  for (int i = 0; i < p.n; ++i) fy += p.d[(size_t)p.k * p.n + i] * p.d[(size_t)p.k * p.n + i];
+  const double up = 1.0 + 1e-5;
+  const double bu = C.nu * up + 1e-5 * std::sqrt(fu), by = (C.ny * up + 1e-5 * std::sqrt(fy)) / P.ynorm;
+  const double bg = (C.ng * up + 1e-5 * fg) / P.ynorm;
+  if (!(bu <= 0.25) || !(by <= 0.2 * std::sqrt(cut)) || (gate && !(bg <= 2e-3))) return false;
+  const double tiny = 1e-12;
+  F.bu = (float)bu;
+  F.mu = (float)(C.mu * up + tiny);
+  F.by = (float)by;
+  F.my = (float)(C.my * up / P.ynorm + tiny);
+  F.bg = (float)bg;
+  F.mg = (float)(C.mg * up / P.ynorm + tiny);
+  for (int l = 0; l < 3; ++l) F.sy[l] = (float)(C.sy[l] / P.ynorm);
+  if (gate)
+    for (int l = 0; l < 4; ++l) F.sg[l] = (float)(C.sg[l] / P.ynorm);
+  for (int j = 0; j < F.ku; ++j)
+    for (int l = 0; l < lu; ++l) F.su[lu * j + l] = (float)C.su[(size_t)j * lu + l];
+  return true;
+}
+
 // State of the many-phenotype path.
 struct Multi {
   int np = 0, n_row = 0, NP = 0, G = 0, kpad = 0, cm = 0, nsteps = 0;
   int PPG = 1;          // phenotypes per group (one MMA of NP * PPG columns)
   bool stationary = false;  // the group image fits in shared memory: kernel_mpb.cu
   bool pair_ok = false;     // kernel_mpb2.cu can run these phenotypes (PPG = 1 images)
-  int kern = 0;             // chosen kernel: 0 image streamed (tb), 1 image resident (mpb), 2 SM pair (mpb2)
+  int kern = 0;             // chosen kernel: 0 image streamed (tb), 1 image resident (mpb), 2 SM pair (mpb2), 3 4-bit screen (fs)
   int bt_scale = 2;         // tile-iterations per L2 block: the 48 MB rule times bt_scale / 2
+  // 4-bit screen: group images and, behind them, the phenotypes' constants;
+  // columns per slot (0: not used), slots per group, groups, samples per image
+  uint8_t* dFs = nullptr;
+  int fs_NP = 0, fs_PPG = 1, fs_G = 0, fs_kpad = 0;
   int8_t* dB = nullptr;
   kg::MPheno* dPh = nullptr;
   double* dV = nullptr;
@@ -126,6 +178,10 @@ struct kg_ctx {
   int8_t* dB = nullptr;      // B image of the smem-A kernel
   int8_t* dBts = nullptr;    // B image of the TMEM-A kernels
   kg::MPheno* dPh1 = nullptr;  // the phenotype's constants for the streamed-image kernel
+  // 4-bit screen: image and, behind it, the phenotype's constants; columns (0:
+  // not used), limbs per U column, samples of the image
+  uint8_t* dFs = nullptr;
+  int fs_N = 0, fs_lu = 0, fs_kpad = 0;
   int nchunk = 0;
   int f64_N = 0;             // limb columns of the FP64 form (dBts holds image and constants); 0: CUDA cores
   // outputs on the device

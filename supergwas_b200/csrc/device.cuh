@@ -624,6 +624,24 @@ __device__ __forceinline__ void table_row_sums(const uint64_t* __restrict__ row,
   }
 }
 
+// Correlation gate of a refinement candidate in FP64 from its lane-distributed
+// column sums (refine_reduce); identical in every lane.
+template <int CM>
+__device__ __forceinline__ bool refine_gate(const EpiParams& P, const double (&acc)[(CM + 31) / 32], int lane, int c,
+                                            double ey) {
+  double gs = 0.0;
+#pragma unroll
+  for (int jj = 0; jj < (CM + 31) / 32; ++jj) {
+    const int j = lane + 32 * jj;
+    if (j >= 1 && j <= P.k) gs += P.g[j - 1] * acc[jj];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) gs += __shfl_xor_sync(0xffffffffu, gs, o);
+  const double xcn2 = (double)c * (double)(P.n - c) / (double)P.n;
+  const double xyc = ey + gs + P.kappa * (double)c;
+  return xyc * xyc >= P.thr2_ynorm2 * xcn2;
+}
+
 // From the lane-distributed column sums (column 0 = count, 1..k = U columns,
 // k+1 = y'): c, ss = sum_j (a_j c + e_j)^2 and ey, identical in every lane.
 template <int CM>
@@ -662,6 +680,15 @@ __device__ __forceinline__ int mp_shard(const DevOutMP& O, unsigned long long gk
     else hi = mid - 1;
   }
   return lo;
+}
+
+// Adds the lanes' counts of phenotype p to their (shard, phenotype) counters:
+// one atomic per distinct shard in the warp.
+__device__ __forceinline__ void tb_count(const DevOutMP& O, int p, int shard, uint32_t cnt) {
+  const unsigned match = __match_any_sync(0xffffffffu, shard);
+  const unsigned tot = __reduce_add_sync(match, cnt);
+  if ((int)(threadIdx.x & 31u) == __ffs(match) - 1 && tot)
+    atomicAdd(O.tested + (size_t)shard * O.n_pheno + p, (unsigned long long)tot);
 }
 
 // Statistic of one (k-mer, phenotype) from the exact integer sums, as the

@@ -9,7 +9,7 @@
 
 namespace kg {
 
-constexpr unsigned long long MP_KMER_MASK = (1ull << 48) - 1;
+constexpr unsigned long long MP_KMER_MASK = (1ull << 47) - 1;  // bit 47: CAND_OPEN_MP
 
 // FP64 recomputation of the candidates of a multi-phenotype launch: one
 // warp per (k-mer, phenotype), the phenotype's byte tables at T + p*tstride
@@ -34,6 +34,11 @@ __global__ void __launch_bounds__(256) mp_refine_kernel(const uint64_t* __restri
     int c;
     double ss, ey;
     refine_reduce<CM>(P, acc, lane, c, ss, ey);
+    if (ent & CAND_OPEN_MP) {
+      if (!refine_gate<CM>(P, acc, lane, c, ey)) continue;
+      if (lane == 0)
+        atomicAdd(O.tested + (size_t)mp_shard(O, gk) * O.n_pheno + p, O.weight ? (unsigned long long)O.weight[gk] : 1ull);
+    }
     if (lane == 0) {
       const double xxM = (double)c - ss, xyM = P.b * (double)c + ey;
       double effect = 0, Tq = 0, pv = 1;

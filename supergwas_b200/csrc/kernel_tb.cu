@@ -63,15 +63,6 @@ __host__ __device__ inline TbSmem tb_smem(int N, int xst, int nb, int rb) {
   return L;
 }
 
-// Adds the lanes' counts of phenotype p to their (shard, phenotype) counters:
-// one atomic per distinct shard in the warp.
-__device__ __forceinline__ void tb_count(const DevOutMP& O, int p, int shard, uint32_t cnt) {
-  const unsigned match = __match_any_sync(0xffffffffu, shard);
-  const unsigned tot = __reduce_add_sync(match, cnt);
-  if ((int)(threadIdx.x & 31u) == __ffs(match) - 1 && tot)
-    atomicAdd(O.tested + (size_t)shard * O.n_pheno + p, (unsigned long long)tot);
-}
-
 // One phenotype, outputs of kernel_ts.cu (DevOut).
 template <int N>
 __device__ __forceinline__ void tb_single(const DevOut& O, const MPheno* ME, uint32_t taddr, unsigned long long local,

@@ -139,13 +139,17 @@ __global__ void __launch_bounds__(256) refine_kernel(const uint64_t* __restrict_
   if (ncand > O.cand_cap) ncand = O.cand_cap;
   for (unsigned long long w = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < ncand;
        w += warps) {
-    const unsigned long long g = O.cand[w];
+    const unsigned long long entry = O.cand[w], g = entry & ~CAND_OPEN;
     const uint64_t* row = x + (g - O.kmer_offset) * (unsigned long long)wpk;
     double acc[(CM + 31) / 32];
     table_row_sums<CM>(row, nwords, T, lane, acc);
     int c;
     double ss, ey;
     refine_reduce<CM>(P, acc, lane, c, ss, ey);
+    if (entry & CAND_OPEN) {
+      if (!refine_gate<CM>(P, acc, lane, c, ey)) continue;
+      if (lane == 0) atomicAdd(O.counters, O.weight ? (unsigned long long)O.weight[g] : 1ull);
+    }
     if (lane == 0) {
       const double xxM = (double)c - ss, xyM = P.b * (double)c + ey;
       double effect = 0, Tq = 0, p = 1;

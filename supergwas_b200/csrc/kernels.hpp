@@ -107,6 +107,39 @@ int tb_tiles(unsigned long long m, int num_sms);  // tiles per item of a launch
 int tb_ring(int N);                               // image chunks in the ring
 cudaError_t launch_tb(const LaunchTb& L, cudaStream_t st);
 
+// 4-bit screen (kernel_fs.cu), one phenotype (O1) or many (O).
+struct LaunchFs {
+  const uint64_t* x;          // packed rows (device), 16-byte aligned
+  unsigned long long m;
+  int wpk;
+  int kpad;                   // samples per image (multiple of 256)
+  int NP, PPG, G;             // columns per phenotype slot, phenotypes per group, groups
+  int lu;                     // limbs per U column
+  bool gate;                  // the columns hold y - mean(y)
+  int bt;                     // tiles of a CTA per pass over the groups (G > 1)
+  const uint8_t* Bimg;        // G images of kpad * NP * PPG / 2 bytes (put_fs_image; device)
+  const FsPheno* ph;          // per-phenotype constants (device)
+  const DevOutMP* O;
+  const DevOut* O1;
+  int num_sms;
+};
+// (columns per phenotype slot, phenotypes per group) with a many-phenotype
+// screen: groups of at most 112 columns.
+#define KG_FS_GROUPS(X)                                                                                    \
+  X(8, 1) X(8, 3) X(8, 8) X(16, 1) X(16, 2) X(16, 4) X(16, 6) X(24, 1) X(24, 2) X(24, 4) X(32, 1) X(32, 2) \
+  X(32, 3) X(40, 1) X(40, 2) X(48, 1) X(48, 2) X(56, 1) X(56, 2) X(64, 1) X(72, 1)
+// (columns, limbs per U column) with a single-phenotype screen.
+#define KG_FS_SINGLE(X)                                                                                         \
+  X(8, 1) X(16, 1) X(24, 1) X(32, 1) X(40, 1) X(48, 1) X(56, 1) X(64, 1) X(72, 1) X(80, 1) X(16, 2) X(32, 2) \
+  X(48, 2) X(64, 2) X(80, 2) X(96, 2) X(112, 2)
+// Columns of one phenotype's slot: a width that has a kernel.
+inline int fs_width(bool gate, int lu, int ku) {
+  const int q = lu == 2 ? 16 : 8, w = (4 + (gate ? 4 : 0) + lu * ku + q - 1) / q * q;
+  return w > 80 ? (w + 15) / 16 * 16 : w;
+}
+bool fs_supported(int N, int kpad, int wpk);
+cudaError_t launch_fs(const LaunchFs& L, cudaStream_t st);
+
 struct LaunchMpRefine {
   const uint64_t* x;
   int wpk;

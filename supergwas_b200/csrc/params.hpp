@@ -1,5 +1,6 @@
 // params.hpp -- kernel parameter blocks shared by host and device code.
 #pragma once
+#include <cmath>
 #include <cstdint>
 
 #include "../../include/kgwas_cuda.h"
@@ -75,7 +76,8 @@ inline void set_screen(EpiParams& P, const LimbMap& L, bool drop0) {
   double cut = P.r2_cand;
   if (P.refine && P.r2_ref < cut) cut = P.r2_ref > P.r2_need ? P.r2_ref : P.r2_need;
   const double yv = P.yyM / (P.ynorm * P.ynorm);
-  if (!drop0 || !(P.ynorm >= 1e-12) || !(P.ynorm < 1e150) || !(cut > 0) || !(yv > 1e-6) || P.n >= 65536) return;
+  // c - s_0^2 = c (n - c) / n, which the screen uses, holds for a unit intercept
+  if (!(drop0 && std::fabs(P.a[0] * P.a[0] * P.n - 1.0) <= 1e-6) || !(P.ynorm >= 1e-12) || !(P.ynorm < 1e150) || !(cut > 0) || !(yv > 1e-6) || P.n >= 65536) return;
   S.on = 1;
   while ((4 << S.shift) < P.n) ++S.shift;
   S.inv_n = (float)(1.0 / P.n);
@@ -104,6 +106,23 @@ inline void set_screen64(EpiParams& P, const LimbMap& L, bool drop0) {
   for (int j = 0; j < KMAX; ++j) P.S.su[j] = (float)(P.S.su[j] * f);
   P.S.sy = (float)(P.S.sy * (f * 256.0 / 65536.0));
 }
+
+// Constants of one phenotype for the 4-bit screen (kernel_fs.cu); everything
+// about y is relative to ynorm.
+struct alignas(16) FsPheno {
+  int n, ku;              // samples; U columns with limbs
+  float inv_n, cut;       // 1 / n; lowest r2 of an emitted row x yyM / ynorm^2
+  float b, kappa, thr;    // b / ynorm, kappa / ynorm, the correlation threshold
+  float bu, mu;           // bounds of what the limbs leave out (fs_verdict): U columns,
+  float by, my, bg;       // y' and
+  float sy[3];            // limb sums of y' -> e_y
+  float mg;               // y - mean(y)
+  float sg[4];            // limb sums of y - mean(y)
+  float su[2 * KMAX];     // limb sums of the U columns, one or two limbs each
+};
+
+// Refinement candidates: marks of entries whose correlation gate is not decided.
+constexpr unsigned long long CAND_OPEN = 1ull << 63, CAND_OPEN_MP = 1ull << 47;
 
 // Device outputs of one launch.
 struct DevOut {

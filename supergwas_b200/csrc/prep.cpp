@@ -231,4 +231,182 @@ void make_b_image(const LimbCols& L, int KC, std::vector<int8_t>& img) {
         }
 }
 
+// ------------------------------------------------------------ 4-bit screen
+// Nearest e2m1 value of t (|t| above 6 becomes 6).
+static inline float e2m1_round(float t) {
+  const float a = std::fabs(t);
+  const float r = a < 2.0f ? std::rint(a * 2.0f) * 0.5f : a < 4.0f ? std::rint(a) : std::min(std::rint(a * 0.5f) * 2.0f, 6.0f);
+  return std::copysign(r, t);
+}
+static inline uint8_t e2m1_code(float v) {
+  const int h = (int)(std::fabs(v) * 2.0f);  // 0 1 2 3 4 6 8 12
+  const int c = h <= 4 ? h : h == 6 ? 5 : h == 8 ? 6 : 7;
+  return (uint8_t)(c | (v < 0 ? 8 : 0));
+}
+
+// Moves codes of the last limb (scale s) to a neighbouring value, where that adds
+// least to the residual r, until the residual's sum is as close to zero as one
+// such step allows.  A row of frequency near one meets the sum: the rest of the
+// bound shrinks with ||x - mean(x)||, c |sum r| / n does not.
+static void fs_balance(std::vector<double>& r, const int* pos, uint8_t* code, double s) {
+  static const float val[8] = {0.0f, 0.5f, 1.0f, 1.5f, 2.0f, 3.0f, 4.0f, 6.0f};
+  const int n = (int)r.size();
+  double D = 0;
+  for (double v : r) D += v;
+  const int dir = D > 0 ? 1 : -1;  // a positive sum: larger limbs
+  struct Move {
+    double cost, step;
+    int i;
+    uint8_t to;
+  };
+  std::vector<Move> mv;
+  mv.reserve(n);
+  for (int i = 0; i < n; ++i) {
+    const uint8_t c = code[pos ? pos[i] : i];
+    const int at = (c & 8) ? -(c & 7) : (c & 7), to = at + dir;
+    if (to > 7 || to < -7) continue;
+    const float q = at < 0 ? -val[-at] : val[at], q2 = to < 0 ? -val[-to] : val[to];
+    const double step = s * (double)(q2 - q), moved = r[i] - step;
+    mv.push_back({(moved * moved - r[i] * r[i]) / std::fabs(step), step, i, (uint8_t)(to < 0 ? 8 | -to : to)});
+  }
+  // steps of s / 2 at least: no more than this many
+  const size_t most = std::min(mv.size(), (size_t)std::min(4.0 * std::fabs(D) / s + 16.0, (double)n));
+  std::partial_sort(mv.begin(), mv.begin() + most, mv.end(),
+                    [](const Move& a, const Move& b) { return a.cost < b.cost || (a.cost == b.cost && a.i < b.i); });
+  for (size_t t = 0; t < most; ++t) {
+    const Move& m = mv[t];
+    if (std::fabs(D - m.step) >= std::fabs(D)) continue;
+    D -= m.step;
+    r[m.i] -= m.step;
+    code[pos ? pos[m.i] : m.i] = m.to;
+  }
+}
+
+// The limbs of column r (n values): the codes (limb l to code + l * stride) and
+// the scales; r keeps what they leave out.  The last two limbs take the nearest
+// e2m1 values, with the scale, of a few below the one that represents the
+// largest value, that leaves the least.  The limbs before it keep to the
+// integers up to 4, whose even spacing leaves the next limb a ninth of the range
+// (the wider steps above would leave it a few large values, and the rest to
+// round to zero).
+static void fs_limbs(std::vector<double>& r, const int* pos, int nl, uint8_t* code, size_t stride, double* scale) {
+  const int n = (int)r.size();
+  for (int l = 0; l < nl; ++l, code += stride) {
+    double mx = 0;
+    for (double v : r) mx = std::max(mx, std::fabs(v));
+    scale[l] = 0.0;
+    if (!(mx > 0)) continue;
+    const bool nearest = l + 2 >= nl;
+    double best = mx / 4.5;
+    if (nearest) {
+      double best_err = HUGE_VAL;
+      for (double f : {1.0, 0.8, 0.6}) {
+        const float up = (float)(6.0 / (f * mx));
+        const double s = 1.0 / (double)up;
+        double err[4] = {0, 0, 0, 0};
+        for (int i = 0; i < n; ++i) {
+          const double d = r[i] - s * (double)e2m1_round((float)r[i] * up);
+          err[i & 3] += d * d;
+        }
+        const double e = err[0] + err[1] + err[2] + err[3];
+        if (e < best_err) best_err = e, best = s;
+      }
+    }
+    const float up = (float)(1.0 / best);
+    for (int i = 0; i < n; ++i) {
+      const float t = (float)r[i] * up;
+      const float q = nearest ? e2m1_round(t) : std::max(-4.0f, std::min(4.0f, std::rint(t)));
+      code[pos ? pos[i] : i] = e2m1_code(q);
+      r[i] -= best * (double)q;
+    }
+    scale[l] = best;
+    if (l + 1 == nl) fs_balance(r, pos, code, best);
+  }
+}
+
+static double sum_of(const std::vector<double>& r) {
+  double s = 0;
+  for (double v : r) s += v;
+  return s;
+}
+static double dot(const double* a, const double* b, int n) {
+  double s[4] = {0, 0, 0, 0};
+  int i = 0;
+  for (; i + 4 <= n; i += 4)
+    for (int t = 0; t < 4; ++t) s[t] += a[i + t] * b[i + t];
+  for (; i < n; ++i) s[0] += a[i] * b[i];
+  return s[0] + s[1] + s[2] + s[3];
+}
+
+void make_fs_cols(const Prepared& p, const int* pos, int n_row, int lu, bool gate, FsCols& F) {
+  const int n = p.n, k = p.k, ku = k > 0 ? k - 1 : 0;
+  F = FsCols();
+  F.kpad = (n_row + 255) / 256 * 256;
+  F.ncol = 1 + 3 + (gate ? 4 : 0) + lu * ku;
+  F.code.assign((size_t)F.ncol * F.kpad, 0);
+  auto col = [&](int c) { return F.code.data() + (size_t)c * F.kpad; };
+  for (int i = 0; i < n; ++i) col(0)[pos ? pos[i] : i] = e2m1_code(1.0f);
+  const double* dy = &p.d[(size_t)k * n];
+  std::vector<double> r(dy, dy + n);
+  fs_limbs(r, pos, 3, col(1), F.kpad, F.sy);
+  F.ny = std::sqrt(dot(r.data(), r.data(), n));
+  F.my = std::fabs(sum_of(r)) / n;
+  if (gate) {
+    for (int i = 0; i < n; ++i) r[i] = dy[i];
+    for (int j = 0; j < k; ++j)
+      for (int i = 0; i < n; ++i) r[i] += p.g[j] * p.d[(size_t)j * n + i];
+    fs_limbs(r, pos, 4, col(4), F.kpad, F.sg);
+    F.ng = std::sqrt(dot(r.data(), r.data(), n));
+    F.mg = std::fabs(sum_of(r)) / n;
+  }
+  F.su.assign((size_t)lu * ku, 0.0);
+  std::vector<double> R((size_t)ku * n);
+  double m2 = 0;
+  for (int j = 0; j < ku; ++j) {
+    const double* d = &p.d[(size_t)(j + 1) * n];
+    r.assign(d, d + n);
+    fs_limbs(r, pos, lu, col(4 + (gate ? 4 : 0) + lu * j), F.kpad, &F.su[(size_t)lu * j]);
+    std::copy(r.begin(), r.end(), R.begin() + (size_t)j * n);
+    const double s = sum_of(r) / n;
+    m2 += s * s;
+  }
+  F.mu = std::sqrt(m2);
+  // largest singular value of R: trace(G^32)^(1/32) with G = R'R / trace(R'R),
+  // never below it and at most ku^(1/64) above
+  std::vector<double> G((size_t)ku * ku), H((size_t)ku * ku);
+  double tr = 0;
+  for (int a = 0; a < ku; ++a) {
+    for (int b = 0; b <= a; ++b) G[(size_t)a * ku + b] = G[(size_t)b * ku + a] = dot(&R[(size_t)a * n], &R[(size_t)b * n], n);
+    tr += G[(size_t)a * ku + a];
+  }
+  if (tr > 0) {
+    for (double& v : G) v /= tr;
+    for (int it = 0; it < 5; ++it) {
+      for (int a = 0; a < ku; ++a)
+        for (int b = 0; b <= a; ++b)
+          H[(size_t)a * ku + b] = H[(size_t)b * ku + a] = dot(&G[(size_t)a * ku], &G[(size_t)b * ku], ku);
+      G.swap(H);
+    }
+    double t = 0;
+    for (int a = 0; a < ku; ++a) t += G[(size_t)a * ku + a];
+    F.nu = std::sqrt(tr * std::pow(t, 1.0 / 32));
+  }
+}
+
+void put_fs_image(const FsCols& F, int col0, int N, uint8_t* img) {
+  for (int c = 0; c < F.ncol; ++c) {
+    const uint8_t* code = &F.code[(size_t)c * F.kpad];
+    const int cc = col0 + c;
+    uint8_t* base = img + (size_t)(cc >> 3) * 128 + (size_t)(cc & 7) * 16;
+    for (int u = 0; u < F.kpad / 256; ++u)
+      for (int cl = 0; cl < 4; ++cl)
+        for (int e = 0; e < 64; e += 2) {
+          // element e of the MMA: word e / 8 of the unit, its sample 4 (e % 8) + cl
+          const int kap = 256 * u + 64 * cl + e;
+          const uint8_t* s = code + 256 * u + 4 * e + cl;
+          base[(size_t)(kap >> 5) * (N * 16) + ((kap & 31) >> 1)] = (uint8_t)(s[0] | s[4] << 4);
+        }
+  }
+}
+
 }  // namespace kg

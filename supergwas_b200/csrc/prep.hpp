@@ -79,4 +79,23 @@ void make_b_image_ts(const LimbCols& L, std::vector<int8_t>& img);
 // side in one MMA.
 void put_b_image_ts(const LimbCols& L, int col0, int N, std::vector<int8_t>& img);
 
+// The contraction columns in e2m1 (4-bit) limbs for the screen of kernel_fs.cu:
+// count, 3 limbs of y', with `gate` 4 of y - mean(y), lu per U column 1 .. k-1
+// (prepare's drop0 must hold).  A limb holds the nearest e2m1 values of what
+// the limbs before it leave out, over its scale.
+struct FsCols {
+  int ncol = 0, kpad = 0;           // columns; n_row rounded up to 256 samples
+  std::vector<uint8_t> code;        // e2m1 codes, code[col * kpad + sample position]
+  double sy[3], sg[4];              // limb scales
+  std::vector<double> su;           // lu per U column
+  // what the limbs leave out: norms of the residual columns (for U the largest
+  // singular value, rounded up) and |sum| / n, in the columns' own units
+  double nu = 0, mu = 0, ny = 0, my = 0, ng = 0, mg = 0;
+};
+void make_fs_cols(const Prepared& p, const int* pos, int n_row, int lu, bool gate, FsCols& out);
+// Columns at col0 .. of an N-column image: core matrices of 8 columns x 32
+// samples (16 bytes), K-major, no swizzle; of a 256-sample unit the samples
+// 4i, then 4i + 1, 4i + 2, 4i + 3 (the order of unpack_unit).
+void put_fs_image(const FsCols& F, int col0, int N, uint8_t* img);
+
 }  // namespace kg

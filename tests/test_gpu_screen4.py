@@ -1,0 +1,73 @@
+"""The 4-bit screen against the kernels that evaluate every k-mer: a row that
+is emitted comes from the FP64 refinement on both sides, so counts and rows are
+equal.  Row widths below and above one TMA box, rows that end inside a unit of
+256 samples or a box, one and two limbs per U column, tiles of one row and many
+per SM, and rows around every decision."""
+import numpy as np
+import pytest
+
+from supergwas_b200 import api, synth
+from test_gpu_ts_shapes import awkward_rows
+
+pytestmark = pytest.mark.gpu
+
+# (samples, U columns, k-mers)
+SHAPES = [(64, 3, 129), (150, 2, 1), (200, 6, 60_001), (257, 5, 127), (640, 11, 20_000), (700, 9, 128),
+          (1000, 17, 40_000), (1024, 30, 3000), (1025, 17, 3001), (2000, 21, 40_001), (2900, 33, 2500),
+          (5000, 33, 20_000), (9000, 9, 2500)]
+
+
+def structure(n, k, rng):
+    pop = np.arange(n) * 4 // n
+    Z = rng.standard_normal((n, k))
+    Z[:, 0] = 1.0
+    for s in range(1, min(4, k)):
+        Z[:, s] = pop == s
+    return pop, Z
+
+
+def both(X, U, y, thr, lt, monkeypatch, kern, *where):
+    monkeypatch.setenv("KG_DEDUP", "0")
+    with api.Kgwas(corr_threshold=thr, log10_thresh=lt) as g:
+        g.set_structure(U, y, *where)
+        monkeypatch.delenv("KG_KERNEL", raising=False)
+        a = g.run_host(X)
+        monkeypatch.setenv("KG_KERNEL", kern)
+        return a, g.run_host(X)
+
+
+@pytest.mark.parametrize("n,k,m", SHAPES, ids=lambda v: str(v))
+@pytest.mark.parametrize("thr,lt", [(0.0, 6.0), (0.2, 4.0), (1e-5, 9.0)])
+def test_same_rows_as_full_kernel(built, n, k, m, thr, lt, monkeypatch):
+    rng = np.random.default_rng(n + k + m)
+    pop, Z = structure(n, k, rng)
+    y = rng.standard_normal(n) + 0.5 * pop + 2.0
+    X = synth.pack_rows(awkward_rows(n, min(m, 4096), pop, y, rng))
+    X = np.ascontiguousarray(X[np.arange(m) % X.shape[0]])
+    a, b = both(X, np.linalg.qr(Z)[0], y, thr, lt, monkeypatch, "full")
+    assert a.n_tested == b.n_tested
+    assert np.array_equal(a.hits, b.hits)
+    if m > 2000:
+        assert b.hits.shape[0] > 0
+
+
+@pytest.mark.parametrize("tail", ["y", "U", "both", "scale"])
+@pytest.mark.parametrize("thr", [0.0, 0.1])
+def test_heavy_tails_and_missing_samples(built, tail, thr, monkeypatch):
+    """Columns whose largest value is far above the rest leave the limbs less
+    to hold the rest with; the bounds follow."""
+    n, k, m = 1200, 12, 30_000
+    rng = np.random.default_rng(len(tail))
+    keep = np.sort(rng.choice(n, n - n // 7, replace=False))
+    pop, Z = structure(n, k, rng)
+    if tail in ("U", "both"):
+        Z[:, 5:] = rng.standard_cauchy((n, k - 5))
+    y = rng.standard_cauchy(n) if tail in ("y", "both") else rng.standard_normal(n) + 0.5 * pop
+    U = np.linalg.qr(Z[keep])[0]
+    if tail == "scale":
+        U = U * 1.5  # not orthonormal: the general statistic
+        y = y * 1e-9
+    x = awkward_rows(n, m, pop, y, rng)
+    a, b = both(synth.pack_rows(x), U, y[keep], thr, 4.0, monkeypatch, "full", keep, n)
+    assert a.n_tested == b.n_tested
+    assert np.array_equal(a.hits, b.hits)

@@ -29,7 +29,7 @@ MERGE = os.path.join(BIN_DIR, "kgwas_index_merge")
 OBJ_DIR = os.path.join(PKG, "_build")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-LIB_SOURCES = ["kernels.cu", "kernel_ts.cu", "kernel_mp.cu", "kernel_tb.cu", "kernel_fs.cu", "kernel_mpb.cu", "kernel_mpb2.cu", "kernel_pairs.cu", "capi_pairs.cpp", "noalloc.cu", "probes.cu", "capi.cpp", "capi_multi.cpp", "prep.cpp"]
+LIB_SOURCES = ["kernels.cu", "kernel_ts.cu", "kernel_mp.cu", "kernel_tb.cu", "kernel_fs.cu", "kernel_fsp.cu", "kernel_mpb.cu", "kernel_mpb2.cu", "kernel_pairs.cu", "capi_pairs.cpp", "noalloc.cu", "probes.cu", "capi.cpp", "capi_multi.cpp", "prep.cpp"]
 CLI_SOURCES = ["kgwas_main.cpp", "kgwas_io.cpp"]
 CLI2_SOURCES = ["kgwas2d_main.cpp", "kgwas_io.cpp"]
 MERGE_SOURCES = ["index_merge_main.cpp", "kgwas_io.cpp"]
@@ -74,7 +74,9 @@ def build_lib(force=False, verbose=False, ptxas_verbose=False) -> str:
         return LIB
     os.makedirs(LIB_DIR, exist_ok=True)
     os.makedirs(OBJ_DIR, exist_ok=True)
-    base = [nvcc(), *ARCH, "-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC,-O3"]
+    # no traps or errno from host arithmetic: the quantiser's selects vectorise (prep.cpp)
+    base = [nvcc(), *ARCH, "-O3", "-std=c++17", "-lineinfo", "-Xcompiler",
+            "-fPIC,-O3,-fno-trapping-math,-fno-math-errno"]
     if ptxas_verbose:
         base.append("-Xptxas=-v")
     objs = [os.path.join(OBJ_DIR, os.path.splitext(s)[0] + ".o") for s in LIB_SOURCES]

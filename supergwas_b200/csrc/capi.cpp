@@ -82,12 +82,11 @@ int set_screen4(kg_ctx* ctx, const int32_t* sample_pos, int n_row) {
     if (!kg::fs_supported(N, kpad, wpk + (wpk & 1))) continue;
     kg::FsCols C;
     kg::make_fs_cols(p, sample_pos, n_row, lu, gate, C);
-    kg::FsPheno F;
+    kg::FsPheno& F = ctx->fsF;
     if (!kgctx::fill_fs(F, ctx->P, p, C, lu, gate)) continue;
     const size_t bytes = (size_t)kpad * N / 2;
-    std::vector<uint8_t> img(bytes + sizeof(F), 0);
+    std::vector<uint8_t> img(bytes, 0);
     kg::put_fs_image(C, 0, N, img.data());
-    std::memcpy(img.data() + bytes, &F, sizeof(F));
     dfree(ctx->dFs);
     KG_CUDA(cudaMalloc((void**)&ctx->dFs, img.size()), "cudaMalloc(screen)");
     KG_CUDA(cudaMemcpy(ctx->dFs, img.data(), img.size(), cudaMemcpyHostToDevice), "copy screen");
@@ -626,7 +625,7 @@ int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64
       L.lu = ctx->fs_lu;
       L.gate = ctx->P.corr_thr > 0.0;
       L.Bimg = ctx->dFs;
-      L.ph = reinterpret_cast<const kg::FsPheno*>(ctx->dFs + (size_t)ctx->fs_kpad * ctx->fs_N / 2);
+      L.F1 = &ctx->fsF;
       L.O1 = &O;
       L.num_sms = ctx->num_sms;
       e = kg::launch_fs(L, st);

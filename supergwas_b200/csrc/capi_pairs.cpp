@@ -177,11 +177,21 @@ int kg_pairs_run_host(kg_ctx* ctx, const uint64_t* xbits, uint64_t n_kmers, uint
   for (int attempt = 0; attempt < 8; ++attempt) {
     kg::DevOutPairs O{ctx->dCounters, ctx->dPairs, ctx->pair_cap, ctx->dCand, ctx->cand_cap, ctx->wait_ns};
     KG_CUDA(cudaMemsetAsync(ctx->dCounters, 0, 4 * sizeof(unsigned long long), st), "memset");
-    kg::LaunchPairs L{ctx->dPX, (int)wd, ctx->limbs.Kpad, ctx->prep.drop0 && ctx->P.k > 0, S, ctx->dBts, &ctx->P,
-                      &ctx->LM, &O, ctx->num_sms};
-    cudaError_t e = kg::launch_pairs(L, st);
-    if (e != cudaSuccess) return ctx->cuda_fail(e, "pair kernel launch");
-    kg::LaunchPairRefine R{ctx->dPX, (int)wd, ctx->dT, ctx->nsteps * 128, ctx->cm, &ctx->P, &O, ctx->num_sms};
+    // the 4-bit screen, unless another kernel is asked for
+    const char* force = std::getenv("KG_KERNEL");
+    const bool fs = ctx->fs_N && !force && kg::fsp_supported(ctx->fs_N, ctx->fs_lu, ctx->fs_kpad, (int)wd, ic);
+    cudaError_t e;
+    if (fs) {
+      kg::LaunchFsPairs L{ctx->dPX, (int)wd, ctx->fs_kpad, ctx->fs_N, ctx->fs_lu, ctx->P.corr_thr > 0.0, S, ctx->dFs,
+                          &ctx->fsF, &O, ctx->num_sms};
+      e = kg::launch_fs_pairs(L, st);
+    } else {
+      kg::LaunchPairs L{ctx->dPX, (int)wd, ctx->limbs.Kpad, ctx->prep.drop0 && ctx->P.k > 0, S, ctx->dBts, &ctx->P,
+                        &ctx->LM, &O, ctx->num_sms};
+      e = kg::launch_pairs(L, st);
+    }
+    kg::LaunchPairRefine R{ctx->dPX, (int)wd, ctx->dT, ctx->nsteps * 128, ctx->cm, &ctx->P, &O, ctx->num_sms, fs,
+                          &ctx->LM, ctx->dV};
     e = kg::launch_pair_refine(R, st);
     if (e != cudaSuccess) return ctx->cuda_fail(e, "pair refinement launch");
     ctx->launches = 2;

@@ -77,8 +77,7 @@ inline bool fill_fs(kg::FsPheno& F, const kg::EpiParams& P, const kg::Prepared& 
   if (!p.drop0 || p.k < 1 || !(std::fabs(P.a[0] * P.a[0] * p.n - 1.0) <= 1e-6) || p.n >= 65536 || !(P.ynorm >= 1e-12) || !(P.ynorm < 1e150) || !(yv > 1e-6) ||
       !(P.r2_cand >= r2_ref) || !(P.r2_cand < 1.0) || P.refine == 0)
     return false;
-  F.n = p.n;
-  F.ku = p.k - 1;
+  F.n = (float)p.n;
   F.inv_n = (float)(1.0 / p.n);
   const double cut = P.r2_cand * yv;
   F.cut = (float)(cut * (1.0 - 1e-4));
@@ -105,7 +104,7 @@ inline bool fill_fs(kg::FsPheno& F, const kg::EpiParams& P, const kg::Prepared& 
   for (int l = 0; l < 3; ++l) F.sy[l] = (float)(C.sy[l] / P.ynorm);
   if (gate)
     for (int l = 0; l < 4; ++l) F.sg[l] = (float)(C.sg[l] / P.ynorm);
-  for (int j = 0; j < F.ku; ++j)
+  for (int j = 0; j + 1 < p.k; ++j)
     for (int l = 0; l < lu; ++l) F.su[lu * j + l] = (float)C.su[(size_t)j * lu + l];
   return true;
 }
@@ -178,9 +177,10 @@ struct kg_ctx {
   int8_t* dB = nullptr;      // B image of the smem-A kernel
   int8_t* dBts = nullptr;    // B image of the TMEM-A kernels
   kg::MPheno* dPh1 = nullptr;  // the phenotype's constants for the streamed-image kernel
-  // 4-bit screen: image and, behind it, the phenotype's constants; columns (0:
-  // not used), limbs per U column, samples of the image
+  // 4-bit screen: image, the phenotype's constants; columns (0: not used), limbs
+  // per U column, samples of the image
   uint8_t* dFs = nullptr;
+  kg::FsPheno fsF{};
   int fs_N = 0, fs_lu = 0, fs_kpad = 0;
   int nchunk = 0;
   int f64_N = 0;             // limb columns of the FP64 form (dBts holds image and constants); 0: CUDA cores

@@ -602,25 +602,41 @@ __device__ __forceinline__ void table_row_sums(const uint64_t* __restrict__ row,
   constexpr int JW = (CM + 31) / 32;
 #pragma unroll
   for (int jj = 0; jj < JW; ++jj) acc[jj] = 0.0;
-  for (int w = 0; w < nwords; ++w) {
-    uint64_t bits = __ldg(row + w);  // one address for the whole warp
-    if (row2) bits &= __ldg(row2 + w);
-    const double* Tw = T + (size_t)w * (8 * 256 * CM);
-    double v[8][JW];
+  // Four words (32 loads) at a time where a lane has one column: a candidate is a
+  // chain of L2 latencies and a launch has few of them.  1e8 k-mers at n = 1000,
+  // r = 16+1: 23 us with one word at a time, 14 us now.  Two columns per lane
+  // (k > 30) gained nothing.  The sums are added in the same order.
+  constexpr int TRW = JW == 1 ? 4 : 1;
+  for (int w0 = 0; w0 < nwords; w0 += TRW) {
+    uint64_t bits[TRW];
 #pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      const unsigned b = (unsigned)(bits >> (8 * t)) & 255u;
-      const double* e = Tw + (size_t)(t * 256 + b) * CM;
+    for (int u = 0; u < TRW; ++u) {
+      const int w = w0 + u < nwords ? w0 + u : nwords - 1;
+      bits[u] = __ldg(row + w);  // one address for the whole warp
+      if (row2) bits[u] &= __ldg(row2 + w);
+      if (w0 + u >= nwords) bits[u] = 0;  // the entries of an empty byte are zero
+    }
+    double v[TRW][8][JW];
 #pragma unroll
-      for (int jj = 0; jj < JW; ++jj) {
-        const int j = lane + 32 * jj;
-        v[t][jj] = (j < CM) ? __ldg(e + j) : 0.0;
+    for (int u = 0; u < TRW; ++u) {
+      const double* Tw = T + (size_t)(w0 + u < nwords ? w0 + u : nwords - 1) * (8 * 256 * CM);
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        const unsigned b = (unsigned)(bits[u] >> (8 * t)) & 255u;
+        const double* e = Tw + (size_t)(t * 256 + b) * CM;
+#pragma unroll
+        for (int jj = 0; jj < JW; ++jj) {
+          const int j = lane + 32 * jj;
+          v[u][t][jj] = (j < CM) ? __ldg(e + j) : 0.0;
+        }
       }
     }
 #pragma unroll
-    for (int t = 0; t < 8; ++t)
+    for (int u = 0; u < TRW; ++u)
 #pragma unroll
-      for (int jj = 0; jj < JW; ++jj) acc[jj] += v[t][jj];
+      for (int t = 0; t < 8; ++t)
+#pragma unroll
+        for (int jj = 0; jj < JW; ++jj) acc[jj] += v[u][t][jj];
   }
 }
 
@@ -897,6 +913,27 @@ __device__ __forceinline__ void mp_emit(const DevOutMP& O, int p, unsigned long 
       atomicAdd(O.tested + (size_t)shard * O.n_pheno + p, (unsigned long long)__popc(tm & match));
   }
   mp_emit_rare(O, p, gk, shard, hit, cand, T, pv, effect);
+}
+
+// ------------------------------------------------------ pair schedule
+struct PairUnit {
+  unsigned long long jb, i0, i1;
+};
+// Unit u -> its j-block (the last block whose first unit is <= u) and i range.
+__device__ __forceinline__ PairUnit pr_unit(const PairSched& S, unsigned long long u) {
+  int lo = 0, hi = S.njb - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (S.unit_off[mid] <= u) lo = mid;
+    else hi = mid - 1;
+  }
+  PairUnit U;
+  U.jb = (unsigned long long)lo;
+  const unsigned long long jend = 128ull * (U.jb + 1) < S.n_kmers ? 128ull * (U.jb + 1) : S.n_kmers;
+  const unsigned long long ihi = S.row_end < jend - 1 ? S.row_end : jend - 1;
+  U.i0 = S.row_start + (u - S.unit_off[lo]) * S.ic;
+  U.i1 = U.i0 + S.ic < ihi ? U.i0 + S.ic : ihi;
+  return U;
 }
 
 }  // namespace kg

@@ -1,5 +1,7 @@
 // fs.cuh -- parts shared by the 4-bit screen kernels (kernel_fs.cu, kernel_fsp.cu).
 #pragma once
+#include <cstddef>
+
 #include "device.cuh"
 
 namespace kg {
@@ -72,55 +74,44 @@ __device__ __forceinline__ void fs_load(uint32_t taddr, uint32_t* d) {
 // are those factors, with room for the rounding of this arithmetic.
 // PAIRS: the columns of y - mean(y), if any, are not read; c = n is left open.
 template <int NP, int LU, bool GATE, bool PAIRS = false>
-__device__ __forceinline__ int fs_verdict(const FsPheno* __restrict__ F, const uint32_t* d, bool valid) {
-  const int4 h0 = __ldg(reinterpret_cast<const int4*>(F));
-  const float4 h1 = __ldg(reinterpret_cast<const float4*>(F) + 1);
-  const float4 h2 = __ldg(reinterpret_cast<const float4*>(F) + 2);
-  const float4 sy = __ldg(reinterpret_cast<const float4*>(F) + 3);
-  const int n = h0.x, ku = h0.y;
-  const float inv_n = __int_as_float(h0.z), cut = __int_as_float(h0.w);
-  const float b = h1.x, kappa = h1.y, thr = h1.z, bu = h1.w;
-  const float mu = h2.x, by = h2.y, my = h2.z;
+__device__ __forceinline__ int fs_verdict(const FsPheno& F, const uint32_t* d, bool valid) {
   auto f = [&](int i) { return __uint_as_float(d[i]); };
-  const float cf = f(0);
-  const int c = (int)cf;
-  const float ey = fmaf(f(3), sy.z, fmaf(f(2), sy.y, f(1) * sy.x));
-  float ss = 0.0f;
   constexpr int U0 = 4 + (GATE ? 4 : 0), KU = (NP - U0) / LU;
+  const float cf = f(0);
+  float s2[2] = {0.0f, 0.0f};
 #pragma unroll
-  for (int j0 = 0; j0 < KU; j0 += 4 / LU) {
-    // slots past the U columns hold zero limbs and zero scales: fewer than 8 / LU
-    if (j0 > KU - 8 / LU && j0 >= ku) break;
-    const float4 s4 = __ldg(reinterpret_cast<const float4*>(F->su) + j0 * LU / 4);
-    const float s[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-    for (int t = 0; t < 4 / LU; ++t) {
-      const int o = U0 + LU * (j0 + t);
-      if (j0 + t < KU) {
-        const float e = LU == 2 ? fmaf(f(o + LU - 1), s[LU * t + LU - 1], f(o) * s[LU * t]) : f(o) * s[t];
-        ss = fmaf(e, e, ss);
-      }
-    }
+  for (int j = 0; j < KU; ++j) {  // slots past the U columns hold zero limbs and zero scales
+    const int o = U0 + LU * j;
+    const float e = LU == 2 ? fmaf(f(o + LU - 1), F.su[LU * j + LU - 1], f(o) * F.su[LU * j]) : f(o) * F.su[j];
+    s2[j & 1] = fmaf(e, e, s2[j & 1]);
   }
-  if (!(valid && c > 0 && (PAIRS || c < n))) return 0;
-  const float xcn = (float)(c * (n - c)) * inv_n;
+  const float xcn = cf * (F.n - cf) * F.inv_n;
   float nx, rs;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(nx) : "f"(xcn));
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(rs) : "f"(ss));
-  bool open = false;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(nx) : "f"(xcn));
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(s2[0] + s2[1]));
+  bool in = valid && cf > 0.0f && (PAIRS || cf < F.n), open = false;
   if (GATE && !PAIRS) {
-    const float4 sg = __ldg(reinterpret_cast<const float4*>(F) + 4);
-    const float bg = h2.w, mg = sy.w;
-    const float eg = fmaf(f(7), sg.w, fmaf(f(6), sg.z, fmaf(f(5), sg.y, f(4) * sg.x)));
-    const float q = fabsf(fmaf(kappa, cf, eg)), err = fmaf(bg, nx, mg * cf), t = thr * nx;
-    if (q + err < t) return 0;
+    const float eg = fmaf(f(7), F.sg[3], fmaf(f(6), F.sg[2], fmaf(f(5), F.sg[1], f(4) * F.sg[0])));
+    const float q = fabsf(fmaf(F.kappa, cf, eg)), err = fmaf(F.bg, nx, F.mg * cf), t = F.thr * nx;
+    in = in && !(q + err < t);
     open = !(q - err > t);
   }
-  const float root = rs + fmaf(bu, nx, mu * cf);
+  const float root = rs + fmaf(F.bu, nx, F.mu * cf);
   const float low = fmaf(-root, root, xcn);  // xxM is at least this
-  const float y = fabsf(fmaf(b, cf, ey)) + fmaf(by, nx, my * cf);
-  const bool below = xcn > 0.0f && low >= 1e-3f * xcn && y * y < cut * low;
-  return open ? 3 : below ? 1 : 2;
+  const float ey = fmaf(f(3), F.sy[2], fmaf(f(2), F.sy[1], f(1) * F.sy[0]));
+  const float y = fabsf(fmaf(F.b, cf, ey)) + fmaf(F.by, nx, F.my * cf);
+  const bool below = xcn > 0.0f && low >= 1e-3f * xcn && y * y < F.cut * low;
+  return !in ? 0 : open ? 3 : below ? 1 : 2;
+}
+// The constants that fs_verdict<NP, LU, GATE> reads, in registers.
+template <int NP, int LU, bool GATE>
+__device__ __forceinline__ void fs_constants(const FsPheno* __restrict__ F, FsPheno& R) {
+  constexpr int U0 = 4 + (GATE ? 4 : 0), HEAD = (int)(offsetof(FsPheno, su) / 16), NV = ((NP - U0) / LU * LU + 3) / 4;
+#pragma unroll
+  for (int i = 0; i < HEAD + NV; ++i) {
+    if (!GATE && i == HEAD - 1) continue;  // sg
+    reinterpret_cast<float4*>(&R)[i] = __ldg(reinterpret_cast<const float4*>(F) + i);
+  }
 }
 
 // Appends the lanes with `take` to the candidate list (warp-aggregated).

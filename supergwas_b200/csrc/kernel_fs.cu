@@ -66,8 +66,8 @@ __host__ __device__ inline FsSmem fs_smem(int b_bytes, int xst, int rb) {
 template <int NP, int PPG, int LU, bool GATE, bool MANY>
 __global__ void __launch_bounds__(fs_threads(NP * PPG), 1)
     fs_kernel(const __grid_constant__ CUtensorMap tmap, unsigned long long m, int nunit, int G, int bt, int xst, int rb,
-              const uint8_t* __restrict__ Bimg, int b_bytes, const FsPheno* __restrict__ ph, const DevOutMP O,
-              const DevOut O1) {
+              const uint8_t* __restrict__ Bimg, int b_bytes, const __grid_constant__ FsPheno F1,
+              const FsPheno* __restrict__ ph, const DevOutMP O, const DevOut O1) {
   constexpr int N = NP * PPG;
   constexpr int NSLOT = fs_nslot(N);
   constexpr int SF0 = 512 - FS_SF, A0 = SF0 - NSLOT * 128;
@@ -338,8 +338,24 @@ __global__ void __launch_bounds__(fs_threads(NP * PPG), 1)
     const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + e * N;
     uint32_t item = 0, jt = 0, tested_local = 0;
     bool ok = true;
+    // MANY: tested counts of the group's phenotypes in the shard of k-mers
+    // [s_lo, s_hi) (one atomic per item and phenotype, after a match of the
+    // lanes' shards, took a quarter of the kernel's time)
+    uint32_t cnt[PPG] = {};
+    int shard = 0;
+    unsigned long long s_lo = 1, s_hi = 0;
+    auto flush = [&](int g) {
+#pragma unroll
+      for (int pp = 0; pp < PPG; ++pp) {
+        const unsigned tot = __reduce_add_sync(0xffffffffu, cnt[pp]);
+        const int p = g * PPG + pp;
+        if (lane == 0 && tot && p < O.n_pheno)
+          atomicAdd(O.tested + (size_t)shard * O.n_pheno + p, (unsigned long long)tot);
+        cnt[pp] = 0;
+      }
+    };
     for (uint32_t i0 = 0; i0 < mine && ok; i0 += bt)
-      for (int g = 0; g < G && ok; ++g)
+      for (int g = 0; g < G && ok; ++g) {
         for (uint32_t i = i0; i < mine && i < i0 + bt; ++i, ++item) {
           if ((item & 1u) != e) continue;
           if (!__all_sync(0xffffffffu, wait_or_abort(acc_full + 8 * e, jt & 1u, s_abort, counters, ERR_TIMEOUT_MMA,
@@ -351,12 +367,18 @@ __global__ void __launch_bounds__(fs_threads(NP * PPG), 1)
           tc_fence_after();
           const unsigned long long local = (unsigned long long)(blockIdx.x + i * gridDim.x) * FS_TM + r;
           const bool valid = local < m;
-          int shard = 0;
           uint32_t wt = 1u;
+          bool same = true;  // the warp's rows lie in one shard, whose counts stay in registers
           if (MANY) {
-            const unsigned long long gk = O.kmer_offset + local;
-            shard = mp_shard(O, valid ? gk : O.kmer_offset);
-            if (O.weight && valid) wt = O.weight[gk];
+            const unsigned long long w0 = O.kmer_offset + local - lane, end = O.kmer_offset + m;
+            if (w0 < end && !(w0 >= s_lo && w0 < s_hi)) {
+              flush(g);
+              shard = mp_shard(O, w0);
+              s_lo = w0;
+              s_hi = shard + 1 < O.n_shards ? O.shard_start[shard + 1] : ~0ull;
+            }
+            same = w0 + 32 <= s_hi || end <= s_hi;
+            if (O.weight && valid) wt = O.weight[O.kmer_offset + local];
           }
 #pragma unroll
           for (int pp = 0; pp < PPG; ++pp) {
@@ -369,19 +391,26 @@ __global__ void __launch_bounds__(fs_threads(NP * PPG), 1)
             }
             const int p = g * PPG + pp;
             if (MANY && p >= O.n_pheno) continue;  // warp-uniform
-            const int v = fs_verdict<NP, LU, GATE>(ph + p, d, valid);
             if constexpr (MANY) {
-              tb_count(O, p, shard, v == 1 || v == 2 ? wt : 0u);
+              FsPheno F;
+              fs_constants<NP, LU, GATE>(ph + p, F);
+              const int v = fs_verdict<NP, LU, GATE>(F, d, valid);
+              const uint32_t t = v == 1 || v == 2 ? wt : 0u;
+              if (same) cnt[pp] += t;
+              else tb_count(O, p, mp_shard(O, valid ? O.kmer_offset + local : O.kmer_offset), t);
               if (__any_sync(0xffffffffu, v >= 2))
                 fs_push(counters, O.cand, O.cand_cap, v >= 2,
                         (O.kmer_offset + local) | ((unsigned long long)p << 48) | (v == 3 ? CAND_OPEN_MP : 0ull));
             } else {
+              const int v = fs_verdict<NP, LU, GATE>(F1, d, valid);
               if (v == 1 || v == 2) tested_local += O1.weight ? O1.weight[O1.kmer_offset + local] : 1u;
               if (__any_sync(0xffffffffu, v >= 2))
                 fs_push(counters, O1.cand, O1.cand_cap, v >= 2, (O1.kmer_offset + local) | (v == 3 ? CAND_OPEN : 0ull));
             }
           }
         }
+        if (MANY) flush(g);
+      }
     if (!MANY) flush_tested(O1, tested_local);
   }
   __syncthreads();
@@ -431,7 +460,7 @@ static cudaError_t launch_fs_t(const LaunchFs& L, const CUtensorMap& tm, cudaStr
   else O1 = *L.O1;
   const int bt = L.G == 1 ? 1 << 30 : L.bt;
   fs_kernel<NP, PPG, LU, GATE, MANY><<<grid, fs_threads(N), smem, st>>>(tm, L.m, L.kpad / FS_UNIT, L.G, bt, xst, rb,
-                                                                      L.Bimg, b_bytes, L.ph, O, O1);
+                                                                      L.Bimg, b_bytes, MANY ? FsPheno() : *L.F1, L.ph, O, O1);
   return cudaGetLastError();
 }
 

@@ -67,26 +67,6 @@ __host__ __device__ inline PrSmem pr_smem(int b_bytes, int xst, bool ibox) {
   return L;
 }
 
-struct PairUnit {
-  unsigned long long jb, i0, i1;
-};
-// Unit u -> its j-block (the last block whose first unit is <= u) and i range.
-__device__ __forceinline__ PairUnit pr_unit(const PairSched& S, unsigned long long u) {
-  int lo = 0, hi = S.njb - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (S.unit_off[mid] <= u) lo = mid;
-    else hi = mid - 1;
-  }
-  PairUnit U;
-  U.jb = (unsigned long long)lo;
-  const unsigned long long jend = 128ull * (U.jb + 1) < S.n_kmers ? 128ull * (U.jb + 1) : S.n_kmers;
-  const unsigned long long ihi = S.row_end < jend - 1 ? S.row_end : jend - 1;
-  U.i0 = S.row_start + (u - S.unit_off[lo]) * S.ic;
-  U.i1 = U.i0 + S.ic < ihi ? U.i0 + S.ic : ihi;
-  return U;
-}
-
 // Warp-aggregated pair records and refinement candidates, one pair per lane.
 __device__ __forceinline__ void pr_emit(const DevOutPairs& O, unsigned long long i, unsigned long long j, bool hit,
                                         bool cand, double T, double p, double effect) {
@@ -474,13 +454,51 @@ __global__ void __launch_bounds__(pr_threads(N), 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
+// xxM of a product row as pairs_kernel has it (drop0): the column sums over the
+// values that the limbs hold -- integers times the column's scale, so exact in
+// any order -- squared in the order of its epilogue.  V: the FP64 columns.
+template <int CM>
+__device__ __noinline__ double pr_split_xxM(const EpiParams& P, const LimbMap& LM, const double* __restrict__ V,
+                                            const uint64_t* __restrict__ ri, const uint64_t* __restrict__ rj,
+                                            int nwords, int lane, int c) {
+  constexpr int JW = (CM + 31) / 32;
+  double e[JW];
+#pragma unroll
+  for (int jj = 0; jj < JW; ++jj) {
+    e[jj] = 0.0;
+    const int col = lane + 32 * jj;  // V: the count, then U column col - 1
+    if (col < 2 || col > P.k) continue;
+    const double scale = LM.scale[col - 1], up = 1.0 / scale;  // a power of two
+    double sum = 0.0;
+    for (int w = 0; w < nwords; ++w)
+      for (uint64_t bits = ri[w] & rj[w]; bits; bits &= bits - 1)
+        sum += round(V[(size_t)(64 * w + __ffsll((long long)bits) - 1) * CM + col] * up);
+    e[jj] = sum * scale;
+  }
+  const double cd = (double)c, s0 = P.a[0] * cd;
+  double ss = s0 * s0;
+#pragma unroll
+  for (int jj = 0; jj < JW; ++jj)
+    for (int l = 0; l < 32; ++l) {
+      const double ej = __shfl_sync(0xffffffffu, e[jj], l);
+      const int col = l + 32 * jj;
+      if (col < 2 || col > P.k) continue;
+      const double sj = fma(P.a[col - 1], cd, ej);
+      ss = fma(sj, sj, ss);
+    }
+  return cd - ss;
+}
+
 // FP64 recomputation of the pair candidates: one warp per pair, column sums
 // of x_i * x_j from the byte tables of V (table_row_sums on the AND of the
-// two rows), then compute_hit in FP64 (src/kgwas_2d.cpp:300-318).
+// two rows), then compute_hit in FP64 (src/kgwas_2d.cpp:300-318).  count: the
+// candidates have not been counted as evaluated yet (the 4-bit screen's).
 template <int CM>
 __global__ void __launch_bounds__(256) pr_refine_kernel(const uint64_t* __restrict__ x, int wpk, int nwords,
                                                         const double* __restrict__ T,
-                                                        const __grid_constant__ EpiParams P, const DevOutPairs O) {
+                                                        const __grid_constant__ EpiParams P, const DevOutPairs O,
+                                                        bool count, const __grid_constant__ LimbMap LM,
+                                                        const double* __restrict__ V) {
   const int lane = threadIdx.x & 31;
   const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
   unsigned long long ncand = O.counters[3];
@@ -494,9 +512,17 @@ __global__ void __launch_bounds__(256) pr_refine_kernel(const uint64_t* __restri
     int c;
     double ss, ey;
     refine_reduce<CM>(P, acc, lane, c, ss, ey);
+    double split_xxM = (double)c - ss;
+    // Whether a pair counts as evaluated is a matter of the limb sums (kernels
+    // of LimbMap columns), which differ where xxM is rounding: products in the
+    // span of U
+    if (count && !(split_xxM >= 0.02 * (double)c * (double)(P.n - c) / (double)P.n))
+      split_xxM = pr_split_xxM<CM>(P, LM, V, x + i * (unsigned long long)wpk, x + j * (unsigned long long)wpk, nwords,
+                                   lane, c);
     if (lane == 0) {
       const double eps = 1e-12;
       const double xxM = (double)c - ss, xyM = P.b * (double)c + ey;
+      if (count && c > 0 && split_xxM > eps && P.yyM > eps) atomicAdd(O.counters, 1ull);
       if (c > 0 && xxM > eps && P.yyM > eps) {
         double r2 = (xyM * xyM) / (xxM * P.yyM);
         if (r2 < 0) r2 = 0;
@@ -608,7 +634,7 @@ static cudaError_t launch_pr_refine_t(const LaunchPairRefine& L, cudaStream_t st
       (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pr_refine_kernel<CM>, 256, 0) != cudaSuccess ||
        per_sm < 1))
     per_sm = 1;
-  pr_refine_kernel<CM><<<(unsigned)(L.num_sms * per_sm), 256, 0, st>>>(L.x, L.wpk, L.vrows / 64, L.T, *L.P, *L.O);
+  pr_refine_kernel<CM><<<(unsigned)(L.num_sms * per_sm), 256, 0, st>>>(L.x, L.wpk, L.vrows / 64, L.T, *L.P, *L.O, L.count, *L.LM, L.V);
   return cudaGetLastError();
 }
 

@@ -118,7 +118,8 @@ struct LaunchFs {
   bool gate;                  // the columns hold y - mean(y)
   int bt;                     // tiles of a CTA per pass over the groups (G > 1)
   const uint8_t* Bimg;        // G images of kpad * NP * PPG / 2 bytes (put_fs_image; device)
-  const FsPheno* ph;          // per-phenotype constants (device)
+  const FsPheno* F1;          // one phenotype: its constants (host)
+  const FsPheno* ph;          // many: per-phenotype constants (device)
   const DevOutMP* O;
   const DevOut* O1;
   int num_sms;
@@ -205,7 +206,25 @@ struct LaunchPairRefine {
   const EpiParams* P;
   const DevOutPairs* O;
   int num_sms;
+  bool count;                 // the candidates are not counted as evaluated yet (4-bit screen)
+  const LimbMap* LM;          // with count: the int8 limb columns,
+  const double* V;            // and the FP64 columns, vrows x cm
 };
+// The pair test with the 4-bit screen (kernel_fsp.cu).
+struct LaunchFsPairs {
+  const uint64_t* x;          // packed rows (device), 16-byte aligned, wpk >= 16
+  int wpk;
+  int kpad;                   // samples of the image (multiple of 256)
+  int N, lu;                  // its columns and limbs per U column
+  bool gate;                  // it holds y - mean(y)
+  PairSched S;
+  const uint8_t* Bimg;
+  const FsPheno* F;           // host
+  const DevOutPairs* O;
+  int num_sms;
+};
+bool fsp_supported(int N, int lu, int kpad, int wpk, unsigned long long ic);
+cudaError_t launch_fs_pairs(const LaunchFsPairs& L, cudaStream_t st);
 bool pairs_supported(int N, int limbs_u, int limbs_y, int kpad, int wpk);
 cudaError_t launch_pairs(const LaunchPairs& L, cudaStream_t st);
 cudaError_t launch_pair_refine(const LaunchPairRefine& L, cudaStream_t st);

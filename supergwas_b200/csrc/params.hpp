@@ -110,8 +110,8 @@ inline void set_screen64(EpiParams& P, const LimbMap& L, bool drop0) {
 // Constants of one phenotype for the 4-bit screen (kernel_fs.cu); everything
 // about y is relative to ynorm.
 struct alignas(16) FsPheno {
-  int n, ku;              // samples; U columns with limbs
-  float inv_n, cut;       // 1 / n; lowest r2 of an emitted row x yyM / ynorm^2
+  float n, inv_n;         // samples
+  float cut, pad;         // lowest r2 of an emitted row x yyM / ynorm^2
   float b, kappa, thr;    // b / ynorm, kappa / ynorm, the correlation threshold
   float bu, mu;           // bounds of what the limbs leave out (fs_verdict): U columns,
   float by, my, bg;       // y' and

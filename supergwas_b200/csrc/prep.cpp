@@ -232,11 +232,14 @@ void make_b_image(const LimbCols& L, int KC, std::vector<int8_t>& img) {
 }
 
 // ------------------------------------------------------------ 4-bit screen
-// Nearest e2m1 value of t (|t| above 6 becomes 6).
+// Nearest integer (|t| < 2^22), in two additions that vectorise.
+static inline float near_int(float t) { return (t + 12582912.0f) - 12582912.0f; }
+// Nearest e2m1 value of t (|t| above 6 becomes 6), without branches.
 static inline float e2m1_round(float t) {
-  const float a = std::fabs(t);
-  const float r = a < 2.0f ? std::rint(a * 2.0f) * 0.5f : a < 4.0f ? std::rint(a) : std::min(std::rint(a * 0.5f) * 2.0f, 6.0f);
-  return std::copysign(r, t);
+  const float a = std::min(std::fabs(t), 6.0f);
+  const float h = near_int(a * 2.0f) * 0.5f, w = near_int(a), d = near_int(a * 0.5f) * 2.0f;
+  const float ge2 = a >= 2.0f ? 1.0f : 0.0f, ge4 = a >= 4.0f ? 1.0f : 0.0f;
+  return std::copysign(h + (w - h) * ge2 + (d - w) * ge4, t);
 }
 static inline uint8_t e2m1_code(float v) {
   const int h = (int)(std::fabs(v) * 2.0f);  // 0 1 2 3 4 6 8 12
@@ -245,7 +248,7 @@ static inline uint8_t e2m1_code(float v) {
 }
 
 // Moves codes of the last limb (scale s) to a neighbouring value, where that adds
-// least to the residual r, until the residual's sum is as close to zero as one
+// little to the residual r, until the residual's sum is as close to zero as one
 // such step allows.  A row of frequency near one meets the sum: the rest of the
 // bound shrinks with ||x - mean(x)||, c |sum r| / n does not.
 static void fs_balance(std::vector<double>& r, const int* pos, uint8_t* code, double s) {
@@ -253,32 +256,20 @@ static void fs_balance(std::vector<double>& r, const int* pos, uint8_t* code, do
   const int n = (int)r.size();
   double D = 0;
   for (double v : r) D += v;
-  const int dir = D > 0 ? 1 : -1;  // a positive sum: larger limbs
-  struct Move {
-    double cost, step;
-    int i;
-    uint8_t to;
-  };
-  std::vector<Move> mv;
-  mv.reserve(n);
-  for (int i = 0; i < n; ++i) {
-    const uint8_t c = code[pos ? pos[i] : i];
-    const int at = (c & 8) ? -(c & 7) : (c & 7), to = at + dir;
-    if (to > 7 || to < -7) continue;
-    const float q = at < 0 ? -val[-at] : val[at], q2 = to < 0 ? -val[-to] : val[to];
-    const double step = s * (double)(q2 - q), moved = r[i] - step;
-    mv.push_back({(moved * moved - r[i] * r[i]) / std::fabs(step), step, i, (uint8_t)(to < 0 ? 8 | -to : to)});
-  }
-  // steps of s / 2 at least: no more than this many
-  const size_t most = std::min(mv.size(), (size_t)std::min(4.0 * std::fabs(D) / s + 16.0, (double)n));
-  std::partial_sort(mv.begin(), mv.begin() + most, mv.end(),
-                    [](const Move& a, const Move& b) { return a.cost < b.cost || (a.cost == b.cost && a.i < b.i); });
-  for (size_t t = 0; t < most; ++t) {
-    const Move& m = mv[t];
-    if (std::fabs(D - m.step) >= std::fabs(D)) continue;
-    D -= m.step;
-    r[m.i] -= m.step;
-    code[pos ? pos[m.i] : m.i] = m.to;
+  // in units of s; passes over the entries, the nearest to a tie first
+  for (float most : {0.02f, 0.1f, 0.3f, 1.0f, 8.0f}) {
+    for (int i = 0; i < n && std::fabs(D) > 0.25 * s; ++i) {
+      const int dir = D > 0 ? 1 : -1;  // a positive sum: larger limbs
+      uint8_t& c = code[pos ? pos[i] : i];
+      const int at = (c & 8) ? -(c & 7) : (c & 7), to = at + dir;
+      if (to > 7 || to < -7) continue;
+      const float q = at < 0 ? -val[-at] : val[at], q2 = to < 0 ? -val[-to] : val[to];
+      const double step = s * (double)(q2 - q), moved = r[i] - step;
+      if (!(moved * moved - r[i] * r[i] <= most * s * s) || std::fabs(D - step) >= std::fabs(D)) continue;
+      D -= step;
+      r[i] = moved;
+      c = (uint8_t)(to < 0 ? 8 | -to : to);
+    }
   }
 }
 
@@ -290,8 +281,10 @@ static void fs_balance(std::vector<double>& r, const int* pos, uint8_t* code, do
 // (the wider steps above would leave it a few large values, and the rest to
 // round to zero).
 static void fs_limbs(std::vector<double>& r, const int* pos, int nl, uint8_t* code, size_t stride, double* scale) {
-  const int n = (int)r.size();
+  const int n = (int)r.size(), n16 = (n + 15) / 16 * 16;
+  std::vector<float> rf((size_t)n16, 0.0f);  // zeros past the end leave nothing
   for (int l = 0; l < nl; ++l, code += stride) {
+    for (int i = 0; i < n; ++i) rf[i] = (float)r[i];
     double mx = 0;
     for (double v : r) mx = std::max(mx, std::fabs(v));
     scale[l] = 0.0;
@@ -303,21 +296,26 @@ static void fs_limbs(std::vector<double>& r, const int* pos, int nl, uint8_t* co
       for (double f : {1.0, 0.8, 0.6}) {
         const float up = (float)(6.0 / (f * mx));
         const double s = 1.0 / (double)up;
-        double err[4] = {0, 0, 0, 0};
-        for (int i = 0; i < n; ++i) {
-          const double d = r[i] - s * (double)e2m1_round((float)r[i] * up);
-          err[i & 3] += d * d;
-        }
-        const double e = err[0] + err[1] + err[2] + err[3];
+        float err[16] = {};
+        for (int i = 0; i + 16 <= n16; i += 16)
+          for (int t = 0; t < 16; ++t) {
+            const float v = rf[i + t] * up, d = v - e2m1_round(v);
+            err[t] += d * d;
+          }
+        double e = 0;
+        for (int t = 0; t < 16; ++t) e += err[t];
+        e *= s * s;
         if (e < best_err) best_err = e, best = s;
       }
     }
     const float up = (float)(1.0 / best);
+    for (int i = 0; i < n16; ++i) {
+      const float t = rf[i] * up;
+      rf[i] = nearest ? e2m1_round(t) : std::max(-4.0f, std::min(4.0f, near_int(t)));
+    }
     for (int i = 0; i < n; ++i) {
-      const float t = (float)r[i] * up;
-      const float q = nearest ? e2m1_round(t) : std::max(-4.0f, std::min(4.0f, std::rint(t)));
-      code[pos ? pos[i] : i] = e2m1_code(q);
-      r[i] -= best * (double)q;
+      code[pos ? pos[i] : i] = e2m1_code(rf[i]);
+      r[i] -= best * (double)rf[i];
     }
     scale[l] = best;
     if (l + 1 == nl) fs_balance(r, pos, code, best);

@@ -71,3 +71,61 @@ def test_heavy_tails_and_missing_samples(built, tail, thr, monkeypatch):
     a, b = both(synth.pack_rows(x), U, y[keep], thr, 4.0, monkeypatch, "full", keep, n)
     assert a.n_tested == b.n_tested
     assert np.array_equal(a.hits, b.hits)
+
+
+@pytest.mark.parametrize("thr,lt", [(0.0, 6.0), (0.2, 4.0)])
+@pytest.mark.parametrize("n,ks,np_", [(900, (12, 15), 5), (2000, (21, 3), 7), (1030, (5, 6), 17), (5000, (33, 30), 3),
+                                      (300, (2, 3), 8)], ids=lambda v: str(v))
+def test_many_phenotypes(built, n, ks, np_, thr, lt, monkeypatch):
+    """Phenotypes of different widths and samples in one launch, several and
+    single tiles per pass over the groups, shards that start inside a tile."""
+    rng = np.random.default_rng(n + np_)
+    pop, Z = structure(n, max(ks), rng)
+    y0 = rng.standard_normal(n) + 0.5 * pop
+    x = awkward_rows(n, 4096, pop, y0, rng)
+    X = synth.pack_rows(np.concatenate([x] * 10)[:40_003], max(16, synth.words_per_kmer(n)))
+    phenos = []
+    for p in range(np_):
+        keep = np.sort(rng.choice(n, n - p * n // 40, replace=False))
+        U = np.linalg.qr(Z[keep][:, :ks[p % 2]])[0]
+        phenos.append((U, (y0 + 0.3 * rng.standard_normal(n))[keep], keep))
+    shards = np.array([0, 7, 100, 100, 20_000, 39_990], dtype=np.uint64)
+    monkeypatch.setenv("KG_DEDUP", "0")
+    out = []
+    for kern, bt in (("mp", None), (None, None), (None, "1"), (None, "3")):
+        for var, val in (("KG_MP_KERNEL", kern), ("KG_MP_BT", bt)):
+            monkeypatch.setenv(var, val) if val else monkeypatch.delenv(var, raising=False)
+        with api.Kgwas(corr_threshold=thr, log10_thresh=lt) as g:
+            g.set_phenotypes(phenos, n)
+            out.append(g.run_multi_host(X, shards))
+            assert (g.multi_shape()["kernel"] == "4-bit screen (fs)") == (kern is None)
+            if kern is None and bt is None:
+                monkeypatch.setenv("KG_DEDUP", "1")
+                out.append(g.run_multi_host(X, shards))
+                monkeypatch.setenv("KG_DEDUP", "0")
+    assert out[0][1].shape[0] > 0
+    for tested, hits in out[1:]:
+        assert np.array_equal(tested, out[0][0])
+        assert np.array_equal(hits, out[0][1])
+
+
+@pytest.mark.parametrize("n,k,m", [(1000, 17, 700), (300, 4, 1501), (2000, 21, 400), (1024, 9, 130)],
+                         ids=lambda v: str(v))
+@pytest.mark.parametrize("thr", [0.0, 0.2])
+def test_pairs(built, n, k, m, thr, monkeypatch):
+    rng = np.random.default_rng(n + m)
+    pop, Z = structure(n, k, rng)
+    y = rng.standard_normal(n) + 0.5 * pop
+    x = awkward_rows(n, m, pop, y, rng)
+    x[10:13] = 1  # products of all ones
+    X = synth.pack_rows(x)
+    with api.Kgwas(corr_threshold=thr, log10_thresh=4.0) as g:
+        g.set_structure(np.linalg.qr(Z)[0], y)
+        for r0, r1 in ((0, m), (m // 3, m // 3 + 33)):
+            monkeypatch.delenv("KG_KERNEL", raising=False)
+            a, ea = g.run_pairs_host(X, r0, r1)
+            monkeypatch.setenv("KG_KERNEL", "full")
+            b, eb = g.run_pairs_host(X, r0, r1)
+            assert ea == eb
+            assert np.array_equal(a, b)
+        assert b.shape[0] > 0 or r1 < m

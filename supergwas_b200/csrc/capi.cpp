@@ -300,6 +300,7 @@ int kg_set_structure_ex(kg_ctx* ctx, const double* U, int n, int k, const double
       LM.scale[j] = ctx->limbs.scale[j];
     }
     kg::set_limb_consts(LM);
+    kg::set_gate_unit(P, LM, p.drop0 && k > 0);
     if (ctx->opts.limbs_u == 3 && ctx->opts.limbs_y == 5) kg::set_screen(P, LM, p.drop0 && k > 0);
     dfree(ctx->dB);
     KG_CUDA(cudaMalloc((void**)&ctx->dB, img.size()), "cudaMalloc(B)");
@@ -649,7 +650,7 @@ int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64
   if (e != cudaSuccess) return ctx->cuda_fail(e, "kernel launch");
   ++ctx->launches;
   if (ctx->P.refine) {
-    kg::LaunchFp64 R{dx, m, (int)wpk, ctx->dV, ctx->nsteps, ctx->cm, &ctx->P, &O, ctx->num_sms, ctx->dT};
+    kg::LaunchFp64 R{dx, m, (int)wpk, ctx->dV, ctx->nsteps, ctx->cm, &ctx->P, &O, ctx->num_sms, ctx->dT, &ctx->LM};
     e = kg::launch_refine(R, st);
     if (e != cudaSuccess) return ctx->cuda_fail(e, "refinement launch");
     ++ctx->launches;

@@ -426,6 +426,7 @@ int kg_set_phenotypes(kg_ctx* ctx, const kg_pheno* ph, int np, int n_row) {
     }
     kg::set_limb_consts(LM);
     mph[p].drop0 = (k > 0 && prep[p].drop0) ? 1 : 0;
+    kg::set_gate_unit(mph[p].P, LM, mph[p].drop0 != 0);
     kg::set_screen(mph[p].P, LM, mph[p].drop0 != 0);
   }
   // FP64 refinement operands: per phenotype, rows = packed-row sample positions,

@@ -100,7 +100,7 @@ inline bool fill_fs(kg::FsPheno& F, const kg::EpiParams& P, const kg::Prepared& 
   F.by = (float)by;
   F.my = (float)(C.my * up / P.ynorm + tiny);
   F.bg = (float)bg;
-  F.mg = (float)(C.mg * up / P.ynorm + tiny);
+  F.mg = (float)((C.mg + 1.01 * P.gate_unit) * up / P.ynorm + tiny);  // the limb sums decide alike outside it
   for (int l = 0; l < 3; ++l) F.sy[l] = (float)(C.sy[l] / P.ynorm);
   if (gate)
     for (int l = 0; l < 4; ++l) F.sg[l] = (float)(C.sg[l] / P.ynorm);

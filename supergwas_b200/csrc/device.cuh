@@ -640,21 +640,72 @@ __device__ __forceinline__ void table_row_sums(const uint64_t* __restrict__ row,
   }
 }
 
-// Correlation gate of a refinement candidate in FP64 from its lane-distributed
-// column sums (refine_reduce); identical in every lane.
+// The column sums of a row (of a product of two, with row2) over the values that
+// the int8 limbs hold: integers times the column's scale, so exact in any order
+// and equal to the recombined limb sums.  V: the FP64 columns, nwords * 64 rows;
+// scale[j]: limb scale of U column j, of y' at k.  For the candidates whose
+// outcome turns on the roundings of the limbs.
 template <int CM>
-__device__ __forceinline__ bool refine_gate(const EpiParams& P, const double (&acc)[(CM + 31) / 32], int lane, int c,
-                                            double ey) {
-  double gs = 0.0;
+__device__ __noinline__ void split_columns(int k, const double* scale, const double* __restrict__ V,
+                                           const uint64_t* __restrict__ row, const uint64_t* __restrict__ row2,
+                                           int nwords, int lane, double (&e)[(CM + 31) / 32]) {
 #pragma unroll
   for (int jj = 0; jj < (CM + 31) / 32; ++jj) {
+    e[jj] = 0.0;
+    const int col = lane + 32 * jj;  // the count, U column col - 1, y' at k + 1
+    if (col < 2 || col > k + 1) continue;
+    const double sc = scale[col - 1], up = 1.0 / sc;  // powers of two
+    double sum = 0.0;
+    for (int w = 0; w < nwords; ++w) {
+      const uint64_t bits = row2 ? row[w] & row2[w] : row[w];
+      const double* v = V + (size_t)(64 * w) * CM + col;
+      for (int b = 0; b < 64; b += 16) {
+        double t[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) t[i] = __ldg(v + (size_t)(b + i) * CM);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sum += (bits >> (b + i)) & 1u ? round(t[i] * up) : 0.0;
+      }
+    }
+    e[jj] = sum * sc;
+  }
+}
+
+// Correlation gate of a refinement candidate, identical in every lane: from its
+// FP64 column sums (refine_reduce), or, where those are so near the threshold
+// that the roundings of the limbs decide (P.gate_unit), from the limb sums in the
+// expressions of the int8 kernels.
+template <int CM>
+__device__ __forceinline__ bool refine_gate(const EpiParams& P, const LimbMap& LM, const double* __restrict__ V,
+                                            const uint64_t* __restrict__ row, int nwords,
+                                            const double (&acc)[(CM + 31) / 32], int lane, int c, double ey) {
+  constexpr int JW = (CM + 31) / 32;
+  double gs = 0.0;
+#pragma unroll
+  for (int jj = 0; jj < JW; ++jj) {
     const int j = lane + 32 * jj;
     if (j >= 1 && j <= P.k) gs += P.g[j - 1] * acc[jj];
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) gs += __shfl_xor_sync(0xffffffffu, gs, o);
-  const double xcn2 = (double)c * (double)(P.n - c) / (double)P.n;
-  const double xyc = ey + gs + P.kappa * (double)c;
+  const double cd = (double)c;
+  const double xcn2 = cd * (double)(P.n - c) / (double)P.n;
+  double xyc = ey + gs + P.kappa * cd;
+  const double t = sqrt(P.thr2_ynorm2 * xcn2);
+  if (!(fabs(fabs(xyc) - t) > 1.01 * P.gate_unit * cd + 1e-11 * t)) {
+    double e[JW];
+    split_columns<CM>(P.k, LM.scale, V, row, nullptr, nwords, lane, e);
+    gs = 0.0;
+#pragma unroll
+    for (int jj = 0; jj < JW; ++jj)
+      for (int l = 0; l < 32; ++l) {
+        const double ej = __shfl_sync(0xffffffffu, e[jj], l);
+        const int col = l + 32 * jj;
+        if (col >= 2 && col <= P.k) gs = fma(P.g[col - 1], ej, gs);
+        if (col == P.k + 1) ey = ej;
+      }
+    xyc = ey + gs + P.kappa * cd;
+  }
   return xyc * xyc >= P.thr2_ynorm2 * xcn2;
 }
 

@@ -17,6 +17,7 @@ constexpr unsigned long long MP_KMER_MASK = (1ull << 47) - 1;  // bit 47: CAND_O
 template <int CM>
 __global__ void __launch_bounds__(256) mp_refine_kernel(const uint64_t* __restrict__ x, int wpk, int nwords,
                                                         const double* __restrict__ T, unsigned long long tstride,
+                                                        const double* __restrict__ V, unsigned long long vstride,
                                                         const MPheno* __restrict__ ph, const DevOutMP O) {
   const int lane = threadIdx.x & 31;
   const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
@@ -35,7 +36,7 @@ __global__ void __launch_bounds__(256) mp_refine_kernel(const uint64_t* __restri
     double ss, ey;
     refine_reduce<CM>(P, acc, lane, c, ss, ey);
     if (ent & CAND_OPEN_MP) {
-      if (!refine_gate<CM>(P, acc, lane, c, ey)) continue;
+      if (!refine_gate<CM>(P, ph[p].LM, V + (size_t)p * vstride, row, nwords, acc, lane, c, ey)) continue;
       if (lane == 0)
         atomicAdd(O.tested + (size_t)mp_shard(O, gk) * O.n_pheno + p, O.weight ? (unsigned long long)O.weight[gk] : 1ull);
     }
@@ -112,7 +113,7 @@ static cudaError_t launch_mp_refine_t(const LaunchMpRefine& L, cudaStream_t st) 
        per_sm < 1))
     per_sm = 1;
   mp_refine_kernel<CM><<<(unsigned)(L.num_sms * per_sm), 256, 0, st>>>(
-      L.x, L.wpk, L.vrows / 64, L.T, (unsigned long long)refine_table_len(L.vrows, L.cm), L.ph, *L.O);
+      L.x, L.wpk, L.vrows / 64, L.T, (unsigned long long)refine_table_len(L.vrows, L.cm), L.V, L.vstride, L.ph, *L.O);
   return cudaGetLastError();
 }
 

@@ -454,27 +454,15 @@ __global__ void __launch_bounds__(pr_threads(N), 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
-// xxM of a product row as pairs_kernel has it (drop0): the column sums over the
-// values that the limbs hold -- integers times the column's scale, so exact in
-// any order -- squared in the order of its epilogue.  V: the FP64 columns.
+// xxM of a product row as pairs_kernel has it (drop0), from the limb sums in the
+// order of its epilogue.
 template <int CM>
 __device__ __noinline__ double pr_split_xxM(const EpiParams& P, const LimbMap& LM, const double* __restrict__ V,
                                             const uint64_t* __restrict__ ri, const uint64_t* __restrict__ rj,
                                             int nwords, int lane, int c) {
   constexpr int JW = (CM + 31) / 32;
   double e[JW];
-#pragma unroll
-  for (int jj = 0; jj < JW; ++jj) {
-    e[jj] = 0.0;
-    const int col = lane + 32 * jj;  // V: the count, then U column col - 1
-    if (col < 2 || col > P.k) continue;
-    const double scale = LM.scale[col - 1], up = 1.0 / scale;  // a power of two
-    double sum = 0.0;
-    for (int w = 0; w < nwords; ++w)
-      for (uint64_t bits = ri[w] & rj[w]; bits; bits &= bits - 1)
-        sum += round(V[(size_t)(64 * w + __ffsll((long long)bits) - 1) * CM + col] * up);
-    e[jj] = sum * scale;
-  }
+  split_columns<CM>(P.k, LM.scale, V, ri, rj, nwords, lane, e);
   const double cd = (double)c, s0 = P.a[0] * cd;
   double ss = s0 * s0;
 #pragma unroll

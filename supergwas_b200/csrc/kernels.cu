@@ -131,8 +131,9 @@ cudaError_t launch_fp64(const LaunchFp64& L, cudaStream_t st) {
 // (src/kgwas.cpp:44-56) in FP64 and emits the row.
 template <int CM>
 __global__ void __launch_bounds__(256) refine_kernel(const uint64_t* __restrict__ x, int wpk, int nwords,
-                                                     const double* __restrict__ T,
-                                                     const __grid_constant__ EpiParams P, const DevOut O) {
+                                                     const double* __restrict__ T, const double* __restrict__ V,
+                                                     const __grid_constant__ EpiParams P,
+                                                     const __grid_constant__ LimbMap LM, const DevOut O) {
   const int lane = threadIdx.x & 31;
   const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
   unsigned long long ncand = O.counters[3];
@@ -147,7 +148,7 @@ __global__ void __launch_bounds__(256) refine_kernel(const uint64_t* __restrict_
     double ss, ey;
     refine_reduce<CM>(P, acc, lane, c, ss, ey);
     if (entry & CAND_OPEN) {
-      if (!refine_gate<CM>(P, acc, lane, c, ey)) continue;
+      if (!refine_gate<CM>(P, LM, V, row, nwords, acc, lane, c, ey)) continue;
       if (lane == 0) atomicAdd(O.counters, O.weight ? (unsigned long long)O.weight[g] : 1ull);
     }
     if (lane == 0) {
@@ -194,12 +195,12 @@ static cudaError_t launch_refine_t(const LaunchFp64& L, cudaStream_t st) {
       (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, refine_kernel<CM>, 256, 0) != cudaSuccess || per_sm < 1))
     per_sm = 1;
   const unsigned grid = (unsigned)(L.num_sms * per_sm);
-  refine_kernel<CM><<<grid, 256, 0, st>>>(L.x, L.wpk, L.nsteps * F64_SCH / 64, L.T, *L.P, *L.O);
+  refine_kernel<CM><<<grid, 256, 0, st>>>(L.x, L.wpk, L.nsteps * F64_SCH / 64, L.T, L.V, *L.P, *L.LM, *L.O);
   return cudaGetLastError();
 }
 
 cudaError_t launch_refine(const LaunchFp64& L, cudaStream_t st) {
-  if (!L.T) return cudaErrorInvalidValue;
+  if (!L.T || !L.LM) return cudaErrorInvalidValue;
   switch (L.cm) {
     case 8: return launch_refine_t<8>(L, st);
     case 12: return launch_refine_t<12>(L, st);

@@ -18,6 +18,7 @@ struct LaunchFp64 {
   const DevOut* O;
   int num_sms;
   const double* T = nullptr;  // refinement byte tables of V (refine_table_len doubles; device)
+  const LimbMap* LM = nullptr;  // refinement: the int8 limb columns
 };
 
 struct LaunchTc {

@@ -35,6 +35,7 @@ struct EpiParams {
   double r2_ref;
   double r2_need;   // refinement may skip k-mers with r2 in [r2_ref, r2_need), see may_refine
   double thr2_ynorm2;  // corr_thr^2 * ynorm^2 (division-free Pearson gate)
+  double gate_unit;    // the limbs' rounding moves x.(y - mean) by at most popcount(x) times this
   double a[KMAX];
   double g[KMAX];
   ScreenParams S;
@@ -66,6 +67,13 @@ inline void set_limb_consts(LimbMap& L) {
 // is not emitted whatever the refinement gives, as long as the split form's
 // xxM is good to a few percent (may_refine).
 inline void set_refine_need(EpiParams& P) { P.r2_need = 0.9 * P.r2_cand; }
+
+// EpiParams::gate_unit: half a unit of the last limb of every column, U columns
+// weighted as the gate sums them.
+inline void set_gate_unit(EpiParams& P, const LimbMap& L, bool drop0) {
+  P.gate_unit = 0.5 * L.scale[P.k];
+  for (int j = drop0 ? 1 : 0; j < P.k; ++j) P.gate_unit += 0.5 * std::fabs(P.g[j]) * L.scale[j];
+}
 
 // Screen constants of a phenotype whose intercept carries no limbs (drop0)
 // and whose limb columns are those of L (3 per U column, 5 for y').  See

@@ -129,3 +129,32 @@ def test_pairs(built, n, k, m, thr, monkeypatch):
             assert ea == eb
             assert np.array_equal(a, b)
         assert b.shape[0] > 0 or r1 < m
+
+
+@pytest.mark.parametrize("n,k", [(200, 6), (1000, 33)])
+def test_gate_decided_by_the_limb_sums(built, n, k, monkeypatch):
+    """A correlation a few 1e-9 from the threshold, less than the roundings of
+    the int8 limbs: the count of tested k-mers is that of the int8 kernels, for
+    one phenotype and for many."""
+    rng = np.random.default_rng(n)
+    pop, Z = structure(n, k, rng)
+    y = rng.standard_normal(n) + 1.5 * pop + 2.0
+    U = np.linalg.qr(Z)[0]
+    X = synth.pack_rows(awkward_rows(n, 2000, pop, y, rng), max(16, synth.words_per_kmer(n)))
+    with api.Kgwas(corr_threshold=0.0, log10_thresh=6.0) as g:
+        g.set_structure(U, y)
+        st = g.run_host(X, stats=True).stats
+    cor = np.abs(st["cor"])
+    pick = rng.choice(np.nonzero((cor > 0.05) & (cor < 0.9))[0], 16, replace=False)
+    for i, eps in zip(pick, [3e-9, -3e-9] * 8):
+        with api.Kgwas(corr_threshold=float(cor[i] * (1 + eps)), log10_thresh=6.0) as g:
+            g.set_structure(U, y)
+            g.set_phenotypes([(U, y, np.arange(n))] * 2, n)
+            monkeypatch.delenv("KG_KERNEL", raising=False)
+            monkeypatch.delenv("KG_MP_KERNEL", raising=False)
+            a, (ta, _) = g.run_host(X), g.run_multi_host(X)
+            monkeypatch.setenv("KG_KERNEL", "full")
+            monkeypatch.setenv("KG_MP_KERNEL", "mp")
+            b, (tb, _) = g.run_host(X), g.run_multi_host(X)
+        assert a.n_tested == b.n_tested
+        assert np.array_equal(ta, tb) and ta[0, 0] == a.n_tested

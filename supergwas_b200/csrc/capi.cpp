@@ -172,6 +172,7 @@ void kg_destroy(kg_ctx* ctx) {
   dfree(ctx->dBts);
   dfree(ctx->dPh1);
   dfree(ctx->dFs);
+  dfree(ctx->dGather);
   dfree(ctx->dCounters);
   dfree(ctx->dHits);
   dfree(ctx->dCand);
@@ -269,6 +270,8 @@ int kg_set_structure_ex(kg_ctx* ctx, const double* U, int n, int k, const double
   ctx->fs_N = 0;
   if (ctx->opts.precision == KG_PREC_FP64) {
     if (int rc = set_f64_limbs(ctx, n_row)) return rc;
+    if (ctx->f64_N)
+      if (int rc = set_screen4(ctx, sample_pos, n_row)) return rc;
   }
   if (ctx->opts.precision == KG_PREC_SPLIT_I8) {
     // byte tables of V for the FP64 refinement of high-chi-square k-mers
@@ -540,6 +543,14 @@ int ensure_cand(kg_ctx* ctx, unsigned long long cap) {
   return KG_OK;
 }
 
+// After a launch with more candidates than room: a longer list, or, in the FP64
+// form, no screen for this structure.
+int cand_overflow(kg_ctx* ctx) {
+  if (ctx->opts.precision != KG_PREC_FP64) return ensure_cand(ctx, 4 * ctx->cand_cap);
+  ctx->fs_N = 0;
+  return KG_OK;
+}
+
 int ensure_stats(kg_ctx* ctx, size_t m) {
   if (ctx->stat_cap >= m && ctx->dTested) return KG_OK;
   dfree(ctx->dTested);
@@ -562,6 +573,29 @@ int check_shape(kg_ctx* ctx, const void* x, uint64_t m, uint32_t wpk) {
     return ctx->fail(KG_ERR_INVALID, "words_per_kmer*64 < samples per row");
   return KG_OK;
 }
+
+cudaError_t launch_screen4(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, const kg::DevOut& O,
+                           cudaStream_t st) {
+  kg::LaunchFs L{};
+  L.x = dx;
+  L.m = m;
+  L.wpk = (int)wpk;
+  L.kpad = ctx->fs_kpad;
+  L.NP = ctx->fs_N;
+  L.PPG = L.G = 1;
+  L.lu = ctx->fs_lu;
+  L.gate = ctx->P.corr_thr > 0.0;
+  L.Bimg = ctx->dFs;
+  L.F1 = &ctx->fsF;
+  L.O1 = &O;
+  L.num_sms = ctx->num_sms;
+  return kg::launch_fs(L, st);
+}
+
+// FP64 form behind the 4-bit screen: smallest work (k-mers x samples x limb
+// columns) and the rows that the screen may leave.
+constexpr double FS64_MIN = 3.2e10;
+constexpr unsigned long long FS64_ROWS = 1ull << 16;
 
 int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64_t offset, bool stats,
                cudaStream_t st) {
@@ -596,6 +630,37 @@ int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64
       kg::LaunchTb L{dx, m, (int)wpk, kpad, ctx->f64_N, 1, 1, ctx->dBts,
                      reinterpret_cast<const kg::MPheno*>(ctx->dBts + (size_t)kpad * ctx->f64_N), nullptr, &O,
                      ctx->num_sms, true};
+      // Batches large enough to be worth two launches more (the line: 4e5 k-mers
+      // at n = 1000, r = 10+1, 80 columns, where the limb kernel takes 35 us): the
+      // 4-bit screen, and the limb kernel on the rows that it leaves undecided.  A
+      // call that returns with more of those than there is room for is repeated
+      // without the screen (ctx->fs_N = 0 from then on).
+      const bool screen = ctx->fs_N && !stats && !force && (double)m * kpad * ctx->f64_N >= FS64_MIN &&
+                          kg::fs_supported(ctx->fs_N, ctx->fs_kpad, (int)wpk);
+      if (screen) {
+        const size_t bytes = (size_t)FS64_ROWS * wpk * 8;
+        if (ctx->gather_bytes < bytes) {
+          dfree(ctx->dGather);
+          ctx->gather_bytes = 0;
+          KG_CUDA(cudaMalloc((void**)&ctx->dGather, bytes), "cudaMalloc(rows)");
+          ctx->gather_bytes = bytes;
+        }
+        KG_CUDA(cudaMemsetAsync(ctx->dCounters + 3, 0, sizeof(unsigned long long), st), "memset");
+        const unsigned long long cap = std::min<unsigned long long>(O.cand_cap, FS64_ROWS);
+        O.cand_cap = cap;
+        O.count_sure = 1;
+        e = launch_screen4(ctx, dx, m, wpk, O, st);
+        if (e != cudaSuccess) return ctx->cuda_fail(e, "kernel launch");
+        e = kg::launch_fs_gather(dx, (int)wpk, ctx->dCand, ctx->dCounters + 3, cap, offset, ctx->dGather, ctx->num_sms,
+                                 st);
+        if (e != cudaSuccess) return ctx->cuda_fail(e, "gather launch");
+        ctx->launches += 2;
+        O.index = ctx->dCand;
+        O.rows = ctx->dCounters + 3;
+        O.stall_loads = 0;
+        L.x = ctx->dGather;
+        L.m = cap;
+      }
       e = kg::launch_tb(L, st);
     } else {
       kg::LaunchFp64 L{dx, m, (int)wpk, ctx->dV, ctx->nsteps, ctx->cm, &ctx->P, &O, ctx->num_sms};
@@ -616,20 +681,7 @@ int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64
     if (force && std::string(force) == "ts" && !ts_ok)
       return ctx->fail(KG_ERR_UNSUPPORTED, "KG_KERNEL=ts: shape not supported by the TMEM-A kernel");
     if (ctx->fs_N && tma_ok && !stats && !force && kg::fs_supported(ctx->fs_N, ctx->fs_kpad, (int)wpk)) {
-      kg::LaunchFs L{};
-      L.x = dx;
-      L.m = m;
-      L.wpk = (int)wpk;
-      L.kpad = ctx->fs_kpad;
-      L.NP = ctx->fs_N;
-      L.PPG = L.G = 1;
-      L.lu = ctx->fs_lu;
-      L.gate = ctx->P.corr_thr > 0.0;
-      L.Bimg = ctx->dFs;
-      L.F1 = &ctx->fsF;
-      L.O1 = &O;
-      L.num_sms = ctx->num_sms;
-      e = kg::launch_fs(L, st);
+      e = launch_screen4(ctx, dx, m, wpk, O, st);
       ctx->last_kernel = "ts";
     } else if (ts_ok && !want_ss) {
       kg::LaunchTs L{dx, m, (int)wpk, ctx->limbs.Kpad, ctx->prep.drop0 && ctx->P.k > 0, ctx->dBts, &ctx->P,
@@ -827,7 +879,7 @@ int kg_run_host(kg_ctx* ctx, const uint64_t* xbits, uint64_t m, uint32_t wpk, kg
     if ((rc = run_host_once(ctx, xbits, m, wpk, stats, runs))) return rc;
     for (int retry = 0; retry < 8 && (ctx->counters[2] & (kg::ERR_HIT_OVERFLOW | kg::ERR_CAND_OVERFLOW)); ++retry) {
       if ((ctx->counters[2] & kg::ERR_HIT_OVERFLOW) && (rc = ensure_hits(ctx, ctx->counters[1]))) return rc;
-      if ((ctx->counters[2] & kg::ERR_CAND_OVERFLOW) && (rc = ensure_cand(ctx, 4 * ctx->cand_cap))) return rc;
+      if ((ctx->counters[2] & kg::ERR_CAND_OVERFLOW) && (rc = cand_overflow(ctx))) return rc;
       if ((rc = run_host_once(ctx, xbits, m, wpk, stats, runs))) return rc;
     }
   }
@@ -916,7 +968,7 @@ extern "C" int kg_fetch(kg_ctx* ctx, kg_result* res, kg_stats* st) {
   for (int retry = 0; retry < 8 && (ctx->counters[2] & (kg::ERR_HIT_OVERFLOW | kg::ERR_CAND_OVERFLOW)); ++retry) {
     int rc = 0;
     if ((ctx->counters[2] & kg::ERR_HIT_OVERFLOW) && (rc = ensure_hits(ctx, ctx->counters[1]))) return rc;
-    if ((ctx->counters[2] & kg::ERR_CAND_OVERFLOW) && (rc = ensure_cand(ctx, 4 * ctx->cand_cap))) return rc;
+    if ((ctx->counters[2] & kg::ERR_CAND_OVERFLOW) && (rc = cand_overflow(ctx))) return rc;
     KG_CUDA(cudaMemsetAsync(ctx->dCounters, 0, 4 * sizeof(unsigned long long), ctx->pend_stream), "memset");
     if ((rc = launch_one(ctx, ctx->pend_x, ctx->pend_m, ctx->pend_wpk, 0, stats, ctx->pend_stream))) return rc;
     KG_CUDA(cudaMemcpyAsync(ctx->counters, ctx->dCounters, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,

@@ -75,7 +75,7 @@ inline bool fill_fs(kg::FsPheno& F, const kg::EpiParams& P, const kg::Prepared& 
   const double r2_ref = -std::expm1(-kg::REFINE_CHISQ / (double)p.n);
   const double yv = P.yyM / (P.ynorm * P.ynorm);
   if (!p.drop0 || p.k < 1 || !(std::fabs(P.a[0] * P.a[0] * p.n - 1.0) <= 1e-6) || p.n >= 65536 || !(P.ynorm >= 1e-12) || !(P.ynorm < 1e150) || !(yv > 1e-6) ||
-      !(P.r2_cand >= r2_ref) || !(P.r2_cand < 1.0) || P.refine == 0)
+      !(P.r2_cand >= r2_ref) || !(P.r2_cand < 1.0))
     return false;
   F.n = (float)p.n;
   F.inv_n = (float)(1.0 / p.n);
@@ -182,6 +182,9 @@ struct kg_ctx {
   uint8_t* dFs = nullptr;
   kg::FsPheno fsF{};
   int fs_N = 0, fs_lu = 0, fs_kpad = 0;
+  // FP64 form behind the screen: the gathered rows of undecided k-mers
+  uint64_t* dGather = nullptr;
+  size_t gather_bytes = 0;
   int nchunk = 0;
   int f64_N = 0;             // limb columns of the FP64 form (dBts holds image and constants); 0: CUDA cores
   // outputs on the device

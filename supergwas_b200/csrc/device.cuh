@@ -343,7 +343,7 @@ __device__ __forceinline__ void emit_rare(const DevOut& O, unsigned long long lo
       const unsigned long long slot = base + __popc(hmask & ((1u << lane) - 1u));
       if (slot < O.hit_cap) {
         kg_hit h;
-        h.kmer = O.kmer_offset + local;
+        h.kmer = O.kmer(local);
         h.effect = effect;
         h.pval = p;
         h.chisq = T;
@@ -372,7 +372,7 @@ __device__ __forceinline__ void emit_kmer(const DevOut& O, unsigned long long lo
                                           double xyM, double cor) {
   const unsigned lane = threadIdx.x & 31u;
   if (O.weight) {
-    const unsigned tot = __reduce_add_sync(0xffffffffu, tested ? O.weight[O.kmer_offset + local] : 0u);
+    const unsigned tot = __reduce_add_sync(0xffffffffu, tested ? O.weight[O.kmer(local)] : 0u);
     if (lane == 0 && tot) atomicAdd(O.counters + 0, (unsigned long long)tot);
   } else {
     const unsigned tmask = __ballot_sync(0xffffffffu, tested);

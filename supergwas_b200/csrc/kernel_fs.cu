@@ -403,9 +403,10 @@ __global__ void __launch_bounds__(fs_threads(NP * PPG), 1)
                         (O.kmer_offset + local) | ((unsigned long long)p << 48) | (v == 3 ? CAND_OPEN_MP : 0ull));
             } else {
               const int v = fs_verdict<NP, LU, GATE>(F1, d, valid);
-              if (v == 1 || v == 2) tested_local += O1.weight ? O1.weight[O1.kmer_offset + local] : 1u;
+              if (v == 1 || (v == 2 && !O1.count_sure))
+                tested_local += O1.weight ? O1.weight[O1.kmer_offset + local] : 1u;
               if (__any_sync(0xffffffffu, v >= 2))
-                fs_push(counters, O1.cand, O1.cand_cap, v >= 2, (O1.kmer_offset + local) | (v == 3 ? CAND_OPEN : 0ull));
+                fs_push(counters, O1.cand, O1.cand_cap, v >= 2, (O1.kmer_offset + local) | (v == 3 && !O1.count_sure ? CAND_OPEN : 0ull));
             }
           }
         }
@@ -419,7 +420,32 @@ __global__ void __launch_bounds__(fs_threads(NP * PPG), 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
+// Copies the rows of the candidates to dst, 16 bytes a thread; none where they
+// are more than cap (ERR_CAND_OVERFLOW has been set then).
+__global__ void __launch_bounds__(256) fs_gather_kernel(const uint4* __restrict__ x, int chunks,
+                                                        const unsigned long long* __restrict__ cand,
+                                                        const unsigned long long* __restrict__ count,
+                                                        unsigned long long cap, unsigned long long offset,
+                                                        uint4* __restrict__ dst) {
+  const unsigned long long rows = *count;
+  if (rows > cap) return;
+  const unsigned long long total = rows * (unsigned)chunks;
+  for (unsigned long long t = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
+       t += (unsigned long long)gridDim.x * blockDim.x) {
+    const unsigned long long r = t / (unsigned)chunks;
+    dst[t] = x[(cand[r] - offset) * (unsigned)chunks + (t - r * (unsigned)chunks)];
+  }
+}
+
 // ------------------------------------------------------------------- host
+
+cudaError_t launch_fs_gather(const uint64_t* x, int wpk, const unsigned long long* cand,
+                             const unsigned long long* count, unsigned long long cap, unsigned long long offset,
+                             uint64_t* dst, int num_sms, cudaStream_t st) {
+  fs_gather_kernel<<<2 * num_sms, 256, 0, st>>>(reinterpret_cast<const uint4*>(x), wpk / 2, cand, count, cap, offset,
+                                                reinterpret_cast<uint4*>(dst));
+  return cudaGetLastError();
+}
 
 static int fs_box_bytes(int wpk) { return wpk * 8 < 128 ? wpk * 8 : 128; }
 

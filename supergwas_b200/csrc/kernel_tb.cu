@@ -154,7 +154,7 @@ __device__ __forceinline__ void tb_single64(const DevOut& O, const MPheno* ME, u
   if (!O.tested && P.S.on) {
     const int v = P.S.gate ? f64_screen<N, true>(P, taddr, ku, valid) : f64_screen<N, false>(P, taddr, ku, valid);
     if (!__any_sync(0xffffffffu, v == 2)) {
-      if (v) tested_local += O.weight ? O.weight[O.kmer_offset + local] : 1u;
+      if (v) tested_local += O.weight ? O.weight[O.kmer(local)] : 1u;
       return;
     }
   }
@@ -246,6 +246,10 @@ __global__ void __launch_bounds__(TB_THREADS, 1)
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   unsigned long long* const counters = SINGLE ? O1.counters : O.counters;
   const unsigned long long lim = wait_limit(SINGLE ? O1.wait_ns : O.wait_ns);
+  if (FORM == TB_ONE64 && O1.rows) {
+    const unsigned long long rows = *O1.rows;
+    m = rows <= m ? rows : 0;
+  }
   const int nsp = (nsub + TB_SUPER - 1) / TB_SUPER;     // super-stages of a tile
   const int nchunk = (nsub + TB_CHUNK - 1) / TB_CHUNK;  // image chunks
   const uint32_t ntg = (uint32_t)((m + (unsigned)(TB_TM * T) - 1) / (unsigned)(TB_TM * T));  // tile groups

@@ -141,6 +141,11 @@ inline int fs_width(bool gate, int lu, int ku) {
 }
 bool fs_supported(int N, int kpad, int wpk);
 cudaError_t launch_fs(const LaunchFs& L, cudaStream_t st);
+// Rows cand[0 .. *count) of x (16-byte aligned, wpk words each; indices from
+// `offset`) to dst, unless they are more than cap.
+cudaError_t launch_fs_gather(const uint64_t* x, int wpk, const unsigned long long* cand,
+                             const unsigned long long* count, unsigned long long cap, unsigned long long offset,
+                             uint64_t* dst, int num_sms, cudaStream_t st);
 
 struct LaunchMpRefine {
   const uint64_t* x;

@@ -153,6 +153,17 @@ struct DevOut {
   // CTA issues this many row loads and then stops, so that the consumers'
   // waits run out (0: off)
   unsigned long long stall_loads;
+  // fs_kernel: no undecided k-mer is counted as tested (the kernel that takes
+  // them counts them)
+  int count_sure;
+  // tb_kernel, FP64 form: the rows are the gathered rows of the k-mers
+  // index[0 .. *rows), of which the launch has room for m; nothing runs when
+  // there are more
+  const unsigned long long* index;
+  const unsigned long long* rows;
+  __host__ __device__ unsigned long long kmer(unsigned long long local) const {
+    return index ? index[local] : kmer_offset + local;
+  }
 };
 
 enum : unsigned { ERR_TIMEOUT_FULL = 1u, ERR_TIMEOUT_MMA = 2u, ERR_HIT_OVERFLOW = 4u, ERR_CAND_OVERFLOW = 8u };

@@ -158,3 +158,33 @@ def test_gate_decided_by_the_limb_sums(built, n, k, monkeypatch):
             b, (tb, _) = g.run_host(X), g.run_multi_host(X)
         assert a.n_tested == b.n_tested
         assert np.array_equal(ta, tb) and ta[0, 0] == a.n_tested
+
+@pytest.mark.parametrize("n,k,m,thr,lt", [(1000, 11, 420_001, 0.0, 6.0), (300, 12, 900_001, 0.2, 9.0),
+                                          (2100, 21, 100_001, 0.2, 6.0), (1000, 11, 800_000, 0.0, 4.0)],
+                         ids=lambda v: str(v))
+def test_fp64_form(built, n, k, m, thr, lt, monkeypatch):
+    """The FP64 form evaluates the rows that the screen leaves (gathered), or,
+    where those are more than it has room for (the last case: every eighth row
+    follows y), all rows."""
+    rng = np.random.default_rng(n + m)
+    pop, Z = structure(n, k, rng)
+    y = rng.standard_normal(n) + 0.5 * pop
+    x = awkward_rows(n, 4096, pop, y, rng)
+    X = synth.pack_rows(x)
+    X = np.ascontiguousarray(X[rng.integers(0, 4096, m)])
+    if lt == 6.0:
+        X[:, :] = X[np.where(np.arange(m) % 97 == 0, np.arange(m), np.arange(m) // 64 * 64 + 1)]
+    monkeypatch.setenv("KG_DEDUP", "0")
+    with api.Kgwas(precision="fp64", corr_threshold=thr, log10_thresh=lt) as g:
+        g.set_structure(np.linalg.qr(Z)[0], y)
+        monkeypatch.delenv("KG_KERNEL", raising=False)
+        a, again = g.run_host(X), g.run_host(X)
+        monkeypatch.setenv("KG_DEDUP", "1")
+        runs = g.run_host(X)
+        monkeypatch.setenv("KG_DEDUP", "0")
+        monkeypatch.setenv("KG_KERNEL", "full")
+        b = g.run_host(X)
+    assert b.hits.shape[0] > 0
+    for r in (a, again, runs):
+        assert r.n_tested == b.n_tested
+        assert np.array_equal(r.hits, b.hits)

@@ -260,7 +260,8 @@ int kg_pairs_run_host(kg_ctx* ctx, const uint64_t* xbits, uint64_t n_kmers, uint
 int kg_last_launch_count(const kg_ctx* ctx);
 
 /* Which association kernel the last launch used: "ts" (tensor cores, x
- * unpacked into tensor memory), "tb" (the same with the limb image streamed,
+ * unpacked into tensor memory: the 4-bit screen where it applies, else int8
+ * limbs), "tb" (the same with the limb image streamed,
  * where it does not fit shared memory), "ss" (tensor cores, x unpacked into
  * shared memory; other limb counts, unaligned rows) or "fp64". */
 const char* kg_last_kernel(const kg_ctx* ctx);

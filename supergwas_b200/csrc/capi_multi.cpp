@@ -651,11 +651,11 @@ int kg_run_multi_host(kg_ctx* ctx, const uint64_t* xbits, uint64_t m, uint32_t w
       if (sel) {
         par_gather(ctx->hStage[b], xbits, sel + s0, cnt, row);
         src = (const char*)ctx->hStage[b];
-      } else if (!pinned) {
-        par_memcpy(ctx->hStage[b], src, nb);
-        src = (const char*)ctx->hStage[b];
       }
-      KG_CUDA(cudaMemcpyAsync(ctx->dChunk[b], src, nb, cudaMemcpyHostToDevice, ctx->copy_stream), "H2D");
+      if (sel || pinned)
+        KG_CUDA(cudaMemcpyAsync(ctx->dChunk[b], src, nb, cudaMemcpyHostToDevice, ctx->copy_stream), "H2D");
+      else
+        KG_CUDA(stage_h2d(ctx->dChunk[b], ctx->hStage[b], src, nb, ctx->copy_stream), "H2D");
       KG_CUDA(cudaEventRecord(ctx->ev_h2d[b], ctx->copy_stream), "record");
       KG_CUDA(cudaStreamWaitEvent(st, ctx->ev_h2d[b], 0), "wait");
       if (i == 0 && (rc = autotune(ctx, ctx->dChunk[b], cnt, wpk, st))) return rc;

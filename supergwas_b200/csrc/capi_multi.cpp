@@ -4,7 +4,9 @@
 #include <chrono>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -296,22 +298,31 @@ int set_screen4_multi(kg_ctx* ctx, const kg_pheno* ph, const std::vector<kg::Pre
   std::vector<uint8_t> img((size_t)G * img_bytes + (size_t)np * sizeof(kg::FsPheno), 0);
   std::atomic<int> next{0}, bad{0};
   auto work = [&] {
-    for (int p; (p = next.fetch_add(1)) < np && !bad.load();) {
-      kg::FsCols C;
-      kg::make_fs_cols(prep[p], ph[p].sample_pos, n_row, 1, gate, C);
-      kg::FsPheno F;
-      if (!fill_fs(F, mph[p].P, prep[p], C, 1, gate)) {
-        bad.store(1);
-        return;
+    try {
+      for (int p; (p = next.fetch_add(1)) < np && !bad.load();) {
+        kg::FsCols C;
+        kg::make_fs_cols(prep[p], ph[p].sample_pos, n_row, 1, gate, C);
+        kg::FsPheno F;
+        if (!fill_fs(F, mph[p].P, prep[p], C, 1, gate)) {
+          bad.store(1);
+          return;
+        }
+        // two columns share no byte: a byte holds two samples of one column
+        kg::put_fs_image(C, (p % PPG) * NP, N, img.data() + (size_t)(p / PPG) * img_bytes);
+        std::memcpy(img.data() + (size_t)G * img_bytes + (size_t)p * sizeof(F), &F, sizeof(F));
       }
-      // two columns share no byte: a byte holds two samples of one column
-      kg::put_fs_image(C, (p % PPG) * NP, N, img.data() + (size_t)(p / PPG) * img_bytes);
-      std::memcpy(img.data() + (size_t)G * img_bytes + (size_t)p * sizeof(F), &F, sizeof(F));
+    } catch (const std::bad_alloc&) {
+      bad.store(1);  // no screen
     }
   };
   const int nt = std::max(1, std::min<int>({8, (int)std::thread::hardware_concurrency(), np}));
   std::vector<std::thread> th;
-  for (int t = 1; t < nt; ++t) th.emplace_back(work);
+  th.reserve((size_t)nt);
+  try {
+    for (int t = 1; t < nt; ++t) th.emplace_back(work);
+  } catch (const std::system_error&) {
+    // as many threads as there are
+  }
   work();
   for (auto& t : th) t.join();
   if (bad.load()) return KG_OK;

@@ -63,7 +63,8 @@ inline void fill_epi(kg::EpiParams& P, const kg::Prepared& p, const kg_opts& o, 
 }
 
 // Constants of the 4-bit screen for one phenotype (fs_verdict).  False where
-// the screen does not apply: the intercept has limbs, the structure or the
+// the screen does not apply: the intercept has limbs or is not of unit norm (the
+// screen takes c (n - c) / n for c - s_0^2: within 1e-9 c), the structure or the
 // phenotype is degenerate, or so much may pass (thresholds at which rows of
 // chi-square below REFINE_CHISQ are emitted, residuals that leave the cut or the
 // gate vague) that refining it would cost more than the screen saves: a
@@ -74,7 +75,7 @@ inline bool fill_fs(kg::FsPheno& F, const kg::EpiParams& P, const kg::Prepared& 
   F = kg::FsPheno();
   const double r2_ref = -std::expm1(-kg::REFINE_CHISQ / (double)p.n);
   const double yv = P.yyM / (P.ynorm * P.ynorm);
-  if (!p.drop0 || p.k < 1 || !(std::fabs(P.a[0] * P.a[0] * p.n - 1.0) <= 1e-6) || p.n >= 65536 || !(P.ynorm >= 1e-12) || !(P.ynorm < 1e150) || !(yv > 1e-6) ||
+  if (!p.drop0 || p.k < 1 || !(std::fabs(P.a[0] * P.a[0] * p.n - 1.0) <= 1e-9) || p.n >= 65536 || !(P.ynorm >= 1e-12) || !(P.ynorm < 1e150) || !(yv > 1e-6) ||
       !(P.r2_cand >= r2_ref) || !(P.r2_cand < 1.0))
     return false;
   F.n = (float)p.n;

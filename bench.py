@@ -49,13 +49,15 @@ def measured_peaks():
     return 6650.0, 1590.0, "fallback"
 
 
-# DRAM bytes (read + write) per k-mer of ts_kernel<64,1> on the bench workload
+# DRAM bytes (read + write) per k-mer of fs_kernel<24> on the bench workload
 # (n=1000, 128-byte rows, r=16+1): dram__bytes_read.sum + dram__bytes_write.sum
-# of one ncu capture of a 4M-k-mer launch (512 MB of rows, > L2) divided by the
+# of one ncu capture of an 8M-k-mer launch (1 GB of rows, > L2) divided by the
 # k-mers it processed; the traffic grows in proportion to the k-mers, so a full
 # launch moves this many bytes per k-mer.  Capture and command:
-# profiles/ts_kernel_n1000_r16.md.
-TS_DRAM_BYTES_PER_KMER = 129.2
+# profiles/fs_kernel.md.
+TS_DRAM_BYTES_PER_KMER = 128.6
+# Emitted rows are evaluated in FP64; the screen tells which k-mers may be emitted.
+SCREEN_DTYPE = "e2m1 screen with error bounds -> f32 TMEM, f64 for every k-mer that may be emitted"
 
 
 class Clocks:
@@ -355,17 +357,14 @@ def run_ours(args):
         alg_bytes = m * ((n + 7) // 8)          # packed x, 1 bit per sample (algorithmic)
         achieved = alg_bytes / t_launch / 1e9
         traffic_pk = TS_DRAM_BYTES_PER_KMER if (n, r) == (1000, 16) else None
-        N = 64
+        cols = (4 + r + 7) // 8 * 8             # e2m1 columns: count, 3 of y', one per PC, rounded up to 8
         kpad = ((n + 255) // 256) * 256
-        tops = 2.0 * m * kpad * N / t_launch / 1e12
-        sm_mhz = clocks.get("sm_mhz") or 0.0
-        n_sm = torch.cuda.get_device_properties(local).multi_processor_count
-        hw_peak = 16384.0 * n_sm * sm_mhz * 1e6 / 1e12 if sm_mhz else None
+        tops = 2.0 * m * kpad * cols / t_launch / 1e12
         cpu = cpu_baseline(n, r, W["seed"], args.cpu_kmers) if not args.no_cpu else None
         line = {
             "metric": METRIC, "value": value, "unit": "k-mer tests/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": 1e3 * t_split_all / args.steps, "higher_is_better": True,
-            "scaling": "weak", "vs_baseline": None, "dtype": "i8 limbs -> i32 TMEM, f64 epilogue",
+            "scaling": "weak", "vs_baseline": None, "dtype": SCREEN_DTYPE,
             "data": "synthetic (seeded Balding-Nichols, generated on device)",
             "config": {"workload": f"n={n} (5% unphenotyped), m={m} k-mers per GPU, r={r}+1, 1 phenotype, "
                                    f"CORR_THRESHOLD=0", "kmers_per_gpu": m, "bytes_per_kmer": wpk * 8,
@@ -376,18 +375,14 @@ def run_ours(args):
                          "frac": achieved / hbm, "peak_source": peak_src,
                          "traffic": (traffic_pk * m if traffic_pk else None),
                          "algorithmic_bytes_per_launch": alg_bytes,
-                         "tensor": {"achieved_tops_int8": tops, "peak_tops_int8": 2 * bf16,
-                                    "frac": tops / (2 * bf16),
-                                    "peak_note": "2x measured bf16 burst (int8 MMA issues at twice the bf16 rate)",
-                                    # 16384 int8 ops per SM-cycle at the median SM clock of the timed
-                                    # region (an N=64 MMA issues at that rate: --workload mma-rate)
-                                    "hw_peak_tops_int8_at_clock": hw_peak,
-                                    "frac_of_hw_peak": tops / hw_peak if hw_peak else None,
-                                    "useful_columns": "54 of N=64 (count, 5 y' limbs, 16 x 3 U limbs)"}},
+                         "tensor": {"achieved_tops_e2m1": tops, "peak_tops_e2m1": 4 * bf16,
+                                    "frac": tops / (4 * bf16),
+                                    "peak_note": "4x measured bf16 burst (block-scaled e2m1 MMA)",
+                                    "useful_columns": f"{4 + r} of {cols} (count, 3 y' limbs, {r} U limbs)"}},
             "fp64_form": {"value": ftested / t_fp64, "unit": "k-mer tests/s", "ms_per_step": 1e3 * t_fp64,
                           "split_speedup": value / world / (ftested / t_fp64),
-                          # the multiply-adds of a plain FP64 evaluation; the form runs in exact
-                          # int8 limbs on the tensor cores
+                          # the multiply-adds of a plain FP64 evaluation of every k-mer; the form
+                          # screens in 4 bits and evaluates what is left in exact int8 limbs
                           "equivalent_fp64_tflops": 2.0 * m * n * (r + 2) / t_fp64 / 1e12},
             "fp64_config2": leg_fp64,
             "files_cols": leg_files,
@@ -481,7 +476,9 @@ def batched_leg(local, rank, m, steps, warmup, acc_kmers):
                     "mlog10p_abs_max": float(ml.max()), "chisq_rel_p99": float(np.percentile(rel, 99)),
                     "chisq_rel_max_T_ge_1e-3": float(rel[T0 >= 1e-3].max()) if (T0 >= 1e-3).any() else 0.0})
     hbm, bf16, peak_src = measured_peaks()
-    ops = 2.0 * m * shape["kpad"] * shape["NP"] * npn   # int8 ops executed (padded columns included)
+    ops = 2.0 * m * shape["kpad"] * shape["NP"] * npn   # ops executed (padded columns included)
+    e2m1 = shape["kernel"].startswith("4-bit")
+    peak, op = (4 * bf16, "e2m1") if e2m1 else (2 * bf16, "int8")
     tops = ops / (t / steps) / 1e12
     return {"metric": "k-mer tests/s (batched: 64 phenotypes x 1e8 k-mers, n=2000, r=20+1, one fused launch)",
             "value": value, "unit": "k-mer tests/s", "steps": steps, "warmup": warmup,
@@ -491,8 +488,8 @@ def batched_leg(local, rank, m, steps, warmup, acc_kmers):
                                    "CORR_THRESHOLD=0",
                        "l2": "inputs (%.1f GB) >> L2; no flush needed" % (m * wpk * 8 / 1e9)},
             "tile_shape": shape,
-            "roofline": {"bound": "tensor", "achieved": tops, "peak": 2 * bf16, "unit": "TOP/s int8",
-                         "frac": tops / (2 * bf16), "peak_source": peak_src + " (2x bf16 burst)",
+            "roofline": {"bound": "tensor", "achieved": tops, "peak": peak, "unit": f"TOP/s {op}",
+                         "frac": tops / peak, "peak_source": peak_src + (" (4x" if e2m1 else " (2x") + " bf16 burst)",
                          "ops_per_launch": ops, "traffic": None},
             "accuracy_vs_fp64_oracle": acc, "clocks": ck.summary(), "gen_seconds": t_gen}
 
@@ -506,7 +503,7 @@ def run_batched(args):
     leg = batched_leg(local, rank, args.kmers, args.steps, args.warmup, args.acc_kmers // 4)
     line = dict(leg)
     line.update({"n_gpus": world, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-                 "dtype": "i8 limbs -> i32 TMEM, f64 epilogue", "data": "synthetic (seeded, generated on device)"})
+                 "dtype": SCREEN_DTYPE, "data": "synthetic (seeded, generated on device)"})
     line["config"]["parallelism"] = f"weak: {world} GPU(s)"
     if rank == 0:
         print(json.dumps(line), flush=True)
@@ -520,7 +517,7 @@ def fp64_config2_leg(X, local, rank, steps, warmup, fp64_peak):
     5e7 rows of the device batch (same generator, 8 subpopulations) with a
     structure of 10 PCs and its own phenotype.  HBM GB/s of the packed rows,
     and the rate of a plain FP64 evaluation's multiply-adds beside the measured
-    DFMA peak (the form runs in exact int8 limbs on the tensor cores)."""
+    DFMA peak (the form screens in 4 bits and evaluates what is left in exact int8 limbs)."""
     import torch
     from supergwas_b200 import api, synth_gpu
     C = FP64_CFG2
@@ -664,7 +661,7 @@ def run_streaming(args):
     line = {"metric": "k-mer tests/s (streaming from pinned host: 8 phenotypes, n=5000, r=32+1, 16 GB chunks)",
             "value": value, "unit": "k-mer tests/s", "n_gpus": world, "steps": nchunks, "warmup": args.warmup,
             "ms_per_step": 1e3 * t / nchunks, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "i8 limbs -> i32 TMEM, f64 epilogue",
+            "dtype": SCREEN_DTYPE,
             "data": "synthetic (seeded Balding-Nichols, each chunk regenerated on the device from its seed)",
             "config": {"workload": f"streaming: n={n} ({S} subpopulations), m=1e9 k-mers as {W['m_total'] // per} "
                                    f"chunks of {per} ({per * row / 1e9:.1f} GB) in pinned host memory, r={r}+1, "
@@ -769,7 +766,7 @@ def run_sorted(args):
             "value": value, "unit": "k-mer tests/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": 1e3 * t / args.steps,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "i8 limbs -> i32 TMEM, f64 epilogue", "data": "synthetic (seeded, generated on device)",
+            "dtype": SCREEN_DTYPE, "data": "synthetic (seeded, generated on device)",
             "config": {"workload": f"sorted: n={n} (5% unphenotyped), {m} k-mers per step from {d} distinct rows "
                                    f"(runs of 1..9, mean {mr}), r={r}+1, 1 phenotype, CORR_THRESHOLD=0",
                        "parallelism": f"weak: {world} GPU(s)"},
@@ -919,7 +916,7 @@ def run_files(args):
     line = {"metric": "k-mer tests/s end to end through the kgwas program (files in, files out)",
             "value": t_c / s_c, "unit": "k-mer tests/s", "n_gpus": 1, "steps": 1, "warmup": 1,
             "ms_per_step": 1e3 * s_c, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "i8 limbs -> i32 TMEM, f64 epilogue", "data": "synthetic (seeded), written as pipeline files",
+            "dtype": SCREEN_DTYPE, "data": "synthetic (seeded), written as pipeline files",
             "config": {"workload": f"files: n={n} (5% unphenotyped), {m} k-mers in one batch_*/ directory "
                                    f"({n} column files) and one ROWS file, r={r}+1, CORR_THRESHOLD=0, "
                                    f"files in the page cache, {threads} host threads for both programs",
@@ -1005,7 +1002,7 @@ def run_pairs(args):
     value = n_eval / t * world
     hbm, bf16, peak_src = measured_peaks()
     kpad = ((n + 255) // 256) * 256
-    ops = 2.0 * kpad * 64 * (N * (N - 1) / 2)
+    ops = 2.0 * kpad * ((4 + r + 7) // 8 * 8) * (N * (N - 1) / 2)
     cpu = None
     if not args.no_cpu and reference_binary() and rank == 0:
         threads = os.cpu_count() or 1
@@ -1017,12 +1014,12 @@ def run_pairs(args):
     line = {"metric": f"pair tests/s (2-D pair test, n={n}, r={r}+1, {N} k-mers)", "value": value,
             "unit": "pair tests/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": 1e3 * t, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "i8 limbs -> i32 TMEM, f64 epilogue", "data": "synthetic (seeded, generated on device)",
+            "dtype": SCREEN_DTYPE, "data": "synthetic (seeded, generated on device)",
             "config": {"workload": f"pairs: n={n}, N={N} k-mers ({N * (N - 1) // 2} pairs), r={r}+1, "
                                    "log10_thresh=6", "parallelism": f"weak: {world} GPU(s)"},
             "pairs_scored": n_eval, "pairs_emitted": int(res.shape[0]),
-            "roofline": {"bound": "tensor", "achieved": ops / t / 1e12, "peak": 2 * bf16, "unit": "TOP/s int8",
-                         "frac": ops / t / 1e12 / (2 * bf16), "peak_source": peak_src + " (2x bf16 burst)",
+            "roofline": {"bound": "tensor", "achieved": ops / t / 1e12, "peak": 4 * bf16, "unit": "TOP/s e2m1",
+                         "frac": ops / t / 1e12 / (4 * bf16), "peak_source": peak_src + " (4x bf16 burst)",
                          "traffic": None},
             "e2e": {"value": value, "unit": "pair tests/s", "h2d_bytes_per_step": int(X.nbytes),
                     "d2h_bytes_per_step": int(res.shape[0]) * 40 + 32, "api": "kg_pairs_run_host"},
@@ -1267,7 +1264,7 @@ def main():
                          "files: the kgwas program against the reference's on the same files; "
                          "profile: a few launches of one kernel for ncu (--kernel, --launches, --n, --r, --pheno); "
                          "mma-rate: tcgen05 MMA rates per SM")
-    ap.add_argument("--kernel", default="ts", choices=["ts", "ss", "fp64", "multi", "pairs"])
+    ap.add_argument("--kernel", default="ts", choices=["ts", "ss", "fp64", "fs", "multi", "pairs"])
     ap.add_argument("--launches", type=int, default=3)
     ap.add_argument("--n", type=int, default=1000, help="samples (profile workload)")
     ap.add_argument("--r", type=int, default=16, help="PCs (profile workload)")

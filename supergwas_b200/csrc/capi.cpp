@@ -59,7 +59,9 @@ int set_f64_limbs(kg_ctx* ctx, int n_row) {
     ph.LM.scale[j] = std::ldexp(1.0, -s);
   }
   kg::set_limb_consts(ph.LM);
-  kg::set_screen64(ph.P, ph.LM, drop0);
+  kg::LimbLoss loss;  // what a double holds, the limbs hold
+  kg::column_norms(p, loss.norm);
+  kg::set_screen(ph.P, ph.LM, drop0, loss, true);
   const int kpad = ctx->nsteps * 128;
   const size_t img = (size_t)kpad * N;
   dfree(ctx->dBts);
@@ -286,7 +288,6 @@ int kg_set_structure_ex(kg_ctx* ctx, const double* U, int n, int k, const double
     KG_CUDA(cudaStreamSynchronize(ctx->stream), "refinement tables");
     P.refine = 1;
     P.r2_ref = -std::expm1(-kg::REFINE_CHISQ / (double)n);
-    kg::set_refine_need(P);
     e = kg::make_limbs(p, sample_pos, n_row, ctx->opts.limbs_u, ctx->opts.limbs_y, kg::tc_kc(), ctx->limbs);
     if (!e.empty()) return ctx->fail(KG_ERR_UNSUPPORTED, e);
     if (!kg::tc_supported_n(ctx->limbs.N))
@@ -305,8 +306,11 @@ int kg_set_structure_ex(kg_ctx* ctx, const double* U, int n, int k, const double
       LM.scale[j] = ctx->limbs.scale[j];
     }
     kg::set_limb_consts(LM);
+    kg::LimbLoss loss;
+    kg::limb_loss(p, LM.scale, loss);
+    kg::set_refine_need(P, loss);
     kg::set_gate_unit(P, LM, p.drop0 && k > 0);
-    if (ctx->opts.limbs_u == 3 && ctx->opts.limbs_y == 5) kg::set_screen(P, LM, p.drop0 && k > 0);
+    if (ctx->opts.limbs_u == 3 && ctx->opts.limbs_y == 5) kg::set_screen(P, LM, p.drop0 && k > 0, loss);
     dfree(ctx->dB);
     KG_CUDA(cudaMalloc((void**)&ctx->dB, img.size()), "cudaMalloc(B)");
     KG_CUDA(cudaMemcpy(ctx->dB, img.data(), img.size(), cudaMemcpyHostToDevice), "copy B");

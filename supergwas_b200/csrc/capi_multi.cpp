@@ -437,8 +437,11 @@ int kg_set_phenotypes(kg_ctx* ctx, const kg_pheno* ph, int np, int n_row) {
     }
     kg::set_limb_consts(LM);
     mph[p].drop0 = (k > 0 && prep[p].drop0) ? 1 : 0;
+    kg::LimbLoss loss;
+    kg::limb_loss(prep[p], LM.scale, loss);
+    kg::set_refine_need(mph[p].P, loss);
     kg::set_gate_unit(mph[p].P, LM, mph[p].drop0 != 0);
-    kg::set_screen(mph[p].P, LM, mph[p].drop0 != 0);
+    kg::set_screen(mph[p].P, LM, mph[p].drop0 != 0, loss);
   }
   // FP64 refinement operands: per phenotype, rows = packed-row sample positions,
   // columns [count, d_0 .. d_{k-1}, d_y]

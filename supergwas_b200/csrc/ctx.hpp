@@ -58,7 +58,6 @@ inline void fill_epi(kg::EpiParams& P, const kg::Prepared& p, const kg_opts& o, 
   if (refine) {
     P.refine = 1;
     P.r2_ref = -std::expm1(-kg::REFINE_CHISQ / (double)p.n);
-    kg::set_refine_need(P);
   }
 }
 

@@ -474,17 +474,13 @@ __device__ __forceinline__ void finish_kmer_fast(const EpiParams& P, const DevOu
 
 // Whether a tested k-mer of the split form goes to the FP64 refinement in a
 // launch that returns emitted rows only: r2 = q / den at least r2_ref, and not
-// so far below the emit cut that refining cannot matter.  The limbs of U are
-// rounded to 2^-23 of a column's largest value, which in the worst case (every
-// rounding of one sign) moves xxM by under 1 % of c(n - c)/n / 50 (up to 12,000
-// samples, 33 columns), so the 10 % below the cut hold where xxM is at least
-// that 50th.
+// so far below the emit cut that refining cannot matter (set_refine_need).
 // Refining every k-mer from chi-square 12 up took 0.1 ms per 4e7 k-mers at
 // n = 1000 (5e-4 of them, 20 KB of byte tables each); from 0.9 of the cut at
 // p = 1e-6 it is 4e-6 of them.
 __device__ __forceinline__ bool may_refine(const EpiParams& P, double cd, double xxM, double q, double den) {
   return q >= P.r2_ref * den &&
-         (q >= P.r2_need * den || !(xxM >= 0.02 * cd * ((double)P.n - cd) / (double)P.n));
+         (q >= P.r2_need * den || !(xxM >= XXM_FLOOR * cd * ((double)P.n - cd) / (double)P.n));
 }
 
 // Fast screen of one k-mer for kernels that count tested k-mers in a
@@ -537,13 +533,12 @@ __device__ __forceinline__ float shifted_float(long long v, int s) {
 // FP64 instructions and the MMAs share one pipe (ncu: pipe_shared), so an FP64
 // instruction waits for the MMA in the pipe, ~36 cycles beside N = 64: the
 // FP64 statistic of 16 U columns took 3100 cycles per 128-k-mer tile.  The
-// screen uses the integer, conversion and FP32 pipes only.  Errors, relative to
-// what is compared: a limb sum shifted into 32 bits is good to 2^-20 of its
-// column's largest value per 1024 samples, and columns of U (and y' over
-// ||y - mean||) hold no value above 1.  With xxM at least 0.02 c(n - c)/n the
-// r2 compared here is within 1 % of the exact one (up to 12,000 samples, 64
-// columns); the cut it is compared with is 10 % low.  The correlation is
-// within 1e-5 per 1024 samples; gate_lo and gate_hi leave 1e-4.
+// screen uses the integer, conversion and FP32 pipes only.  The r2 compared here
+// is within a few percent of that of the limb sums where xxM is at least XXM_FLOOR
+// of c (n - c) / n, and the cut it is compared with is 10 % low; the correlation is
+// within half the room of gate_lo and gate_hi.  set_screen checks both for the
+// phenotype (a limb sum shifted into 32 bits is good to 2^-20 of its column's
+// largest value per 1024 samples).
 // PAIRS: no correlation gate, and c = n is left to the FP64 form.
 template <bool GATE, bool PAIRS>
 __device__ __forceinline__ int screen_verdict(const ScreenParams& S, int n, int c, float ey, float ss, float gs,
@@ -558,7 +553,7 @@ __device__ __forceinline__ int screen_verdict(const ScreenParams& S, int n, int 
     if (!(q > S.gate_hi * xcn)) return 2;
   }
   const float xxM = xcn - ss, xyM = fmaf(S.b, cf, ey);
-  return xxM >= 0.02f * xcn && xcn > 0.0f && xyM * xyM < S.cut * xxM ? 1 : 2;
+  return xxM >= (float)XXM_FLOOR * xcn && xcn > 0.0f && xyM * xyM < S.cut * xxM ? 1 : 2;
 }
 // e_y / ynorm from the y' limb sums d[1..5], without the lowest limb.
 __device__ __forceinline__ float screen_ey(const ScreenParams& S, const uint32_t* d) {

@@ -33,7 +33,7 @@ struct EpiParams {
   double r2_cand;   // r2 below this cannot give p <= p_thresh (log/erfc skipped)
   int refine;       // 1: k-mers with r2 >= r2_ref go to the FP64 refinement list
   double r2_ref;
-  double r2_need;   // refinement may skip k-mers with r2 in [r2_ref, r2_need), see may_refine
+  double r2_need;   // refinement may skip k-mers with r2 in [r2_ref, r2_need), see may_refine; 0: none
   double thr2_ynorm2;  // corr_thr^2 * ynorm^2 (division-free Pearson gate)
   double gate_unit;    // the limbs' rounding moves x.(y - mean) by at most popcount(x) times this
   double a[KMAX];
@@ -62,11 +62,29 @@ inline void set_limb_consts(LimbMap& L) {
   }
 }
 
+// Smallest share of c (n - c) / n at which xxM is used to place a k-mer below a
+// cut, and how far below the cut it has to be.
+constexpr double XXM_FLOOR = 0.02, CUT_ROOM = 0.9;
+
+// Whether r2 = xyM^2 / (xxM yyM) below CUT_ROOM of a cut means that the exact r2
+// is below the cut, where xxM is at least XXM_FLOOR of xcn = c (n - c) / n.  u and
+// y: errors of (s_1 ..) and of xyM over sqrt(yyM cut), in units of sqrt(xcn).
+// xxM = xcn - |s|^2 with |s|^2 <= xcn is then off by at most (2 u + u^2) xcn.
+inline bool cut_room_covers(double u, double y) {
+  const double rho = (2.0 * u + u * u) / XXM_FLOOR, root = std::sqrt(CUT_ROOM) + y / std::sqrt(XXM_FLOOR);
+  return rho < 1.0 && root * root <= 0.999 * (1.0 - rho);
+}
+
 // The part of the refinement range that a launch without per-k-mer outputs
-// leaves out: a k-mer whose r2 in the split form is below 0.9 of the emit cut
+// leaves out: a k-mer whose r2 in the split form is below CUT_ROOM of the emit cut
 // is not emitted whatever the refinement gives, as long as the split form's
-// xxM is good to a few percent (may_refine).
-inline void set_refine_need(EpiParams& P) { P.r2_need = 0.9 * P.r2_cand; }
+// xxM is at least XXM_FLOOR of c (n - c) / n (may_refine) and the limbs are good
+// enough for that.  They are not where many values of a column are rounded the
+// same way (columns that mark single samples, n above about 10,000): there
+// every k-mer from r2_ref up is refined.
+inline void set_refine_need(EpiParams& P, const LimbLoss& B) {
+  P.r2_need = cut_room_covers(B.u, B.y / std::sqrt(P.yyM * P.r2_cand)) ? CUT_ROOM * P.r2_cand : 0.0;
+}
 
 // EpiParams::gate_unit: half a unit of the last limb of every column, U columns
 // weighted as the gate sums them.
@@ -76,43 +94,55 @@ inline void set_gate_unit(EpiParams& P, const LimbMap& L, bool drop0) {
 }
 
 // Screen constants of a phenotype whose intercept carries no limbs (drop0)
-// and whose limb columns are those of L (3 per U column, 5 for y').  See
-// screen_kmer for the error bounds behind the margins.
-inline void set_screen(EpiParams& P, const LimbMap& L, bool drop0) {
+// and whose limb columns are those of L: 3 per U column and 5 for y', of which
+// the lowest is not read, or with f64 the FP64 form's 7 and 8, of which the four
+// highest are read.  No screen where its margins (screen_verdict) do not cover
+// its rounding: the limb sums, shifted into 32 bits, and the digits that are not
+// read are off by at most two units S.su (S.sy) each, single precision by a few
+// 2^-24 of every term, and 1 / sqrt(xcn) is at most 1.5.
+inline void set_screen(EpiParams& P, const LimbMap& L, bool drop0, const LimbLoss& B, bool f64 = false) {
   ScreenParams& S = P.S;
   S = ScreenParams();
-  double cut = P.r2_cand;
-  if (P.refine && P.r2_ref < cut) cut = P.r2_ref > P.r2_need ? P.r2_ref : P.r2_need;
+  // a cut from r2_need stands for the exact r2, the others for the limb sums' own
+  double cut = P.r2_cand, lost_u = 0.0, lost_y = 0.0;
+  if (P.refine && P.r2_ref < cut) {
+    cut = P.r2_ref;
+    if (P.r2_need > cut) {
+      cut = P.r2_need;
+      lost_u = B.u;
+      lost_y = B.y / P.ynorm;
+    }
+  }
   const double yv = P.yyM / (P.ynorm * P.ynorm);
   // c - s_0^2 = c (n - c) / n, which the screen uses, holds for a unit intercept
   if (!(drop0 && std::fabs(P.a[0] * P.a[0] * P.n - 1.0) <= 1e-6) || !(P.ynorm >= 1e-12) || !(P.ynorm < 1e150) || !(cut > 0) || !(yv > 1e-6) || P.n >= 65536) return;
-  S.on = 1;
   while ((4 << S.shift) < P.n) ++S.shift;
   S.inv_n = (float)(1.0 / P.n);
   S.b = (float)(P.b / P.ynorm);
   S.kappa = (float)(P.kappa / P.ynorm);
-  S.cut = (float)(0.9 * cut * yv);
+  S.cut = (float)(CUT_ROOM * cut * yv);
   const double eps = 1e-4 * (P.n > 1024 ? P.n / 1024.0 : 1.0);
   const double lo = P.corr_thr > eps ? P.corr_thr - eps : 0.0, hi = P.corr_thr + eps;
   S.gate_lo = (float)(lo * lo);
   S.gate_hi = (float)(hi * hi);
   S.gate = P.corr_thr > 0.0;
-  // accumulators hold -128 x the digit sums; y' drops its lowest limb
-  const double unit = -(double)(1 << S.shift) / 128.0;
-  S.sy = (float)(unit * 65536.0 * L.scale[P.k] / P.ynorm);
+  // accumulators hold -128 x the digit sums
+  const double unit = -(double)(1 << S.shift) / 128.0, low3 = f64 ? 4294967296.0 : 1.0;  // 2^8 of the shift, 256^3
+  S.sy = (float)(unit * (f64 ? low3 * 256.0 : 65536.0) * L.scale[P.k] / P.ynorm);
+  double units2 = 0.0, gate = 0.0;
+  const double round = (P.k + 16) * 5.97e-8;  // of every term of a sum
   for (int j = 1; j < P.k; ++j) {
-    S.su[j - 1] = (float)(unit * L.scale[j]);
+    S.su[j - 1] = (float)(unit * low3 * L.scale[j]);
     S.g[j - 1] = (float)(P.g[j] / P.ynorm);
+    const double e = 2.0 * std::fabs((double)S.su[j - 1]);
+    units2 += e * e;
+    gate += std::fabs((double)S.g[j - 1]) * (1.5 * e + round * B.norm[j]);
   }
-}
-
-// The same for limb columns of the FP64 form (7 limbs per U column, 8 for y'),
-// of which the screen reads the four highest.
-inline void set_screen64(EpiParams& P, const LimbMap& L, bool drop0) {
-  set_screen(P, L, drop0);
-  const double f = 65536.0 * 65536.0;  // 2^8 of the shift, 256^3 of the lower limbs
-  for (int j = 0; j < KMAX; ++j) P.S.su[j] = (float)(P.S.su[j] * f);
-  P.S.sy = (float)(P.S.sy * (f * 256.0 / 65536.0));
+  const double ey = 3.0 * std::fabs((double)S.sy) + round * B.norm[P.k] / P.ynorm;
+  const double u = lost_u + 1.5 * std::sqrt(units2) + round;
+  const double y = lost_y + ey + round * std::fabs((double)S.b) * P.n;
+  gate += ey + round * std::fabs((double)S.kappa) * P.n;
+  S.on = cut_room_covers(u, y / std::sqrt(cut * yv)) && (!S.gate || gate <= 0.5 * eps);
 }
 
 // Constants of one phenotype for the 4-bit screen (kernel_fs.cu); everything

@@ -336,6 +336,37 @@ static double dot(const double* a, const double* b, int n) {
   return s[0] + s[1] + s[2] + s[3];
 }
 
+void column_norms(const Prepared& p, double* norm) {
+  for (int j = 0; j <= p.k; ++j) {
+    const double* d = &p.d[(size_t)j * p.n];
+    norm[j] = std::sqrt(dot(d, d, p.n));
+  }
+}
+
+void limb_loss(const Prepared& p, const double* scale, LimbLoss& B) {
+  B = LimbLoss();
+  column_norms(p, B.norm);
+  double n2 = 0, m2 = 0;
+  for (int j = 0; j <= p.k; ++j) {
+    if (!(scale[j] > 0)) continue;
+    const double* d = &p.d[(size_t)j * p.n];
+    const double sc = scale[j], up = 1.0 / sc;  // powers of two
+    double sq = 0, sum = 0;
+    for (int i = 0; i < p.n; ++i) {
+      const double r = d[i] - sc * std::round(d[i] * up);
+      sq += r * r;
+      sum += r;
+    }
+    if (j == p.k) {
+      B.y = std::sqrt(sq) + std::fabs(sum);
+    } else {
+      n2 += sq;
+      m2 += sum * sum;
+    }
+  }
+  B.u = std::sqrt(n2) + std::sqrt(m2);
+}
+
 void make_fs_cols(const Prepared& p, const int* pos, int n_row, int lu, bool gate, FsCols& F) {
   const int n = p.n, k = p.k, ku = k > 0 ? k - 1 : 0;
   F = FsCols();

@@ -79,6 +79,21 @@ void make_b_image_ts(const LimbCols& L, std::vector<int8_t>& img);
 // side in one MMA.
 void put_b_image_ts(const LimbCols& L, int col0, int N, std::vector<int8_t>& img);
 
+// What the limb columns leave out of a row's sums, as multiples of
+// ||x - mean(x)|| (limb_loss in prep.cpp; at most, whatever the row), and the
+// norms of the columns themselves.
+struct LimbLoss {
+  double u = 0, y = 0;       // the U columns together; y', in its own units
+  double norm[KMAX + 1] = {};  // [k]: y'
+};
+
+// LimbLoss of the columns d with limb scales `scale` (k + 1 values, y' last; 0: a
+// column without limbs, which is left out): with r the part of a column that its
+// limbs do not hold, |r.x| <= ||r|| ||x - mean(x)|| + c |sum r| / n, and c is at
+// most n ||x - mean(x)|| (a row of c = n - 1 samples has that of a single one).
+void column_norms(const Prepared& p, double* norm);
+void limb_loss(const Prepared& p, const double* scale, LimbLoss& B);
+
 // The contraction columns in e2m1 (4-bit) limbs for the screen of kernel_fs.cu:
 // count, 3 limbs of y', with `gate` 4 of y - mean(y), lu per U column 1 .. k-1
 // (prepare's drop0 must hold).  A limb holds the nearest e2m1 values of what

@@ -190,6 +190,7 @@ int kg_pairs_run_host(kg_ctx* ctx, const uint64_t* xbits, uint64_t n_kmers, uint
                         &ctx->LM, &O, ctx->num_sms};
       e = kg::launch_pairs(L, st);
     }
+    if (e != cudaSuccess) return ctx->cuda_fail(e, "pair kernel launch");
     kg::LaunchPairRefine R{ctx->dPX, (int)wd, ctx->dT, ctx->nsteps * 128, ctx->cm, &ctx->P, &O, ctx->num_sms, fs,
                           &ctx->LM, ctx->dV};
     e = kg::launch_pair_refine(R, st);

@@ -177,9 +177,10 @@ int kg_pairs_run_host(kg_ctx* ctx, const uint64_t* xbits, uint64_t n_kmers, uint
   for (int attempt = 0; attempt < 8; ++attempt) {
     kg::DevOutPairs O{ctx->dCounters, ctx->dPairs, ctx->pair_cap, ctx->dCand, ctx->cand_cap, ctx->wait_ns};
     KG_CUDA(cudaMemsetAsync(ctx->dCounters, 0, 4 * sizeof(unsigned long long), st), "memset");
-    // the 4-bit screen, unless another kernel is asked for
+    // the 4-bit screen, unless another kernel is asked for; no pair is evaluated
+    // where yyM is rounding (the kernels' eps), which the screen does not look at
     const char* force = std::getenv("KG_KERNEL");
-    const bool fs = ctx->fs_N && !force && kg::fsp_supported(ctx->fs_N, ctx->fs_lu, ctx->fs_kpad, (int)wd, ic);
+    const bool fs = ctx->fs_N && !force && ctx->P.yyM > 1e-12 && kg::fsp_supported(ctx->fs_N, ctx->fs_lu, ctx->fs_kpad, (int)wd, ic);
     cudaError_t e;
     if (fs) {
       kg::LaunchFsPairs L{ctx->dPX, (int)wd, ctx->fs_kpad, ctx->fs_N, ctx->fs_lu, ctx->P.corr_thr > 0.0, S, ctx->dFs,

@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(pr_threads(N), 1)
         if (lane == 0) mbar_arrive(acc_empty + 8 * e);
         const unsigned long long j = U.jb * PR_TM + r;
         const bool valid = j < S.n_kmers && j > i;
-        if (DROP0 && P.S.on) {
+        if (DROP0 && P.S.on && P.yyM > 1e-12) {  // a screened pair counts as evaluated
           const int v2 = screen_kmer<KU_MAX, 5, false, true>(P.S, P.n, d, ku, valid);
           if (!__any_sync(0xffffffffu, v2 == 2)) {
             evaluated += v2 ? 1u : 0u;

@@ -36,9 +36,10 @@ int set_f64_limbs(kg_ctx* ctx, int n_row) {
   std::vector<double> mx((size_t)k + 1, 0.0);
   for (int j = 0; j <= k; ++j)
     for (int i = 0; i < n; ++i) mx[j] = std::max(mx[j], std::fabs(p.d[(size_t)j * n + i]));
-  // the intercept's centred part is left out only where it is rounding noise of
-  // U itself: below 1e-14 it moves xxM by less than a rounding of the count
-  const bool drop0 = k > 0 && mx[0] <= 1e-14 * std::fabs(p.a[0]);
+  // the intercept's centred part has a single limb where it is rounding noise of U
+  // itself: below 5e-15 of the column, what that limb leaves out (a 63rd of it)
+  // moves xxM by at most 1.6e-16 of the count
+  const bool drop0 = k > 0 && mx[0] <= 5e-15 * std::fabs(p.a[0]);
   const int N = kg::f64_limb_cols(k, drop0);
   const int wpk = ((n_row + 63) / 64 + 1) / 2 * 2;
   if (major != 10 || minor != 0 || !kg::f64_limbs_supported(N, n_row, wpk)) return KG_OK;
@@ -46,14 +47,16 @@ int set_f64_limbs(kg_ctx* ctx, int n_row) {
   ph.P = ctx->P;
   ph.drop0 = drop0;
   double up[kg::KMAX + 1] = {};
-  for (int j = drop0; j <= k; ++j) {
+  for (int j = 0; j <= k; ++j) {
     // half the largest magnitude of the limbs, as in make_limbs
-    const double lim = 127.0 * std::ldexp(1.0, 8 * (j == k ? 7 : 6) - 1);
+    const bool noise = j == 0 && drop0;
+    const double lim = 127.0 * std::ldexp(1.0, 8 * (j == k ? 7 : noise ? 0 : 6) - 1);
     int s = 0;
     if (mx[j] > 0) {
       std::frexp(lim / mx[j], &s);
       --s;
     }
+    if (noise) s = std::min(s, 1000);
     if (s > 1000 || s < -1000) return KG_OK;
     up[j] = std::ldexp(1.0, s);
     ph.LM.scale[j] = std::ldexp(1.0, -s);

@@ -85,16 +85,18 @@ __device__ __forceinline__ void tb_single(const DevOut& O, const MPheno* ME, uin
 }
 
 // ---------------------------------------------------- FP64 form in limbs
-// Columns: the count, 8 limbs of y', 7 of every U column with limbs (62 and 54
+// Columns: the count, 8 limbs of y', one for the centred part of U column 0 where
+// that is rounding noise of U itself (drop0), 7 of every other U column (62 and 54
 // bits below the column's largest value, so at least what a double holds of
 // it).  The sums are exact and rounded once, where fp64_kernel rounds after
 // every sample: the error against 64 bits is that of fp64_kernel or below it
 // (8.2e-14 and 3.1e-13 in p-values at n = 1000 were the same on both).
 // fp64_kernel does n (k + 2) FP64 multiply-adds per k-mer, half of whose time
 // goes to broadcasting the columns from shared memory; here they are int8 MMAs
-// of 8 + 7 k columns.  5e6 k-mers, r = 10+1, n = 1000: 9.70 -> 0.37 ms; 3e5 at
+// of 9 + 7 k columns.  5e6 k-mers, r = 10+1, n = 1000: 9.70 -> 0.37 ms; 3e5 at
 // n = 5000, r = 32+1: 6.79 -> 0.22 ms; 5e6 at n = 200, r = 5+1: 1.25 -> 0.16 ms.
 constexpr int F64_LY = 8, F64_LU = 7;
+constexpr int F64_E0 = 1 + F64_LY, F64_U = F64_E0 + 1;  // the noise column, the first U column with 7 limbs
 
 __device__ __forceinline__ long long limb4(const uint32_t* d) {
   return mad_wide<(1 << 24)>(d[0], limb3(d[1], d[2], d[3]));
@@ -105,7 +107,7 @@ __device__ __forceinline__ long long limb4(const uint32_t* d) {
 // (column(j, d)) as they arrive.
 template <int N, class F, class G>
 __device__ __forceinline__ void f64_columns(uint32_t taddr, int ku, F first, G column) {
-  constexpr int KU = (N - 1 - F64_LY) / F64_LU;
+  constexpr int KU = (N - F64_U) / F64_LU;
   uint32_t d[N];
 #pragma unroll
   for (int q = 0; q < N; q += 32) {
@@ -117,7 +119,7 @@ __device__ __forceinline__ void f64_columns(uint32_t taddr, int ku, F first, G c
     if (q == 0) first(d);
 #pragma unroll
     for (int j = 0; j < KU; ++j) {
-      const int o = 1 + F64_LY + F64_LU * j;
+      const int o = F64_U + F64_LU * j;
       // N is rounded up to 16: at most two groups past the last column
       if (o + F64_LU - 1 >= q && o + F64_LU - 1 < q + 32 && (j < KU - 2 || j < ku)) column(j, d + o);
     }
@@ -168,8 +170,9 @@ __device__ __forceinline__ void tb_single64(const DevOut& O, const MPheno* ME, u
         const double sy = ME->LM.esc[P.k];
         ey = fma(i2d_exact(limb4(d + 1)), sy * 4294967296.0, i2d_exact(limb4(d + 5)) * sy);
         if (drop0) {
-          const double s0 = P.a[0] * cd;
+          const double e0 = i2d_exact((int)d[F64_E0]) * ME->LM.esc[0], s0 = fma(P.a[0], cd, e0);
           ss = s0 * s0;
+          gs = P.g[0] * e0;
         }
       },
       [&](int jj, const uint32_t* d) {
@@ -199,10 +202,11 @@ __global__ void __launch_bounds__(128) f64_image_kernel(const double* __restrict
   if (i >= kpad) return;
   const int a = i >> 7, q = (i >> 5) & 3, t = (i >> 3) & 3, jj = 7 - (i & 7);
   const int kap = 128 * a + 4 * (8 * q + jj) + t;
-  const int j = col < 2 ? k : col - 2 + drop0;  // U column (k: y')
+  if (col == 2 && !drop0) return;
+  const int j = col < 2 ? k : col == 2 ? 0 : col - 3 + drop0;  // U column (k: y')
   const int vc = col == 0 ? 0 : 1 + j;
-  const int L = col == 0 ? 1 : col == 1 ? F64_LY : F64_LU;
-  const int first = col == 0 ? 0 : col == 1 ? 1 : 1 + F64_LY + F64_LU * (col - 2);
+  const int L = col == 0 || col == 2 ? 1 : col == 1 ? F64_LY : F64_LU;
+  const int first = col == 0 ? 0 : col == 1 ? 1 : col == 2 ? F64_E0 : F64_U + F64_LU * (col - 3);
   long long v = 0;
   if (i < vrows) v = __double2ll_rn(V[(size_t)i * cm + vc] * (col == 0 ? 1.0 : S.up[j]));
   if (jj & 1) v *= -2;
@@ -593,7 +597,7 @@ int tb_ring(int N) {
 }
 
 int f64_limb_cols(int k, bool drop0) {
-  const int used = 1 + F64_LY + F64_LU * (k - (drop0 ? 1 : 0));
+  const int used = F64_U + F64_LU * (k - (drop0 ? 1 : 0));
   return (used + 15) / 16 * 16;
 }
 
@@ -607,7 +611,7 @@ cudaError_t launch_f64_image(const LaunchF64Image& L, cudaStream_t st) {
   for (int j = 0; j <= L.k; ++j) S.up[j] = L.up[j];
   cudaError_t e = cudaMemsetAsync(L.img, 0, (size_t)L.kpad * L.N, st);
   if (e != cudaSuccess) return e;
-  const dim3 grid((unsigned)((L.kpad + 127) / 128), (unsigned)(2 + L.k - (L.drop0 ? 1 : 0)));
+  const dim3 grid((unsigned)((L.kpad + 127) / 128), (unsigned)(3 + L.k - (L.drop0 ? 1 : 0)));
   f64_image_kernel<<<grid, 128, 0, st>>>(L.V, L.vrows, L.cm, L.k, L.drop0 ? 1 : 0, L.kpad, L.N, S, L.img);
   return cudaGetLastError();
 }

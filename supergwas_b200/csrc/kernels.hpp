@@ -95,7 +95,7 @@ struct LaunchTb {
 struct LaunchF64Image {
   const double* V;            // FP64 columns (LaunchFp64::V), vrows x cm
   int vrows, cm, k;
-  bool drop0;                 // U column 0 has no limbs
+  bool drop0;                 // U column 0 has a single limb
   int kpad, N;                // f64_limb_cols columns
   const double* up;           // k + 1 scales 2^s (powers of two) of the columns, y' last
   int8_t* img;                // kpad x N bytes (device)

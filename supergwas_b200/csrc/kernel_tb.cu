@@ -601,9 +601,16 @@ int f64_limb_cols(int k, bool drop0) {
   return (used + 15) / 16 * 16;
 }
 
+// Samples up to which the sum of four limbs is an exact double: digits of
+// magnitude 128 enter every second sample as 128 x and the others as 64 x, and
+// i2d_exact takes integers below 2^51.
+constexpr int F64_NMAX = 10880;
+static_assert((long long)F64_NMAX / 2 * 128 * (128 + 64) * ((1ll << 24) + (1ll << 16) + (1ll << 8) + 1) < (1ll << 51),
+              "limb4 sums");
+
 bool f64_limbs_supported(int N, int n_row, int wpk) {
   int xst, nb;
-  return N <= 256 && n_row <= 12288 && tb_rings(N, tb_box_bytes(wpk), xst, nb);
+  return N <= 256 && n_row <= F64_NMAX && tb_rings(N, tb_box_bytes(wpk), xst, nb);
 }
 
 cudaError_t launch_f64_image(const LaunchF64Image& L, cudaStream_t st) {

@@ -343,7 +343,8 @@ int check_multi(kg_ctx* ctx, const void* x, uint64_t m, uint32_t wpk) {
   if ((uint64_t)wpk * 64 < (uint64_t)M.n_row) return ctx->fail(KG_ERR_INVALID, "words_per_kmer*64 < samples per row");
   if (!kg::mp_supported(M.NP, M.PPG, (int)wpk))
     return ctx->fail(KG_ERR_UNSUPPORTED, "rows must be at least 128 bytes (pad words_per_kmer to 16)");
-  if (m >= (1ull << 48)) return ctx->fail(KG_ERR_UNSUPPORTED, "more than 2^48 k-mers in one call");
+  // bit 47 of a refinement candidate marks an open gate (CAND_OPEN_MP)
+  if (m >= (1ull << 47)) return ctx->fail(KG_ERR_UNSUPPORTED, "2^47 k-mers or more in one call");
   return KG_OK;
 }
 

@@ -4,8 +4,10 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
+#include <memory>
+#include <new>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -353,11 +355,20 @@ namespace kgctx {
 cudaError_t stage_h2d(void* dst, void* stage, const void* src, size_t bytes, cudaStream_t st) {
   const size_t B = (size_t)4 << 20, nb = (bytes + B - 1) / B;
   const unsigned nt = (unsigned)std::min<size_t>(std::min<unsigned>(16, std::max(1u, std::thread::hardware_concurrency())), nb);
-  if (nt <= 1) {
+  std::unique_ptr<std::atomic<int>[]> filled;
+  std::vector<std::thread> th;
+  try {
+    if (nt > 1) {
+      th.reserve(nt);
+      filled.reset(new std::atomic<int>[nb]());
+    }
+  } catch (const std::bad_alloc&) {
+    // no room for threads
+  }
+  if (!filled) {
     std::memcpy(stage, src, bytes);
     return cudaMemcpyAsync(dst, stage, bytes, cudaMemcpyHostToDevice, st);
   }
-  std::vector<std::atomic<int>> filled(nb);
   std::atomic<size_t> next{0};
   auto fill_one = [&] {
     const size_t i = next.fetch_add(1);
@@ -366,12 +377,10 @@ cudaError_t stage_h2d(void* dst, void* stage, const void* src, size_t bytes, cud
     filled[i].store(1, std::memory_order_release);
     return true;
   };
-  std::vector<std::thread> th;
-  th.reserve(nt);
   try {
     for (unsigned t = 1; t < nt; ++t) th.emplace_back([&] { while (fill_one()) {} });
-  } catch (const std::system_error&) {
-    // as many threads as there are; this one fills blocks too
+  } catch (const std::exception&) {
+    // as many threads as there are resources for; this one fills blocks too
   }
   cudaError_t e = cudaSuccess;
   for (size_t i = 0; i < nb; ++i) {

@@ -4,9 +4,9 @@
 #include <chrono>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <new>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -317,11 +317,11 @@ int set_screen4_multi(kg_ctx* ctx, const kg_pheno* ph, const std::vector<kg::Pre
   };
   const int nt = std::max(1, std::min<int>({8, (int)std::thread::hardware_concurrency(), np}));
   std::vector<std::thread> th;
-  th.reserve((size_t)nt);
   try {
+    th.reserve((size_t)nt);
     for (int t = 1; t < nt; ++t) th.emplace_back(work);
-  } catch (const std::system_error&) {
-    // as many threads as there are
+  } catch (const std::exception&) {
+    // as many threads as there are resources for
   }
   work();
   for (auto& t : th) t.join();

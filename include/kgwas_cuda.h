@@ -266,6 +266,11 @@ int kg_last_launch_count(const kg_ctx* ctx);
  * shared memory; other limb counts, unaligned rows) or "fp64". */
 const char* kg_last_kernel(const kg_ctx* ctx);
 
+/* Limbs per U column of the 4-bit screen that ran before that kernel in the last
+ * launch (kg_run_host, kg_launch_device, kg_pairs_run_host and the many-phenotype
+ * calls); 0: every k-mer or pair was evaluated by the kernel itself. */
+int kg_last_screen(const kg_ctx* ctx);
+
 /* Rows the last kg_run_host tested on the device when it used runs of equal
  * adjacent rows (0 when it tested every row).  Batches sorted by bit pattern
  * (src/convert_matrix.cpp:366-368) hold such runs; one row per run is tested,

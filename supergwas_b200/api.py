@@ -117,6 +117,8 @@ def lib():
     L.kg_last_launch_count.argtypes = [vp]
     L.kg_last_kernel.argtypes = [vp]
     L.kg_last_kernel.restype = ctypes.c_char_p
+    L.kg_last_screen.argtypes = [vp]
+    L.kg_last_screen.restype = ctypes.c_int
     L.kg_last_unique_rows.argtypes = [vp]
     L.kg_last_unique_rows.restype = ctypes.c_uint64
     L.kg_last_error.argtypes = [vp]
@@ -357,6 +359,10 @@ class Kgwas:
 
     def last_kernel(self) -> str:
         return self._L.kg_last_kernel(self._h).decode()
+
+    def last_screen(self) -> int:
+        """Limbs per U column of the last launch's 4-bit screen, 0 without one (kg_last_screen)."""
+        return int(self._L.kg_last_screen(self._h))
 
     def reserve_host(self, n_kmers: int, words_per_kmer: int):
         """Allocate now the buffers run_host needs for a batch of this shape (kg_reserve_host)."""

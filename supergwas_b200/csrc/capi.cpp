@@ -210,6 +210,8 @@ int kg_last_launch_count(const kg_ctx* ctx) { return ctx ? ctx->launches : 0; }
 
 const char* kg_last_kernel(const kg_ctx* ctx) { return ctx ? ctx->last_kernel : ""; }
 
+int kg_last_screen(const kg_ctx* ctx) { return ctx ? ctx->last_screen : 0; }
+
 int kg_set_wait_limit(kg_ctx* ctx, uint64_t wait_ns) {
   if (!ctx) return KG_ERR_INVALID;
   ctx->wait_ns = wait_ns;
@@ -662,6 +664,7 @@ int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64
     O.cor = ctx->dStat[6];
   }
   cudaError_t e;
+  ctx->last_screen = 0;
   if (ctx->opts.precision == KG_PREC_FP64) {
     const char* force = std::getenv("KG_KERNEL");
     if (ctx->f64_N && ((uintptr_t)dx % 16) == 0 && m <= 0x7fffff00ull &&
@@ -695,6 +698,7 @@ int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64
                                  st);
         if (e != cudaSuccess) return ctx->cuda_fail(e, "gather launch");
         ctx->launches += 2;
+        ctx->last_screen = ctx->fs_lu;
         O.index = ctx->dCand;
         O.rows = ctx->dCounters + 3;
         O.stall_loads = 0;
@@ -723,6 +727,7 @@ int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64
     if (ctx->fs_N && tma_ok && !stats && !force && kg::fs_supported(ctx->fs_N, ctx->fs_kpad, (int)wpk)) {
       e = launch_screen4(ctx, dx, m, wpk, O, st);
       ctx->last_kernel = "ts";
+      ctx->last_screen = ctx->fs_lu;
     } else if (ts_ok && !want_ss) {
       kg::LaunchTs L{dx, m, (int)wpk, ctx->limbs.Kpad, ctx->prep.drop0 && ctx->P.k > 0, ctx->dBts, &ctx->P,
                      &ctx->LM, &O, ctx->num_sms};

@@ -197,6 +197,7 @@ int kg_pairs_run_host(kg_ctx* ctx, const uint64_t* xbits, uint64_t n_kmers, uint
     e = kg::launch_pair_refine(R, st);
     if (e != cudaSuccess) return ctx->cuda_fail(e, "pair refinement launch");
     ctx->launches = 2;
+    ctx->last_screen = fs ? ctx->fs_lu : 0;
     KG_CUDA(cudaMemcpyAsync(cnt, ctx->dCounters, sizeof(cnt), cudaMemcpyDeviceToHost, st), "copy counters");
     KG_CUDA(cudaStreamSynchronize(st), "pair kernels");
     if (cnt[2] & ~(unsigned long long)(kg::ERR_HIT_OVERFLOW | kg::ERR_CAND_OVERFLOW))

@@ -208,6 +208,7 @@ struct kg_ctx {
   cudaStream_t pend_stream = nullptr;
   int launches = 0;
   const char* last_kernel = "";
+  int last_screen = 0;       // limbs per U column of the last launch's 4-bit screen
   // bounded device waits: pipeline wait limit (0: the default) and the
   // one-launch stall of the row producer that the failure tests use
   unsigned long long wait_ns = 0;

@@ -268,7 +268,9 @@ const char* kg_last_kernel(const kg_ctx* ctx);
 
 /* Limbs per U column of the 4-bit screen that ran before that kernel in the last
  * launch (kg_run_host, kg_launch_device, kg_pairs_run_host and the many-phenotype
- * calls); 0: every k-mer or pair was evaluated by the kernel itself. */
+ * calls); 0: every k-mer or pair was evaluated by the kernel itself.  Negative,
+ * once the results have been read, where the screen left too much undecided in a
+ * part of the launch and gave up: the kernel has evaluated that part. */
 int kg_last_screen(const kg_ctx* ctx);
 
 /* Rows the last kg_run_host tested on the device when it used runs of equal

@@ -361,7 +361,8 @@ class Kgwas:
         return self._L.kg_last_kernel(self._h).decode()
 
     def last_screen(self) -> int:
-        """Limbs per U column of the last launch's 4-bit screen, 0 without one (kg_last_screen)."""
+        """Limbs per U column of the last launch's 4-bit screen, 0 without one, negative where it
+        gave up (kg_last_screen)."""
         return int(self._L.kg_last_screen(self._h))
 
     def reserve_host(self, n_kmers: int, words_per_kmer: int):

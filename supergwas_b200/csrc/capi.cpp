@@ -146,7 +146,7 @@ int kg_create(kg_ctx** out, const kg_opts* opts) {
       cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, ctx->opts.device) != cudaSuccess ||
       cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMalloc((void**)&ctx->dCounters, 4 * sizeof(unsigned long long)) != cudaSuccess) {
+      cudaMalloc((void**)&ctx->dCounters, kg::NCOUNT * sizeof(unsigned long long)) != cudaSuccess) {
     kg_destroy(ctx);
     return KG_ERR_CUDA;
   }
@@ -418,6 +418,21 @@ void par_gather(void* dst, const uint64_t* x, const uint64_t* sel, uint64_t cnt,
   for (auto& t : th) t.join();
 }
 
+unsigned long long open_base() {
+  const char* v = std::getenv("KG_SCREEN_OPEN");
+  return v ? std::strtoull(v, nullptr, 10) : kg::FS_OPEN_BASE;
+}
+
+int ensure_cand(kg_ctx* ctx, unsigned long long cap) {
+  if (ctx->cand_cap >= cap && ctx->dCand) return KG_OK;
+  drop_graph(ctx->mp);  // it holds the list's address
+  dfree(ctx->dCand);
+  ctx->cand_cap = 0;
+  KG_CUDA(cudaMalloc((void**)&ctx->dCand, cap * sizeof(unsigned long long)), "cudaMalloc(candidates)");
+  ctx->cand_cap = cap;
+  return KG_OK;
+}
+
 bool is_pinned(const void* p) {
   cudaPointerAttributes attr{};
   const bool pinned = cudaPointerGetAttributes(&attr, p) == cudaSuccess &&
@@ -576,23 +591,6 @@ int ensure_hits(kg_ctx* ctx, unsigned long long cap) {
   return KG_OK;
 }
 
-int ensure_cand(kg_ctx* ctx, unsigned long long cap) {
-  if (ctx->cand_cap >= cap && ctx->dCand) return KG_OK;
-  dfree(ctx->dCand);
-  ctx->cand_cap = 0;
-  KG_CUDA(cudaMalloc((void**)&ctx->dCand, cap * sizeof(unsigned long long)), "cudaMalloc(candidates)");
-  ctx->cand_cap = cap;
-  return KG_OK;
-}
-
-// After a launch with more candidates than room: a longer list, or, in the FP64
-// form, no screen for this structure.
-int cand_overflow(kg_ctx* ctx) {
-  if (ctx->opts.precision != KG_PREC_FP64) return ensure_cand(ctx, 4 * ctx->cand_cap);
-  ctx->fs_N = 0;
-  return KG_OK;
-}
-
 int ensure_stats(kg_ctx* ctx, size_t m) {
   if (ctx->stat_cap >= m && ctx->dTested) return KG_OK;
   dfree(ctx->dTested);
@@ -635,13 +633,17 @@ cudaError_t launch_screen4(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t
 }
 
 // FP64 form behind the 4-bit screen: smallest work (k-mers x samples x limb
-// columns) and the rows that the screen may leave.
+// columns), and the most bytes of rows that the screen may leave.
 constexpr double FS64_MIN = 3.2e10;
-constexpr unsigned long long FS64_ROWS = 1ull << 16;
+constexpr size_t FS64_BYTES = (size_t)256 << 20;
 
-int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64_t offset, bool stats,
-               cudaStream_t st) {
+// One launch on the rows dx.  fresh: the counters have just been cleared.
+int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64_t offset, bool stats, bool fresh,
+               Screen mode, cudaStream_t st) {
+  ctx->last_screen = 0;
   if (m == 0) return KG_OK;
+  // refinement candidates and the screen's counts of this launch start from zero
+  if (!fresh) KG_CUDA(cudaMemsetAsync(ctx->dCounters + 3, 0, 4 * sizeof(unsigned long long), st), "memset");
   kg::DevOut O{};
   O.counters = ctx->dCounters;
   O.hits = ctx->dHits;
@@ -651,6 +653,7 @@ int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64
   O.cand_cap = ctx->cand_cap;
   O.weight = ctx->cur_weight;
   O.wait_ns = ctx->wait_ns;
+  O.open_base = open_base();
   O.stall_loads = ctx->stall_once;
   ctx->stall_once = 0;
   if (stats) {
@@ -664,7 +667,6 @@ int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64
     O.cor = ctx->dStat[6];
   }
   cudaError_t e;
-  ctx->last_screen = 0;
   if (ctx->opts.precision == KG_PREC_FP64) {
     const char* force = std::getenv("KG_KERNEL");
     if (ctx->f64_N && ((uintptr_t)dx % 16) == 0 && m <= 0x7fffff00ull &&
@@ -675,45 +677,51 @@ int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64
                      ctx->num_sms, true};
       // Batches large enough to be worth two launches more (the line: 4e5 k-mers
       // at n = 1000, r = 10+1, 80 columns, where the limb kernel takes 35 us): the
-      // 4-bit screen, and the limb kernel on the rows that it leaves undecided.  A
-      // call that returns with more of those than there is room for is repeated
-      // without the screen (ctx->fs_N = 0 from then on).
-      const bool screen = ctx->fs_N && !stats && !force && (double)m * kpad * ctx->f64_N >= FS64_MIN &&
+      // 4-bit screen, and the limb kernel on the rows that it leaves undecided, or on
+      // all of them where it gives up.  65536 rows of room (1e8 k-mers at 6e-4
+      // undecided filled them) made the whole call repeat.
+      const bool screen = ctx->fs_N && mode != SCREEN_OFF && !stats && !force &&
+                          (double)m * kpad * ctx->f64_N >= FS64_MIN &&
                           kg::fs_supported(ctx->fs_N, ctx->fs_kpad, (int)wpk);
       if (screen) {
-        const size_t bytes = (size_t)FS64_ROWS * wpk * 8;
+        const size_t row = (size_t)wpk * 8;
+        const unsigned long long cap =
+            std::min<unsigned long long>(kg::fs_open_limit(O.open_base, m, m, O.cand_cap), FS64_BYTES / row);
+        const size_t bytes = cap * row;
         if (ctx->gather_bytes < bytes) {
           dfree(ctx->dGather);
           ctx->gather_bytes = 0;
           KG_CUDA(cudaMalloc((void**)&ctx->dGather, bytes), "cudaMalloc(rows)");
           ctx->gather_bytes = bytes;
         }
-        KG_CUDA(cudaMemsetAsync(ctx->dCounters + 3, 0, sizeof(unsigned long long), st), "memset");
-        const unsigned long long cap = std::min<unsigned long long>(O.cand_cap, FS64_ROWS);
-        O.cand_cap = cap;
-        O.count_sure = 1;
-        e = launch_screen4(ctx, dx, m, wpk, O, st);
+        kg::DevOut S = O;
+        S.cand_cap = cap;
+        S.count_sure = 1;
+        e = launch_screen4(ctx, dx, m, wpk, S, st);
         if (e != cudaSuccess) return ctx->cuda_fail(e, "kernel launch");
-        e = kg::launch_fs_gather(dx, (int)wpk, ctx->dCand, ctx->dCounters + 3, cap, offset, ctx->dGather, ctx->num_sms,
-                                 st);
+        e = kg::launch_fs_gather(dx, (int)wpk, ctx->dCand, ctx->dCounters, offset, ctx->dGather, ctx->num_sms, st);
         if (e != cudaSuccess) return ctx->cuda_fail(e, "gather launch");
-        ctx->launches += 2;
-        ctx->last_screen = ctx->fs_lu;
-        O.index = ctx->dCand;
-        O.rows = ctx->dCounters + 3;
+        O.over = ctx->dCounters + kg::CNT_FS_OVER;
         O.stall_loads = 0;
-        L.x = ctx->dGather;
-        L.m = cap;
+        S = O;
+        S.index = ctx->dCand;
+        S.rows = ctx->dCounters + kg::CNT_FS_OPEN;
+        kg::LaunchTb Lg = L;
+        Lg.x = ctx->dGather;
+        Lg.m = cap;
+        Lg.O1 = &S;
+        e = kg::launch_tb(Lg, st);
+        if (e != cudaSuccess) return ctx->cuda_fail(e, "kernel launch");
+        ctx->launches += mode == SCREEN_BEHIND ? 3 : 2;
+        ctx->last_screen = ctx->fs_lu;
       }
-      e = kg::launch_tb(L, st);
+      if (!screen || mode == SCREEN_BEHIND) e = kg::launch_tb(L, st);
     } else {
       kg::LaunchFp64 L{dx, m, (int)wpk, ctx->dV, ctx->nsteps, ctx->cm, &ctx->P, &O, ctx->num_sms};
       e = kg::launch_fp64(L, st);
     }
     ctx->last_kernel = "fp64";
   } else {
-    // refinement candidates of this launch start from zero
-    KG_CUDA(cudaMemsetAsync(ctx->dCounters + 3, 0, sizeof(unsigned long long), st), "memset");
     const char* force = std::getenv("KG_KERNEL");
     const bool want_ss = force && std::string(force) == "ss";
     // 16-byte aligned rows with 31-bit row coordinates: the TMA kernels
@@ -724,10 +732,19 @@ int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64
     const bool tb_ok = tma_ok && !ts_ok && ctx->dPh1 && kg::tb_supported(ctx->limbs.N, (int)wpk);
     if (force && std::string(force) == "ts" && !ts_ok)
       return ctx->fail(KG_ERR_UNSUPPORTED, "KG_KERNEL=ts: shape not supported by the TMEM-A kernel");
-    if (ctx->fs_N && tma_ok && !stats && !force && kg::fs_supported(ctx->fs_N, ctx->fs_kpad, (int)wpk)) {
+    const bool screen = ctx->fs_N && mode != SCREEN_OFF && tma_ok && !stats && !force &&
+                        kg::fs_supported(ctx->fs_N, ctx->fs_kpad, (int)wpk);
+    if (screen) {
       e = launch_screen4(ctx, dx, m, wpk, O, st);
-      ctx->last_kernel = "ts";
+      if (e != cudaSuccess) return ctx->cuda_fail(e, "kernel launch");
       ctx->last_screen = ctx->fs_lu;
+      O.over = ctx->dCounters + kg::CNT_FS_OVER;
+      O.stall_loads = 0;
+    }
+    const bool behind = screen && mode == SCREEN_BEHIND && m > O.open_base;  // with fewer it cannot give up
+    if (behind) ++ctx->launches;
+    if (screen && !behind) {
+      // the screen alone
     } else if (ts_ok && !want_ss) {
       kg::LaunchTs L{dx, m, (int)wpk, ctx->limbs.Kpad, ctx->prep.drop0 && ctx->P.k > 0, ctx->dBts, &ctx->P,
                      &ctx->LM, &O, ctx->num_sms};
@@ -743,6 +760,7 @@ int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64
       e = kg::launch_tc(L, st);
       ctx->last_kernel = "ss";
     }
+    if (screen) ctx->last_kernel = "ts";
   }
   if (e != cudaSuccess) return ctx->cuda_fail(e, "kernel launch");
   ++ctx->launches;
@@ -818,6 +836,15 @@ int ensure_chunks(kg_ctx* ctx, size_t bytes, bool staging) {
   return KG_OK;
 }
 
+// The counters of the launches on st, and what became of their screens.
+int read_counters(kg_ctx* ctx, cudaStream_t st) {
+  KG_CUDA(cudaMemcpyAsync(ctx->counters, ctx->dCounters, sizeof(ctx->counters), cudaMemcpyDeviceToHost, st),
+          "copy counters");
+  KG_CUDA(cudaStreamSynchronize(st), "kernel");
+  if (ctx->counters[kg::CNT_FS_EVER] && ctx->last_screen > 0) ctx->last_screen = -ctx->last_screen;
+  return KG_OK;
+}
+
 int run_host_once(kg_ctx* ctx, const uint64_t* xbits, uint64_t m, uint32_t wpk, bool stats, bool runs) {
   const size_t row = (size_t)wpk * 8;
   const uint64_t per = host_chunk_rows(m, wpk);
@@ -845,7 +872,7 @@ int run_host_once(kg_ctx* ctx, const uint64_t* xbits, uint64_t m, uint32_t wpk, 
     }
     ctx->cur_weight = ctx->dWeight;
   }
-  KG_CUDA(cudaMemsetAsync(ctx->dCounters, 0, 4 * sizeof(unsigned long long), ctx->stream), "memset");
+  KG_CUDA(cudaMemsetAsync(ctx->dCounters, 0, sizeof(ctx->counters), ctx->stream), "memset");
   const uint64_t nch = (m + per - 1) / per;
   uint64_t u0 = 0;  // runs before this chunk
   std::vector<StageSeg> segs;
@@ -882,16 +909,12 @@ int run_host_once(kg_ctx* ctx, const uint64_t* xbits, uint64_t m, uint32_t wpk, 
     }
     KG_CUDA(cudaEventRecord(ctx->ev_h2d[b], ctx->copy_stream), "record");
     KG_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->ev_h2d[b], 0), "wait");
-    int rc = launch_one(ctx, ctx->dChunk[b], rows, wpk, offset, stats, ctx->stream);
+    int rc = launch_one(ctx, ctx->dChunk[b], rows, wpk, offset, stats, i == 0, SCREEN_BEHIND, ctx->stream);
     if (rc) return rc;
     KG_CUDA(cudaEventRecord(ctx->ev_k[b], ctx->stream), "record");
   }
   if (runs) ctx->unique_rows = u0;
-  KG_CUDA(cudaMemcpyAsync(ctx->counters, ctx->dCounters, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                          ctx->stream),
-          "copy counters");
-  KG_CUDA(cudaStreamSynchronize(ctx->stream), "kernel");
-  return KG_OK;
+  return read_counters(ctx, ctx->stream);
 }
 
 }  // namespace
@@ -909,7 +932,7 @@ int kg_run_host(kg_ctx* ctx, const uint64_t* xbits, uint64_t m, uint32_t wpk, kg
   const bool stats = want_stats(st);
   if (stats && (rc = ensure_stats(ctx, m))) return rc;
   if ((rc = ensure_hits(ctx, std::max<unsigned long long>(ctx->hit_cap, 1ull << 16)))) return rc;
-  if ((rc = ensure_cand(ctx, std::max<unsigned long long>(ctx->cand_cap, 1ull << 20)))) return rc;
+  if ((rc = ensure_cand(ctx, std::max(ctx->cand_cap, kg::fs_cand_room(open_base(), host_chunk_rows(m, wpk)))))) return rc;
   std::memset(ctx->counters, 0, sizeof(ctx->counters));
   // per-k-mer outputs are kept for every row, so runs are only used without them
   const bool runs = !stats && use_runs(xbits, m, wpk, !is_pinned(xbits));
@@ -921,7 +944,7 @@ int kg_run_host(kg_ctx* ctx, const uint64_t* xbits, uint64_t m, uint32_t wpk, kg
     if ((rc = run_host_once(ctx, xbits, m, wpk, stats, runs))) return rc;
     for (int retry = 0; retry < 8 && (ctx->counters[2] & (kg::ERR_HIT_OVERFLOW | kg::ERR_CAND_OVERFLOW)); ++retry) {
       if ((ctx->counters[2] & kg::ERR_HIT_OVERFLOW) && (rc = ensure_hits(ctx, ctx->counters[1]))) return rc;
-      if ((ctx->counters[2] & kg::ERR_CAND_OVERFLOW) && (rc = cand_overflow(ctx))) return rc;
+      if ((ctx->counters[2] & kg::ERR_CAND_OVERFLOW) && (rc = ensure_cand(ctx, 4 * ctx->cand_cap))) return rc;
       if ((rc = run_host_once(ctx, xbits, m, wpk, stats, runs))) return rc;
     }
   }
@@ -947,11 +970,11 @@ int kg_launch_device(kg_ctx* ctx, const uint64_t* d_x, uint64_t m, uint32_t wpk,
   int rc = check_shape(ctx, d_x, m, wpk);
   if (rc) return rc;
   if ((rc = ensure_hits(ctx, std::max<unsigned long long>(ctx->hit_cap, 1ull << 16)))) return rc;
-  if ((rc = ensure_cand(ctx, std::max<unsigned long long>(ctx->cand_cap, 1ull << 20)))) return rc;
+  if ((rc = ensure_cand(ctx, std::max(ctx->cand_cap, kg::fs_cand_room(open_base(), m))))) return rc;
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
   ctx->launches = 0;
-  KG_CUDA(cudaMemsetAsync(ctx->dCounters, 0, 4 * sizeof(unsigned long long), st), "memset");
-  if ((rc = launch_one(ctx, d_x, m, wpk, 0, ctx->pend_stats, st))) return rc;
+  KG_CUDA(cudaMemsetAsync(ctx->dCounters, 0, sizeof(ctx->counters), st), "memset");
+  if ((rc = launch_one(ctx, d_x, m, wpk, 0, ctx->pend_stats, true, SCREEN_REPEAT, st))) return rc;
   ctx->pending = true;
   ctx->pend_x = d_x;
   ctx->pend_m = m;
@@ -1003,20 +1026,20 @@ extern "C" int kg_fetch(kg_ctx* ctx, kg_result* res, kg_stats* st) {
   ctx->pending = false;
   const bool stats = ctx->pend_stats;
   ctx->pend_stats = false;
-  KG_CUDA(cudaMemcpyAsync(ctx->counters, ctx->dCounters, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                          ctx->pend_stream),
-          "copy counters");
-  KG_CUDA(cudaStreamSynchronize(ctx->pend_stream), "kernel");
-  for (int retry = 0; retry < 8 && (ctx->counters[2] & (kg::ERR_HIT_OVERFLOW | kg::ERR_CAND_OVERFLOW)); ++retry) {
-    int rc = 0;
+  int rc = read_counters(ctx, ctx->pend_stream);
+  if (rc) return rc;
+  const int screen = ctx->last_screen;  // negative: it gave up
+  for (int retry = 0; retry < 8 && ((ctx->counters[2] & (kg::ERR_HIT_OVERFLOW | kg::ERR_CAND_OVERFLOW)) ||
+                                    ctx->counters[kg::CNT_FS_EVER]);
+       ++retry) {
     if ((ctx->counters[2] & kg::ERR_HIT_OVERFLOW) && (rc = ensure_hits(ctx, ctx->counters[1]))) return rc;
-    if ((ctx->counters[2] & kg::ERR_CAND_OVERFLOW) && (rc = cand_overflow(ctx))) return rc;
-    KG_CUDA(cudaMemsetAsync(ctx->dCounters, 0, 4 * sizeof(unsigned long long), ctx->pend_stream), "memset");
-    if ((rc = launch_one(ctx, ctx->pend_x, ctx->pend_m, ctx->pend_wpk, 0, stats, ctx->pend_stream))) return rc;
-    KG_CUDA(cudaMemcpyAsync(ctx->counters, ctx->dCounters, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                            ctx->pend_stream),
-            "copy counters");
-    KG_CUDA(cudaStreamSynchronize(ctx->pend_stream), "kernel");
+    if ((ctx->counters[2] & kg::ERR_CAND_OVERFLOW) && (rc = ensure_cand(ctx, 4 * ctx->cand_cap))) return rc;
+    KG_CUDA(cudaMemsetAsync(ctx->dCounters, 0, sizeof(ctx->counters), ctx->pend_stream), "memset");
+    if ((rc = launch_one(ctx, ctx->pend_x, ctx->pend_m, ctx->pend_wpk, 0, stats, true,
+                         screen < 0 ? SCREEN_OFF : SCREEN_REPEAT, ctx->pend_stream)))
+      return rc;
+    if ((rc = read_counters(ctx, ctx->pend_stream))) return rc;
   }
+  ctx->last_screen = screen;
   return collect(ctx, ctx->pend_m, res, st, stats);
 }

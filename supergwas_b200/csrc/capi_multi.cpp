@@ -36,15 +36,15 @@ void free_multi(kg_ctx* ctx) {
   M.np = 0;
 }
 
-}  // namespace kgctx
-
-namespace {
-
 void drop_graph(Multi& M) {
   if (M.graph) cudaGraphExecDestroy(M.graph);
   M.graph = nullptr;
   M.g_seen = 0;
 }
+
+}  // namespace kgctx
+
+namespace {
 
 int ensure_multi_out(kg_ctx* ctx, int n_shards, unsigned long long hit_cap) {
   Multi& M = ctx->mp;
@@ -52,7 +52,7 @@ int ensure_multi_out(kg_ctx* ctx, int n_shards, unsigned long long hit_cap) {
   if (M.tested_cap < need || !M.dTested) {
     dfree(M.dTested);
     M.tested_cap = 0;
-    KG_CUDA(cudaMalloc((void**)&M.dTested, need * sizeof(unsigned long long)), "cudaMalloc(tested)");
+    KG_CUDA(cudaMalloc((void**)&M.dTested, 2 * need * sizeof(unsigned long long)), "cudaMalloc(tested)");
     M.tested_cap = need;
     drop_graph(M);
   }
@@ -71,7 +71,7 @@ int ensure_multi_out(kg_ctx* ctx, int n_shards, unsigned long long hit_cap) {
     M.shard_cap = n_shards;
     drop_graph(M);
   }
-  if (!M.dCounters) KG_CUDA(cudaMalloc((void**)&M.dCounters, 4 * sizeof(unsigned long long)), "cudaMalloc");
+  if (!M.dCounters) KG_CUDA(cudaMalloc((void**)&M.dCounters, kg::NCOUNT * sizeof(unsigned long long)), "cudaMalloc");
   return KG_OK;
 }
 
@@ -110,18 +110,24 @@ kg::DevOutMP dev_out(kg_ctx* ctx, unsigned long long offset) {
   O.kmer_offset = offset;
   O.weight = ctx->cur_weight;
   O.wait_ns = ctx->wait_ns;
+  O.open_base = open_base();
   return O;
 }
 
-// Enqueue: candidate reset, the phenotype-tile kernel and its FP64 refinement.
-int enqueue_multi(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, unsigned long long offset,
-                  cudaStream_t st) {
+// Enqueue: candidate reset (unless fresh: the counters have just been cleared), the
+// 4-bit screen where that is on, the phenotype-tile kernel (mode: only without the
+// screen, or behind it too) and the FP64 refinement.
+int enqueue_multi(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, unsigned long long offset, bool fresh,
+                  Screen mode, cudaStream_t st) {
   Multi& M = ctx->mp;
   if (m == 0) return KG_OK;
   kg::DevOutMP O = dev_out(ctx, offset);
-  KG_CUDA(cudaMemsetAsync(M.dCounters + 3, 0, sizeof(unsigned long long), st), "memset");
+  if (!fresh) KG_CUDA(cudaMemsetAsync(M.dCounters + 3, 0, 4 * sizeof(unsigned long long), st), "memset");
   cudaError_t e;
-  if (M.kern == 3) {
+  // for rows that leave too much undecided, the kernel that the autotuner's order
+  // starts with
+  int kern = M.kern == 3 ? (M.pair_ok ? 2 : M.stationary ? 1 : 0) : M.kern;
+  if (M.kern == 3 && mode != SCREEN_OFF) {
     // a block's packed rows (every CTA's) stay in L2 across the passes
     const unsigned long long grid = std::min<unsigned long long>((m + 127) / 128, (unsigned long long)ctx->num_sms);
     unsigned long long bt = (64ull << 20) / std::max<unsigned long long>(1, grid * 128ull * wpk * 8);
@@ -140,10 +146,20 @@ int enqueue_multi(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uns
     L.bt = M.bt;
     L.Bimg = M.dFs;
     L.ph = reinterpret_cast<const kg::FsPheno*>(M.dFs + (size_t)M.fs_G * M.fs_kpad * M.fs_NP * M.fs_PPG / 2);
-    L.O = &O;
+    kg::DevOutMP S = O;
+    S.tested = M.dTested + (size_t)M.n_shards * M.np;
+    L.O = &S;
     L.num_sms = ctx->num_sms;
     e = kg::launch_fs(L, st);
-  } else if (M.kern >= 1) {
+    if (e != cudaSuccess) return ctx->cuda_fail(e, "multi-phenotype kernel launch");
+    O.over = M.dCounters + kg::CNT_FS_OVER;
+    O.fs_tested = S.tested;
+    if (mode == SCREEN_REPEAT || m * M.np <= O.open_base) kern = 3;  // with so few it cannot give up
+    else ++ctx->launches;
+  }
+  if (kern == 3) {
+    // the screen alone
+  } else if (kern >= 1) {
     // tile-iterations per block: the block's packed rows (every CTA's) stay in L2
     // across the G passes; the autotuner scales the 48 MB rule by bt_scale / 2
     const unsigned long long tiles = (m + 127) / 128;
@@ -153,12 +169,12 @@ int enqueue_multi(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uns
                             std::max<unsigned long long>(1, grid * tile_bytes);
     if (const char* v = std::getenv("KG_MP_BT")) bt = (unsigned long long)std::max(1, std::atoi(v));
     bt = std::max<unsigned long long>(1, std::min<unsigned long long>(bt, 1024));
-    M.bt = (int)bt;
+    if (M.kern != 3) M.bt = (int)bt;
     kg::LaunchMpb L{dx, m, (int)wpk, M.kpad, M.NP, M.PPG, M.G, (int)bt, M.dB, M.dPh, &O, ctx->num_sms};
-    e = M.kern == 2 ? kg::launch_mpb2(L, st) : kg::launch_mpb(L, st);
+    e = kern == 2 ? kg::launch_mpb2(L, st) : kg::launch_mpb(L, st);
   } else {
-    M.xs = kg::tb_tiles(m, ctx->num_sms);
-    M.nb = kg::tb_ring(M.NP * M.PPG);
+    if (M.kern != 3) M.xs = kg::tb_tiles(m, ctx->num_sms);
+    if (M.kern != 3) M.nb = kg::tb_ring(M.NP * M.PPG);
     kg::LaunchTb L{dx, m, (int)wpk, M.kpad, M.NP, M.PPG, M.G, M.dB, M.dPh, &O, nullptr, ctx->num_sms};
     e = kg::launch_tb(L, st);
   }
@@ -170,10 +186,25 @@ int enqueue_multi(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uns
   return KG_OK;
 }
 
+// Room for the candidates of launches of m k-mers.
+int ensure_multi_cand(kg_ctx* ctx, uint64_t m) {
+  const unsigned long long tests = ctx->mp.fs_NP ? m * ctx->mp.np : 0;
+  return ensure_cand(ctx, std::max(ctx->cand_cap, kg::fs_cand_room(open_base(), tests)));
+}
+
+// The counters of the launches on st, and what became of their screens.
+int read_multi_counters(kg_ctx* ctx, cudaStream_t st) {
+  Multi& M = ctx->mp;
+  KG_CUDA(cudaMemcpyAsync(M.counters, M.dCounters, sizeof(M.counters), cudaMemcpyDeviceToHost, st), "copy counters");
+  KG_CUDA(cudaStreamSynchronize(st), "kernel");
+  ctx->last_screen = M.kern != 3 ? 0 : M.counters[kg::CNT_FS_EVER] ? -1 : 1;
+  return KG_OK;
+}
+
 int reset_outputs(kg_ctx* ctx, cudaStream_t st) {
   Multi& M = ctx->mp;
-  KG_CUDA(cudaMemsetAsync(M.dCounters, 0, 4 * sizeof(unsigned long long), st), "memset");
-  KG_CUDA(cudaMemsetAsync(M.dTested, 0, (size_t)M.n_shards * M.np * sizeof(unsigned long long), st), "memset");
+  KG_CUDA(cudaMemsetAsync(M.dCounters, 0, sizeof(M.counters), st), "memset");
+  KG_CUDA(cudaMemsetAsync(M.dTested, 0, 2 * (size_t)M.n_shards * M.np * sizeof(unsigned long long), st), "memset");
   return KG_OK;
 }
 
@@ -227,9 +258,9 @@ int autotune(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, cudaStre
     M.bt_scale = c.bt_scale;
     int rc = reset_outputs(ctx, st);
     if (rc) return rc;
-    if ((rc = enqueue_multi(ctx, dx, sample, wpk, 0, st))) return rc;  // warm
+    if ((rc = enqueue_multi(ctx, dx, sample, wpk, 0, true, SCREEN_OFF, st))) return rc;  // warm
     KG_CUDA(cudaEventRecord(a, st), "event");
-    if ((rc = enqueue_multi(ctx, dx, sample, wpk, 0, st))) return rc;
+    if ((rc = enqueue_multi(ctx, dx, sample, wpk, 0, false, SCREEN_OFF, st))) return rc;
     KG_CUDA(cudaEventRecord(b, st), "event");
     KG_CUDA(cudaEventSynchronize(b), "autotune");
     float ms = 0;
@@ -501,12 +532,7 @@ int kg_launch_multi_device(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t
   if (rc) return rc;
   if ((rc = set_shards(ctx, shard_start, n_shards, m))) return rc;
   if ((rc = ensure_multi_out(ctx, M.n_shards, std::max<unsigned long long>(M.hit_cap, 1ull << 16)))) return rc;
-  if (!ctx->dCand || ctx->cand_cap < (1ull << 20)) {
-    dfree(ctx->dCand);
-    KG_CUDA(cudaMalloc((void**)&ctx->dCand, (1ull << 20) * sizeof(unsigned long long)), "cudaMalloc(candidates)");
-    ctx->cand_cap = 1ull << 20;
-    drop_graph(M);
-  }
+  if ((rc = ensure_multi_cand(ctx, m))) return rc;
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
   KG_CUDA(cudaMemcpyAsync(M.dShard, M.shard_host.data(), M.shard_host.size() * sizeof(unsigned long long),
                           cudaMemcpyHostToDevice, st),
@@ -525,12 +551,12 @@ int kg_launch_multi_device(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t
   }
   if (M.graph) {
     KG_CUDA(cudaGraphLaunch(M.graph, st), "graph launch");
-    ctx->launches = 2;
+    ctx->launches = M.g_launches;
   } else if (same && M.g_seen >= 1 && !std::getenv("KG_NO_GRAPH")) {
     cudaGraph_t g = nullptr;
     KG_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "capture");
     int r1 = reset_outputs(ctx, st);
-    int r2 = r1 ? r1 : enqueue_multi(ctx, dx, m, wpk, 0, st);
+    int r2 = r1 ? r1 : enqueue_multi(ctx, dx, m, wpk, 0, true, SCREEN_REPEAT, st);
     cudaError_t ec = cudaStreamEndCapture(st, &g);
     if (r2) {
       if (g) cudaGraphDestroy(g);
@@ -540,11 +566,11 @@ int kg_launch_multi_device(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t
     ec = cudaGraphInstantiate(&M.graph, g, 0);
     cudaGraphDestroy(g);
     if (ec != cudaSuccess) return ctx->cuda_fail(ec, "graph instantiate");
+    M.g_launches = ctx->launches;
     KG_CUDA(cudaGraphLaunch(M.graph, st), "graph launch");
-    ctx->launches = 2;
   } else {
     if ((rc = reset_outputs(ctx, st))) return rc;
-    if ((rc = enqueue_multi(ctx, dx, m, wpk, 0, st))) return rc;
+    if ((rc = enqueue_multi(ctx, dx, m, wpk, 0, true, SCREEN_REPEAT, st))) return rc;
     M.g_seen++;
   }
   M.pending = true;
@@ -561,29 +587,22 @@ int kg_fetch_multi(kg_ctx* ctx, kg_multi_result* res) {
   if (!M.pending) return ctx->fail(KG_ERR_STATE, "kg_fetch_multi without a pending kg_launch_multi_device");
   KG_CUDA(cudaSetDevice(ctx->opts.device), "cudaSetDevice");
   M.pending = false;
-  KG_CUDA(cudaMemcpyAsync(M.counters, M.dCounters, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                          M.pend_stream),
-          "copy counters");
-  KG_CUDA(cudaStreamSynchronize(M.pend_stream), "kernel");
-  for (int retry = 0; retry < 8 && (M.counters[2] & (kg::ERR_HIT_OVERFLOW | kg::ERR_CAND_OVERFLOW)); ++retry) {
-    int rc = 0;
+  int rc = read_multi_counters(ctx, M.pend_stream);
+  if (rc) return rc;
+  const int screen = ctx->last_screen;  // negative: it gave up
+  for (int retry = 0; retry < 8 && ((M.counters[2] & (kg::ERR_HIT_OVERFLOW | kg::ERR_CAND_OVERFLOW)) ||
+                                    M.counters[kg::CNT_FS_EVER]);
+       ++retry) {
     if ((M.counters[2] & kg::ERR_HIT_OVERFLOW) && (rc = ensure_multi_out(ctx, M.n_shards, M.counters[1])))
       return rc;
-    if (M.counters[2] & kg::ERR_CAND_OVERFLOW) {
-      const unsigned long long cap = 4 * ctx->cand_cap;
-      dfree(ctx->dCand);
-      ctx->cand_cap = 0;
-      KG_CUDA(cudaMalloc((void**)&ctx->dCand, cap * sizeof(unsigned long long)), "cudaMalloc(candidates)");
-      ctx->cand_cap = cap;
-    }
-    drop_graph(M);
+    if ((M.counters[2] & kg::ERR_CAND_OVERFLOW) && (rc = ensure_cand(ctx, 4 * ctx->cand_cap))) return rc;
     if ((rc = reset_outputs(ctx, M.pend_stream))) return rc;
-    if ((rc = enqueue_multi(ctx, M.pend_x, M.pend_m, M.pend_wpk, 0, M.pend_stream))) return rc;
-    KG_CUDA(cudaMemcpyAsync(M.counters, M.dCounters, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                            M.pend_stream),
-            "copy counters");
-    KG_CUDA(cudaStreamSynchronize(M.pend_stream), "kernel");
+    if ((rc = enqueue_multi(ctx, M.pend_x, M.pend_m, M.pend_wpk, 0, true, screen < 0 ? SCREEN_OFF : SCREEN_REPEAT,
+                            M.pend_stream)))
+      return rc;
+    if ((rc = read_multi_counters(ctx, M.pend_stream))) return rc;
   }
+  ctx->last_screen = screen;
   return collect_multi(ctx, M.pend_m, res);
 }
 
@@ -617,11 +636,11 @@ int kg_run_multi_host(kg_ctx* ctx, const uint64_t* xbits, uint64_t m, uint32_t w
     ~Reset() { c->cur_weight = nullptr; }
   } reset{ctx};
   if ((rc = ensure_multi_out(ctx, M.n_shards, std::max<unsigned long long>(M.hit_cap, 1ull << 16)))) return rc;
-  if (!ctx->dCand || ctx->cand_cap < (1ull << 20)) {
-    dfree(ctx->dCand);
-    KG_CUDA(cudaMalloc((void**)&ctx->dCand, (1ull << 20) * sizeof(unsigned long long)), "cudaMalloc(candidates)");
-    ctx->cand_cap = 1ull << 20;
-  }
+  const size_t row = (size_t)wpk * 8;
+  size_t want = (size_t)512 << 20;  // small chunks: less copy and compute left unoverlapped at the ends
+  if (const char* v = std::getenv("KG_CHUNK_MB")) want = (size_t)std::max(1, std::atoi(v)) << 20;
+  const uint64_t per = std::min(m, std::max<uint64_t>(1, want / row));
+  if ((rc = ensure_multi_cand(ctx, per))) return rc;
   KG_CUDA(cudaMemcpyAsync(M.dShard, M.shard_host.data(), M.shard_host.size() * sizeof(unsigned long long),
                           cudaMemcpyHostToDevice, st),
           "copy shards");
@@ -630,11 +649,6 @@ int kg_run_multi_host(kg_ctx* ctx, const uint64_t* xbits, uint64_t m, uint32_t w
     if ((rc = reset_outputs(ctx, st))) return rc;
     // Chunks of the rows stream through two device buffers: the copy of
     // chunk i+1 (copy stream) overlaps the kernels of chunk i (compute stream).
-    const size_t row = (size_t)wpk * 8;
-    size_t want = (size_t)512 << 20;  // small chunks: less copy and compute left unoverlapped at the ends
-    if (const char* v = std::getenv("KG_CHUNK_MB")) want = (size_t)std::max(1, std::atoi(v)) << 20;
-    uint64_t per = std::max<uint64_t>(1, want / row);
-    if (per > m) per = m;
     const size_t bytes = (size_t)per * row;
     cudaPointerAttributes attr{};
     const bool pinned = !sel && (m == 0 || (cudaPointerGetAttributes(&attr, xbits) == cudaSuccess &&
@@ -676,23 +690,14 @@ int kg_run_multi_host(kg_ctx* ctx, const uint64_t* xbits, uint64_t m, uint32_t w
       KG_CUDA(cudaStreamWaitEvent(st, ctx->ev_h2d[b], 0), "wait");
       if (i == 0 && (rc = autotune(ctx, ctx->dChunk[b], cnt, wpk, st))) return rc;
       if (i == 0 && (rc = reset_outputs(ctx, st))) return rc;  // the autotuner's trial launches wrote outputs
-      if ((rc = enqueue_multi(ctx, ctx->dChunk[b], cnt, wpk, s0, st))) return rc;
-      ctx->last_screen = M.kern == 3 ? 1 : 0;
+      if ((rc = enqueue_multi(ctx, ctx->dChunk[b], cnt, wpk, s0, i == 0, SCREEN_BEHIND, st))) return rc;
       KG_CUDA(cudaEventRecord(ctx->ev_k[b], st), "record");
     }
-    KG_CUDA(cudaMemcpyAsync(M.counters, M.dCounters, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st),
-            "copy counters");
-    KG_CUDA(cudaStreamSynchronize(st), "kernel");
+    if ((rc = read_multi_counters(ctx, st))) return rc;
     if (!(M.counters[2] & (kg::ERR_HIT_OVERFLOW | kg::ERR_CAND_OVERFLOW))) break;
     if ((M.counters[2] & kg::ERR_HIT_OVERFLOW) && (rc = ensure_multi_out(ctx, M.n_shards, M.counters[1])))
       return rc;
-    if (M.counters[2] & kg::ERR_CAND_OVERFLOW) {
-      const unsigned long long cap = 4 * ctx->cand_cap;
-      dfree(ctx->dCand);
-      ctx->cand_cap = 0;
-      KG_CUDA(cudaMalloc((void**)&ctx->dCand, cap * sizeof(unsigned long long)), "cudaMalloc(candidates)");
-      ctx->cand_cap = cap;
-    }
+    if ((M.counters[2] & kg::ERR_CAND_OVERFLOW) && (rc = ensure_cand(ctx, 4 * ctx->cand_cap))) return rc;
   }
   drop_graph(M);
   M.g_x = nullptr;

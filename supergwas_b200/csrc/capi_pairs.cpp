@@ -33,15 +33,6 @@ int ensure_pairs(kg_ctx* ctx, unsigned long long cap) {
   return KG_OK;
 }
 
-int ensure_pair_cand(kg_ctx* ctx, unsigned long long cap) {
-  if (ctx->cand_cap >= cap && ctx->dCand) return KG_OK;
-  dfree(ctx->dCand);
-  ctx->cand_cap = 0;
-  KG_CUDA(cudaMalloc((void**)&ctx->dCand, cap * sizeof(unsigned long long)), "cudaMalloc(candidates)");
-  ctx->cand_cap = cap;
-  return KG_OK;
-}
-
 // Sorts the emitted pairs by (a, b).  a lies in the task's row range
 // [row_start, row_end): a counting sort on a, then each row's few pairs
 // sorted by b.  The scatter is bound by cache misses, so host threads each
@@ -172,42 +163,47 @@ int kg_pairs_run_host(kg_ctx* ctx, const uint64_t* xbits, uint64_t n_kmers, uint
   kg::PairSched S{ctx->dUnitOff, njb, off.back(), n_kmers, row_start, row_end, ic};
   int rc;
   if ((rc = ensure_pairs(ctx, std::max<unsigned long long>(ctx->pair_cap, 1ull << 16)))) return rc;
-  if ((rc = ensure_pair_cand(ctx, std::max<unsigned long long>(ctx->cand_cap, 1ull << 20)))) return rc;
-  unsigned long long cnt[4] = {0, 0, 0, 0};
-  for (int attempt = 0; attempt < 8; ++attempt) {
-    kg::DevOutPairs O{ctx->dCounters, ctx->dPairs, ctx->pair_cap, ctx->dCand, ctx->cand_cap, ctx->wait_ns};
-    KG_CUDA(cudaMemsetAsync(ctx->dCounters, 0, 4 * sizeof(unsigned long long), st), "memset");
+  const unsigned long long tests = S.n_units * ic * 128;
+  if ((rc = ensure_cand(ctx, std::max(ctx->cand_cap, kg::fs_cand_room(open_base(), tests))))) return rc;
+  unsigned long long cnt[kg::NCOUNT] = {};
+  bool gave_up = false;  // the screen, in an earlier attempt
+  for (int attempt = 0; attempt < 9; ++attempt) {
+    kg::DevOutPairs O{ctx->dCounters, ctx->dPairs, ctx->pair_cap, ctx->dCand, ctx->cand_cap, ctx->wait_ns, nullptr,
+                      open_base()};
+    KG_CUDA(cudaMemsetAsync(ctx->dCounters, 0, sizeof(cnt), st), "memset");
     // the 4-bit screen, unless another kernel is asked for; no pair is evaluated
     // where yyM is rounding (the kernels' eps), which the screen does not look at
     const char* force = std::getenv("KG_KERNEL");
-    const bool fs = ctx->fs_N && !force && ctx->P.yyM > 1e-12 && kg::fsp_supported(ctx->fs_N, ctx->fs_lu, ctx->fs_kpad, (int)wd, ic);
+    const bool fs = ctx->fs_N && !force && !gave_up && ctx->P.yyM > 1e-12 && kg::fsp_supported(ctx->fs_N, ctx->fs_lu, ctx->fs_kpad, (int)wd, ic);
     cudaError_t e;
+    ctx->launches = 2;
     if (fs) {
       kg::LaunchFsPairs L{ctx->dPX, (int)wd, ctx->fs_kpad, ctx->fs_N, ctx->fs_lu, ctx->P.corr_thr > 0.0, S, ctx->dFs,
                           &ctx->fsF, &O, ctx->num_sms};
       e = kg::launch_fs_pairs(L, st);
+      O.over = ctx->dCounters + kg::CNT_FS_OVER;
     } else {
       kg::LaunchPairs L{ctx->dPX, (int)wd, ctx->limbs.Kpad, ctx->prep.drop0 && ctx->P.k > 0, S, ctx->dBts, &ctx->P,
                         &ctx->LM, &O, ctx->num_sms};
       e = kg::launch_pairs(L, st);
     }
     if (e != cudaSuccess) return ctx->cuda_fail(e, "pair kernel launch");
-    kg::LaunchPairRefine R{ctx->dPX, (int)wd, ctx->dT, ctx->nsteps * 128, ctx->cm, &ctx->P, &O, ctx->num_sms, fs,
+    kg::LaunchPairRefine R{ctx->dPX, (int)wd, ctx->dT, ctx->nsteps * 128, ctx->cm, &ctx->P, &O, ctx->num_sms,
                           &ctx->LM, ctx->dV};
     e = kg::launch_pair_refine(R, st);
     if (e != cudaSuccess) return ctx->cuda_fail(e, "pair refinement launch");
-    ctx->launches = 2;
-    ctx->last_screen = fs ? ctx->fs_lu : 0;
     KG_CUDA(cudaMemcpyAsync(cnt, ctx->dCounters, sizeof(cnt), cudaMemcpyDeviceToHost, st), "copy counters");
     KG_CUDA(cudaStreamSynchronize(st), "pair kernels");
+    if (cnt[kg::CNT_FS_EVER]) gave_up = true;  // the pair kernel takes every pair
+    ctx->last_screen = gave_up ? -ctx->fs_lu : fs ? ctx->fs_lu : 0;
     if (cnt[2] & ~(unsigned long long)(kg::ERR_HIT_OVERFLOW | kg::ERR_CAND_OVERFLOW))
       return ctx->fail(KG_ERR_TIMEOUT, "a bounded device-side wait gave up (error bits " + std::to_string(cnt[2]) + ")");
-    if (!(cnt[2] & (kg::ERR_HIT_OVERFLOW | kg::ERR_CAND_OVERFLOW))) break;
-    if ((cnt[2] & kg::ERR_CAND_OVERFLOW) && (rc = ensure_pair_cand(ctx, std::max(cnt[3], 4 * ctx->cand_cap))))
+    if (!cnt[kg::CNT_FS_EVER] && !(cnt[2] & (kg::ERR_HIT_OVERFLOW | kg::ERR_CAND_OVERFLOW))) break;
+    if ((cnt[2] & kg::ERR_CAND_OVERFLOW) && (rc = ensure_cand(ctx, std::max(cnt[3], 4 * ctx->cand_cap))))
       return rc;
     if ((cnt[2] & kg::ERR_HIT_OVERFLOW) && (rc = ensure_pairs(ctx, std::max(cnt[1] + (1ull << 16), 2 * ctx->pair_cap))))
       return rc;
-    if (attempt == 7) return ctx->fail(KG_ERR_NOMEM, "pair or candidate buffer still too small");
+    if (attempt == 8) return ctx->fail(KG_ERR_NOMEM, "pair or candidate buffer still too small");
   }
   ctx->pairs.resize(cnt[1]);
   if (cnt[1])

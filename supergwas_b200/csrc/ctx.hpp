@@ -127,7 +127,7 @@ struct Multi {
   double* dT = nullptr;  // byte tables of V (refinement), one block per phenotype
   size_t vstride = 0;
   unsigned long long* dCounters = nullptr;
-  unsigned long long* dTested = nullptr;
+  unsigned long long* dTested = nullptr;  // counts, and behind them the screen's
   size_t tested_cap = 0;
   kg_phit* dHits = nullptr;
   unsigned long long hit_cap = 0;
@@ -137,7 +137,7 @@ struct Multi {
   std::vector<unsigned long long> shard_host;
   std::vector<kg_phit> hits;
   std::vector<uint64_t> tested;
-  unsigned long long counters[4] = {0, 0, 0, 0};
+  unsigned long long counters[kg::NCOUNT] = {};
   // shape of the last streamed-image launch: tiles per item, image chunks in the ring
   int xs = 1, nb = 4;
   int bt = 0;  // B-stationary kernel: tile-iterations per L2 block of the last launch
@@ -154,7 +154,7 @@ struct Multi {
   uint64_t g_m = 0;
   uint32_t g_wpk = 0;
   cudaStream_t g_stream = nullptr;
-  int g_seen = 0;
+  int g_seen = 0, g_launches = 0;
 };
 
 }  // namespace kgctx
@@ -198,7 +198,7 @@ struct kg_ctx {
   size_t stat_cap = 0;
   // host result
   std::vector<kg_hit> hits;
-  unsigned long long counters[3] = {0, 0, 0};
+  unsigned long long counters[kg::NCOUNT] = {};
   // pending device launch
   bool pending = false;
   const uint64_t* pend_x = nullptr;
@@ -208,7 +208,7 @@ struct kg_ctx {
   cudaStream_t pend_stream = nullptr;
   int launches = 0;
   const char* last_kernel = "";
-  int last_screen = 0;       // limbs per U column of the last launch's 4-bit screen
+  int last_screen = 0;       // limbs per U column of the last launch's 4-bit screen, negative where it gave up
   // bounded device waits: pipeline wait limit (0: the default) and the
   // one-launch stall of the row producer that the failure tests use
   unsigned long long wait_ns = 0;
@@ -257,6 +257,7 @@ struct kg_ctx {
 
 namespace kgctx {
 void free_multi(kg_ctx* ctx);  // capi_multi.cpp
+void drop_graph(Multi& M);
 }  // namespace kgctx
 
 namespace kgctx {
@@ -294,6 +295,15 @@ uint64_t scan_gather(const uint64_t* x, uint64_t s0, uint64_t cnt, uint32_t wpk,
 bool find_runs(kg_ctx* ctx, const uint64_t* x, uint64_t m, uint32_t wpk, const std::vector<unsigned long long>& bounds,
                bool pageable);
 bool is_pinned(const void* p);
+// What a launch does about rows that the 4-bit screen cannot place: it is repeated
+// without the screen once its counters have been read (the rows stay where they
+// are), or the kernel for that case is launched behind the screen.
+enum Screen { SCREEN_REPEAT, SCREEN_BEHIND, SCREEN_OFF };
+// The base of kg::fs_open_limit: FS_OPEN_BASE, or KG_SCREEN_OPEN (0: the shares
+// alone; 16777216: never reached).
+unsigned long long open_base();
+// The candidate list, at least cap entries (all paths share it; what it held is lost).
+int ensure_cand(kg_ctx* ctx, unsigned long long cap);
 // Copies the run lengths to the device and makes them the tested-count
 // weights of the following launches (ctx->cur_weight).
 int upload_run_lengths(kg_ctx* ctx, cudaStream_t st);

@@ -92,8 +92,9 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 // As mbar_try, letting the hardware suspend the thread until the phase
-// completes (or about 1 ms passes) instead of returning at once, so that a
+// completes (or NS, about 1 ms, passes) instead of returning at once, so that a
 // waiting warp takes no issue slots from the warps doing the work.
+template <uint32_t NS = 1000000u>
 __device__ __forceinline__ bool mbar_try_sleep(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -101,7 +102,7 @@ __device__ __forceinline__ bool mbar_try_sleep(uint32_t bar, uint32_t parity) {
       "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2, %3;\n\t"
       "selp.b32 %0, 1, 0, P1;\n\t}"
       : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(1000000u)
+      : "r"(bar), "r"(parity), "r"(NS)
       : "memory");
   return ok != 0;
 }

@@ -8,7 +8,11 @@
 // undecided, which goes to the FP64 refinement list.  The refinement kernel
 // evaluates the statistic (src/kgwas.cpp:44-56, 182-218) in FP64 and emits:
 // every value that leaves the device is FP64, and no decision rests on a sum
-// whose bound does not carry it.
+// whose bound does not carry it.  Where too many tests stay undecided
+// (fs_open_limit) the screen gives up: its CTAs leave by the path of a wait that
+// ran out, without an error, and another kernel evaluates every test: one launched
+// behind it, which otherwise ends at once (5 us), where rows stream through, and a
+// second launch where the rows stay on the device.
 //
 // Operands: A = the packed bits spread over 4-bit floats, 8 per 32-bit word,
 // in tensor memory: of a word w, w & 0x11111111 holds its samples 4i as 0.5,
@@ -149,7 +153,7 @@ __global__ void __launch_bounds__(fs_threads(NP * PPG), 1)
         for (int g = 0; g < G && ok; ++g)
           for (uint32_t i = i0; i < mine && i < i0 + bt && ok; ++i)
             for (int bx = 0; bx < nsp; ++bx, xr.next()) {
-              if (xr.used && !wait_or_abort(x_empty + 8 * xr.slot, xr.phase ^ 1u, s_abort, counters, ERR_TIMEOUT_FULL,
+              if (xr.used && !fs_wait(x_empty + 8 * xr.slot, xr.phase ^ 1u, s_abort, counters, ERR_TIMEOUT_FULL,
                                             lim)) {
                 ok = false;
                 break;
@@ -178,7 +182,7 @@ __global__ void __launch_bounds__(fs_threads(NP * PPG), 1)
         for (int g = 0; g < G && ok; ++g, ++pass) {
           const uint8_t* src = Bimg + (size_t)g * (uint32_t)b_bytes;
           for (int c = 0; c < nsp; ++c) {
-            if (pass && !wait_or_abort(b_empty + 8 * c, (pass - 1) & 1u, s_abort, counters, ERR_TIMEOUT_FULL, lim)) {
+            if (pass && !fs_wait(b_empty + 8 * c, (pass - 1) & 1u, s_abort, counters, ERR_TIMEOUT_FULL, lim)) {
               ok = false;
               break;
             }
@@ -216,24 +220,24 @@ __global__ void __launch_bounds__(fs_threads(NP * PPG), 1)
             continue;
           }
           const bool lastone = G > 1 && i + 2 >= cnt;  // this warp's last item of the pass
-          if (i2 >= 1 && !__all_sync(0xffffffffu, wait_or_abort(acc_empty + 8 * b, (i2 - 1) & 1u, s_abort, counters,
+          if (i2 >= 1 && !__all_sync(0xffffffffu, fs_wait(acc_empty + 8 * b, (i2 - 1) & 1u, s_abort, counters,
                                                                 ERR_TIMEOUT_MMA, lim))) {
             ok = false;
             break;
           }
-          if ((b || i2 >= 1) && !__all_sync(0xffffffffu, wait_or_abort(turn + 8 * b, b ? i2 & 1u : (i2 - 1) & 1u,
+          if ((b || i2 >= 1) && !__all_sync(0xffffffffu, fs_wait(turn + 8 * b, b ? i2 & 1u : (i2 - 1) & 1u,
                                                                        s_abort, counters, ERR_TIMEOUT_MMA, lim))) {
             ok = false;
             break;
           }
           uint64_t bd = bdesc0;
           for (int sp = 0; sp < nsp; ++sp, ar.next()) {
-            if (first && !__all_sync(0xffffffffu, wait_or_abort(b_full + 8 * sp, bpar, s_abort, counters,
+            if (first && !__all_sync(0xffffffffu, fs_wait(b_full + 8 * sp, bpar, s_abort, counters,
                                                                 ERR_TIMEOUT_FULL, lim))) {
               ok = false;
               break;
             }
-            if (!__all_sync(0xffffffffu, wait_or_abort(a_full + 8 * ar.slot, ar.phase, s_abort, counters,
+            if (!__all_sync(0xffffffffu, fs_wait(a_full + 8 * ar.slot, ar.phase, s_abort, counters,
                                                        ERR_TIMEOUT_MMA, lim))) {
               ok = false;
               break;
@@ -287,7 +291,7 @@ __global__ void __launch_bounds__(fs_threads(NP * PPG), 1)
       for (sp += step; sp >= nsp; sp -= nsp)
         if (left) --left;
       if (!left) break;
-      if (!__all_sync(0xffffffffu, wait_or_abort(x_full + 8 * xslot, xphase, s_abort, counters, ERR_TIMEOUT_FULL, lim)))
+      if (!__all_sync(0xffffffffu, fs_wait(x_full + 8 * xslot, xphase, s_abort, counters, ERR_TIMEOUT_FULL, lim)))
         break;
       const uint32_t xrow = row0 + xslot * xbytes;
       const int here = nunit - sp * FS_SUPER;
@@ -310,7 +314,7 @@ __global__ void __launch_bounds__(fs_threads(NP * PPG), 1)
           unpack_unit(w, o);
           if (u == 0 && used &&
               !__all_sync(0xffffffffu,
-                          wait_or_abort(a_empty + 8 * grp, aphase ^ 1u, s_abort, counters, ERR_TIMEOUT_MMA, lim))) {
+                          fs_wait(a_empty + 8 * grp, aphase ^ 1u, s_abort, counters, ERR_TIMEOUT_MMA, lim))) {
             ok = false;
             break;
           }
@@ -358,7 +362,7 @@ __global__ void __launch_bounds__(fs_threads(NP * PPG), 1)
       for (int g = 0; g < G && ok; ++g) {
         for (uint32_t i = i0; i < mine && i < i0 + bt; ++i, ++item) {
           if ((item & 1u) != e) continue;
-          if (!__all_sync(0xffffffffu, wait_or_abort(acc_full + 8 * e, jt & 1u, s_abort, counters, ERR_TIMEOUT_MMA,
+          if (!__all_sync(0xffffffffu, fs_wait(acc_full + 8 * e, jt & 1u, s_abort, counters, ERR_TIMEOUT_MMA,
                                                      lim))) {
             ok = false;
             break;
@@ -368,6 +372,9 @@ __global__ void __launch_bounds__(fs_threads(NP * PPG), 1)
           const unsigned long long local = (unsigned long long)(blockIdx.x + i * gridDim.x) * FS_TM + r;
           const bool valid = local < m;
           uint32_t wt = 1u;
+          const unsigned long long limit =
+              fs_open_limit(MANY ? O.open_base : O1.open_base, (item + 1ull) * gridDim.x * (FS_TM * PPG),
+                            MANY ? m * (unsigned)O.n_pheno : m, MANY ? O.cand_cap : O1.cand_cap);
           bool same = true;  // the warp's rows lie in one shard, whose counts stay in registers
           if (MANY) {
             const unsigned long long w0 = O.kmer_offset + local - lane, end = O.kmer_offset + m;
@@ -398,21 +405,32 @@ __global__ void __launch_bounds__(fs_threads(NP * PPG), 1)
               const uint32_t t = v == 1 || v == 2 ? wt : 0u;
               if (same) cnt[pp] += t;
               else tb_count(O, p, mp_shard(O, valid ? O.kmer_offset + local : O.kmer_offset), t);
-              if (__any_sync(0xffffffffu, v >= 2))
-                fs_push(counters, O.cand, O.cand_cap, v >= 2,
-                        (O.kmer_offset + local) | ((unsigned long long)p << 48) | (v == 3 ? CAND_OPEN_MP : 0ull));
+              if (__any_sync(0xffffffffu, v >= 2) &&
+                  !fs_push(counters, O.cand, limit, v >= 2,
+                           (O.kmer_offset + local) | ((unsigned long long)p << 48) | (v == 3 ? CAND_OPEN_MP : 0ull))) {
+                ok = false;
+                break;
+              }
             } else {
               const int v = fs_verdict<NP, LU, GATE>(F1, d, valid);
               if (v == 1 || (v == 2 && !O1.count_sure))
                 tested_local += O1.weight ? O1.weight[O1.kmer_offset + local] : 1u;
-              if (__any_sync(0xffffffffu, v >= 2))
-                fs_push(counters, O1.cand, O1.cand_cap, v >= 2, (O1.kmer_offset + local) | (v == 3 && !O1.count_sure ? CAND_OPEN : 0ull));
+              if (__any_sync(0xffffffffu, v >= 2) &&
+                  !fs_push(counters, O1.cand, limit, v >= 2,
+                           (O1.kmer_offset + local) | (v == 3 && !O1.count_sure ? CAND_OPEN : 0ull))) {
+                ok = false;
+                break;
+              }
             }
+          }
+          if (!ok) {  // given up: the CTA's other roles leave too
+            if (lane == 0) *s_abort = 1;
+            break;
           }
         }
         if (MANY) flush(g);
       }
-    if (!MANY) flush_tested(O1, tested_local);
+    if (!MANY) fs_flush(counters, tested_local);
   }
   __syncthreads();
   tc_fence_after();
@@ -420,15 +438,14 @@ __global__ void __launch_bounds__(fs_threads(NP * PPG), 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
-// Copies the rows of the candidates to dst, 16 bytes a thread; none where they
-// are more than cap (ERR_CAND_OVERFLOW has been set then).
+// Copies the rows of the screen's candidates to dst, 16 bytes a
+// thread; none where it has given up.
 __global__ void __launch_bounds__(256) fs_gather_kernel(const uint4* __restrict__ x, int chunks,
                                                         const unsigned long long* __restrict__ cand,
-                                                        const unsigned long long* __restrict__ count,
-                                                        unsigned long long cap, unsigned long long offset,
-                                                        uint4* __restrict__ dst) {
-  const unsigned long long rows = *count;
-  if (rows > cap) return;
+                                                        const unsigned long long* __restrict__ counters,
+                                                        unsigned long long offset, uint4* __restrict__ dst) {
+  if (counters[CNT_FS_OVER]) return;
+  const unsigned long long rows = counters[CNT_FS_OPEN];
   const unsigned long long total = rows * (unsigned)chunks;
   for (unsigned long long t = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (unsigned long long)gridDim.x * blockDim.x) {
@@ -440,9 +457,9 @@ __global__ void __launch_bounds__(256) fs_gather_kernel(const uint4* __restrict_
 // ------------------------------------------------------------------- host
 
 cudaError_t launch_fs_gather(const uint64_t* x, int wpk, const unsigned long long* cand,
-                             const unsigned long long* count, unsigned long long cap, unsigned long long offset,
-                             uint64_t* dst, int num_sms, cudaStream_t st) {
-  fs_gather_kernel<<<2 * num_sms, 256, 0, st>>>(reinterpret_cast<const uint4*>(x), wpk / 2, cand, count, cap, offset,
+                             const unsigned long long* counters, unsigned long long offset, uint64_t* dst, int num_sms,
+                             cudaStream_t st) {
+  fs_gather_kernel<<<2 * num_sms, 256, 0, st>>>(reinterpret_cast<const uint4*>(x), wpk / 2, cand, counters, offset,
                                                 reinterpret_cast<uint4*>(dst));
   return cudaGetLastError();
 }

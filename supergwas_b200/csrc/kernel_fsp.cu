@@ -2,7 +2,8 @@
 // screen of kernel_fs.cu: A = the AND of two packed rows, spread over 4-bit
 // floats, against the phenotype's screen image.  Pairs that the screen cannot
 // place below the emit cut go to the FP64 refinement list, which
-// pr_refine_kernel recomputes, counts and emits.
+// pr_refine_kernel recomputes, counts and emits; with too many of them
+// (fs_open_limit) pairs_kernel evaluates every pair instead.
 //
 // Schedule and roles are those of kernel_pairs.cu: a tile is 128 pairs (i, j)
 // sharing i, j in one 128-row j-block; the unit's boxes (its j-block and up to
@@ -113,7 +114,7 @@ __global__ void __launch_bounds__(fsp_threads(N), 1)
       for (unsigned long long u = blockIdx.x; u < S.n_units && ok; u += gridDim.x) {
         const PairUnit U = pr_unit(S, u);
         for (int bx = 0; bx < nsp; ++bx, xr.next()) {
-          if (xr.used && !wait_or_abort(x_empty + 8 * xr.slot, xr.phase ^ 1u, s_abort, O.counters, ERR_TIMEOUT_FULL,
+          if (xr.used && !fs_wait(x_empty + 8 * xr.slot, xr.phase ^ 1u, s_abort, O.counters, ERR_TIMEOUT_FULL,
                                         lim)) {
             ok = false;
             break;
@@ -135,7 +136,7 @@ __global__ void __launch_bounds__(fsp_threads(N), 1)
     // two warps taking alternate tiles, in the order of kernel_ts.cu
     const bool leader = elect_one();
     const uint32_t b = (uint32_t)(warp - W_MMA);
-    bool ok = __all_sync(0xffffffffu, wait_or_abort(b_full, 0, s_abort, O.counters, ERR_TIMEOUT_FULL, lim));
+    bool ok = __all_sync(0xffffffffu, fs_wait(b_full, 0, s_abort, O.counters, ERR_TIMEOUT_FULL, lim));
     const uint64_t bdesc0 = sdesc_noswz(sb, N * 16, 128);
     const uint32_t d_t = tmem + b * N, sf = tmem + SF0;
     Ring<NSLOT> ar;
@@ -148,12 +149,12 @@ __global__ void __launch_bounds__(fsp_threads(N), 1)
           for (int sp = 0; sp < nsp; ++sp) ar.next();
           continue;
         }
-        if (t >= 1 && !__all_sync(0xffffffffu, wait_or_abort(acc_empty + 8 * b, (t - 1) & 1u, s_abort, O.counters,
+        if (t >= 1 && !__all_sync(0xffffffffu, fs_wait(acc_empty + 8 * b, (t - 1) & 1u, s_abort, O.counters,
                                                              ERR_TIMEOUT_MMA, lim))) {
           ok = false;
           break;
         }
-        if ((b || t >= 1) && !__all_sync(0xffffffffu, wait_or_abort(turn + 8 * b, b ? t & 1u : (t - 1) & 1u, s_abort,
+        if ((b || t >= 1) && !__all_sync(0xffffffffu, fs_wait(turn + 8 * b, b ? t & 1u : (t - 1) & 1u, s_abort,
                                                                     O.counters, ERR_TIMEOUT_MMA, lim))) {
           ok = false;
           break;
@@ -162,7 +163,7 @@ __global__ void __launch_bounds__(fsp_threads(N), 1)
         uint64_t bd = bdesc0;
         for (int sp = 0; sp < nsp; ++sp, ar.next()) {
           if (!__all_sync(0xffffffffu,
-                          wait_or_abort(a_full + 8 * ar.slot, ar.phase, s_abort, O.counters, ERR_TIMEOUT_MMA, lim))) {
+                          fs_wait(a_full + 8 * ar.slot, ar.phase, s_abort, O.counters, ERR_TIMEOUT_MMA, lim))) {
             ok = false;
             break;
           }
@@ -205,7 +206,7 @@ __global__ void __launch_bounds__(fsp_threads(N), 1)
       // box bx of the unit is slot slot0 + bx of the ring
       const uint32_t slot0 = xr.slot;
       for (int bx = 0; bx < nsp; ++bx, xr.next())
-        if (ok && !__all_sync(0xffffffffu, wait_or_abort(x_full + 8 * xr.slot, xr.phase, s_abort, O.counters,
+        if (ok && !__all_sync(0xffffffffu, fs_wait(x_full + 8 * xr.slot, xr.phase, s_abort, O.counters,
                                                          ERR_TIMEOUT_FULL, lim)))
           ok = false;
       int ii = 0, sp = skip;  // tile of the unit, super-stage of the tile
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(fsp_threads(N), 1)
             uint32_t o[32];
             unpack_unit(w, o);
             if (un == 0 && used &&
-                !__all_sync(0xffffffffu, wait_or_abort(a_empty + 8 * grp, aphase ^ 1u, s_abort, O.counters,
+                !__all_sync(0xffffffffu, fs_wait(a_empty + 8 * grp, aphase ^ 1u, s_abort, O.counters,
                                                        ERR_TIMEOUT_MMA, lim))) {
               ok = false;
               break;
@@ -276,7 +277,7 @@ __global__ void __launch_bounds__(fsp_threads(N), 1)
       const unsigned long long j = U.jb * FS_TM + r;
       for (unsigned long long i = U.i0; i < U.i1; ++i, ++v) {
         if ((v & 1u) != e) continue;
-        if (!__all_sync(0xffffffffu, wait_or_abort(acc_full + 8 * e, jt & 1u, s_abort, O.counters, ERR_TIMEOUT_MMA,
+        if (!__all_sync(0xffffffffu, fs_wait(acc_full + 8 * e, jt & 1u, s_abort, O.counters, ERR_TIMEOUT_MMA,
                                                    lim))) {
           ok = false;
           break;
@@ -290,11 +291,17 @@ __global__ void __launch_bounds__(fsp_threads(N), 1)
         mbar_arrive_if(acc_empty + 8 * e, lane == 0);
         const int vd = fs_verdict<N, LU, GATE, true>(F, d, j < S.n_kmers && j > i);
         evaluated += vd == 1 ? 1u : 0u;
-        if (__any_sync(0xffffffffu, vd >= 2)) fs_push(O.counters, O.cand, O.cand_cap, vd >= 2, (i << 32) | j);
+        if (__any_sync(0xffffffffu, vd >= 2) &&
+            !fs_push(O.counters, O.cand,
+                     fs_open_limit(O.open_base, (v + 1ull) * gridDim.x * FS_TM, S.n_units * S.ic * FS_TM, O.cand_cap),
+                     vd >= 2, (i << 32) | j)) {
+          ok = false;  // given up, as in kernel_fs.cu
+          if (lane == 0) *s_abort = 1;
+          break;
+        }
       }
     }
-    const unsigned tot = __reduce_add_sync(0xffffffffu, evaluated);
-    if (lane == 0 && tot) atomicAdd(O.counters + 0, (unsigned long long)tot);
+    fs_flush(O.counters, evaluated);
   }
   __syncthreads();
   tc_fence_after();

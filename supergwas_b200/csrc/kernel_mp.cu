@@ -21,7 +21,18 @@ __global__ void __launch_bounds__(256) mp_refine_kernel(const uint64_t* __restri
                                                         const MPheno* __restrict__ ph, const DevOutMP O) {
   const int lane = threadIdx.x & 31;
   const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
-  unsigned long long ncand = O.counters[3];
+  const bool fs = O.over && !*O.over;  // the 4-bit screen's candidates and counts
+  if (O.over) {
+    const unsigned long long nc = (unsigned long long)O.n_shards * O.n_pheno;
+    for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < nc;
+         i += (unsigned long long)gridDim.x * blockDim.x) {
+      const unsigned long long c = O.fs_tested[i];
+      if (!c) continue;
+      if (fs) atomicAdd(O.tested + i, c);
+      O.fs_tested[i] = 0;  // for the next launch
+    }
+  }
+  unsigned long long ncand = O.counters[fs ? CNT_FS_OPEN : 3];
   if (ncand > O.cand_cap) ncand = O.cand_cap;
   for (unsigned long long w = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < ncand;
        w += warps) {

@@ -122,6 +122,7 @@ __global__ void __launch_bounds__(mb_threads(NP * PPG), 1)
   const unsigned long long nt =
       ntiles > blockIdx.x ? (ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0ull;
 
+  if (O.over && !*O.over) return;  // the screen has decided
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(s_tmem))
                  : "memory");

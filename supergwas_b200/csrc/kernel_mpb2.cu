@@ -193,6 +193,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(M2_THREADS, 1)
   const unsigned long long npt = (m + 2 * M2_TM - 1) / (2 * M2_TM);
   const unsigned long long nt = npt > pair ? (npt - pair + npairs - 1) / npairs : 0ull;
 
+  if (O.over && !*O.over) return;  // the screen has decided
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(s_tmem))
                  : "memory");

@@ -479,17 +479,19 @@ __device__ __noinline__ double pr_split_xxM(const EpiParams& P, const LimbMap& L
 
 // FP64 recomputation of the pair candidates: one warp per pair, column sums
 // of x_i * x_j from the byte tables of V (table_row_sums on the AND of the
-// two rows), then compute_hit in FP64 (src/kgwas_2d.cpp:300-318).  count: the
-// candidates have not been counted as evaluated yet (the 4-bit screen's).
+// two rows), then compute_hit in FP64 (src/kgwas_2d.cpp:300-318).  The 4-bit
+// screen's candidates have not been counted as evaluated yet (count).
 template <int CM>
 __global__ void __launch_bounds__(256) pr_refine_kernel(const uint64_t* __restrict__ x, int wpk, int nwords,
                                                         const double* __restrict__ T,
                                                         const __grid_constant__ EpiParams P, const DevOutPairs O,
-                                                        bool count, const __grid_constant__ LimbMap LM,
+                                                        const __grid_constant__ LimbMap LM,
                                                         const double* __restrict__ V) {
   const int lane = threadIdx.x & 31;
   const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
-  unsigned long long ncand = O.counters[3];
+  const bool count = O.over && !*O.over;
+  if (count && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(O.counters, O.counters[CNT_FS_TESTED]);
+  unsigned long long ncand = O.counters[count ? CNT_FS_OPEN : 3];
   if (ncand > O.cand_cap) ncand = O.cand_cap;
   for (unsigned long long w = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < ncand;
        w += warps) {
@@ -622,7 +624,7 @@ static cudaError_t launch_pr_refine_t(const LaunchPairRefine& L, cudaStream_t st
       (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pr_refine_kernel<CM>, 256, 0) != cudaSuccess ||
        per_sm < 1))
     per_sm = 1;
-  pr_refine_kernel<CM><<<(unsigned)(L.num_sms * per_sm), 256, 0, st>>>(L.x, L.wpk, L.vrows / 64, L.T, *L.P, *L.O, L.count, *L.LM, L.V);
+  pr_refine_kernel<CM><<<(unsigned)(L.num_sms * per_sm), 256, 0, st>>>(L.x, L.wpk, L.vrows / 64, L.T, *L.P, *L.O, *L.LM, L.V);
   return cudaGetLastError();
 }
 

@@ -250,9 +250,14 @@ __global__ void __launch_bounds__(TB_THREADS, 1)
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   unsigned long long* const counters = SINGLE ? O1.counters : O.counters;
   const unsigned long long lim = wait_limit(SINGLE ? O1.wait_ns : O.wait_ns);
-  if (FORM == TB_ONE64 && O1.rows) {
-    const unsigned long long rows = *O1.rows;
-    m = rows <= m ? rows : 0;
+  // behind the screen: the rows that it has left (FP64 form), or every row where it
+  // has given up
+  const unsigned long long* const over = SINGLE ? O1.over : O.over;
+  const bool left = FORM == TB_ONE64 && O1.rows;
+  if (over && (*over != 0) == left) return;
+  if (left) {
+    m = *O1.rows;
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(O1.counters, O1.counters[CNT_FS_TESTED]);
   }
   const int nsp = (nsub + TB_SUPER - 1) / TB_SUPER;     // super-stages of a tile
   const int nchunk = (nsub + TB_CHUNK - 1) / TB_CHUNK;  // image chunks

@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(ts_threads(N), 1)
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int nsp = (nsub + TS_SUPER - 1) / TS_SUPER;  // super-stages per tile
 
+  if (O.over && !*O.over) return;  // the screen has decided
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(s_tmem))
                  : "memory");

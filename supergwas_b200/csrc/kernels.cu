@@ -136,7 +136,9 @@ __global__ void __launch_bounds__(256) refine_kernel(const uint64_t* __restrict_
                                                      const __grid_constant__ LimbMap LM, const DevOut O) {
   const int lane = threadIdx.x & 31;
   const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
-  unsigned long long ncand = O.counters[3];
+  const bool fs = O.over && !*O.over;  // the 4-bit screen's candidates
+  if (fs && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(O.counters, O.counters[CNT_FS_TESTED]);
+  unsigned long long ncand = O.counters[fs ? CNT_FS_OPEN : 3];
   if (ncand > O.cand_cap) ncand = O.cand_cap;
   for (unsigned long long w = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < ncand;
        w += warps) {
@@ -294,6 +296,7 @@ __global__ void __launch_bounds__(TC_TM, 1)
   const int tid = threadIdx.x, warp = tid >> 5;
   const uint32_t full0 = smem_u32(bars), done0 = smem_u32(bars + TC_NST);
 
+  if (O.over && !*O.over) return;  // the screen has decided
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)),
                  "r"(TCOLS)

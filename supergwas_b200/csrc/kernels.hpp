@@ -141,11 +141,11 @@ inline int fs_width(bool gate, int lu, int ku) {
 }
 bool fs_supported(int N, int kpad, int wpk);
 cudaError_t launch_fs(const LaunchFs& L, cudaStream_t st);
-// Rows cand[0 .. *count) of x (16-byte aligned, wpk words each; indices from
-// `offset`) to dst, unless they are more than cap.
+// The rows of x (16-byte aligned, wpk words each; indices from `offset`) that a
+// screen with these counters has listed in cand, to dst.
 cudaError_t launch_fs_gather(const uint64_t* x, int wpk, const unsigned long long* cand,
-                             const unsigned long long* count, unsigned long long cap, unsigned long long offset,
-                             uint64_t* dst, int num_sms, cudaStream_t st);
+                             const unsigned long long* counters, unsigned long long offset, uint64_t* dst, int num_sms,
+                             cudaStream_t st);
 
 struct LaunchMpRefine {
   const uint64_t* x;
@@ -212,8 +212,7 @@ struct LaunchPairRefine {
   const EpiParams* P;
   const DevOutPairs* O;
   int num_sms;
-  bool count;                 // the candidates are not counted as evaluated yet (4-bit screen)
-  const LimbMap* LM;          // with count: the int8 limb columns,
+  const LimbMap* LM;          // behind the 4-bit screen: the int8 limb columns,
   const double* V;            // and the FP64 columns, vrows x cm
 };
 // The pair test with the 4-bit screen (kernel_fsp.cu).

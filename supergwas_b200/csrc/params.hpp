@@ -162,9 +162,36 @@ struct alignas(16) FsPheno {
 // Refinement candidates: marks of entries whose correlation gate is not decided.
 constexpr unsigned long long CAND_OPEN = 1ull << 63, CAND_OPEN_MP = 1ull << 47;
 
+// Counters of a launch (device): [0] tested, [1] hits, [2] error bits, [3]
+// refinement candidates, and those of the 4-bit screen: the tests that it has
+// decided, its undecided ones (candidates in the place of [3]'s), whether it has
+// given up in this launch and in any launch of the call.
+constexpr int CNT_FS_TESTED = 4, CNT_FS_OPEN = 5, CNT_FS_OVER = 6, CNT_FS_EVER = 7, NCOUNT = 8;
+
+// Undecided tests at which the screen gives up, and a kernel that evaluates every
+// test runs in its place.  A row near the span of U (a marker of a lineage) is
+// undecided whatever its statistic, and refining one costs as much as screening a
+// hundred (3 ns and 0.03 ns on the whole device at n = 1000, r = 16+1).  While an
+// eighth of the tests are done the limit is one in 128 of those, so that rows of one
+// kind are found out early, later one in 64 of all; calls of up to `base` tests never
+// give up.  1e7 rows at n = 1000, r = 16+1, of which 0, 1, 3, 10 and 100 % are lineage
+// markers, about half of them undecided: 0.30, 0.46, 0.79, 1.9 and 16 ms with all
+// of those refined; now 0.30, 0.47, 0.52, 0.51 and 0.52; 0.47 without the screen.
+constexpr unsigned long long FS_OPEN_BASE = 4096;
+__host__ __device__ inline unsigned long long fs_open_limit(unsigned long long base, unsigned long long done,
+                                                            unsigned long long total, unsigned long long cap) {
+  const unsigned long long v = total > base && 8 * done <= total ? base / 4 + done / 128 : base + total / 64;
+  return v < cap ? v : cap;
+}
+// Candidates that a launch of so many tests may have to list (at most 128 MB).
+inline unsigned long long fs_cand_room(unsigned long long base, unsigned long long total) {
+  const unsigned long long v = fs_open_limit(base, total, total, 1ull << 24);
+  return v > (1ull << 20) ? v : 1ull << 20;
+}
+
 // Device outputs of one launch.
 struct DevOut {
-  unsigned long long* counters;  // [0] tested, [1] hits, [2] error bits, [3] refinement candidates
+  unsigned long long* counters;
   kg_hit* hits;
   unsigned long long hit_cap;
   unsigned long long kmer_offset;  // added to the launch-local k-mer index
@@ -183,14 +210,18 @@ struct DevOut {
   // CTA issues this many row loads and then stops, so that the consumers'
   // waits run out (0: off)
   unsigned long long stall_loads;
-  // fs_kernel: no undecided k-mer is counted as tested (the kernel that takes
-  // them counts them)
+  // fs_kernel: the base of fs_open_limit; no undecided k-mer is counted as tested
+  // (the kernel that takes them counts them)
+  unsigned long long open_base;
   int count_sure;
   // tb_kernel, FP64 form: the rows are the gathered rows of the k-mers
-  // index[0 .. *rows), of which the launch has room for m; nothing runs when
-  // there are more
+  // index[0 .. *rows), at most m
   const unsigned long long* index;
   const unsigned long long* rows;
+  // a launch behind the screen: its counter CNT_FS_OVER.  The kernels run only
+  // where the screen has given up, the refinement and what reads `rows` take its
+  // candidates where it has not
+  const unsigned long long* over;
   __host__ __device__ unsigned long long kmer(unsigned long long local) const {
     return index ? index[local] : kmer_offset + local;
   }
@@ -213,7 +244,7 @@ struct MPheno {
 
 // Outputs of a multi-phenotype launch.
 struct DevOutMP {
-  unsigned long long* counters;      // [1] hits, [2] error bits, [3] refinement candidates
+  unsigned long long* counters;
   unsigned long long* tested;        // [shard * n_pheno + pheno]
   kg_phit* hits;
   unsigned long long hit_cap;
@@ -230,16 +261,23 @@ struct DevOutMP {
   unsigned long long wait_ns;
   // test hook of the bounded waits, as DevOut::stall_loads (0: off)
   unsigned long long stall_loads;
+  // behind the screen, as DevOut::over; its counts, which the refinement adds to
+  // `tested` where it has not given up, and clears
+  const unsigned long long* over;
+  unsigned long long* fs_tested;
+  unsigned long long open_base;      // of fs_open_limit
 };
 
 // Outputs of the 2-D pair test (kernel_pairs.cu).
 struct DevOutPairs {
-  unsigned long long* counters;  // [0] evaluated pairs, [1] hits, [2] error bits, [3] refinement candidates
+  unsigned long long* counters;  // [0]: evaluated pairs
   kg_pair* hits;
   unsigned long long hit_cap;
   unsigned long long* cand;      // i << 32 | j
   unsigned long long cand_cap;
   unsigned long long wait_ns;    // pipeline wait limit in ns (0: WAIT_LIMIT_NS)
+  const unsigned long long* over;  // behind the screen, as DevOut::over
+  unsigned long long open_base;    // of fs_open_limit
 };
 
 // Pair schedule: pairs (i, j), i < j, row_start <= i < row_end, j < n_kmers.

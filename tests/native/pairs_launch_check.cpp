@@ -30,6 +30,12 @@ cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) {
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "stand-in"; }
 
+unsigned long long kgctx::open_base() { return kg::FS_OPEN_BASE; }
+int kgctx::ensure_cand(kg_ctx* ctx, unsigned long long cap) {
+  ctx->cand_cap = cap;
+  return cudaMalloc((void**)&ctx->dCand, cap * sizeof(unsigned long long)) == cudaSuccess ? KG_OK : KG_ERR_NOMEM;
+}
+
 namespace kg {
 bool pairs_supported(int, int, int, int, int) { return true; }
 bool fsp_supported(int, int, int, int, unsigned long long) { return true; }

@@ -6,13 +6,12 @@ import pytest
 
 from supergwas_b200 import api, synth
 from test_gpu_screen4 import SHAPES, structure
-from test_gpu_ts_shapes import awkward_rows
 
 pytestmark = pytest.mark.gpu
 
 
-def rows_of(n, m, pop, y, rng):
-    X = synth.pack_rows(awkward_rows(n, min(m, 2048), pop, y, rng))
+def rows_of(n, m, rng):
+    X = synth.pack_rows((rng.random((2048, n)) < rng.random((2048, 1))).astype(np.uint8))
     return np.ascontiguousarray(X[np.arange(m) % X.shape[0]])
 
 
@@ -22,7 +21,7 @@ def test_one_phenotype(built, n, k, m, thr, lt, monkeypatch):
     rng = np.random.default_rng(n + k + m)
     pop, Z = structure(n, k, rng)
     y = rng.standard_normal(n) + 0.5 * pop + 2.0
-    X = rows_of(n, m, pop, y, rng)
+    X = rows_of(n, m, rng)
     monkeypatch.setenv("KG_DEDUP", "0")
     with api.Kgwas(corr_threshold=thr, log10_thresh=lt) as g:
         g.set_structure(np.linalg.qr(Z)[0], y)
@@ -47,7 +46,7 @@ def test_structures_that_need_more_or_are_refused(built, tail, limbs):
     U = np.linalg.qr(Z[keep])[0] * (1.5 if tail == "scale" else 1.0)
     with api.Kgwas(corr_threshold=0.0, log10_thresh=2.0 if tail == "threshold" else 6.0) as g:
         g.set_structure(U, y[keep], keep, n)
-        g.run_host(rows_of(n, 3000, pop, y, rng))
+        g.run_host(rows_of(n, 3000, rng))
         assert g.last_screen() == limbs
 
 
@@ -58,7 +57,7 @@ def test_pairs(built, n, k, m, thr, monkeypatch):
     rng = np.random.default_rng(n + m)
     pop, Z = structure(n, k, rng)
     y = rng.standard_normal(n) + 0.5 * pop
-    X = rows_of(n, m, pop, y, rng)
+    X = rows_of(n, m, rng)
     with api.Kgwas(corr_threshold=thr, log10_thresh=4.0) as g:
         g.set_structure(np.linalg.qr(Z)[0], y)
         g.run_pairs_host(X, 0, 40)
@@ -89,7 +88,7 @@ def test_many_phenotypes(built, monkeypatch):
     pop, Z = structure(n, k, rng)
     y = rng.standard_normal(n) + 0.5 * pop
     U = np.linalg.qr(Z)[0]
-    X = rows_of(n, 3000, pop, y, rng)
+    X = rows_of(n, 3000, rng)
     with api.Kgwas(corr_threshold=0.0, log10_thresh=6.0) as g:
         g.set_phenotypes([(U, y, np.arange(n))] * 3, n)
         g.run_multi_host(X)

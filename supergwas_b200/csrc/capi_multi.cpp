@@ -501,6 +501,7 @@ int kg_set_phenotypes(kg_ctx* ctx, const kg_pheno* ph, int np, int n_row) {
   kg::LaunchTable LT{M.dV, vrows, cm, (unsigned long long)M.vstride, np, M.dT};
   KG_CUDA(kg::launch_refine_table(LT, ctx->stream), "refinement tables");
   KG_CUDA(cudaStreamSynchronize(ctx->stream), "refinement tables");
+  if (std::getenv("KG_MP_STREAMED")) return KG_OK;  // the streamed kernel, without a screen
   return set_screen4_multi(ctx, ph, prep, mph, n_row);
 }
 

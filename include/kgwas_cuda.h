@@ -296,9 +296,10 @@ int kg_set_wait_limit(kg_ctx* ctx, uint64_t wait_ns);
 
 /* Failure test hook of the bounded waits, off by default: for the next
  * launch of a single-phenotype tensor-memory kernel or of the 4-bit screen of
- * many phenotypes only, the row producer of every CTA issues its first stop_after_loads row loads and then no more,
- * so that the waits of the roles it feeds run out (KG_ERR_TIMEOUT) instead of
- * completing.  No counterpart in the reference. */
+ * many phenotypes only, the row producer of every CTA issues its first
+ * stop_after_loads row loads and then no more, so that the waits of the roles it
+ * feeds run out (KG_ERR_TIMEOUT) instead of completing.  No counterpart in the
+ * reference. */
 int kg_inject_stall(kg_ctx* ctx, uint64_t stop_after_loads);
 
 const char* kg_last_error(const kg_ctx* ctx);

@@ -257,10 +257,10 @@ __device__ __forceinline__ void unpack_stage(const uint32_t (&w)[4], uint32_t (&
     }
 }
 
-// Bounded wait that also gives up when another role has aborted.  The first
-// test is inline (the common case: the phase is already complete), the rest a
-// call, so that the waits of all roles do not fill the instruction cache; the
-// abort flag and the clock are read only every 16 failed tests.  limit_ns:
+// Bounded wait that also gives up when another role has aborted: one test (the
+// common case: the phase is already complete), then tests that let the hardware
+// suspend the warp; the abort flag and the clock are read only every 16 of
+// those.  limit_ns:
 // how long to wait before giving up (a launch parameter, see wait_limit).
 static __device__ __forceinline__ bool wait_more(uint32_t bar, uint32_t parity, volatile int* abort,
                                               unsigned long long* counters, unsigned code,
@@ -433,46 +433,6 @@ __device__ __forceinline__ void finish_kmer(const EpiParams& P, const DevOut& O,
   emit_kmer(O, local, valid, tested, tested && p <= P.p_thresh, cand, T, p, effect, xxM, xyM, cor);
 }
 
-
-// As finish_kmer, for launches without per-k-mer outputs: the Pearson gate
-// and the emit / refinement screens compare squares instead of dividing
-// (|cor| >= thr  <=>  xyc^2 >= thr^2 ||xc||^2 ||yc||^2;  r2 >= t  <=>
-// xyM^2 >= t xxM yyM), and only k-mers that may reach the emit cut evaluate
-// the reference formula (src/kgwas.cpp:47-53) exactly.
-__device__ __forceinline__ void finish_kmer_fast(const EpiParams& P, const DevOut& O, unsigned long long local,
-                                                 bool valid, int c, double ss, double gs, double ey) {
-  const int n = P.n;
-  bool tested = valid && c > 0 && c < n && !(P.ynorm < 1e-12);
-  if (tested && P.corr_thr > 0.0) {
-    const double xcn2 = (double)c * (double)(n - c) / (double)n;
-    const double xyc = ey + gs + P.kappa * (double)c;
-    tested = xyc * xyc >= P.thr2_ynorm2 * xcn2;
-  }
-  double xxM = 0, xyM = 0, effect = 0, T = 0, p = 1;
-  bool cand = false, hit = false;
-  if (tested) {
-    const double cd = i2d_exact(c);
-    xxM = cd - ss;
-    xyM = P.b * cd + ey;
-    const double eps = 1e-12;
-    if (xxM > eps && P.yyM > eps) {
-      const double q = xyM * xyM, den = xxM * P.yyM;
-      if (P.refine && q >= P.r2_ref * den) {
-        cand = true;
-      } else if (q >= P.r2_cand * den) {
-        double r2 = q / den;
-        if (r2 < 0) r2 = 0;
-        if (r2 >= 1) r2 = 1 - 1e-15;
-        T = (double)n * log(1.0 / (1.0 - r2));
-        p = erfc(sqrt(0.5 * T));
-        effect = xyM / den;
-        hit = p <= P.p_thresh;
-      }
-    }
-  }
-  emit_kmer(O, local, valid, tested, hit, cand, T, p, effect, xxM, xyM, 0.0);
-}
-
 // Whether a tested k-mer of the split form goes to the FP64 refinement in a
 // launch that returns emitted rows only: r2 = q / den at least r2_ref, and not
 // so far below the emit cut that refining cannot matter (set_refine_need).
@@ -484,10 +444,13 @@ __device__ __forceinline__ bool may_refine(const EpiParams& P, double cd, double
          (q >= P.r2_need * den || !(xxM >= XXM_FLOOR * cd * ((double)P.n - cd) / (double)P.n));
 }
 
-// Fast screen of one k-mer for kernels that count tested k-mers in a
-// register (tested_local, flushed once per warp by the caller): in the common
+// As finish_kmer, for launches without per-k-mer outputs: the Pearson gate
+// and the emit / refinement screens compare squares instead of dividing
+// (|cor| >= thr  <=>  xyc^2 >= thr^2 ||xc||^2 ||yc||^2;  r2 >= t  <=>
+// xyM^2 >= t xxM yyM), and only k-mers that may reach the emit cut evaluate
+// the reference formula (src/kgwas.cpp:47-53) exactly.  Tested k-mers are counted
+// in a register (tested_local, flushed once per warp by the caller): in the common
 // case (no hit, no refinement candidate in the warp) it costs one ballot.
-// Same decisions and values as finish_kmer_fast.
 __device__ __forceinline__ void finish_kmer_lean(const EpiParams& P, const DevOut& O, unsigned long long local,
                                                  bool valid, int c, double cd, double ss, double gs, double ey,
                                                  uint32_t& tested_local) {
@@ -755,7 +718,7 @@ __device__ __forceinline__ void tb_count(const DevOutMP& O, int p, int shard, ui
 }
 
 // Statistic of one (k-mer, phenotype) from the exact integer sums, as the
-// division-free screen of finish_kmer_fast; writes the outcome flags.
+// division-free screen of finish_kmer_lean; writes the outcome flags.
 __device__ __forceinline__ void mp_eval(const EpiParams& P, bool valid, int c, double ss, double gs, double ey,
                                         bool& tested, bool& hit, bool& cand, double& T, double& p, double& effect) {
   const int n = P.n;
@@ -904,10 +867,8 @@ __device__ __forceinline__ bool mp_test(const DevOutMP& O, const MPheno* ME, uin
 }
 
 // Warp-aggregated hit records and FP64 refinement candidates (k-mer |
-// phenotype << 48) of one (k-mer, phenotype) per lane.  mp_emit adds the
-// tested count of (shard, phenotype) with one atomic per shard present in the
-// warp (match = the lanes of this lane's shard, leader = the lowest of them).
-// All 32 lanes of the warp must call them.
+// phenotype << 48) of one (k-mer, phenotype) per lane.  All 32 lanes of the warp
+// must call it.
 __device__ __forceinline__ void mp_emit_rare(const DevOutMP& O, int p, unsigned long long gk, int shard, bool hit,
                                              bool cand, double T, double pv, double effect) {
   const unsigned lane = threadIdx.x & 31u;
@@ -945,21 +906,6 @@ __device__ __forceinline__ void mp_emit_rare(const DevOutMP& O, int p, unsigned 
       else atomicOr(O.counters + 2, (unsigned long long)ERR_CAND_OVERFLOW);
     }
   }
-}
-
-__device__ __forceinline__ void mp_emit(const DevOutMP& O, int p, unsigned long long gk, int shard, unsigned match,
-                                        bool leader, bool tested, bool hit, bool cand, double T, double pv,
-                                        double effect) {
-  if (O.weight) {
-    // the lanes of one shard (match) add their rows' weights
-    const unsigned tot = __reduce_add_sync(match, tested ? O.weight[gk] : 0u);
-    if (leader && tot) atomicAdd(O.tested + (size_t)shard * O.n_pheno + p, (unsigned long long)tot);
-  } else {
-    const unsigned tm = __ballot_sync(0xffffffffu, tested);
-    if (leader && (tm & match))
-      atomicAdd(O.tested + (size_t)shard * O.n_pheno + p, (unsigned long long)__popc(tm & match));
-  }
-  mp_emit_rare(O, p, gk, shard, hit, cand, T, pv, effect);
 }
 
 // ------------------------------------------------------ pair schedule

@@ -166,49 +166,41 @@ def run_reference_arm(args):
     rank, world, _ = rank_env()
     if rank != 0:
         return
+    if not reference_binary():
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's kgwas program is not on this machine"}),
+              flush=True)
+        return
     W = WORKLOAD
     threads = os.cpu_count() or 1
     m_sample = args.ref_kmers
     vals = []
-    kind = "reference" if reference_binary() else "port"
     with tempfile.TemporaryDirectory() as d:
-        if kind == "reference":
-            from oracle import oracle as O
-            tested, dt, paths = cpu_reference_run(W["n"], m_sample, W["r"], W["seed"], threads, d)
-            env = {"CORR_THRESHOLD": "0", "LOAD_THREADS": threads, "BLAS_THREADS": threads,
-                   "EMIT_THREADS": threads}
-            out = os.path.join(d, "out", "batch_000.tsv")
-            for i in range(args.warmup + args.steps):
-                t0 = time.perf_counter()
-                res = O.run_reference([paths["samples"], paths["pheno"], paths["batch"], paths["ubin"], out,
-                                       "6"], env)
-                dt = time.perf_counter() - t0
-                if res.returncode != 0:
-                    raise RuntimeError(res.stderr[-500:])
-                if i >= args.warmup:
-                    vals.append((int(open(out + ".count").read().split("\t")[1]), dt))
-        else:
-            for i in range(args.warmup + args.steps):
-                tested, dt = cpu_port_run(W["n"], max(1000, m_sample // 20), W["r"], W["seed"])
-                if i >= args.warmup:
-                    vals.append((tested, dt))
+        from oracle import oracle as O
+        tested, dt, paths = cpu_reference_run(W["n"], m_sample, W["r"], W["seed"], threads, d)
+        env = {"CORR_THRESHOLD": "0", "LOAD_THREADS": threads, "BLAS_THREADS": threads, "EMIT_THREADS": threads}
+        out = os.path.join(d, "out", "batch_000.tsv")
+        for i in range(args.warmup + args.steps):
+            t0 = time.perf_counter()
+            res = O.run_reference([paths["samples"], paths["pheno"], paths["batch"], paths["ubin"], out, "6"], env)
+            dt = time.perf_counter() - t0
+            if res.returncode != 0:
+                raise RuntimeError(res.stderr[-500:])
+            if i >= args.warmup:
+                vals.append((int(open(out + ".count").read().split("\t")[1]), dt))
     tests = sum(t for t, _ in vals)
     secs = sum(s for _, s in vals)
     v = tests / secs
-    ms = m_sample if kind == "reference" else max(1000, m_sample // 20)
     line = {"impl": "reference", "metric": METRIC, "value": v, "unit": "k-mer tests/s", "n_gpus": args.gpus,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1e3 * secs / len(vals),
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "f32 (reference COLS mode)" if kind == "reference" else "f64",
+            "dtype": "f32 (reference COLS mode)",
             "data": "synthetic",
             "config": {"workload": f"n={W['n']} (5% unphenotyped), r={W['r']}+1, 1 phenotype, "
-                                   f"CORR_THRESHOLD=0; each step one {ms}-k-mer batch of that workload",
+                                   f"CORR_THRESHOLD=0; each step one {m_sample}-k-mer batch of that workload",
                        "parallelism": "host cores"},
-            "cpu_baseline": {"value": v, "unit": "k-mer tests/s", "cores": threads if kind == "reference" else 1,
-                             "kind": kind,
-                             "sample": (f"shipped reference kgwas --mode cols on {ms} k-mers per step, wall "
-                                        "clock of the process (file load included)") if kind == "reference"
-                             else f"FP64 C oracle on {ms} k-mers per step"},
+            "cpu_baseline": {"value": v, "unit": "k-mer tests/s", "cores": threads, "kind": "reference",
+                             "sample": f"shipped reference kgwas --mode cols on {m_sample} k-mers per step, wall "
+                                       "clock of the process (file load included)"},
             "e2e": {"value": v, "unit": "k-mer tests/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
     print(json.dumps(line), flush=True)
 

@@ -14,22 +14,21 @@ constexpr int FS_XST_MAX = 12, FS_CH_MAX = 24, FS_MAXSLOT = 3;
 __host__ __device__ constexpr int fs_nslot(int N) { return 2 * N + FS_SF <= 128 ? 3 : 2; }
 __host__ __device__ constexpr int fs_threads(int N) { return 32 * (8 + 4 * fs_nslot(N) + 4); }
 
-// As wait_or_abort, but returns within a few microseconds of the abort flag: the
-// screen gives up through it, and at 16 suspensions of 1 ms per look at the flag a
-// launch that gave up took 13 ms.
+// As wait_or_abort, but looks at the abort flag before every suspension, and
+// suspends for a few microseconds at most: the screen gives up through the flag (at
+// 16 suspensions of 1 ms per look a launch that gave up took 13 ms).
 __device__ __forceinline__ bool fs_wait(uint32_t bar, uint32_t parity, volatile int* abort,
                                         unsigned long long* counters, unsigned code, unsigned long long limit_ns) {
   if (mbar_try(bar, parity)) return true;
   const unsigned long long t0 = gtimer_ns();
-  while (!mbar_try_sleep<4000u>(bar, parity)) {
-    if (*abort) return false;
+  while (!*abort) {
+    if (mbar_try_sleep<4000u>(bar, parity)) return true;
     if (gtimer_ns() - t0 > limit_ns) {
       atomicOr(counters + 2, (unsigned long long)code);
       *abort = 1;
-      return false;
     }
   }
-  return true;
+  return false;
 }
 
 // D[tmem] (+)= A[tmem] * B[smem desc], e2m1 x e2m1 in blocks of 32 with ue8m0
@@ -132,25 +131,36 @@ __device__ __forceinline__ void fs_constants(const FsPheno* __restrict__ F, FsPh
   }
 }
 
-// Appends the lanes with `take` to the candidate list (warp-aggregated).  False
-// where the list holds more than `limit` then (fs_open_limit): the screen gives up.
-__device__ __forceinline__ bool fs_push(unsigned long long* counters, unsigned long long* cand,
-                                        unsigned long long limit, bool take, unsigned long long entry) {
+// Appends the lanes with `take` to the candidate list (warp-aggregated).  Where that
+// is too many for the tests done (fs_open_limit) the screen gives up: the counters
+// say so and the CTA's waits end.
+__device__ __forceinline__ void fs_push(unsigned long long* counters, volatile int* abort,
+                                            unsigned long long* cand, unsigned long long cap,
+                                            unsigned long long base_open, unsigned long long done,
+                                            unsigned long long total, bool take, unsigned long long entry) {
   const unsigned lane = threadIdx.x & 31u;
   const unsigned mask = __ballot_sync(0xffffffffu, take);
   unsigned long long base = 0;
   const int leader = __ffs(mask) - 1;
   if ((int)lane == leader) base = atomicAdd(counters + CNT_FS_OPEN, (unsigned long long)__popc(mask));
   base = __shfl_sync(0xffffffffu, base, leader);
-  if (base + __popc(mask) > limit) {
+  if (base + __popc(mask) > fs_open_limit(base_open, done, total, cap)) {
     if ((int)lane == leader) {
       atomicExch(counters + CNT_FS_OVER, 1ull);
       atomicExch(counters + CNT_FS_EVER, 1ull);
+      *abort = 1;
     }
-    return false;
+  } else if (take) {
+    cand[base + __popc(mask & ((1u << lane) - 1u))] = entry;
   }
-  if (take) cand[base + __popc(mask & ((1u << lane) - 1u))] = entry;
-  return true;
+}
+// The same as a call: where a warp has one test per item, few warps come here, and
+// inlined it cost the rest of the kernel 2 % (1e8 k-mers at n = 1000).
+static __device__ __noinline__ void fs_push_call(unsigned long long* counters, volatile int* abort,
+                                                 unsigned long long* cand, unsigned long long cap,
+                                                 unsigned long long base_open, unsigned long long done,
+                                                 unsigned long long total, bool take, unsigned long long entry) {
+  fs_push(counters, abort, cand, cap, base_open, done, total, take, entry);
 }
 // Adds a warp's counts of decided tests (32 bits in all, as flush_tested).
 __device__ __forceinline__ void fs_flush(unsigned long long* counters, uint32_t cnt) {

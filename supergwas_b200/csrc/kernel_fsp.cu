@@ -291,14 +291,9 @@ __global__ void __launch_bounds__(fsp_threads(N), 1)
         mbar_arrive_if(acc_empty + 8 * e, lane == 0);
         const int vd = fs_verdict<N, LU, GATE, true>(F, d, j < S.n_kmers && j > i);
         evaluated += vd == 1 ? 1u : 0u;
-        if (__any_sync(0xffffffffu, vd >= 2) &&
-            !fs_push(O.counters, O.cand,
-                     fs_open_limit(O.open_base, (v + 1ull) * gridDim.x * FS_TM, S.n_units * S.ic * FS_TM, O.cand_cap),
-                     vd >= 2, (i << 32) | j)) {
-          ok = false;  // given up, as in kernel_fs.cu
-          if (lane == 0) *s_abort = 1;
-          break;
-        }
+        if (__any_sync(0xffffffffu, vd >= 2))
+          fs_push_call(O.counters, s_abort, O.cand, O.cand_cap, O.open_base, (v + 1ull) * gridDim.x * FS_TM,
+                  S.n_units * S.ic * FS_TM, vd >= 2, (i << 32) | j);
       }
     }
     fs_flush(O.counters, evaluated);

@@ -11,6 +11,19 @@ namespace kg {
 
 constexpr unsigned long long MP_KMER_MASK = (1ull << 47) - 1;  // bit 47: CAND_OPEN_MP
 
+// Adds the screen's counts to the launch's, unless it gave up, and clears them for
+// the next launch.  A call: inlined, it changes the registers that the compiler
+// gives the candidates' loop (8 phenotypes at n = 5000: 65 -> 101 us).
+static __device__ __noinline__ void mp_add_counts(const DevOutMP& O, unsigned nc) {
+  const bool fs = !*O.over;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < nc; i += gridDim.x * blockDim.x) {
+    const unsigned long long c = O.fs_tested[i];
+    if (!c) continue;
+    if (fs) atomicAdd(O.tested + i, c);
+    O.fs_tested[i] = 0;
+  }
+}
+
 // FP64 recomputation of the candidates of a multi-phenotype launch: one
 // warp per (k-mer, phenotype), the phenotype's byte tables at T + p*tstride
 // (lanes own the FP64 columns, one table row per byte of the packed row).
@@ -21,17 +34,9 @@ __global__ void __launch_bounds__(256) mp_refine_kernel(const uint64_t* __restri
                                                         const MPheno* __restrict__ ph, const DevOutMP O) {
   const int lane = threadIdx.x & 31;
   const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
-  const bool fs = O.over && !*O.over;  // the 4-bit screen's candidates and counts
-  if (O.over) {
-    const unsigned long long nc = (unsigned long long)O.n_shards * O.n_pheno;
-    for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < nc;
-         i += (unsigned long long)gridDim.x * blockDim.x) {
-      const unsigned long long c = O.fs_tested[i];
-      if (!c) continue;
-      if (fs) atomicAdd(O.tested + i, c);
-      O.fs_tested[i] = 0;  // for the next launch
-    }
-  }
+  const unsigned nc = O.over ? (unsigned)O.n_shards * (unsigned)O.n_pheno : 0u;
+  if (blockIdx.x * blockDim.x < nc) mp_add_counts(O, nc);
+  const bool fs = O.over && !*O.over;  // the 4-bit screen's candidates
   unsigned long long ncand = O.counters[fs ? CNT_FS_OPEN : 3];
   if (ncand > O.cand_cap) ncand = O.cand_cap;
   for (unsigned long long w = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < ncand;

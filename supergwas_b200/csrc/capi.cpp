@@ -871,6 +871,8 @@ int run_host_once(kg_ctx* ctx, const uint64_t* xbits, uint64_t m, uint32_t wpk, 
   }
   KG_CUDA(cudaMemsetAsync(ctx->dCounters, 0, sizeof(ctx->counters), ctx->stream), "memset");
   const uint64_t nch = (m + per - 1) / per;
+  // the rows of a single chunk are still there for a repeat
+  const Screen mode = nch == 1 ? SCREEN_REPEAT : SCREEN_BEHIND;
   uint64_t u0 = 0;  // runs before this chunk
   std::vector<StageSeg> segs;
   for (uint64_t i = 0; i < nch; ++i) {
@@ -906,12 +908,19 @@ int run_host_once(kg_ctx* ctx, const uint64_t* xbits, uint64_t m, uint32_t wpk, 
     }
     KG_CUDA(cudaEventRecord(ctx->ev_h2d[b], ctx->copy_stream), "record");
     KG_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->ev_h2d[b], 0), "wait");
-    int rc = launch_one(ctx, ctx->dChunk[b], rows, wpk, offset, stats, i == 0, SCREEN_BEHIND, ctx->stream);
+    int rc = launch_one(ctx, ctx->dChunk[b], rows, wpk, offset, stats, i == 0, mode, ctx->stream);
     if (rc) return rc;
     KG_CUDA(cudaEventRecord(ctx->ev_k[b], ctx->stream), "record");
   }
   if (runs) ctx->unique_rows = u0;
-  return read_counters(ctx, ctx->stream);
+  if (int rc = read_counters(ctx, ctx->stream)) return rc;
+  if (mode != SCREEN_REPEAT || !ctx->counters[kg::CNT_FS_EVER]) return KG_OK;
+  const int screen = ctx->last_screen;
+  KG_CUDA(cudaMemsetAsync(ctx->dCounters, 0, sizeof(ctx->counters), ctx->stream), "memset");
+  if (int rc = launch_one(ctx, ctx->dChunk[0], runs ? u0 : m, wpk, 0, stats, true, SCREEN_OFF, ctx->stream)) return rc;
+  if (int rc = read_counters(ctx, ctx->stream)) return rc;
+  ctx->last_screen = screen;
+  return KG_OK;
 }
 
 }  // namespace

@@ -694,10 +694,18 @@ int kg_run_multi_host(kg_ctx* ctx, const uint64_t* xbits, uint64_t m, uint32_t w
       KG_CUDA(cudaStreamWaitEvent(st, ctx->ev_h2d[b], 0), "wait");
       if (i == 0 && (rc = autotune(ctx, ctx->dChunk[b], cnt, wpk, st))) return rc;
       if (i == 0 && (rc = reset_outputs(ctx, st))) return rc;  // the autotuner's trial launches wrote outputs
-      if ((rc = enqueue_multi(ctx, ctx->dChunk[b], cnt, wpk, s0, i == 0, SCREEN_BEHIND, st))) return rc;
+      if ((rc = enqueue_multi(ctx, ctx->dChunk[b], cnt, wpk, s0, i == 0, nch == 1 ? SCREEN_REPEAT : SCREEN_BEHIND, st)))
+        return rc;
       KG_CUDA(cudaEventRecord(ctx->ev_k[b], st), "record");
     }
     if ((rc = read_multi_counters(ctx, st))) return rc;
+    if (nch == 1 && M.counters[kg::CNT_FS_EVER]) {  // the rows of a single chunk are still there
+      const int screen = ctx->last_screen;
+      if ((rc = reset_outputs(ctx, st))) return rc;
+      if ((rc = enqueue_multi(ctx, ctx->dChunk[0], m, wpk, 0, true, SCREEN_OFF, st))) return rc;
+      if ((rc = read_multi_counters(ctx, st))) return rc;
+      ctx->last_screen = screen;
+    }
     if (!(M.counters[2] & (kg::ERR_HIT_OVERFLOW | kg::ERR_CAND_OVERFLOW))) break;
     if ((M.counters[2] & kg::ERR_HIT_OVERFLOW) && (rc = ensure_multi_out(ctx, M.n_shards, M.counters[1])))
       return rc;

@@ -353,7 +353,8 @@ void limb_loss(const Prepared& p, const double* scale, LimbLoss& B) {
     const double sc = scale[j], up = 1.0 / sc;  // powers of two
     double sq = 0, sum = 0;
     for (int i = 0; i < p.n; ++i) {
-      const double r = d[i] - sc * std::round(d[i] * up);
+      const double t = d[i] * up;  // to the nearest integer, in make_limbs' way and inline
+      const double r = sc * (t - (double)(long long)(t + std::copysign(0.5, t)));
       sq += r * r;
       sum += r;
     }

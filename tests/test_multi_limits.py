@@ -14,7 +14,7 @@ def test_number_of_kmers():
     out = os.path.join(HERE, "native", "_build", "libmulti_limits_check.so")
     os.makedirs(os.path.dirname(out), exist_ok=True)
     cuda = os.path.join(os.path.dirname(os.path.dirname(build.nvcc())), "include")
-    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I" + cuda, "-o", out,
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic-functions", "-I" + cuda, "-o", out,
                     os.path.join(HERE, "native", "multi_limits_check.cpp"), "-lpthread"], check=True)
     call = ctypes.CDLL(out, mode=os.RTLD_LAZY).multi_call
     call.argtypes = [ctypes.c_uint64]

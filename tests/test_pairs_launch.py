@@ -18,7 +18,7 @@ def pairs_call():
     out = os.path.join(HERE, "native", "_build", "libpairs_launch_check.so")
     os.makedirs(os.path.dirname(out), exist_ok=True)
     cuda = os.path.join(os.path.dirname(os.path.dirname(build.nvcc())), "include")
-    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-I" + cuda, "-o", out,
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic-functions", "-I" + cuda, "-o", out,
                     os.path.join(HERE, "native", "pairs_launch_check.cpp"), "-lpthread"], check=True)
     fn = ctypes.CDLL(out).pairs_call
 

@@ -351,9 +351,9 @@ namespace kgctx {
 
 // Copies bytes from pageable memory to the device through the pinned buffer
 // `stage`, 4 MB at a time: up to 16 host threads fill the blocks in order and
-// each goes to `st` as soon as it is filled.  With the whole staging copy before
-// the transfer a call on 128 MB (1e6 k-mers at n = 1000) took 7.05 ms, now 6.5;
-// the host's memory bounds it (the rows are read, staged and read again).
+// each goes to `st` as soon as it is filled.  A call on 128 MB (1e6 k-mers at
+// n = 1000) takes 6.5 to 6.9 ms, 7.0 with the whole staging copy before the
+// transfer, which is within what runs differ by (6 %); the link would take 2.3.
 cudaError_t stage_h2d(void* dst, void* stage, const void* src, size_t bytes, cudaStream_t st) {
   const size_t B = (size_t)4 << 20, nb = (bytes + B - 1) / B;
   const unsigned nt = (unsigned)std::min<size_t>(std::min<unsigned>(16, std::max(1u, std::thread::hardware_concurrency())), nb);

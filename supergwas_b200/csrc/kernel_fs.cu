@@ -34,11 +34,11 @@
 //
 // What bounds it: one phenotype, the rows' bytes (1e8 k-mers at n = 1000,
 // r = 16+1: 12.8 GB at 6.5 TB/s are 1.96 ms; the kernel takes 2.2 ms); many,
-// the MMAs (64 phenotypes x 4e6 at n = 2000, r = 20+1: 3.7 of 5.3 ms at 24
+// the MMAs (64 phenotypes x 4e6 at n = 2000, r = 20+1: 3.7 of 4.6 ms at 24
 // columns a phenotype).  Whole calls, before (int8 limbs, kernel_ts.cu,
-// kernel_tb.cu, kernel_mpb2.cu) and now: 1e8 at n = 1000 4.80 -> 2.60 ms; 1e7
-// at n = 2000 1.12 -> 0.54; 2e6 at n = 5000, r = 32+1 0.99 -> 0.41; 64
-// phenotypes x 4e6 at n = 2000 22.9 -> 5.7; 8 x 1e6 at n = 5000 3.38 -> 1.13.
+// kernel_tb.cu, kernel_mpb2.cu) and now: 1e8 at n = 1000 4.80 -> 2.7 ms; 1e7
+// at n = 2000 1.12 -> 0.56; 2e6 at n = 5000, r = 32+1 0.99 -> 0.37; 64
+// phenotypes x 4e6 at n = 2000 22.9 -> 5.4; 8 x 1e6 at n = 5000 3.38 -> 1.06.
 // One limb per U column: with two (48 columns instead of 24 at n = 1000) the MMAs
 // bound it (2.6 ms); the few more undecided k-mers cost 0.01 ms.
 #include <cuda.h>

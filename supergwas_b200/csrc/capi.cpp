@@ -980,7 +980,7 @@ int kg_launch_device(kg_ctx* ctx, const uint64_t* d_x, uint64_t m, uint32_t wpk,
   cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
   ctx->launches = 0;
   KG_CUDA(cudaMemsetAsync(ctx->dCounters, 0, sizeof(ctx->counters), st), "memset");
-  if ((rc = launch_one(ctx, d_x, m, wpk, 0, ctx->pend_stats, true, SCREEN_REPEAT, st))) return rc;
+  if ((rc = launch_one(ctx, d_x, m, wpk, 0, ctx->pend_stats, true, SCREEN_BEHIND, st))) return rc;
   ctx->pending = true;
   ctx->pend_x = d_x;
   ctx->pend_m = m;
@@ -1034,18 +1034,13 @@ extern "C" int kg_fetch(kg_ctx* ctx, kg_result* res, kg_stats* st) {
   ctx->pend_stats = false;
   int rc = read_counters(ctx, ctx->pend_stream);
   if (rc) return rc;
-  const int screen = ctx->last_screen;  // negative: it gave up
-  for (int retry = 0; retry < 8 && ((ctx->counters[2] & (kg::ERR_HIT_OVERFLOW | kg::ERR_CAND_OVERFLOW)) ||
-                                    ctx->counters[kg::CNT_FS_EVER]);
-       ++retry) {
+  for (int retry = 0; retry < 8 && (ctx->counters[2] & (kg::ERR_HIT_OVERFLOW | kg::ERR_CAND_OVERFLOW)); ++retry) {
     if ((ctx->counters[2] & kg::ERR_HIT_OVERFLOW) && (rc = ensure_hits(ctx, ctx->counters[1]))) return rc;
     if ((ctx->counters[2] & kg::ERR_CAND_OVERFLOW) && (rc = ensure_cand(ctx, 4 * ctx->cand_cap))) return rc;
     KG_CUDA(cudaMemsetAsync(ctx->dCounters, 0, sizeof(ctx->counters), ctx->pend_stream), "memset");
-    if ((rc = launch_one(ctx, ctx->pend_x, ctx->pend_m, ctx->pend_wpk, 0, stats, true,
-                         screen < 0 ? SCREEN_OFF : SCREEN_REPEAT, ctx->pend_stream)))
+    if ((rc = launch_one(ctx, ctx->pend_x, ctx->pend_m, ctx->pend_wpk, 0, stats, true, SCREEN_BEHIND, ctx->pend_stream)))
       return rc;
     if ((rc = read_counters(ctx, ctx->pend_stream))) return rc;
   }
-  ctx->last_screen = screen;
   return collect(ctx, ctx->pend_m, res, st, stats);
 }

@@ -560,7 +560,7 @@ int kg_launch_multi_device(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t
     cudaGraph_t g = nullptr;
     KG_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "capture");
     int r1 = reset_outputs(ctx, st);
-    int r2 = r1 ? r1 : enqueue_multi(ctx, dx, m, wpk, 0, true, SCREEN_REPEAT, st);
+    int r2 = r1 ? r1 : enqueue_multi(ctx, dx, m, wpk, 0, true, SCREEN_BEHIND, st);
     cudaError_t ec = cudaStreamEndCapture(st, &g);
     if (r2) {
       if (g) cudaGraphDestroy(g);
@@ -574,7 +574,7 @@ int kg_launch_multi_device(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t
     KG_CUDA(cudaGraphLaunch(M.graph, st), "graph launch");
   } else {
     if ((rc = reset_outputs(ctx, st))) return rc;
-    if ((rc = enqueue_multi(ctx, dx, m, wpk, 0, true, SCREEN_REPEAT, st))) return rc;
+    if ((rc = enqueue_multi(ctx, dx, m, wpk, 0, true, SCREEN_BEHIND, st))) return rc;
     M.g_seen++;
   }
   M.pending = true;
@@ -593,20 +593,14 @@ int kg_fetch_multi(kg_ctx* ctx, kg_multi_result* res) {
   M.pending = false;
   int rc = read_multi_counters(ctx, M.pend_stream);
   if (rc) return rc;
-  const int screen = ctx->last_screen;  // negative: it gave up
-  for (int retry = 0; retry < 8 && ((M.counters[2] & (kg::ERR_HIT_OVERFLOW | kg::ERR_CAND_OVERFLOW)) ||
-                                    M.counters[kg::CNT_FS_EVER]);
-       ++retry) {
+  for (int retry = 0; retry < 8 && (M.counters[2] & (kg::ERR_HIT_OVERFLOW | kg::ERR_CAND_OVERFLOW)); ++retry) {
     if ((M.counters[2] & kg::ERR_HIT_OVERFLOW) && (rc = ensure_multi_out(ctx, M.n_shards, M.counters[1])))
       return rc;
     if ((M.counters[2] & kg::ERR_CAND_OVERFLOW) && (rc = ensure_cand(ctx, 4 * ctx->cand_cap))) return rc;
     if ((rc = reset_outputs(ctx, M.pend_stream))) return rc;
-    if ((rc = enqueue_multi(ctx, M.pend_x, M.pend_m, M.pend_wpk, 0, true, screen < 0 ? SCREEN_OFF : SCREEN_REPEAT,
-                            M.pend_stream)))
-      return rc;
+    if ((rc = enqueue_multi(ctx, M.pend_x, M.pend_m, M.pend_wpk, 0, true, SCREEN_BEHIND, M.pend_stream))) return rc;
     if ((rc = read_multi_counters(ctx, M.pend_stream))) return rc;
   }
-  ctx->last_screen = screen;
   return collect_multi(ctx, M.pend_m, res);
 }
 

@@ -296,8 +296,9 @@ bool find_runs(kg_ctx* ctx, const uint64_t* x, uint64_t m, uint32_t wpk, const s
                bool pageable);
 bool is_pinned(const void* p);
 // What a launch does about rows that the 4-bit screen cannot place: it is repeated
-// without the screen once its counters have been read (the rows stay where they
-// are), or the kernel for that case is launched behind the screen.
+// without the screen once its counters have been read (rows in buffers of the
+// context), or the kernel for that case is launched behind the screen (rows that a
+// caller, or the next chunk, may overwrite as soon as the launch is done).
 enum Screen { SCREEN_REPEAT, SCREEN_BEHIND, SCREEN_OFF };
 // The base of kg::fs_open_limit: FS_OPEN_BASE, or KG_SCREEN_OPEN (0: the shares
 // alone; 16777216: never reached).

@@ -292,6 +292,12 @@ __device__ __forceinline__ unsigned long long wait_limit(unsigned long long ns) 
   return ns ? ns : WAIT_LIMIT_NS;
 }
 
+// A launch behind the 4-bit screen may start while the one before it still runs
+// (launch_behind in kernels.hpp): waits until that one is done and its writes are
+// seen.  next_may_start: a launch that follows in this way may be set up.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Ring position: slot index and phase parity, advanced without division.
 template <int NS>
 struct Ring {

@@ -10,9 +10,9 @@
 // every value that leaves the device is FP64, and no decision rests on a sum
 // whose bound does not carry it.  Where too many tests stay undecided
 // (fs_open_limit) the screen gives up: its CTAs leave by the path of a wait that
-// ran out, without an error, and another kernel evaluates every test: one launched
-// behind it, which otherwise ends at once (5 us), where rows stream through, and a
-// second launch where the rows stay on the device.
+// ran out, without an error, and another kernel evaluates every test: launched
+// behind it, where it ends at once otherwise, or by a second call where the rows are
+// in a buffer of the context.
 //
 // Operands: A = the packed bits spread over 4-bit floats, 8 per 32-bit word,
 // in tensor memory: of a word w, w & 0x11111111 holds its samples 4i as 0.5,
@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(fs_threads(NP * PPG), 1)
   const uint32_t ntiles = (uint32_t)((m + FS_TM - 1) / FS_TM);
   const uint32_t mine = ntiles > blockIdx.x ? (ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;  // tiles of this CTA
 
+  next_may_start();
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(s_tmem))
                  : "memory");

@@ -122,7 +122,10 @@ __global__ void __launch_bounds__(mb_threads(NP * PPG), 1)
   const unsigned long long nt =
       ntiles > blockIdx.x ? (ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0ull;
 
-  if (O.over && !*O.over) return;  // the screen has decided
+  if (O.over) {
+    wait_for_previous();
+    if (!*O.over) return;  // the screen has decided
+  }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(s_tmem))
                  : "memory");
@@ -414,10 +417,8 @@ static cudaError_t launch_mpb_t(const LaunchMpb& L, const CUtensorMap& tm, cudaS
   unsigned long long grid = (unsigned long long)L.num_sms;
   if (grid > tiles) grid = tiles;
   const int nbox = (L.wpk * 8 + 127) / 128;
-  mpb_kernel<NP, PPG><<<(unsigned)grid, mb_threads(N), smem, st>>>(tm, L.m, nbox, L.kpad / MB_KS, L.G,
-                                                                   L.bt > 0 ? L.bt : 1, L.Bimg, b_bytes, L.ph,
-                                                                   *L.O);
-  return cudaGetLastError();
+  return launch_behind(L.O->over != nullptr, mpb_kernel<NP, PPG>, (unsigned)grid, mb_threads(N), smem, st, tm, L.m,
+                       nbox, L.kpad / MB_KS, L.G, L.bt > 0 ? L.bt : 1, L.Bimg, b_bytes, L.ph, *L.O);
 }
 
 cudaError_t launch_mpb(const LaunchMpb& L, cudaStream_t st) {

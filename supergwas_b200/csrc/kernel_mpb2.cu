@@ -193,7 +193,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(M2_THREADS, 1)
   const unsigned long long npt = (m + 2 * M2_TM - 1) / (2 * M2_TM);
   const unsigned long long nt = npt > pair ? (npt - pair + npairs - 1) / npairs : 0ull;
 
-  if (O.over && !*O.over) return;  // the screen has decided
+  if (O.over) {
+    wait_for_previous();
+    if (!*O.over) return;  // the screen has decided
+  }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(s_tmem))
                  : "memory");
@@ -513,9 +516,8 @@ static cudaError_t launch_mpb2_t(const LaunchMpb& L, const CUtensorMap& tm, cuda
   if (pairs < 1) pairs = 1;
   const int nbox = (L.wpk * 8 + 127) / 128;
   const int G = (L.G + 1) / 2;  // L.G phenotypes (one image each), two per MMA
-  mpb2_kernel<NP><<<(unsigned)(2 * pairs), M2_THREADS, smem, st>>>(tm, L.m, nbox, L.kpad / M2_KS, G,
-                                                                    L.bt > 0 ? L.bt : 1, L.Bimg, b_bytes, L.ph, *L.O);
-  return cudaGetLastError();
+  return launch_behind(L.O->over != nullptr, mpb2_kernel<NP>, (unsigned)(2 * pairs), M2_THREADS, smem, st, tm, L.m, nbox,
+                       L.kpad / M2_KS, G, L.bt > 0 ? L.bt : 1, L.Bimg, b_bytes, L.ph, *L.O);
 }
 
 cudaError_t launch_mpb2(const LaunchMpb& L, cudaStream_t st) {

@@ -254,7 +254,10 @@ __global__ void __launch_bounds__(TB_THREADS, 1)
   // has given up
   const unsigned long long* const over = SINGLE ? O1.over : O.over;
   const bool left = FORM == TB_ONE64 && O1.rows;
-  if (over && (*over != 0) == left) return;
+  if (over) {
+    wait_for_previous();
+    if ((*over != 0) == left) return;
+  }
   if (left) {
     m = *O1.rows;
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(O1.counters, O1.counters[CNT_FS_TESTED]);
@@ -647,9 +650,9 @@ static cudaError_t launch_tb_t(const LaunchTb& L, const CUtensorMap& tm, cudaStr
   DevOut O1{};
   if (FORM == TB_MANY) O = *L.O;
   else O1 = *L.O1;
-  tb_kernel<NP, PPG, FORM><<<grid, TB_THREADS, smem, st>>>(tm, L.m, nbox, nsub, L.G, T, xst, nb, rb, L.Bimg,
-                                                           (unsigned long long)L.kpad * N, L.ph, O, O1);
-  return cudaGetLastError();
+  return launch_behind((FORM == TB_MANY ? O.over : O1.over) != nullptr, tb_kernel<NP, PPG, FORM>, grid, TB_THREADS,
+                       smem, st, tm, L.m, nbox, nsub, L.G, T, xst, nb, rb, L.Bimg, (unsigned long long)L.kpad * N,
+                       L.ph, O, O1);
 }
 
 cudaError_t launch_tb(const LaunchTb& L, cudaStream_t st) {

@@ -128,7 +128,10 @@ __global__ void __launch_bounds__(ts_threads(N), 1)
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int nsp = (nsub + TS_SUPER - 1) / TS_SUPER;  // super-stages per tile
 
-  if (O.over && !*O.over) return;  // the screen has decided
+  if (O.over) {
+    wait_for_previous();
+    if (!*O.over) return;  // the screen has decided
+  }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(s_tmem))
                  : "memory");
@@ -537,9 +540,8 @@ static cudaError_t launch_ts_w(const LaunchTs& L, const CUtensorMap& tm, cudaStr
   unsigned long long grid = (unsigned long long)L.num_sms;
   if (grid > tiles) grid = tiles;
   const int nbox = (nsub * 16 + 127) / 128;
-  ts_kernel<N, D0, GATE, WIDE><<<(unsigned)grid, ts_threads(N), smem, st>>>(tm, L.m, nbox, nsub, xst, ug, rb, L.Bimg, b_bytes,
-                                                                   *L.P, *L.LM, *L.O);
-  return cudaGetLastError();
+  return launch_behind(L.O->over != nullptr, ts_kernel<N, D0, GATE, WIDE>, (unsigned)grid, ts_threads(N), smem, st, tm,
+                       L.m, nbox, nsub, xst, ug, rb, L.Bimg, b_bytes, *L.P, *L.LM, *L.O);
 }
 
 template <int N, bool D0, bool GATE>

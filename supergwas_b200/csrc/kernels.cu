@@ -296,7 +296,10 @@ __global__ void __launch_bounds__(TC_TM, 1)
   const int tid = threadIdx.x, warp = tid >> 5;
   const uint32_t full0 = smem_u32(bars), done0 = smem_u32(bars + TC_NST);
 
-  if (O.over && !*O.over) return;  // the screen has decided
+  if (O.over) {
+    wait_for_previous();
+    if (!*O.over) return;  // the screen has decided
+  }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)),
                  "r"(TCOLS)
@@ -416,8 +419,8 @@ static cudaError_t launch_tc_ss_t(const LaunchTc& L, cudaStream_t st) {
   unsigned long long grid = (unsigned long long)L.num_sms;
   if (grid > tiles) grid = tiles;
   if (grid < 1) grid = 1;
-  tc_ss_kernel<N><<<(unsigned)grid, TC_TM, smem, st>>>(L.x, L.m, L.wpk, L.nchunk, L.Bimg, *L.P, *L.LM, *L.O);
-  return cudaGetLastError();
+  return launch_behind(L.O->over != nullptr, tc_ss_kernel<N>, (unsigned)grid, TC_TM, smem, st, L.x, L.m, L.wpk, L.nchunk,
+                       L.Bimg, *L.P, *L.LM, *L.O);
 }
 
 int tc_kc() { return TC_KC; }

@@ -34,12 +34,12 @@ CASES = [(0.0, None, False), (0.002, None, False), (0.1, None, True), (1.0, None
 
 
 @pytest.mark.parametrize("share,base,over", CASES)
-@pytest.mark.parametrize("n,k,m,thr", [(200, 6, 200_001, 0.2), (1000, 17, 150_000, 0.0), (5000, 33, 80_000, 0.0)])
+@pytest.mark.parametrize("n,k,m,thr", [(200, 6, 400_001, 0.2), (1000, 17, 150_000, 0.0), (5000, 33, 80_000, 0.0)])
 def test_one_phenotype(built, n, k, m, thr, share, base, over, monkeypatch):
     import torch
     rng = np.random.default_rng(n)
     U, y, X = batch(n, k, m, share, rng)
-    plain = batch(n, k, 20_000, 0.0, np.random.default_rng(1))[2]
+    plain = batch(n, k, 4000, 0.0, np.random.default_rng(1))[2]
     monkeypatch.setenv("KG_DEDUP", "0")
     if base is not None:
         monkeypatch.setenv("KG_SCREEN_OPEN", base)
@@ -196,3 +196,34 @@ def test_longer_candidate_list_between_graph_replays(built):
                 assert g.last_screen() == 1
     for tested, hits in out[1:]:
         assert np.array_equal(tested, out[0][0]) and np.array_equal(hits, out[0][1])
+
+
+@pytest.mark.parametrize("prec,m", [("split", 150_000), ("fp64", 420_000), ("many", 30_000)])
+@pytest.mark.parametrize("share", [0.0, 0.3])
+def test_rows_overwritten_behind_the_launch(built, prec, m, share, monkeypatch):
+    """A launch has read its rows when the stream is past it, whether the screen
+    gives up or not: the next rows may go to the same buffer before the fetch."""
+    import torch
+    n, k = (1000, 11) if prec == "fp64" else (1000, 17)
+    U, y, X = batch(n, k, m, share, np.random.default_rng(m))
+    dx = torch.from_numpy(X.view(np.int64)).cuda()
+    st = torch.cuda.current_stream().cuda_stream
+    with api.Kgwas(precision="split" if prec == "many" else prec, corr_threshold=0.0, log10_thresh=6.0) as g:
+        if prec == "many":
+            g.set_phenotypes([(U, y + 0.1 * p, np.arange(n)) for p in range(3)], n)
+            ref = g.run_multi_host(X)
+            for _ in range(3):
+                dx.copy_(torch.from_numpy(X.view(np.int64)))
+                g.launch_multi_device(dx.data_ptr(), m, X.shape[1], None, st)
+                dx.zero_()
+                tested, hits = g.fetch_multi()
+                assert np.array_equal(tested, ref[0]) and np.array_equal(hits, ref[1])
+        else:
+            g.set_structure(U, y)
+            g.launch_device(dx.data_ptr(), m, X.shape[1], st)
+            dx.zero_()
+            r = g.fetch()
+            monkeypatch.setenv("KG_KERNEL", "full")
+            ref = g.run_host(X)
+            assert r.n_tested == ref.n_tested and np.array_equal(r.hits, ref.hits)
+        assert ref[1].shape[0] > 0 if prec == "many" else ref.hits.shape[0] > 0

@@ -629,6 +629,12 @@ cudaError_t launch_screen4(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t
   return kg::launch_fs(L, st);
 }
 
+// Smallest work (k-mers x samples x limb columns) of a launch of more than
+// open_base() k-mers that the 4-bit screen takes: below it the kernel behind costs
+// more than the screen saves (calls with and without: 77 and 75 us for 2e4 k-mers at
+// n = 200 and 1.6e8, 77 and 72 for 5e4 at n = 700 and 1.2e9, 77 and 81 for 2e5 at
+// n = 700 and 4.9e9, 80 and 86 for 1e5 at n = 1000 and 6.6e9).
+constexpr double FS_MIN = 3e9;
 // FP64 form behind the 4-bit screen: smallest work (k-mers x samples x limb
 // columns), and the most bytes of rows that the screen may leave.
 constexpr double FS64_MIN = 3.2e10;
@@ -730,6 +736,7 @@ int launch_one(kg_ctx* ctx, const uint64_t* dx, uint64_t m, uint32_t wpk, uint64
     if (force && std::string(force) == "ts" && !ts_ok)
       return ctx->fail(KG_ERR_UNSUPPORTED, "KG_KERNEL=ts: shape not supported by the TMEM-A kernel");
     const bool screen = ctx->fs_N && mode != SCREEN_OFF && tma_ok && !stats && !force &&
+                        (m <= O.open_base || (double)m * ctx->limbs.Kpad * ctx->limbs.N >= FS_MIN) &&
                         kg::fs_supported(ctx->fs_N, ctx->fs_kpad, (int)wpk);
     if (screen) {
       e = launch_screen4(ctx, dx, m, wpk, O, st);

@@ -15,6 +15,10 @@ def rows_of(n, m, rng):
     return np.ascontiguousarray(X[np.arange(m) % X.shape[0]])
 
 
+# work that the screen would not save its cost on (3e9 k-mers x samples x limb columns, above 4096 k-mers)
+SMALL = {(200, 6, 60_001), (640, 11, 20_000), (1000, 17, 40_000)}
+
+
 @pytest.mark.parametrize("n,k,m", SHAPES, ids=lambda v: str(v))
 @pytest.mark.parametrize("thr,lt", [(0.0, 6.0), (0.2, 4.0), (1e-5, 9.0)])
 def test_one_phenotype(built, n, k, m, thr, lt, monkeypatch):
@@ -26,7 +30,11 @@ def test_one_phenotype(built, n, k, m, thr, lt, monkeypatch):
     with api.Kgwas(corr_threshold=thr, log10_thresh=lt) as g:
         g.set_structure(np.linalg.qr(Z)[0], y)
         g.run_host(X)
+        assert g.last_screen() == ((n, k, m) not in SMALL)
+        monkeypatch.setenv("KG_SCREEN_OPEN", str(1 << 24))
+        g.run_host(X)
         assert g.last_screen() == 1
+        monkeypatch.delenv("KG_SCREEN_OPEN")
         g.run_host(X[:1], stats=True)
         assert g.last_screen() == 0
         monkeypatch.setenv("KG_KERNEL", "full")

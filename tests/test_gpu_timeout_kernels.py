@@ -15,7 +15,7 @@ ERR_TIMEOUT = 5  # include/kgwas_cuda.h
 
 # samples, U columns, k-mers, precision, -log10 p, kg_last_kernel, limbs of the screen
 CASES = {"screen": (1000, 17, 100_000, "split", 6.0, "ts", 1),
-         "screen, short rows": (200, 6, 200_000, "split", 6.0, "ts", 1),
+         "screen, short rows": (200, 6, 400_000, "split", 6.0, "ts", 1),
          "screen, long rows": (5000, 33, 40_000, "split", 6.0, "ts", 1),
          "streamed image": (5000, 33, 40_000, "split", 2.0, "tb", 0),
          "fp64": (1000, 11, 100_000, "fp64", 6.0, "fp64", 0),

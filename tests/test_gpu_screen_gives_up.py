@@ -206,14 +206,18 @@ def test_rows_overwritten_behind_the_launch(built, prec, m, share, monkeypatch):
     import torch
     n, k = (1000, 11) if prec == "fp64" else (1000, 17)
     U, y, X = batch(n, k, m, share, np.random.default_rng(m))
-    dx = torch.from_numpy(X.view(np.int64)).cuda()
-    st = torch.cuda.current_stream().cuda_stream
-    with api.Kgwas(precision="split" if prec == "many" else prec, corr_threshold=0.0, log10_thresh=6.0) as g:
+    rows = torch.from_numpy(X.view(np.int64)).cuda()
+    dx = rows.clone()
+    stream = torch.cuda.Stream()  # 0 would be the context's own stream
+    st = stream.cuda_stream
+    stream.wait_stream(torch.cuda.current_stream())
+    form = "split" if prec == "many" else prec
+    with torch.cuda.stream(stream), api.Kgwas(precision=form, corr_threshold=0.0, log10_thresh=6.0) as g:
         if prec == "many":
             g.set_phenotypes([(U, y + 0.1 * p, np.arange(n)) for p in range(3)], n)
             ref = g.run_multi_host(X)
             for _ in range(3):
-                dx.copy_(torch.from_numpy(X.view(np.int64)))
+                dx.copy_(rows)
                 g.launch_multi_device(dx.data_ptr(), m, X.shape[1], None, st)
                 dx.zero_()
                 tested, hits = g.fetch_multi()

@@ -176,7 +176,7 @@ constexpr int CNT_FS_TESTED = 4, CNT_FS_OPEN = 5, CNT_FS_OVER = 6, CNT_FS_EVER =
 // kind are found out early, later one in 64 of all; calls of up to `base` tests never
 // give up.  1e7 rows at n = 1000, r = 16+1, of which 0, 1, 3, 10 and 100 % are lineage
 // markers, about half of them undecided: 0.30, 0.46, 0.79, 1.9 and 16 ms with all
-// of those refined; now 0.30, 0.47, 0.52, 0.51 and 0.52; 0.47 without the screen.
+// of those refined; now 0.30, 0.47, 0.49, 0.50 and 0.49; 0.47 without the screen.
 constexpr unsigned long long FS_OPEN_BASE = 4096;
 __host__ __device__ inline unsigned long long fs_open_limit(unsigned long long base, unsigned long long done,
                                                             unsigned long long total, unsigned long long cap) {
